@@ -82,6 +82,7 @@ EXPORTS = (
     "mla_fp4_cp_close",
     "mla_fp4_cp_free",
     "mla_fp4_cp_exchange_merge",
+    "mla_fp4_step_metadata",
 )
 CP_MAX_RANKS = 8
 CP_HANDLE_BYTES = 64
@@ -132,6 +133,9 @@ def _load() -> C.CDLL:
     lib.mla_fp4_cache_write.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p,
                                         C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mla_fp4_cache_write.restype = C.c_int
+    lib.mla_fp4_step_metadata.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32,
+                                          C.c_int32, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]
+    lib.mla_fp4_step_metadata.restype = C.c_int
     v = lib.mla_fp4_abi_version()
     if v != ABI_VERSION:
         raise ImportError(f"{LIB_PATH} has ABI version {v}, expected {ABI_VERSION}: rebuild it")
@@ -139,6 +143,23 @@ def _load() -> C.CDLL:
 
 
 lib = _load()
+
+
+def _load_native():
+    """The native call path (csrc/py_native.cpp), bound to the functions of the library loaded above."""
+    import torch  # noqa: F401  (the module links against torch's libraries, which importing torch loads)
+
+    try:
+        from . import _native
+    except ImportError as e:
+        raise ImportError(f"the native call path is missing or does not load ({e}): build it with "
+                          "`python -m flashinfer_mla_fp4_b200.build`. There is no fallback path.") from e
+    names = ("mla_fp4_decode", "mla_fp4_workspace_bytes", "mla_fp4_cache_write", "mla_fp4_step_metadata", "mla_fp4_last_error")
+    _native.bind(*(C.cast(getattr(lib, n), C.c_void_p).value for n in names))
+    return _native
+
+
+native = _load_native()
 
 
 def last_error() -> str:

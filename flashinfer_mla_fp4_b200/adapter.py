@@ -93,6 +93,8 @@ class FP4MLADecodeBackend:
         self.block_tables = torch.zeros(max_batch, self.max_pages, dtype=torch.int32, device=self.device)
         self.seq_lens = torch.zeros(max_batch, dtype=torch.int32, device=self.device)
         self.slot_mapping = torch.full((max_batch * q_len,), -1, dtype=torch.int64, device=self.device)
+        self._step_metadata = _cabi.native.step_metadata
+        self._views = (0, None, None, None)  # (batch, block_tables, seq_lens, slot_mapping) of the last forward()
 
     # ------------------------------------------------------------------ metadata
     def clear(self) -> None:
@@ -115,10 +117,14 @@ class FP4MLADecodeBackend:
             raise ValueError(f"batch {batch} exceeds max_batch {self.max_batch}")
         if block_tables.dim() != 2 or block_tables.shape[0] != batch or block_tables.shape[1] > self.max_pages:
             raise ValueError(f"block_tables must be [batch, <= {self.max_pages}], got {tuple(block_tables.shape)}")
+        if slot_mapping is not None and slot_mapping.numel() != batch * self.q_len:
+            raise ValueError(f"slot_mapping must hold batch * q_len = {batch * self.q_len} slots")
+        # Device or pinned host tensors of the usual types: one kernel writes all three buffers.
+        if self._step_metadata(block_tables, seq_lens, slot_mapping, self.block_tables, self.seq_lens, self.slot_mapping,
+                               self.page_size, self.q_len):
+            return batch
         if slot_mapping is None:
             slot_mapping = decode_slot_mapping(block_tables, seq_lens, self.page_size, self.q_len)
-        elif slot_mapping.numel() != batch * self.q_len:
-            raise ValueError(f"slot_mapping must hold batch * q_len = {batch * self.q_len} slots")
         self.block_tables[:batch, : block_tables.shape[1]].copy_(block_tables, non_blocking=True)
         self.seq_lens[:batch].copy_(seq_lens, non_blocking=True)
         self.seq_lens[batch:].zero_()
@@ -152,9 +158,12 @@ class FP4MLADecodeBackend:
             raise ValueError(f"latent must be [{n}, {LATENT_DIM}] and rope [{n}, {ROPE_DIM}]")
         if cache.page_size != self.page_size:
             raise ValueError(f"cache page size {cache.page_size} does not match the backend's {self.page_size}")
-        write_tokens(latent, rope, self.slot_mapping[:n], cache.kv_cache, cache.kv_cache_sf)
-        return self._runner.run(q, cache.kv_cache, self.block_tables[:batch], self.seq_lens[:batch], self.max_seq_len,
-                                self.softmax_scale, output_scale=self.output_scale, out=out, kv_cache_sf=cache.kv_cache_sf)
+        views = self._views  # one attribute read: a batch and the views of the same batch, whatever another thread does
+        if views[0] != batch or views[1] is None:
+            views = self._views = (batch, self.block_tables[:batch], self.seq_lens[:batch], self.slot_mapping[:n])
+        write_tokens(latent, rope, views[3], cache.kv_cache, cache.kv_cache_sf)
+        return self._runner.run(q, cache.kv_cache, views[1], views[2], self.max_seq_len, self.softmax_scale,
+                                output_scale=self.output_scale, out=out, kv_cache_sf=cache.kv_cache_sf)
 
     def capture(self, cache: FP4MLAPagedCache, batch: Optional[int] = None, in_dtype: torch.dtype = torch.bfloat16,
                 warmup: int = 2) -> "CapturedDecodeStep":

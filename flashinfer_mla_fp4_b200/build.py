@@ -1,4 +1,5 @@
-"""Build libmla_fp4_b200.so in-tree with nvcc for sm_100a (no torch dependency in the library)."""
+"""Build the two in-tree binaries: libmla_fp4_b200.so (nvcc, sm_100a: kernels and C ABI, no torch dependency) and
+_native.so (g++: the native call path of the Python entry points, against torch's headers)."""
 from __future__ import annotations
 
 import os
@@ -11,6 +12,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = Path(os.environ.get("MLA_FP4_B200_LIB") or (PKG_DIR / "libmla_fp4_b200.so"))
 SOURCES = ["abi.cu", "kernels_simt.cu", "combine.cu", "cache_write.cu", "cp_exchange.cu", "decode_sm100.cu"]
+NATIVE_PATH = PKG_DIR / "_native.so"
+NATIVE_SOURCE = CSRC / "py_native.cpp"
 HEADERS = ["common.cuh", "dequant.cuh", "launch.h", "ptx_sm100.cuh", "../../include/mla_fp4_b200.h"]
 
 
@@ -19,6 +22,26 @@ def _nvcc() -> str:
     if not Path(cand).exists():
         raise RuntimeError("nvcc not found; set NVCC")
     return cand
+
+
+def _native_command(out: Path) -> list:
+    import sysconfig
+
+    import torch
+
+    base = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    includes = [base / "include", base / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+    libs = ["c10", "c10_cuda", "torch_cpu", "torch_cuda", "torch_python"]
+    return ([os.environ.get("CXX") or "g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", "-DNDEBUG",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+            + [f"-isystem{i}" for i in includes] + [str(NATIVE_SOURCE), "-o", str(out), f"-L{base / 'lib'}"] + [f"-l{x}" for x in libs]
+            + [f"-L{cuda / 'lib64'}", "-lcudart_static", "-lrt", "-ldl", "-lpthread"])
+
+
+def native_needs_build() -> bool:
+    deps = [NATIVE_SOURCE, PKG_DIR.parent / "include" / "mla_fp4_b200.h"]
+    return not NATIVE_PATH.exists() or any(d.stat().st_mtime > NATIVE_PATH.stat().st_mtime for d in deps)
 
 
 def needs_build() -> bool:
@@ -30,9 +53,25 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every CUDA source for sm_100a into one shared library next to this file."""
-    if not force and not needs_build():
-        return LIB_PATH
+    """Compile every CUDA source for sm_100a into one shared library next to this file, and the native call path."""
+    native = None
+    if force or native_needs_build():  # runs beside the CUDA compilation
+        native = subprocess.Popen(_native_command(NATIVE_PATH.with_suffix(".tmp")), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    try:
+        if force or needs_build():
+            _build_library(verbose)
+    finally:
+        if native is not None:
+            out, _ = native.communicate()
+    if native is not None:
+        if native.returncode != 0:
+            sys.stderr.write(f"--- {NATIVE_SOURCE.name}\n{out}\n")
+            raise RuntimeError("the native call path failed to compile")
+        os.replace(NATIVE_PATH.with_suffix(".tmp"), NATIVE_PATH)
+    return LIB_PATH
+
+
+def _build_library(verbose: bool) -> None:
     objs = []
     build_dir = PKG_DIR / "build"
     build_dir.mkdir(exist_ok=True)
@@ -61,7 +100,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if r.returncode != 0:
         sys.stderr.write(r.stdout)
         raise RuntimeError("link failed")
-    return LIB_PATH
 
 
 if __name__ == "__main__":

@@ -383,6 +383,25 @@ int mla_fp4_cache_write(const void* latent, int64_t latent_stride, const void* r
   return MLA_FP4_OK;
 }
 
+int mla_fp4_step_metadata(const int32_t* block_tables, int64_t block_table_stride, int32_t width, const void* seq_lens,
+                          int32_t seq_lens_is_64, const int64_t* slot_mapping, int32_t batch, int32_t page_size,
+                          int32_t q_len, int32_t* dst_block_tables, int64_t dst_block_table_stride,
+                          int32_t* dst_seq_lens, int64_t* dst_slot_mapping, int32_t max_batch, void* stream) {
+  if (batch < 0 || max_batch < batch || width < 0 || page_size <= 0 || q_len <= 0) return fail(MLA_FP4_ERR_BAD_ARG, "batch/max_batch/width/page_size/q_len out of range");
+  if (max_batch == 0) return MLA_FP4_OK;
+  if (!dst_block_tables || !dst_seq_lens || !dst_slot_mapping || (batch > 0 && (!seq_lens || (width > 0 && !block_tables))))
+    return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
+  if (batch > 0 && width == 0 && !slot_mapping) return fail(MLA_FP4_ERR_BAD_ARG, "a slot mapping cannot be derived from empty block tables");
+  mla::StepMetadataParams p;
+  p.block_tables = block_tables; p.block_table_stride = block_table_stride; p.seq_lens = seq_lens; p.slot_mapping = slot_mapping;
+  p.dst_block_tables = dst_block_tables; p.dst_block_table_stride = dst_block_table_stride;
+  p.dst_seq_lens = dst_seq_lens; p.dst_slot_mapping = dst_slot_mapping;
+  p.width = width; p.seq_lens_is_64 = seq_lens_is_64; p.batch = batch; p.max_batch = max_batch; p.page_size = page_size; p.q_len = q_len;
+  cudaError_t e = mla::launch_step_metadata(p, reinterpret_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(MLA_FP4_ERR_CUDA, std::string("step metadata launch: ") + cudaGetErrorString(e));
+  return MLA_FP4_OK;
+}
+
 int mla_fp4_dequant_e2m1_to_e4m3(const void* packed, void* out, int64_t n_bytes, void* stream) {
   if (n_bytes < 0 || (n_bytes % 4)) return fail(MLA_FP4_ERR_BAD_ARG, "n_bytes must be a non-negative multiple of 4");
   if (n_bytes == 0) return MLA_FP4_OK;

@@ -1599,87 +1599,97 @@ bool encode_map(CUtensorMap* m, const void* base, int rank, const uint64_t* dims
   return r == CUDA_SUCCESS;
 }
 
-// The four tensor maps of a launch depend only on the query's address and strides, the cache's address and the
-// shapes.  A serving loop calls with the same ones step after step, and encoding four maps cost more host time than
-// the rest of the call: the last set is kept per thread and reused when its key matches.
-struct MapKey {
+// The four tensor maps of a launch depend only on addresses, strides and shapes: two on the query, two on the cache.
+// Encoding a map costs about a microsecond of host time, and a serving program calls with the same sets again and again,
+// one cache per layer: each thread keeps the last maps in a small direct-mapped table (a bounded 2 x 64 entries; one
+// entry, the form before, was overwritten by every layer's call).
+struct QKey {
   const void* q;
-  const void* kv;
-  int64_t sb, sq, sh, num_pages;
-  int32_t batch, q_len, num_heads, page_size;
-  bool operator==(const MapKey& o) const {
-    return q == o.q && kv == o.kv && sb == o.sb && sq == o.sq && sh == o.sh && num_pages == o.num_pages && batch == o.batch &&
-           q_len == o.q_len && num_heads == o.num_heads && page_size == o.page_size;
+  int64_t sb, sq, sh;
+  int32_t batch, q_len, num_heads, dev;
+  bool operator==(const QKey& o) const {
+    return q == o.q && sb == o.sb && sq == o.sq && sh == o.sh && batch == o.batch && q_len == o.q_len && num_heads == o.num_heads && dev == o.dev;
   }
 };
-struct MapSet {
-  MapKey key;
-  bool valid = false;
-  CUtensorMap q_lat, q_rope, rope, lat;
+struct KvKey {
+  const void* kv;
+  int64_t num_pages;
+  int32_t page_size, dev;
+  bool operator==(const KvKey& o) const { return kv == o.kv && num_pages == o.num_pages && page_size == o.page_size && dev == o.dev; }
 };
+template <typename Key>
+struct MapPair {
+  CUtensorMap a, b;  // (aligned first)
+  Key key;
+  bool valid = false;
+};
+constexpr uint32_t kMapEntries = 64;
+uint32_t map_slot(const void* p) {
+  return uint32_t((reinterpret_cast<uintptr_t>(p) >> 8) * 0x9E3779B97F4A7C15ull >> 58);
+}
+
+// q viewed as [576, H, q_len, B] bytes: a box of 128 latent values (or the 64 RoPE values) of 64 heads
+bool encode_q_maps(const DecodeParams& p, CUtensorMap* lat, CUtensorMap* rope) {
+  const uint64_t sq = p.q_len > 1 ? uint64_t(p.q_stride_qpos) : uint64_t(p.q_stride_head) * uint64_t(p.num_heads);
+  const uint64_t sb = p.batch > 1 ? uint64_t(p.q_stride_batch) : sq * uint64_t(p.q_len);
+  const uint64_t dims[4] = {uint64_t(kQDim), uint64_t(p.num_heads), uint64_t(p.q_len), uint64_t(p.batch)};
+  const uint64_t strides[3] = {uint64_t(p.q_stride_head), sq, sb};
+  const uint32_t box_lat[4] = {128, uint32_t(kGroupHeads), 1, 1};
+  const uint32_t box_rope[4] = {64, uint32_t(kGroupHeads), 1, 1};
+  return encode_map(lat, p.q, 4, dims, strides, box_lat, CU_TENSOR_MAP_SWIZZLE_128B) &&
+         encode_map(rope, p.q, 4, dims, strides, box_rope, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+// the RoPE bytes of a page, and the cache as 4-bit elements: 640 per row (the 512 latent codes, then the RoPE bytes seen as
+// nibbles and never fetched through this map), page_size rows per page; a box is one 128-dim block of one page
+bool encode_kv_maps(const DecodeParams& p, CUtensorMap* lat, CUtensorMap* rope) {
+  const uint64_t dims[3] = {uint64_t(kRowBytes), uint64_t(p.page_size), uint64_t(p.num_pages)};
+  const uint64_t strides[2] = {uint64_t(kRowBytes), uint64_t(kRowBytes) * uint64_t(p.page_size)};
+  const uint32_t box[3] = {64, uint32_t(p.page_size), 1};
+  if (!encode_map(rope, p.kv_cache, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B)) return false;
+  EncodeTiledFn fn = get_encode_fn();
+  cuuint64_t gd[3] = {cuuint64_t(2 * kRowBytes), cuuint64_t(p.page_size), cuuint64_t(p.num_pages)};
+  cuuint64_t gs[2] = {cuuint64_t(kRowBytes), cuuint64_t(kRowBytes) * cuuint64_t(p.page_size)};
+  cuuint32_t bx[3] = {128, cuuint32_t(p.page_size), 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  return fn(lat, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<void*>(p.kv_cache), gd, gs, bx, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 }  // namespace
 
 cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_t stream, const char** err) {
   *err = nullptr;
-  static thread_local MapSet cache;
-  const MapKey key{p.q, p.kv_cache, p.q_stride_batch, p.q_stride_qpos, p.q_stride_head, p.num_pages, p.batch, p.q_len, p.num_heads, p.page_size};
-  if (!(cache.valid && cache.key == key)) {
-    cache.valid = false;
-    CUtensorMap& map_q_lat = cache.q_lat;
-    CUtensorMap& map_q_rope = cache.q_rope;
-    CUtensorMap& map_rope = cache.rope;
-    CUtensorMap& map_lat = cache.lat;
-    {
-      // q viewed as [576, H, q_len, B] bytes
-      uint64_t sq = p.q_len > 1 ? uint64_t(p.q_stride_qpos) : uint64_t(p.q_stride_head) * uint64_t(p.num_heads);
-      uint64_t sb = p.batch > 1 ? uint64_t(p.q_stride_batch) : sq * uint64_t(p.q_len);
-      uint64_t dims[4] = {uint64_t(kQDim), uint64_t(p.num_heads), uint64_t(p.q_len), uint64_t(p.batch)};
-      uint64_t strides[3] = {uint64_t(p.q_stride_head), sq, sb};
-      uint32_t box_lat[4] = {128, uint32_t(kGroupHeads), 1, 1};
-      uint32_t box_rope[4] = {64, uint32_t(kGroupHeads), 1, 1};
-      if (!encode_map(&map_q_lat, p.q, 4, dims, strides, box_lat, CU_TENSOR_MAP_SWIZZLE_128B) ||
-          !encode_map(&map_q_rope, p.q, 4, dims, strides, box_rope, CU_TENSOR_MAP_SWIZZLE_64B)) {
-        *err = "cuTensorMapEncodeTiled failed for q (check alignment and strides)";
-        return cudaErrorInvalidValue;
-      }
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  static thread_local MapPair<QKey> q_maps[kMapEntries];
+  static thread_local MapPair<KvKey> kv_maps[kMapEntries];
+  MapPair<QKey>& qm = q_maps[map_slot(p.q)];
+  MapPair<KvKey>& km = kv_maps[map_slot(p.kv_cache)];
+  const QKey qkey{p.q, p.q_stride_batch, p.q_stride_qpos, p.q_stride_head, p.batch, p.q_len, p.num_heads, dev};
+  const KvKey kvkey{p.kv_cache, p.num_pages, p.page_size, dev};
+  if (!(qm.valid && qm.key == qkey)) {
+    qm.valid = false;
+    if (!encode_q_maps(p, &qm.a, &qm.b)) {
+      *err = "cuTensorMapEncodeTiled failed for q (check alignment and strides)";
+      return cudaErrorInvalidValue;
     }
-    {
-      uint64_t dims[3] = {uint64_t(kRowBytes), uint64_t(p.page_size), uint64_t(p.num_pages)};
-      uint64_t strides[2] = {uint64_t(kRowBytes), uint64_t(kRowBytes) * uint64_t(p.page_size)};
-      uint32_t box[3] = {64, uint32_t(p.page_size), 1};
-      if (!encode_map(&map_rope, p.kv_cache, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B)) {
-        *err = "cuTensorMapEncodeTiled failed for kv_cache (check alignment)";
-        return cudaErrorInvalidValue;
-      }
-    }
-    {
-      // the cache as 4-bit elements: 640 per row (the 512 latent codes, then the RoPE bytes seen as nibbles and
-      // never fetched through this map), page_size rows per page; a box is one 128-dim block of one page
-      EncodeTiledFn fn = get_encode_fn();
-      cuuint64_t gd[3] = {cuuint64_t(2 * kRowBytes), cuuint64_t(p.page_size), cuuint64_t(p.num_pages)};
-      cuuint64_t gs[2] = {cuuint64_t(kRowBytes), cuuint64_t(kRowBytes) * cuuint64_t(p.page_size)};
-      cuuint32_t bx[3] = {128, cuuint32_t(p.page_size), 1};
-      cuuint32_t es[3] = {1, 1, 1};
-      if (!fn || fn(&map_lat, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<void*>(p.kv_cache), gd, gs, bx, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-        *err = "cuTensorMapEncodeTiled failed for the packed latent (kv_cache must be 32-byte aligned)";
-        return cudaErrorInvalidValue;
-      }
-    }
-    cache.key = key;
-    cache.valid = true;
+    qm.key = qkey;
+    qm.valid = true;
   }
-  const CUtensorMap& map_q_lat = cache.q_lat;
-  const CUtensorMap& map_q_rope = cache.q_rope;
-  const CUtensorMap& map_rope = cache.rope;
-  const CUtensorMap& map_lat = cache.lat;
+  if (!(km.valid && km.key == kvkey)) {
+    km.valid = false;
+    if (!encode_kv_maps(p, &km.a, &km.b)) {
+      *err = "cuTensorMapEncodeTiled failed for kv_cache (it must be 32-byte aligned)";
+      return cudaErrorInvalidValue;
+    }
+    km.key = kvkey;
+    km.valid = true;
+  }
+  const CUtensorMap &map_q_lat = qm.a, &map_q_rope = qm.b, &map_rope = km.b, &map_lat = km.a;
   {
     static std::atomic<bool> attr_done[64];  // zero-initialised; setting the attribute twice is harmless
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64 || !attr_done[dev].load(std::memory_order_acquire)) {
       e = cudaFuncSetAttribute(mla_fp4_decode_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
       if (e != cudaSuccess) return e;

@@ -2,6 +2,7 @@
 //   * merge_partials_kernel- context-parallel merge of per-rank partial outputs + LSE
 //   * fp32_check_kernel    - plain-FP32 decode over the same work partition; a slow, exact-
 //                            arithmetic cross-check of the tcgen05 kernel used by tests
+//   * step_metadata_kernel - a decode step's persistent metadata refreshed from the scheduler's tensors
 //   * dequant_kernel       - E2M1 -> E4M3 byte dequantisation (the routine fp32_check_kernel uses), for the
 //                            bit-exact table test; the tcgen05 kernel hands the packed codes to the MMA unchanged
 #include "common.cuh"
@@ -246,6 +247,38 @@ __global__ void __launch_bounds__(256) fp32_check_kernel(DecodeParams p) {
   }
 }
 
+// One CTA per row of the persistent buffers.  The step's metadata is a few kilobytes, so the launch is all latency: the
+// torch form of it was about twenty kernels or copies and 150 us of host time.  Sources in pinned host memory are read in
+// place over PCIe; the row, the length and a given slot mapping are independent loads, and only a derived slot waits for
+// the length before it reads its page id.
+__global__ void __launch_bounds__(128) step_metadata_kernel(StepMetadataParams p) {
+  const int b = blockIdx.x;
+  if (b >= p.batch) {  // padding rows: no tokens, no cache write
+    if (threadIdx.x == 0) p.dst_seq_lens[b] = 0;
+    for (int j = threadIdx.x; j < p.q_len; j += blockDim.x) p.dst_slot_mapping[int64_t(b) * p.q_len + j] = -1;
+    return;
+  }
+  const int32_t* row = p.block_tables + int64_t(b) * p.block_table_stride;
+  const int64_t len = p.seq_lens_is_64 ? static_cast<const int64_t*>(p.seq_lens)[b] : int64_t(static_cast<const int32_t*>(p.seq_lens)[b]);
+  for (int j = threadIdx.x; j < p.q_len; j += blockDim.x) {
+    int64_t slot = -1;
+    if (p.slot_mapping) {
+      slot = p.slot_mapping[int64_t(b) * p.q_len + j];
+    } else {
+      const int64_t pos = len - p.q_len + j;
+      if (pos >= 0) {
+        const int64_t page = pos / p.page_size;
+        slot = int64_t(row[page < p.width ? page : p.width - 1]) * p.page_size + pos % p.page_size;
+      }
+    }
+    p.dst_slot_mapping[int64_t(b) * p.q_len + j] = slot;
+  }
+  if (threadIdx.x == 0) p.dst_seq_lens[b] = int32_t(len);
+  int32_t* dst = p.dst_block_tables + int64_t(b) * p.dst_block_table_stride;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < p.width; i += blockDim.x) dst[i] = row[i];
+}
+
 __global__ void dequant_kernel(const uint32_t* __restrict__ in, uint2* __restrict__ out, int64_t n_words) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (i < n_words) {
@@ -270,6 +303,11 @@ cudaError_t launch_fp32_check(const DecodeParams& p, int num_ctas, cudaStream_t 
   cudaError_t e = cudaFuncSetAttribute(fp32_check_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   fp32_check_kernel<<<num_ctas, 256, smem, stream>>>(p);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_step_metadata(const StepMetadataParams& p, cudaStream_t stream) {
+  step_metadata_kernel<<<unsigned(p.max_batch), 128, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

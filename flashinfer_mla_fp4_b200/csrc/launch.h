@@ -78,6 +78,18 @@ cudaError_t launch_fp32_check(const DecodeParams& p, int num_ctas, cudaStream_t 
 cudaError_t launch_cache_write(const void* latent, int64_t latent_stride, const void* rope, int64_t rope_stride, int in_dtype,
                                const float* scale_in, const int64_t* slot_mapping, int64_t num_tokens, void* cache,
                                float* cache_sf, int64_t num_slots, cudaStream_t stream);
+struct StepMetadataParams {
+  const int32_t* block_tables;
+  int64_t block_table_stride;
+  const void* seq_lens;
+  const int64_t* slot_mapping;
+  int32_t* dst_block_tables;
+  int64_t dst_block_table_stride;
+  int32_t* dst_seq_lens;
+  int64_t* dst_slot_mapping;
+  int32_t width, seq_lens_is_64, batch, max_batch, page_size, q_len;
+};
+cudaError_t launch_step_metadata(const StepMetadataParams& p, cudaStream_t stream);
 cudaError_t launch_dequant(const void* in, void* out, int64_t n_bytes, cudaStream_t stream);
 // tcgen05 decode kernel (decode_sm100.cu). Returns cudaErrorNotSupported-like codes through `err`.
 cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_t stream, const char** err);

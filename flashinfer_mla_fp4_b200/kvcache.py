@@ -53,7 +53,6 @@ def quantize_tokens(
 
 
 @api_logged
-@torch.no_grad()
 def write_tokens(
     latent: torch.Tensor,
     rope: torch.Tensor,
@@ -74,6 +73,8 @@ def write_tokens(
     """
     from . import _cabi
 
+    if _cabi.native.write_tokens(latent, rope, slot_mapping, kv_cache, kv_cache_sf, token_scale):
+        return  # the common form, checked and launched natively; otherwise nothing was done
     if not (latent.is_cuda and rope.is_cuda and kv_cache.is_cuda and kv_cache_sf.is_cuda):
         raise ValueError("write_tokens needs CUDA tensors (use quantize_tokens to build a cache on the host)")
     if latent.ndim != 2 or latent.shape[1] != LATENT_DIM or rope.ndim != 2 or rope.shape[1] != ROPE_DIM or rope.shape[0] != latent.shape[0]:

@@ -25,6 +25,7 @@ from .api_log import api_logged
 from .kvcache import LATENT_DIM, ROPE_DIM, ROW_BYTES
 from .variants import resolve as resolve_variant
 
+_native_decode = _cabi.native.decode
 _OUT_DTYPES = {torch.bfloat16: _cabi.OUT_BF16, torch.float32: _cabi.OUT_F32, torch.float8_e4m3fn: _cabi.OUT_E4M3}
 
 
@@ -104,6 +105,7 @@ class BatchMLADecodeCuteDSLFP4Wrapper:
         self._page_size = page_size
         self._q_dtype = q_dtype
         self._o_dtype = o_dtype
+        self._out_code = _OUT_DTYPES[o_dtype]
         self._is_var_seq = is_var_seq
         self._enable_pdl = True if enable_pdl is None else bool(enable_pdl)
         self._num_ctas = torch.cuda.get_device_properties(self._device).multi_processor_count
@@ -164,6 +166,14 @@ class BatchMLADecodeCuteDSLFP4Wrapper:
         place when ``return_lse`` is set, instead of a freshly allocated tensor."""
         if not self._planned:
             raise RuntimeError("Call plan() before run().")
+        # The common form of the call is checked and launched natively (csrc/py_native.cpp); None: nothing was done, and what
+        # follows either words the error or handles the less common layouts (4-D caches, int64 or strided seq_lens).
+        done = _native_decode(self._workspace_buffer, self._status, self._num_heads, self._page_size, self._out_code, self._kernel,
+                              self._num_ctas, self._enable_pdl, self._phase_mask, self._soft_cap, self._sink, self._wait_polls,
+                              q, kv_cache, block_tables, seq_lens, max_seq_len, softmax_scale, output_scale, out, kv_cache_sf,
+                              return_lse, lse_out)
+        if done is not None:
+            return done
         self._validate_run_inputs(q, kv_cache, kv_cache_sf, out)
 
         if kv_cache.dim() == 4:
@@ -247,7 +257,7 @@ class BatchMLADecodeCuteDSLFP4Wrapper:
         a.batch, a.q_len, a.num_heads, a.page_size = batch_size, q_len, num_heads, self._page_size
         a.num_pages = kv_cache.shape[0]
         a.softmax_scale, a.output_scale = float(softmax_scale), float(output_scale)
-        a.out_dtype = _OUT_DTYPES[self._o_dtype]
+        a.out_dtype = self._out_code
         a.kernel = self._kernel
         a.num_ctas = self._num_ctas
         a.enable_pdl = 1 if self._enable_pdl else 0

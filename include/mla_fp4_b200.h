@@ -235,6 +235,19 @@ int mla_fp4_cache_write(const void* latent, int64_t latent_stride, const void* r
                         int64_t num_tokens, void* kv_cache, float* kv_cache_sf, int64_t num_slots,
                         void* stream);
 
+/* Refresh the persistent metadata of a decode step (what a captured step reads) from a scheduler's tensors, in one
+   launch: block_tables int32 [batch][width] with row stride block_table_stride -> dst_block_tables (row stride
+   dst_block_table_stride, columns beyond width untouched); seq_lens [batch] (int32, or int64 when seq_lens_is_64) ->
+   dst_seq_lens int32 [max_batch], zero beyond the batch; slot_mapping int64 [batch * q_len], or NULL to derive it (the
+   q_len newest positions of each request, seq_len counting them, through the request's block-table row; -1 below
+   position zero) -> dst_slot_mapping int64 [max_batch * q_len], -1 beyond the batch.  The sources may be device memory
+   or pinned host memory as the device addresses it.  Stands in for nothing in the reference, whose serving side is
+   private (README.md:124-126). */
+int mla_fp4_step_metadata(const int32_t* block_tables, int64_t block_table_stride, int32_t width, const void* seq_lens,
+                          int32_t seq_lens_is_64, const int64_t* slot_mapping, int32_t batch, int32_t page_size,
+                          int32_t q_len, int32_t* dst_block_tables, int64_t dst_block_table_stride,
+                          int32_t* dst_seq_lens, int64_t* dst_slot_mapping, int32_t max_batch, void* stream);
+
 /* Largest decode grid the allocation-free variant below accepts, and the bytes of device memory
    its built-in scratch occupies on every GPU that loads the library (until the process exits). */
 #define MLA_FP4_STATIC_MAX_CTAS 148
