@@ -175,6 +175,7 @@ int mla_fp4_decode(const MlaFp4DecodeArgs* a) {
   cudaError_t e = cudaSuccess;
   const bool fused = a->kernel == MLA_FP4_KERNEL_TCGEN05;
   p.fused_merge = fused ? 1 : 0;
+  p.merge_last = fused && (a->phase_mask & 4) ? 1 : 0;
   const bool do_decode = fused || a->phase_mask == 0 || (a->phase_mask & 1);
   const bool do_combine = !fused && (a->phase_mask == 0 || (a->phase_mask & 2));
   if (!do_decode) {

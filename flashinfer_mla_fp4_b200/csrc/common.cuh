@@ -25,7 +25,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 //     scale (the decode kernel's lanes own one dim each: with this order a warp stores 32 dims x 8 heads =
 //     512 contiguous bytes at a time; with heads innermost over all 64 it would store 16 bytes every 128).
 //   * tail of slot s (272 bytes): the base-2 LSE of the 64 heads as f32, that scale (f32), the slot's flag
-//     (int32, see below), 8 bytes of padding.  The tails of all slots lie side by side, so the tails of the
+//     (int32, see below), an arrival counter (int32), 4 bytes of padding.  The tails of all slots lie side by side, so the tails of the
 //     consecutive slots of one split request are one contiguous range (one bulk copy for a merging CTA).
 // The scale is 6 * max|token scale| * |output_scale| / 32768 rounded up to a power of two: an
 // upper bound of |O| mapped below the fp16 maximum, so the 11-bit partials can neither overflow nor
@@ -39,7 +39,8 @@ constexpr int kMaxCombineSlots = 148;
 constexpr int kMaxSlots = 2 * kMaxCombineSlots;
 // The workspace starts with a header.  Header words (int32):
 //   [0]  generation of the last decode step that completed on this workspace
-//   [1]  CTAs of the running step that have finished (zero whenever no step is running)
+//   [1]  CTAs of the running step that have finished, [2] CTAs that have started, [3] how the step merges its partials
+//        (chosen by the first CTA that gets there); all zero whenever no step is running
 // Every slot's tail holds a flag: the generation of the step that last published the slot.  A step uses
 // generation g = header[0] + 1.  A writer stamps the flag of a slot with g once the slot's bytes are
 // visible; a merger waits until the flags of a request's slots equal g.  Flags of earlier steps never
@@ -50,6 +51,8 @@ constexpr size_t kWsTailsBytes = size_t(kMaxSlots) * kSlotTailBytes;
 constexpr size_t kWsFixedBytes = kWsHeaderBytes + kWsTailsBytes;  // what mla_fp4_workspace_init zeroes
 MLA_HD int32_t* ws_generation(void* ws) { return static_cast<int32_t*>(ws); }
 MLA_HD int32_t* ws_finished(void* ws) { return static_cast<int32_t*>(ws) + 1; }
+MLA_HD int32_t* ws_started(void* ws) { return static_cast<int32_t*>(ws) + 2; }
+MLA_HD int32_t* ws_mode(void* ws) { return static_cast<int32_t*>(ws) + 3; }
 MLA_HD uint16_t* slot_o(void* ws, int slot) { return reinterpret_cast<uint16_t*>(static_cast<char*>(ws) + kWsFixedBytes + size_t(slot) * kSlotOBytes); }
 MLA_HD const uint16_t* slot_o(const void* ws, int slot) { return reinterpret_cast<const uint16_t*>(static_cast<const char*>(ws) + kWsFixedBytes + size_t(slot) * kSlotOBytes); }
 MLA_HD float* slot_lse(void* ws, int slot) { return reinterpret_cast<float*>(static_cast<char*>(ws) + kWsHeaderBytes + size_t(slot) * kSlotTailBytes); }
@@ -57,12 +60,17 @@ MLA_HD const float* slot_lse(const void* ws, int slot) { return reinterpret_cast
 MLA_HD float* slot_scale(void* ws, int slot) { return slot_lse(ws, slot) + kGroupHeads; }
 MLA_HD const float* slot_scale(const void* ws, int slot) { return slot_lse(ws, slot) + kGroupHeads; }
 MLA_HD int32_t* slot_flag(void* ws, int slot) { return reinterpret_cast<int32_t*>(slot_scale(ws, slot) + 1); }
+MLA_HD int32_t* slot_arrivals(void* ws, int slot) { return slot_flag(ws, slot) + 1; }  // of the request whose first writer owns the slot
 // element (dim, head) of a slot's partial O
 MLA_HD size_t slot_o_index(int dim, int head) { return (size_t(head >> 3) * kLatent + size_t(dim)) * 8 + size_t(head & 7); }
 // bytes a grid of num_ctas CTAs needs: the fixed part and two partial-O slots per CTA
 __host__ __device__ constexpr size_t workspace_bytes_for(int num_ctas) { return kWsFixedBytes + size_t(2) * size_t(num_ctas) * kSlotOBytes; }
 // power-of-two scale that maps `bound` (an upper bound of |O|) to at most kSlotHalfRange
-MLA_HD float slot_scale_for(float bound) { return exp2f(ceilf(log2f(fmaxf(bound, 1e-30f) / kSlotHalfRange))); }
+#ifdef __CUDACC__
+__device__ __forceinline__ float slot_scale_for(float bound) {  // (round up to the next power of two: carry the mantissa into the exponent)
+  return __uint_as_float((__float_as_uint(fmaxf(bound, 1e-30f) / kSlotHalfRange) + 0x7fffffu) & 0x7f800000u);
+}
+#endif
 
 MLA_HD int out_elem_bytes(int out_dtype) { return out_dtype == MLA_FP4_OUT_F32 ? 4 : (out_dtype == MLA_FP4_OUT_BF16 ? 2 : 1); }
 

@@ -105,7 +105,8 @@ typedef struct MlaFp4DecodeArgs {
   int32_t enable_pdl;  /* programmatic dependent launch: lets the next kernel on the stream start its
                           prologue while the decode kernel drains (0/1) */
   int32_t phase_mask;  /* two-kernel modes only: 0 = decode + combine; 1 = decode kernel only;
-                          2 = combine kernel only (profiling) */
+                          2 = combine kernel only (profiling).  MLA_FP4_KERNEL_TCGEN05: 4 = merge split
+                          requests by their last writer even when the whole grid is resident (tests) */
   void* stream;        /* cudaStream_t */
   /* Width of a block-table row in pages (block_tables.shape[1]).  The kernels never read a row
      beyond it: a seq_lens entry larger than max_pages_per_request * page_size is treated as
@@ -155,8 +156,9 @@ int mla_fp4_plan_partition(const int32_t* seq_lens_host, int32_t batch, int32_t 
 int mla_fp4_workspace_init(void* workspace, size_t workspace_bytes, void* stream);
 
 /* One decode step on args->stream: one persistent kernel that computes the attention and merges
-   the split-KV partials (its CTAs wait for one another at the end, so it is launched
-   cooperatively: the grid must fit the device).  Stands in for the compiled callable invoked at
+   the split-KV partials.  Its CTAs wait for one another at the end only when the whole grid has
+   started by then; otherwise the last writer of each split request merges it, so steps on several
+   streams cannot block one another.  Stands in for the compiled callable invoked at
    wrappers/batch_mla_fp4.py:441-457 (mla_decode_fp4.py:60-305: split_kv_kernel +
    reduction_kernel). */
 int mla_fp4_decode(const MlaFp4DecodeArgs* args);

@@ -1,0 +1,41 @@
+"""The two forms in which the decode kernel merges split requests (shared by their CTAs, or by the last writer alone): both
+against the oracle, and reproducible to the bit, whatever the number of partials and of units per merging CTA."""
+import pytest
+import torch
+
+from oracle import mla_fp4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("lens,heads,page_size,max_ctas", [
+    ([1300], 64, 64, 2),            # two writers, one of them merges whole slots
+    ([700, 129, 64, 2500], 40, 64, None),   # fewer tiles than CTAs: the writers are not consecutive CTAs
+    ([9000, 1, 0, 600], 128, 32, None),     # two head groups, a request cut at both of a CTA's ends
+    ([33000], 64, 128, None),       # every CTA a writer: several threads per unit of the merge
+    ([5000] * 9, 16, 16, 31),       # partials at both ends of most CTAs
+])
+def test_both_merge_forms(lens, heads, page_size, max_ctas):
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("merge", [max(n, 1) for n in lens], heads, page_size, seed=sum(lens), device=dev)
+    case.seq_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=heads, page_size=page_size, max_ctas=max_ctas)
+    got = []
+    for mask in (0, 4, 4, 0):  # twice in a row: the arrival counters are back to zero after a step
+        w._phase_mask = mask
+        got.append(w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale,
+                         kv_cache_sf=case.kv_cache_sf, return_lse=True))
+        torch.cuda.synchronize()
+        w.check_device_status()
+    ref, ref_lse = O.mla_decode(case.q, case.kv_cache, case.kv_cache_sf, case.block_tables, case.seq_lens, case.softmax_scale)
+    live = torch.isfinite(ref_lse)
+    for out, lse in got:
+        O.assert_parity(out, ref, "merge forms")
+        torch.testing.assert_close(lse.cpu()[live], ref_lse[live], atol=2e-3, rtol=1e-4)
+    for i, j in ((0, 3), (1, 2)):
+        assert torch.equal(got[i][0], got[j][0]) and torch.equal(got[i][1], got[j][1])
