@@ -23,14 +23,15 @@
 // is arranged to stay under that:
 //   * latent blocks are handled in pairs (32 KiB, five pair slots = two and a half tiles in flight): one barrier, one wait
 //     and one commit per pair;
-//   * ONE warp issues all MMAs, in the order PV(t), QK(t+2): a PV pair is never torn apart by another MMA, which would
-//     cost it its collector, and the tensor pipe has QK(t+2) to work on while P(t+1) travels to shared memory;
+//   * QK^T and PV are issued by a warp each: the queue of the tensor pipe is short, so a gap in one warp's issue (a wait, the
+//     bookkeeping of a tile) is a gap of the pipe unless the other warp has something queued.  (One warp for both, in the
+//     order PV(t), QK(t+2), measured 120 us where two take XXX.)
 //   * two warps issue the copies of a tile (pair 0 and scales | RoPE and pair 1).  Each issues from one elected lane with
 //     page ids fetched 32 at a time.  (With per-lane copies, per-line L2 prefetches and a vote per wait, the one copy warp of
 //     an earlier version took 3500 clk per tile and bounded the whole kernel: 51.6 us for the north star, 138 us for B=2,
 //     H=128, q_len=2, 131072 tokens.  The TMA unit itself needs 870 clk for a tile that is in L2.)
 //
-// Warp roles (384 threads): 0 MMA issue, 1 and 3 TMA issue, 2 Q loads, merge plan, zero rows (issue warps run
+// Warp roles (384 threads): 0 QK^T issue and Q loads, 1 and 3 TMA issue, 2 merge plan and PV issue (issue warps run
 // warp-uniform code, one elected lane per instruction), 4-11 softmax / O rescale / epilogue (TMEM lane = token or dim; two
 // warps share a lane quarter and split the 64 heads).
 //
@@ -57,7 +58,7 @@ namespace mla {
 
 namespace {
 
-constexpr int kWarpMMA = 0, kWarpTMA = 1, kWarpQ = 2, kWarpTMA2 = 3;
+constexpr int kWarpQK = 0, kWarpTMA = 1, kWarpPV = 2, kWarpTMA2 = 3;
 constexpr int kWarpSoftmax0 = 4;       // 8 warps; warp & 3 is the TMEM lane quarter the warp may access
 constexpr int kThreads = 384;          // 12 warps, three per scheduler
 constexpr int kSoftmaxWarps = 8;       // warp w works on TMEM lanes 32*(w%4).. and heads 32*(w/4)..
@@ -91,10 +92,11 @@ constexpr uint32_t kOffBars = kOffScMax + kSoftmaxWarps * 4;              // mba
 __device__ __forceinline__ constexpr int bar_kv_full(int slot) { return slot; }            // a pair (and, pair 0, the tile's scales) has landed
 __device__ __forceinline__ constexpr int bar_kv_empty(int slot) { return kRing + slot; }   // PV has finished with it
 __device__ __forceinline__ constexpr int bar_s_full(int s) { return 2 * kRing + s; }       // QK^T of a tile is in TMEM
-constexpr int kBarRopeFull = 2 * kRing + 2, kBarRopeEmpty = 2 * kRing + 3, kBarPFull = 2 * kRing + 4, kBarPvDone = 2 * kRing + 5,
-              kBarQFull = 2 * kRing + 6, kBarQEmpty = 2 * kRing + 7, kBarOFree = 2 * kRing + 8, kBarDrain = 2 * kRing + 9,
-              kBarTail = 2 * kRing + 10;
-constexpr int kNumBars = 2 * kRing + 11;
+__device__ __forceinline__ constexpr int bar_s_empty(int s) { return 2 * kRing + 2 + s; }  // ... and has been read
+constexpr int kBarRopeFull = 2 * kRing + 4, kBarRopeEmpty = 2 * kRing + 5, kBarPFull = 2 * kRing + 6, kBarPvDone = 2 * kRing + 7,
+              kBarQFull = 2 * kRing + 8, kBarQEmpty = 2 * kRing + 9, kBarOFree = 2 * kRing + 10, kBarDrain = 2 * kRing + 11,
+              kBarTail = 2 * kRing + 12;
+constexpr int kNumBars = 2 * kRing + 13;
 constexpr uint32_t kOffTail = (kOffBars + kNumBars * 8 + 15u) & ~15u;     // merge plan: [148] slot ids
 constexpr uint32_t kOffSegs = kOffTail + kMaxCombineSlots * 4;            // Segment[kMaxSeg]
 constexpr uint32_t kOffMisc = kOffSegs + kMaxSeg * 24;
@@ -390,7 +392,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
 }
 
 // ------------------------------------------------------------------------------------------
-// role: MMA issue (warp 0).  The whole warp runs this code with uniform control flow; only the
+// roles: MMA issue.  The whole warp runs this code with uniform control flow; only the
 // tcgen05 instructions sit under elect_one(), so their operands stay in uniform registers.
 // ------------------------------------------------------------------------------------------
 // A shared-memory descriptor as two words.  Only the 14-bit address field (bytes >> 4) in the low word
@@ -405,123 +407,115 @@ __device__ __forceinline__ Desc make_desc(uint32_t addr, uint32_t lbo, uint32_t 
   return Desc{uint32_t(d), uint32_t(d >> 32)};
 }
 
-// QK^T of the role's next tile: RoPE first (its commit frees the one RoPE buffer for the next tile), then the two pairs.
-__device__ __forceinline__ bool issue_qk(uint32_t smem, uint32_t tmem, uint32_t it, RoleState& q) {
-  const uint32_t s64 = 64u * (it & 1);
-  const Desc rope = make_desc(smem + kOffRope, 16, 512, 4), q_rope = make_desc(smem + kOffQRope, 16, 512, 4);
-  const Desc kv = make_desc(smem + kOffKV, 16, 1024, 2), q_lat = make_desc(smem + kOffQLat, 16, 1024, 2);  // K-major, 128B swizzle
-  if (!wait(smem, kBarRopeFull, it & 1)) return false;
-  MLA_STAMP(0, it, 0);
-  ptx::tc_fence_after();
-  if (ptx::elect_one()) {
-#pragma unroll
-    for (uint32_t ks = 0; ks < 2; ++ks) ptx::umma_f8(tmem + kColSRope + s64, rope.at(2 * ks), q_rope.at(2 * ks), kIdescQKRope, ks);
-    ptx::umma_commit(bar_addr(smem, kBarRopeEmpty));
-  }
-  __syncwarp();
-#pragma unroll 1
-  for (uint32_t pr = 0; pr < 2; ++pr) {
-    if (!wait(smem, bar_kv_full(q.slot), q.lap & 1)) return false;
-    ptx::tc_fence_after();
-    const uint32_t a = q.slot * (kPairBytes >> 4), b = pr * ((2 * kGroupHeads * 128) >> 4);
-    if (ptx::elect_one()) {
-#pragma unroll
-      for (uint32_t j = 0; j < 2; ++j)
-#pragma unroll
-        for (uint32_t ks = 0; ks < 4; ++ks)
-          ptx::umma_f8(tmem + kColSLat + s64, kv.at(a + j * (kBlockBytes >> 4) + 2 * ks), q_lat.at(b + j * ((kGroupHeads * 128) >> 4) + 2 * ks),
-                       kIdescQK, (pr | j | ks) ? 1u : 0u);
-      if (pr) ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
-    }
-    __syncwarp();
-    q.advance(1);
-  }
-  MLA_STAMP(0, it, 1);
-  return true;
-}
-
-// PV of the role's next tile: per block of 128 dims 4 token steps x (hi, lo), which share A through the collector; the
-// commit after a pair frees its slot.
-__device__ __forceinline__ void issue_pv(uint32_t smem, uint32_t tmem, bool first_of_segment, RoleState& v) {
-  const Desc kv = make_desc(smem + kOffKV, kBlockBytes, 1024, 2);  // V^T: MN-major, 128B swizzle; 32 tokens per step = 4 groups of 8 rows (4096 B)
-  const Desc pd = make_desc(smem + kOffP, 512, 512, 4);            // P^T: MN-major (64 heads contiguous), 64B swizzle; 2048 B per step
-  ptx::tc_fence_after();
-#pragma unroll 1
-  for (uint32_t pr = 0; pr < 2; ++pr) {
-    const uint32_t a = v.slot * (kPairBytes >> 4), d = tmem + kColO + 128u * pr;
-    if (ptx::elect_one()) {
-#pragma unroll
-      for (uint32_t j = 0; j < 2; ++j)
-#pragma unroll
-        for (uint32_t ks = 0; ks < 4; ++ks) {
-          const uint64_t ad = kv.at(a + j * (kBlockBytes >> 4) + 256 * ks);
-          ptx::umma_f8_a_fill(d + 64u * j, ad, pd.at(128 * ks), kIdescPV, (ks || !first_of_segment) ? 1u : 0u);
-          ptx::umma_f8_a_lastuse(d + 64u * j, ad, pd.at(((kTile * 64) >> 4) + 128 * ks), kIdescPV, 1u);
-        }
-      ptx::umma_commit(bar_addr(smem, bar_kv_empty(v.slot)));
-      if (pr) ptx::umma_commit(bar_addr(smem, kBarPvDone));
-    }
-    __syncwarp();
-    v.advance(1);
-  }
-}
-
-// Order: QK(0), QK(1), then PV(t), QK(t+2).  A P that is full tells that the softmax has read S of its tile, so the S stage
-// that QK(t+2) overwrites is free without a barrier of its own.
-__device__ __forceinline__ void mma_role(uint32_t smem, uint32_t tmem, RoleState& q, RoleState& v) {
+// role: QK^T issue and Q loads (warp 0).  RoPE first (its commit frees the one RoPE buffer for the next tile), then the two
+// pairs.  There is one Q buffer, so Q of a segment is loaded by the warp that needs it, when the last QK^T of the segment
+// before has completed.
+__device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, uint32_t tmem, const CUtensorMap* map_q_lat,
+                                        const CUtensorMap* map_q_rope, RoleState& st) {
   const int nseg = misc_of(smem)->nseg;
   const Segment* sg = segs_of(smem);
+  const Desc rope = make_desc(smem + kOffRope, 16, 512, 4), q_rope = make_desc(smem + kOffQRope, 16, 512, 4);
+  const Desc kv = make_desc(smem + kOffKV, 16, 1024, 2), q_lat = make_desc(smem + kOffQLat, 16, 1024, 2);  // K-major, 128B swizzle
+  bool ok = true;
 #pragma unroll 1
-  for (int si = 0; si < nseg; ++si, ++v.seg) {
-    const uint32_t n = uint32_t(sg[si].tile_end - sg[si].tile_begin);
-    if (!wait(smem, kBarQFull, v.seg & 1)) return;
+  for (int si = 0; si < nseg && ok; ++si, ++st.seg) {
+    const Segment g = sg[si];
+    if (st.seg >= 1 && !wait(smem, kBarQEmpty, (st.seg - 1) & 1)) break;
+    int qpos, head0;
+    group_coords(g.g, p.num_heads, qpos, head0);
+    if (ptx::elect_one()) {
+      const uint32_t bar = bar_addr(smem, kBarQFull);
+      ptx::mbar_arrive_expect_tx(bar, kGroupHeads * kQDim);
+      ptx::tma_load_4d(smem + kOffQRope, map_q_rope, bar, kLatent, head0, qpos, g.b);
 #pragma unroll 1
-    for (uint32_t t = 0; t < n + 2; ++t) {  // step t: PV of tile t-2, QK of tile t
-      if (t >= 2) {
-        if (t == 2 && v.seg >= 1 && !wait(smem, kBarOFree, (v.seg - 1) & 1)) return;  // O^T of the previous segment has been read out
-        if (!wait(smem, kBarPFull, v.it & 1)) return;
-        MLA_STAMP(0, v.it, 2);
-        issue_pv(smem, tmem, t == 2, v);
-        MLA_STAMP(0, v.it, 3);
-        ++v.it;
-      }
-      if (t < n) {
-        if (!issue_qk(smem, tmem, q.it, q)) return;
-        ++q.it;
-        if (t == n - 1) {  // every QK^T of this segment has been issued: Q may be overwritten once they complete
-          if (ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarQEmpty));
-          __syncwarp();
-        }
-      }
+      for (int j = 0; j < kBlocks; ++j)
+        ptx::tma_load_4d(smem + kOffQLat + j * kGroupHeads * 128, map_q_lat, bar, 128 * j, head0, qpos, g.b);
     }
+    __syncwarp();
+    ok = wait(smem, kBarQFull, st.seg & 1);
+#pragma unroll 1
+    for (int t = g.tile_begin; t < g.tile_end && ok; ++t, ++st.it) {
+      const uint32_t it = st.it, s64 = 64u * (it & 1);
+      // S of this stage has been read by the softmax of tile it-2; the RoPE bytes of this tile have landed
+      if (it >= 2) ok = wait(smem, bar_s_empty(it & 1), ((it >> 1) - 1) & 1);
+      ok = ok && wait(smem, kBarRopeFull, it & 1);
+      if (!ok) break;
+      MLA_STAMP(0, it, 0);
+      ptx::tc_fence_after();
+      if (ptx::elect_one()) {
+#pragma unroll
+        for (uint32_t ks = 0; ks < 2; ++ks) ptx::umma_f8(tmem + kColSRope + s64, rope.at(2 * ks), q_rope.at(2 * ks), kIdescQKRope, ks);
+        ptx::umma_commit(bar_addr(smem, kBarRopeEmpty));
+      }
+      __syncwarp();
+#pragma unroll 1
+      for (uint32_t pr = 0; pr < 2 && ok; ++pr) {
+        ok = wait(smem, bar_kv_full(st.slot), st.lap & 1);
+        if (!ok) break;
+        ptx::tc_fence_after();
+        const uint32_t a = st.slot * (kPairBytes >> 4), b = pr * ((2 * kGroupHeads * 128) >> 4);
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j)
+#pragma unroll
+            for (uint32_t ks = 0; ks < 4; ++ks)
+              ptx::umma_f8(tmem + kColSLat + s64, kv.at(a + j * (kBlockBytes >> 4) + 2 * ks), q_lat.at(b + j * ((kGroupHeads * 128) >> 4) + 2 * ks),
+                           kIdescQK, (pr | j | ks) ? 1u : 0u);
+          if (pr) ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
+        }
+        __syncwarp();
+        st.advance(1);
+      }
+      MLA_STAMP(0, it, 1);
+    }
+    // every QK^T of this segment has been issued: Q may be overwritten once they complete
+    if (ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarQEmpty));
+    __syncwarp();
   }
+  if (misc_of(smem)->abort && (threadIdx.x & 31) == 0) {  // a Q load in flight lands (one of the two waits runs to its bound)
+    drain_wait(smem, kBarQFull, 0);
+    drain_wait(smem, kBarQFull, 1);
+  }
+  __syncwarp();
 }
 
-// role: Q loads (warp 2)
-__device__ __forceinline__ void issue_q(const DecodeParams& p, uint32_t smem, const Segment& g, const CUtensorMap* map_q_lat, const CUtensorMap* map_q_rope) {
-  int qpos, head0;
-  group_coords(g.g, p.num_heads, qpos, head0);
-  const uint32_t bar = bar_addr(smem, kBarQFull);
-  if (ptx::elect_one()) {
-    ptx::mbar_arrive_expect_tx(bar, kGroupHeads * kQDim);
-#pragma unroll 1
-    for (int j = 0; j < kBlocks; ++j)
-      ptx::tma_load_4d(smem + kOffQLat + j * kGroupHeads * 128, map_q_lat, bar, 128 * j, head0, qpos, g.b);
-    ptx::tma_load_4d(smem + kOffQRope, map_q_rope, bar, kLatent, head0, qpos, g.b);
-  }
-  __syncwarp();
-}
-__device__ __forceinline__ void q_role(const DecodeParams& p, uint32_t smem, const CUtensorMap* map_q_lat, const CUtensorMap* map_q_rope,
-                                       RoleState& st, int issued) {
+// role: PV issue (warp 2).  Per block of 128 dims 4 token steps x (hi, lo), which share A through the collector; the commit
+// after a pair frees its slot.
+__device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState& st) {
   const int nseg = misc_of(smem)->nseg;
-  if (nseg > 0) st.seg += uint32_t(issued);  // the caller has issued the first one
+  const Segment* sg = segs_of(smem);
+  const Desc kv = make_desc(smem + kOffKV, kBlockBytes, 1024, 2);  // V^T: MN-major, 128B swizzle; 32 tokens per step = 4 groups of 8 rows (4096 B)
+  const Desc pd = make_desc(smem + kOffP, 512, 512, 4);            // P^T: MN-major (64 heads contiguous), 64B swizzle; 2048 B per step
 #pragma unroll 1
-  for (int si = issued; si < nseg; ++si, ++st.seg) {
-    if (st.seg >= 1 && !wait(smem, kBarQEmpty, (st.seg - 1) & 1)) break;
-    issue_q(p, smem, segs_of(smem)[si], map_q_lat, map_q_rope);
+  for (int si = 0; si < nseg; ++si, ++st.seg) {
+    const uint32_t n = uint32_t(sg[si].tile_end - sg[si].tile_begin);
+    if (st.seg >= 1 && !wait(smem, kBarOFree, (st.seg - 1) & 1)) return;  // O^T of the previous segment has been read out
+#pragma unroll 1
+    for (uint32_t t = 0; t < n; ++t, ++st.it) {
+      if (!wait(smem, kBarPFull, st.it & 1)) return;
+      MLA_STAMP(0, st.it, 2);
+      ptx::tc_fence_after();
+#pragma unroll 1
+      for (uint32_t pr = 0; pr < 2; ++pr) {
+        const uint32_t a = st.slot * (kPairBytes >> 4), d = tmem + kColO + 128u * pr;
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j)
+#pragma unroll
+            for (uint32_t ks = 0; ks < 4; ++ks) {
+              const uint64_t ad = kv.at(a + j * (kBlockBytes >> 4) + 256 * ks);
+              ptx::umma_f8_a_fill(d + 64u * j, ad, pd.at(128 * ks), kIdescPV, (ks || t) ? 1u : 0u);
+              ptx::umma_f8_a_lastuse(d + 64u * j, ad, pd.at(((kTile * 64) >> 4) + 128 * ks), kIdescPV, 1u);
+            }
+          ptx::umma_commit(bar_addr(smem, bar_kv_empty(st.slot)));
+          if (pr) ptx::umma_commit(bar_addr(smem, kBarPvDone));
+        }
+        __syncwarp();
+        st.advance(1);
+      }
+      MLA_STAMP(0, st.it, 3);
+    }
   }
-  if (misc_of(smem)->abort && st.seg >= 1 && (threadIdx.x & 31) == 0) drain_wait(smem, kBarQFull, (st.seg - 1) & 1);
-  __syncwarp();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -900,6 +894,9 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       }
 #pragma unroll
       for (int h = 0; h < kPairs; ++h) l2[h] = add2(l2[h], e2[h]);
+      ptx::tc_fence_before();  // orders the S reads before the arrival
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar_addr(smem, bar_s_empty(s)));
       if (tid == 0) MLA_STAMP(3, it, 1);
       // The one P buffer (and, for a rescale, O^T) is free once the PV of the previous tile has completed; until then
       // this tile's P' stays in registers.
@@ -917,7 +914,7 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
                      "r"(pr.lo[4 * cidx + 2]), "r"(pr.lo[4 * cidx + 3]) : "memory");
       }
       ptx::fence_proxy_async_smem();
-      ptx::tc_fence_before();  // orders the S reads (and the O^T writes of a rescale) before the arrival
+      ptx::tc_fence_before();  // orders the O^T writes of a rescale before the arrival
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar_addr(smem, kBarPFull));
       if (tid == 0) MLA_STAMP(3, it, 2);
@@ -1280,13 +1277,14 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
 
   // What needs nothing an earlier kernel wrote comes first: with a programmatic dependent launch this part runs
   // while the kernel before this one on the stream is still draining.
-  if (warp == kWarpMMA) {
+  if (warp == kWarpQK) {
     ptx::tmem_alloc(smem + kOffMisc + offsetof(Misc, tmem_base), 512);
     ptx::tmem_relinquish();
-  } else if (warp == kWarpQ) {
+  } else if (warp == kWarpPV) {
     if (lane < kNumBars) {  // lane i: barrier i
       uint32_t count = 1;
-      if (lane == kBarPFull || lane == kBarOFree) count = kSoftmaxWarps;
+      if (lane == kBarPFull || lane == kBarOFree || lane == bar_s_empty(0) || lane == bar_s_empty(1)) count = kSoftmaxWarps;
+      if (lane == kBarDrain) count = 2;  // the two MMA warps
       if (lane == kBarTail) count = 4;
       ptx::mbar_init(bar_addr(smem, lane), count);
     }
@@ -1312,7 +1310,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) MLA_STAMP(4, 1u, 1);
 
-  RoleState st{0, 0, 0, 0}, sv{0, 0, 0, 0};
+  RoleState st{0, 0, 0, 0};
   if (warp == kWarpTMA2) st.slot = 1;
   // Rounds: almost always exactly one; more only when a CTA's range spans more than kMaxSeg requests.
   // The partition is walked by the warp that issues the first copies: it goes on to them without waiting for the others.
@@ -1323,7 +1321,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   } else {
     // The generation of this step: one more than that of the last completed step.  No CTA of this step
     // can have advanced it yet (that takes every CTA of the grid to have finished).
-    if (warp == kWarpQ && lane == 0 && p.fused_merge) {
+    if (warp == kWarpPV && lane == 0 && p.fused_merge) {
       atomicAdd(ws_started(p.workspace), 1);
       misc->gen = ld_acquire(ws_generation(p.workspace)) + 1;
     }
@@ -1335,17 +1333,14 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   for (;;) {
     if (warp >= kWarpSoftmax0) {
       softmax_role<kSoftCap>(p, smem, tmem, tid - 32 * kWarpSoftmax0, st);
-    } else if (warp == kWarpMMA) {
-      mma_role(smem, tmem, st, sv);
-    } else if (warp == kWarpQ) {
-      if (first_round && misc->nseg > 0) {  // ahead of the planning: the first tile waits for it
-        issue_q(p, smem, segs_of(smem)[0], &map_q_lat, &map_q_rope);
-      }
-      if (first_round && p.fused_merge) {  // (the two-kernel modes leave both to the combine kernel)
+    } else if (warp == kWarpQK) {
+      qk_role(p, smem, tmem, &map_q_lat, &map_q_rope, st);
+    } else if (warp == kWarpPV) {
+      if (first_round && p.fused_merge) {  // (the two-kernel modes leave both to the combine kernel); the first P is far away
         plan_merge(smem, 0, lane);
         zero_empty_requests(p, lane);
       }
-      q_role(p, smem, &map_q_lat, &map_q_rope, st, first_round ? 1 : 0);
+      pv_role(smem, tmem, st);
     } else {
       tma_role(p, smem, warp == kWarpTMA2 ? 1u : 0u, &map_rope, &map_lat, st);
     }
@@ -1354,12 +1349,12 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       // Last round: drain (everything issued has completed before TMEM is released and before shared memory is reused:
       // a commit covers the MMAs of the thread that executes it), then these four warps, idle from here on, fetch the
       // partials of the request this CTA merges while the softmax warps finish with its own.
-      if (warp == kWarpMMA && ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
+      if ((warp == kWarpQK || warp == kWarpPV) && ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
       __syncwarp();
       if (lane == 0) drain_wait(smem, kBarDrain, 0);
       __syncwarp();
       if (p.fused_merge) {
-        if (warp == kWarpQ && lane == 0 && (misc->merge[0].vtiles | misc->merge[1].vtiles)) misc->mode = merge_mode(p);
+        if (warp == kWarpPV && lane == 0 && (misc->merge[0].vtiles | misc->merge[1].vtiles)) misc->mode = merge_mode(p);
         ptx::bar_sync(3, 128);
         if (misc->n_slots > 0 && misc->mode == kMergeShared) tail_fetch(p, smem, warp, lane, true);
         if (tid == 0) MLA_STAMP(4, 0u, 1);
@@ -1371,7 +1366,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     if (warp == kWarpTMA) stage_segments(p, smem, lane, false);
     __syncthreads();
   }
-  if (warp == kWarpMMA) {
+  if (warp == kWarpQK) {
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
