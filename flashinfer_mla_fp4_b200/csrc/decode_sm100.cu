@@ -613,11 +613,6 @@ struct SoftmaxTile {
   uint64_t cap2, rcap2;    // soft-cap variant: (cap, cap), (1/cap, 1/cap)
   bool valid;
 };
-// A thread's P' of one tile: 32 heads x (hi, lo) as bytes, kept in registers until the P buffer is free.
-struct PRegs {
-  uint32_t hi[8], lo[8];
-};
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -633,63 +628,59 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// One pass over the 32 heads this thread owns of its token: e = exp2(x*c - m) and P' = e*scale_t split into two
-// E4M3 terms.  Speculative: the largest exponent argument seen is returned for the lazy-reference check, and e is added
-// to the row sums by the caller only once the reference stands (a score may beat it by hundreds of binades, heavy-tailed
-// token scales: such an e is infinite and is thrown away).  Bound by instruction issue (two softmax warps per scheduler).
+// First half of a tile's softmax, over the 32 heads this thread owns of its token: e = exp2(x*c - m) with the reference as it
+// stands; returns the largest exponent argument for the lazy-reference check.  Nothing has been summed or converted yet, so
+// a reference that turns out to be beaten costs a scaling of e, not a second pass.  The S columns of the second 16 heads are
+// on their way while the first are exponentiated.
 // kSoftCap: the raw score x = q.k passes through cap * tanh(x / cap) first (compiled only into the soft-cap kernel).
 template <bool kSoftCap>
-__device__ __forceinline__ float softmax_pass(const SoftmaxTile& t, uint64_t (&e2)[kPairs], PRegs& pr) {
+__device__ __forceinline__ float exp_pass(const SoftmaxTile& t, uint64_t (&e2)[kPairs]) {
   float mx = -INFINITY;
+  uint32_t a[2][16], b[2][16];
+  ptx::tmem_ld16(t.t_lat, a[0]);
+  ptx::tmem_ld16(t.t_rope, b[0]);
+  ptx::tmem_wait_ld();
 #pragma unroll
   for (int cidx = 0; cidx < 2; ++cidx) {
-    uint32_t a[16], b[16];
-    ptx::tmem_ld16(t.t_lat + 16 * cidx, a);
-    ptx::tmem_ld16(t.t_rope + 16 * cidx, b);
-    ptx::tmem_wait_ld();
-    uint32_t hi16[8], lo16[8];
-    if (!t.valid) {  // token beyond seq_len: weight exactly zero, whatever its row holds (its RoPE bytes may decode to NaN)
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        hi16[q] = lo16[q] = 0u;
-        e2[8 * cidx + q] = 0ull;
-      }
+    if (cidx == 0) {
+      ptx::tmem_ld16(t.t_lat + 16, a[1]);
+      ptx::tmem_ld16(t.t_rope + 16, b[1]);
     } else {
+      ptx::tmem_wait_ld();
+    }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {  // 4 heads per shared load of the references
-        uint64_t nm[2];
-        lds_pairs(t.negm + 64 * cidx + 16 * q, nm[0], nm[1]);
+    for (int q = 0; q < 4; ++q) {  // 4 heads per shared load of the references
+      uint64_t nm[2];
+      lds_pairs(t.negm + 64 * cidx + 16 * q, nm[0], nm[1]);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int i = 4 * q + 2 * h;
-          uint64_t x2 = fma2(pack2u(a[i], a[i + 1]), t.sc2, pack2u(b[i], b[i + 1]));
-          if (kSoftCap) {
-            float x0, x1;
-            unpack2(mul2(x2, t.rcap2), x0, x1);
-            x2 = mul2(pack2(tanh_approx(x0), tanh_approx(x1)), t.cap2);
-          }
-          float a0, a1;
-          unpack2(fma2(x2, t.cs2, nm[h]), a0, a1);
-          mx = max3(mx, a0, a1);
-          const uint64_t e = pack2(ptx::ex2(a0), ptx::ex2(a1));
-          e2[8 * cidx + 2 * q + h] = e;
-          hi16[2 * q + h] = split_e4m3x2(mul2(e, t.sc2), lo16[2 * q + h]);
+      for (int h = 0; h < 2; ++h) {
+        const int i = 4 * q + 2 * h;
+        uint64_t x2 = fma2(pack2u(a[cidx][i], a[cidx][i + 1]), t.sc2, pack2u(b[cidx][i], b[cidx][i + 1]));
+        if (kSoftCap) {
+          float x0, x1;
+          unpack2(mul2(x2, t.rcap2), x0, x1);
+          x2 = mul2(pack2(tanh_approx(x0), tanh_approx(x1)), t.cap2);
         }
+        float a0, a1;
+        unpack2(fma2(x2, t.cs2, nm[h]), a0, a1);
+        mx = max3(mx, a0, a1);
+        e2[8 * cidx + 2 * q + h] = pack2(ptx::ex2(a0), ptx::ex2(a1));
       }
     }
+  }
+  if (!t.valid) {  // token beyond seq_len: weight exactly zero, whatever its row holds (its RoPE bytes may decode to NaN)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      pr.hi[4 * cidx + q] = hi16[2 * q] | (hi16[2 * q + 1] << 16);
-      pr.lo[4 * cidx + q] = lo16[2 * q] | (lo16[2 * q + 1] << 16);
-    }
+    for (int q = 0; q < kPairs; ++q) e2[q] = 0ull;
+    mx = -INFINITY;
   }
   return mx;
 }
 
-// Refresh the per-head reference: column max of y = x*c + log2(scale_t) over the tile's tokens,
-// m = max(m_old, colmax - shift); f = 2^(m_old - m) (0 when there was no reference yet).
+// Set the per-head reference from the scores: column max of y = x*c + log2(scale_t) over the tile's tokens,
+// m = max(m_old, colmax - shift); f = 2^(m_old - m) (0 when there was no reference yet).  Used by the first tile of a segment
+// and when a score beats the reference by so much that its exponential overflows.
 template <bool kSoftCap>
-__device__ __noinline__ void refresh_reference(uint32_t smem, uint32_t t_lat, uint32_t t_rope, float sc, bool valid,
+__device__ __noinline__ void reference_from_scores(uint32_t smem, uint32_t t_lat, uint32_t t_rope, float sc, bool valid,
                                                float cscale, float lg, bool have_m, int tid, float cap) {
   const float rcap = kSoftCap ? 1.f / cap : 0.f;
   const int warp = tid >> 5, lane = tid & 31;
@@ -724,19 +715,73 @@ __device__ __noinline__ void refresh_reference(uint32_t smem, uint32_t t_lat, ui
   ptx::bar_sync(1, kSoftmaxThreads);
 }
 
-// O^T *= f per head column, in TMEM (all four 128-dim blocks of this thread's lane)
-__device__ __noinline__ void rescale_output(uint32_t smem, uint32_t tmem_lane, uint32_t half) {
-#pragma unroll 1
-  for (int jc = 0; jc < kBlocks * 2; ++jc) {
-    uint32_t o[16];
-    const uint32_t col = 64u * (jc >> 1) + 32u * half + 16u * (jc & 1);
-    const uint32_t ta = tmem_lane + kColO + col;
-    ptx::tmem_ld16(ta, o);
-    ptx::tmem_wait_ld();
-    const uint32_t f = smem + kOffF + 4 * (col & 63);
+// Move the references that were beaten by more than the lazy threshold, from the exponentials at hand: column max of
+// P' = e * |scale_t| over the tile's tokens; m += log2(colmax) - shift and f = its inverse for those heads, f = 1 for all others.
+__device__ __forceinline__ void refresh_beaten(uint32_t smem, const uint64_t (&e2)[kPairs], float sc_abs, int tid) {
+  const int warp = tid >> 5, lane = tid & 31;
+  const int quarter = warp & 3, half = warp >> 2;
+  const uint32_t wred = smem + kOffWmax;
+  uint32_t mine = 0;  // lane i: head 32*half + i (non-negative floats compare as integers)
 #pragma unroll
-    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * lds_f32(f + 4 * i));
-    ptx::tmem_st16(ta, o);
+  for (int i = 0; i < kPairs; ++i) {
+    float e0, e1;
+    unpack2(e2[i], e0, e1);
+    const uint32_t r0 = __reduce_max_sync(0xffffffffu, __float_as_uint(e0 * sc_abs)), r1 = __reduce_max_sync(0xffffffffu, __float_as_uint(e1 * sc_abs));
+    if ((lane >> 1) == i) mine = (lane & 1) ? r1 : r0;
+  }
+  sts_f32(wred + 4 * (quarter * kGroupHeads + 32 * half + lane), __uint_as_float(mine));
+  ptx::bar_sync(1, kSoftmaxThreads);
+  if (tid < kGroupHeads) {
+    const float cm = fmaxf(fmaxf(lds_f32(wred + 4 * tid), lds_f32(wred + 4 * (kGroupHeads + tid))),
+                           fmaxf(lds_f32(wred + 4 * (2 * kGroupHeads + tid)), lds_f32(wred + 4 * (3 * kGroupHeads + tid))));
+    float f = 1.f;
+    if (cm > 430.f) {  // 2^(shift + threshold)
+      const float d = __log2f(cm) - kPShift;
+      f = ptx::ex2(-d);
+      sts_f32(smem + kOffM + 4 * tid, lds_f32(smem + kOffM + 4 * tid) - d);
+    }
+    sts_f32(smem + kOffF + 4 * tid, f);
+  }
+  ptx::bar_sync(1, kSoftmaxThreads);
+}
+
+// O^T *= f per head column, in TMEM (all four 128-dim blocks of this thread's lane).  With few heads moved, as a new maximum
+// usually has it, column by column.
+__device__ __noinline__ void rescale_output(uint32_t smem, uint32_t tmem_lane, uint32_t half, int lane) {
+  const uint32_t base = tmem_lane + kColO + 32u * half;
+  const float mine = lds_f32(smem + kOffF + 4 * (32u * half + uint32_t(lane)));
+  uint32_t moved = __ballot_sync(0xffffffffu, mine != 1.f);
+  if (__popc(moved) <= 8) {
+#pragma unroll 1
+    while (moved) {
+      const uint32_t h = uint32_t(__ffs(moved)) - 1u;
+      moved &= moved - 1u;
+      const float f = __shfl_sync(0xffffffffu, mine, int(h));
+      uint32_t o[kBlocks];
+#pragma unroll
+      for (int j = 0; j < kBlocks; ++j) ptx::tmem_ld1(base + 64u * j + h, o[j]);
+      ptx::tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < kBlocks; ++j) ptx::tmem_st1(base + 64u * j + h, __float_as_uint(__uint_as_float(o[j]) * f));
+    }
+  } else {
+#pragma unroll 1
+    for (uint32_t jc = 0; jc < kBlocks * 2; ++jc) {
+      uint32_t o[16];
+      const uint32_t ta = base + 64u * (jc >> 1) + 16u * (jc & 1);
+      ptx::tmem_ld16(ta, o);
+      const uint32_t f = smem + kOffF + 4 * (32u * half + 16u * (jc & 1));
+      ptx::tmem_wait_ld();
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 v = lds_f32x4(f + 16 * q);
+        o[4 * q] = __float_as_uint(__uint_as_float(o[4 * q]) * v.x);
+        o[4 * q + 1] = __float_as_uint(__uint_as_float(o[4 * q + 1]) * v.y);
+        o[4 * q + 2] = __float_as_uint(__uint_as_float(o[4 * q + 2]) * v.z);
+        o[4 * q + 3] = __float_as_uint(__uint_as_float(o[4 * q + 3]) * v.w);
+      }
+      ptx::tmem_st16(ta, o);
+    }
   }
   ptx::tmem_wait_st();
 }
@@ -866,52 +911,63 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       if (tid == 0) MLA_STAMP(3, it, 0);
       ptx::tc_fence_after();
 
-      // The pass runs with the reference as it stands, which holds unless some score beat it by more than the lazy threshold
-      // (P' would leave the E4M3 range; the second test catches a large score of a token with a vanishing scale, whose e
-      // would overflow).  Then the reference is refreshed, sums and O^T are rescaled and the pass runs once more.  The
-      // first tile of a segment sets the reference before anything is exponentiated.
-      PRegs pr;
+      // The exponentials are taken with the reference as it stands, which holds unless some score beat it by more than the lazy
+      // threshold (P' would leave the E4M3 range; the second test catches a large score of a token with a vanishing scale).
+      // Then the references of the heads concerned are moved, and e, the sums and, below, O^T are scaled.  Latents with
+      // heavy-tailed scales do that in every other tile: recomputing the whole pass there cost 3900 clk each time.
       uint64_t e2[kPairs];
-      bool refresh = first;
+      bool moved = false;
+      if (first) reference_from_scores<kSoftCap>(smem, t.t_lat, t.t_rope, sc, t.valid, cscale, lg, false, tid, cap);
 #pragma unroll 1
-      for (int rep = 0;; ++rep) {
-        if (refresh) {
-          refresh_reference<kSoftCap>(smem, t.t_lat, t.t_rope, sc, t.valid, cscale, lg, !first, tid, cap);
-          if (!first) {
+      for (;;) {
+        const float mx = exp_pass<kSoftCap>(t, e2);
+        if (first || moved) break;
+        if (!ptx::bar_or(1, kSoftmaxThreads, mx + lg > kPShift + kLazyThreshold || mx > 100.f)) break;
+        moved = true;
+        const bool overflow = ptx::bar_or(1, kSoftmaxThreads, mx > 100.f);
+        if (overflow) reference_from_scores<kSoftCap>(smem, t.t_lat, t.t_rope, sc, t.valid, cscale, lg, true, tid, cap);
+        else refresh_beaten(smem, e2, fabsf(sc), tid);
 #pragma unroll
-            for (int q = 0; q < kPairs / 2; ++q) {
-              uint64_t f0, f1;
-              lds_pairs(smem + kOffF + 4 * kHalfHeads * half + 16 * q, f0, f1);
-              l2[2 * q] = mul2(l2[2 * q], f0);
-              l2[2 * q + 1] = mul2(l2[2 * q + 1], f1);
-            }
+        for (int q = 0; q < kPairs / 2; ++q) {
+          uint64_t f[2];
+          lds_pairs(smem + kOffF + 4 * kHalfHeads * half + 16 * q, f[0], f[1]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            l2[2 * q + h] = mul2(l2[2 * q + h], f[h]);
+            e2[2 * q + h] = mul2(e2[2 * q + h], f[h]);
           }
         }
-        const float mx = softmax_pass<kSoftCap>(t, e2, pr);
-        if (refresh) break;
-        refresh = ptx::bar_or(1, kSoftmaxThreads, t.valid && (mx + lg > kPShift + kLazyThreshold || mx > 100.f));
-        if (!refresh) break;
+        if (!overflow) break;
       }
-#pragma unroll
-      for (int h = 0; h < kPairs; ++h) l2[h] = add2(l2[h], e2[h]);
       ptx::tc_fence_before();  // orders the S reads before the arrival
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar_addr(smem, bar_s_empty(s)));
+      // Second half: row sums, and P' = e * scale_t split into two E4M3 terms
+      uint32_t hi[8], lo[8];
+#pragma unroll
+      for (int q = 0; q < kPairs / 2; ++q) {
+        uint32_t l0, l1;
+        const uint32_t h0 = split_e4m3x2(mul2(e2[2 * q], t.sc2), l0), h1 = split_e4m3x2(mul2(e2[2 * q + 1], t.sc2), l1);
+        hi[q] = h0 | (h1 << 16);
+        lo[q] = l0 | (l1 << 16);
+        l2[2 * q] = add2(l2[2 * q], e2[2 * q]);
+        l2[2 * q + 1] = add2(l2[2 * q + 1], e2[2 * q + 1]);
+      }
       if (tid == 0) MLA_STAMP(3, it, 1);
       // The one P buffer (and, for a rescale, O^T) is free once the PV of the previous tile has completed; until then
       // this tile's P' stays in registers.
       if (it >= 1) (void)wait(smem, kBarPvDone, (it - 1) & 1);
-      if (refresh && !first) {  // O^T holds earlier tiles of the segment: rescale it
+      if (moved) {  // O^T holds earlier tiles of the segment
         ptx::tc_fence_after();
-        rescale_output(smem, tmem_lane, uint32_t(half));
+        rescale_output(smem, tmem_lane, uint32_t(half), lane);
       }
 #pragma unroll
       for (int cidx = 0; cidx < 2; ++cidx) {
         const uint32_t at = p_row + (((2 * uint32_t(half) + uint32_t(cidx)) ^ psw) << 4);
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(pr.hi[4 * cidx]), "r"(pr.hi[4 * cidx + 1]),
-                     "r"(pr.hi[4 * cidx + 2]), "r"(pr.hi[4 * cidx + 3]) : "memory");
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + kTile * 64), "r"(pr.lo[4 * cidx]), "r"(pr.lo[4 * cidx + 1]),
-                     "r"(pr.lo[4 * cidx + 2]), "r"(pr.lo[4 * cidx + 3]) : "memory");
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(hi[4 * cidx]), "r"(hi[4 * cidx + 1]),
+                     "r"(hi[4 * cidx + 2]), "r"(hi[4 * cidx + 3]) : "memory");
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + kTile * 64), "r"(lo[4 * cidx]), "r"(lo[4 * cidx + 1]),
+                     "r"(lo[4 * cidx + 2]), "r"(lo[4 * cidx + 3]) : "memory");
       }
       ptx::fence_proxy_async_smem();
       ptx::tc_fence_before();  // orders the O^T writes of a rescale before the arrival
