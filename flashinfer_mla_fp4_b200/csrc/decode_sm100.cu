@@ -219,17 +219,27 @@ struct RoleState {
 // partition: the segments of this CTA (one warp; common.cuh has the same walk as a sequential loop)
 // ------------------------------------------------------------------------------------------
 // Lane i looks at request base + i: a scan gives its place in the flat tile space, the overlap with the CTA's range its
-// segment, a ballot the segment's number.  Two passes over seq_lens (the second from L1); the flat positions of whole chunks
-// of 32 requests are skipped with one reduction.  A sequential walk by one thread took 2500 clk of every CTA's prologue.
-__device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem, int lane, bool first_round) {
+// segment, a ballot the segment's number.  The lengths are kept in shared memory (the latent ring is idle now) for the second
+// pass and for plan_still_valid; whole chunks of 32 requests outside the range are skipped with one reduction.  A sequential
+// walk by one thread took 2500 clk of every CTA's prologue.
+constexpr int kLensMax = int(kRing * kPairBytes / 4);
+__device__ __forceinline__ int fresh_len(const DecodeParams& p, int i) {  // from L2: an earlier, speculative read must leave nothing in L1
+  const int n = __ldcg(p.seq_lens + i);
+  return n < p.seq_cap ? n : p.seq_cap;
+}
+__device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem, int lane, bool first_round, bool report) {
   Misc* misc = misc_of(smem);
   Segment* out = reinterpret_cast<Segment*>(smem_ptr(smem) + kOffSegs);
+  int* lens = reinterpret_cast<int*>(smem_ptr(smem) + kOffKV);
   const int n = gridDim.x, cta = blockIdx.x;
+  auto len_of = [&](int i) { return i < kLensMax ? lens[i] : fresh_len(p, i); };
   unsigned long long acc = 0;
   uint32_t mx = 0;
 #pragma unroll 4
   for (int i = lane; i < p.batch; i += 32) {
-    const uint32_t v = uint32_t(vtiles_of(capped_len(p.seq_lens, i, p.seq_cap)));
+    const int len = fresh_len(p, i);
+    if (i < kLensMax) lens[i] = len;
+    const uint32_t v = uint32_t(vtiles_of(len));
     acc += v;
     mx = max(mx, v);
   }
@@ -242,12 +252,12 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
   __syncwarp();
   if (!partition_fits(int64_t(T64) * p.groups, n)) {  // never with real caches: nothing is decoded, the status says why
     Tt = -1;
-    if (lane == 0 && p.status && first_round) atomicCAS(p.status, 0, MLA_FP4_ERR_UNSUPPORTED);
+    if (lane == 0 && p.status && report) atomicCAS(p.status, 0, MLA_FP4_ERR_UNSUPPORTED);
   } else if (whole_requests(mx > 0 ? int(mx) - kPhantom : 0, int64_t(p.batch) * p.groups, n)) {  // CTA v: pair v, whole
     Tt = flat_t(T64) * p.groups;
     if (cta < p.batch * p.groups) {
       const int g = cta / p.batch, b = cta - g * p.batch;
-      const int len = capped_len(p.seq_lens, b, p.seq_cap);
+      const int len = len_of(b);
       if (len > 0) {
         if (lane == 0) out[0] = Segment{b, g, 0, tiles_of(len), len, -1};
         nseg = 1;
@@ -264,7 +274,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
 #pragma unroll 1
       for (int base = 0; base < p.batch && run < hi && !more; base += 32) {
         const int b = base + lane;
-        const int len = b < p.batch ? capped_len(p.seq_lens, b, p.seq_cap) : 0;
+        const int len = b < p.batch ? len_of(b) : 0;
         const flat_t v = vtiles_of(len);
         const flat_t tot = __reduce_add_sync(0xffffffffu, v);
         if (run + tot > lo) {
@@ -307,6 +317,15 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
   __syncwarp();
 }
 
+// A plan made before the kernel ahead on the stream had ended stands if the lengths are what it was made from.
+__device__ __forceinline__ bool plan_still_valid(const DecodeParams& p, uint32_t smem, int lane) {
+  if (p.batch > kLensMax) return false;
+  const int* lens = reinterpret_cast<const int*>(smem_ptr(smem) + kOffKV);
+  bool same = true;
+#pragma unroll 4
+  for (int i = lane; i < p.batch; i += 32) same &= fresh_len(p, i) == lens[i];
+  return __all_sync(0xffffffffu, same);
+}
 // ------------------------------------------------------------------------------------------
 // role: TMA issue (warp 1: pair 0 and scales of every tile; warp 3: RoPE and pair 1)
 // ------------------------------------------------------------------------------------------
@@ -316,6 +335,13 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
 // Pair position 2t + w (tile t, pair w) lives in slot (2t + w) mod 5 and is filled once PV of the position five back has
 // completed, which lies in tile t-3 or t-2.  So when pair 0 of tile t is issued the softmax of tile t-3 is over, and the scale
 // stage t mod 4, last read by tile t-4, is free: it needs no barrier of its own and its bytes count on the pair's barrier.
+// page id `at + lane` of a segment, -1 beyond its pages or outside the pool
+__device__ __forceinline__ int page_window(const DecodeParams& p, const Segment& g, int at) {
+  const int ppt = kTile / p.page_size;
+  const int lp = g.tile_begin * ppt + at + int(threadIdx.x & 31);
+  const int id = lp < min((g.seq_len - 1) / p.page_size + 1, g.tile_end * ppt) ? __ldcg(p.block_tables + size_t(g.b) * p.block_table_stride + lp) : -1;
+  return int64_t(id) < p.num_pages ? id : -1;
+}
 __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, uint32_t which, const CUtensorMap* map_rope,
                                          const CUtensorMap* map_lat, RoleState& st) {
   const int nseg = misc_of(smem)->nseg;
@@ -328,14 +354,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
   for (int si = 0; si < nseg && ok; ++si, ++st.seg) {
     const Segment g = sg[si];
     const int total = (g.seq_len - 1) / p.page_size + 1;
-    const int first = g.tile_begin * ppt, last = min(total, g.tile_end * ppt);
-    const int32_t* bt_req = p.block_tables + size_t(g.b) * p.block_table_stride;
-    auto window = [&](int at) {
-      const int lp = first + at + lane;
-      const int id = lp < last ? __ldg(bt_req + lp) : -1;
-      return int64_t(id) < p.num_pages ? id : -1;
-    };
-    int cur = window(0), nxt = window(32), ahead = 64, at = 0;
+    int cur = page_window(p, g, 0), nxt = page_window(p, g, 32), ahead = 64, at = 0;
 #pragma unroll 1
     for (int t = g.tile_begin; t < g.tile_end; ++t, ++st.it) {
       const int np = min(ppt, total - t * ppt);
@@ -369,12 +388,23 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
         }
       }
       MLA_STAMP(1 + which, st.it, 1);
+      // The rows of the tile four ahead are brought into L2: the ring holds two and a half tiles, and a pair's slot comes free
+      // two tiles before the pair is needed, so a load that comes from DRAM (2000 clk instead of 900) shows in every tile:
+      // 2x131072 tokens, H=128, q_len=2: 97.5 -> 92.6 us; 8x32768: 37.6 -> 36.8.
+      if (which) {
+        const int i = at + 4 * ppt + lane;
+        const int in_cur = __shfl_sync(0xffffffffu, cur, i & 31), in_nxt = __shfl_sync(0xffffffffu, nxt, i & 31);
+        const int page = i < 32 ? in_cur : (i < 64 ? in_nxt : -1);
+        if (lane < ppt && page >= 0)
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(static_cast<const uint8_t*>(p.kv_cache) + size_t(page) * ps * kRowBytes),
+                       "r"(ps * kRowBytes) : "memory");
+      }
       st.advance(2);
       at += ppt;
       if (at == 32) {
         at = 0;
         cur = nxt;
-        nxt = window(ahead);
+        nxt = page_window(p, g, ahead);
         ahead += 32;
       }
     }
@@ -1141,7 +1171,7 @@ __device__ __noinline__ int merge_mode(const DecodeParams& p) {
 }
 
 // Fetching the partials, by the four issue warps: slot i (and i + 128) belongs to lane i / 4 of helper warp i % 4, which waits
-// for its flag (shared form) and fetches this CTA's share of it and its tail with two bulk copies.  In the shared form that
+// for its flag (shared form) and fetches this CTA's share of it with a bulk copy.  In the shared form that
 // starts as soon as the last tile's MMAs have drained, while the softmax warps still write and publish this CTA's own
 // partial.  A bulk copy costs about fifty clocks to issue whatever its size and the lanes of a warp issue theirs one after the
 // other, so the slots are dealt round the warps.  The lanes of a warp poll in step.
@@ -1150,7 +1180,7 @@ __device__ __noinline__ void tail_fetch(const DecodeParams& p, uint32_t smem, in
   void* ws = p.workspace;
   const int ns = misc->n_slots, gen = misc->gen;
   const uint32_t U0 = uint32_t(misc->unit0), share = (uint32_t(misc->unit1) - U0) * 16u;
-  const uint32_t rows = smem + kTailStage, tails = rows + uint32_t(ns) * share;
+  const uint32_t rows = smem + kTailStage;
   const uint32_t bar = bar_addr(smem, kBarTail), polls = misc->polls;
 #pragma unroll 1
   for (int i = lane * 4 + hw; __any_sync(0xffffffffu, i < ns); i += 128) {
@@ -1162,9 +1192,8 @@ __device__ __noinline__ void tail_fetch(const DecodeParams& p, uint32_t smem, in
       // writer's release put them: no proxy fence is needed for that (a full one here cost microseconds).
       if (!done && (!flags || ld_acquire(slot_flag(ws, slot)) == gen)) {
         done = true;
-        ptx::mbar_expect_tx(bar, share + kTailBytes);
+        ptx::mbar_expect_tx(bar, share);
         ptx::bulk_load(rows + uint32_t(i) * share, reinterpret_cast<const char*>(slot_o(ws, slot)) + size_t(U0) * 16, share, bar);
-        ptx::bulk_load(tails + uint32_t(i) * kTailBytes, slot_lse(ws, slot), kTailBytes, bar);  // its LSEs and scale
       }
       if (__all_sync(0xffffffffu, done) || __any_sync(0xffffffffu, misc->abort)) break;
       __nanosleep(32);
@@ -1186,9 +1215,64 @@ __device__ __forceinline__ void store_unit(const float (&acc)[8], const float4& 
     if (e < heads) store(e, acc[e] * inv[e]);
 }
 
-// out = sum_i w_i * O_i / sum  with  w_i = 2^(lse_i - max) * slot scale, over the staged shares, in slot order whatever the
-// order of arrival (bit-reproducible).  All threads of the CTA.
-__device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, int tid, uint32_t parity, bool with_lse) {
+// The merge weights w_i = 2^(lse_i - max) * slot scale of the 64 heads, and the inverse of their sum, by the eight softmax
+// warps: four lanes per head split the slots, butterflies give all four the results.  They are computed while the shares of the
+// slots are on their way: the LSEs come straight from L2.
+__device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem, int tid, bool with_lse) {
+  Misc* misc = misc_of(smem);
+  const int ns = misc->n_slots;
+  const uint32_t tails = smem + kTailStage + uint32_t(ns) * (uint32_t(misc->unit1 - misc->unit0) * 16u);
+  const int h = tid >> 2, j = tid & 3;
+  const uint32_t col = tails + 4u * uint32_t(h);
+  float mx = -INFINITY;
+#pragma unroll 1
+  for (int i0 = j; i0 < ns; i0 += 20) {  // five slots' loads in flight together
+    const float* tail[5];
+    float l[5], sc[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) tail[k] = slot_lse(p.workspace, int(lds_u32(smem + kOffTail + 4u * uint32_t(min(i0 + 4 * k, ns - 1)))));
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      l[k] = __ldcg(tail[k] + h);
+      sc[k] = __ldcg(tail[k] + kGroupHeads);  // the slot scale
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const int i = i0 + 4 * k;
+      mx = fmaxf(mx, l[k]);  // (a repeated last slot changes nothing)
+      if (i < ns) {
+        sts_f32(col + uint32_t(i) * kTailBytes, l[k]);
+        if (h == 0) sts_f32(tails + uint32_t(i) * kTailBytes + 4u * kGroupHeads, sc[k]);
+      }
+    }
+  }
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+  ptx::bar_sync(1, kSoftmaxThreads);
+  float dsum = 0.f;
+#pragma unroll 2
+  for (int i = j; i < ns; i += 4) {
+    const uint32_t at = uint32_t(i) * kTailBytes;
+    const float l = lds_f32(col + at);
+    const float e = (l == -INFINITY) ? 0.f : ptx::ex2(l - mx);
+    sts_f32(col + at, e * lds_f32(tails + at + 4u * kGroupHeads));
+    dsum += e;
+  }
+  dsum += __shfl_xor_sync(0xffffffffu, dsum, 1);
+  dsum += __shfl_xor_sync(0xffffffffu, dsum, 2);
+  if (j == 0) {
+    sts_f32(smem + kOffLinv + 4u * uint32_t(h), dsum > 0.f ? __frcp_rn(dsum) : 0.f);
+    const MergeReq m = misc->m;
+    int qpos, head0;
+    group_coords(m.g, p.num_heads, qpos, head0);
+    if (with_lse && p.lse && head0 + h < p.num_heads)
+      p.lse[(size_t(m.b) * p.q_len + qpos) * p.num_heads + head0 + h] = (dsum > 0.f) ? (__log2f(dsum) + mx) : -INFINITY;
+  }
+}
+
+// out = sum_i w_i * O_i / sum, over the staged shares, in slot order whatever the order of arrival (bit-reproducible).  All
+// threads of the CTA; the weights are there.
+__device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, int tid, uint32_t parity) {
   Misc* misc = misc_of(smem);
   const int ns = misc->n_slots;
   const MergeReq m = misc->m;
@@ -1201,34 +1285,7 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
   const bool landed = wait(smem, kBarTail, parity);
   if (!landed && (tid & 31) == 0) drain_wait(smem, kBarTail, parity);  // giving up: copies in flight land first
   if (tid == 0) MLA_STAMP(4, 0u, 2);
-  if (__syncthreads_or(!landed || misc->abort)) return;  // (uniform: the barriers below are for all threads)
-  // weights: four lanes per head split the slots; butterflies give all four the results
-  if (tid < 4 * kGroupHeads) {
-    const int h = tid >> 2, j = tid & 3;
-    const uint32_t col = tails + 4u * uint32_t(h);
-    float mx = -INFINITY;
-#pragma unroll 4
-    for (int i = j; i < ns; i += 4) mx = fmaxf(mx, lds_f32(col + uint32_t(i) * kTailBytes));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    float dsum = 0.f;
-#pragma unroll 2
-    for (int i = j; i < ns; i += 4) {
-      const uint32_t at = uint32_t(i) * kTailBytes;
-      const float l = lds_f32(col + at);
-      const float e = (l == -INFINITY) ? 0.f : ptx::ex2(l - mx);
-      sts_f32(col + at, e * lds_f32(tails + at + 4u * kGroupHeads));
-      dsum += e;
-    }
-    dsum += __shfl_xor_sync(0xffffffffu, dsum, 1);
-    dsum += __shfl_xor_sync(0xffffffffu, dsum, 2);
-    if (j == 0) {
-      sts_f32(smem + kOffLinv + 4u * uint32_t(h), dsum > 0.f ? __frcp_rn(dsum) : 0.f);
-      if (with_lse && p.lse && h < heads_here) p.lse[row0 + h] = (dsum > 0.f) ? (__log2f(dsum) + mx) : -INFINITY;
-    }
-  }
-  __syncthreads();
-  if (tid == 0) MLA_STAMP(4, 0u, 3);
+  if (__syncthreads_or(!landed || misc->abort)) return;  // (uniform: there is a barrier below)
   // A thread per unit, or, when there are fewer units than threads, S threads per unit, each with every S-th slot.
   const int S = min(max(kThreads / nu, 1), ns);
   const int s = S > 1 ? tid / nu : 0;
@@ -1240,7 +1297,7 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (active) {
       uint32_t src = rows + uint32_t(s) * share + uint32_t(u) * 16u, w = tails + uint32_t(s) * kTailBytes + 32u * uint32_t(hg);
-#pragma unroll 2
+#pragma unroll 4
       for (int i = s; i < ns; i += S) {
         const uint4 v = lds_u32x4(src);
         const float4 w0 = lds_f32x4(w), w1 = lds_f32x4(w + 16u);
@@ -1310,7 +1367,9 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
       }
       __syncthreads();
       if (tid < 128) tail_fetch(p, smem, tid >> 5, tid & 31, false);
-      tail_merge(p, smem, tid, parity, r == 0);
+      else merge_weights(p, smem, tid - 128, r == 0);
+      __syncthreads();
+      tail_merge(p, smem, tid, parity);
       __syncthreads();
     }
   }
@@ -1349,7 +1408,10 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       misc->abort = 0;
       misc->polls = p.wait_polls;
       misc->status = p.status;
+      misc->n_slots = 0;
     }
+  } else if (warp == kWarpTMA) {
+    if (p.pdl_wait) stage_segments(p, smem, lane, true, false);  // a first plan, from the lengths as they are in memory
   } else if (warp == kWarpTMA2 && lane == 0) {
     ptx::prefetch_tensormap(&map_q_lat);
     ptx::prefetch_tensormap(&map_q_rope);
@@ -1368,31 +1430,39 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
 
   RoleState st{0, 0, 0, 0};
   if (warp == kWarpTMA2) st.slot = 1;
-  // Rounds: almost always exactly one; more only when a CTA's range spans more than kMaxSeg requests.
-  // The partition is walked by the warp that issues the first copies: it goes on to them without waiting for the others.
+  // The plan made before the wait stands if the lengths have not changed.  The partition is walked by the warp that issues the
+  // first copies: it goes on to them without waiting for the others.
   if (warp == kWarpTMA) {
-    stage_segments(p, smem, lane, true);
+    if (!p.pdl_wait || misc->Tt < 0 || !plan_still_valid(p, smem, lane)) stage_segments(p, smem, lane, true, true);
+    ptx::fence_proxy_async_smem();  // the lengths give way to the first copies
     __threadfence_block();
     asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
   } else {
-    // The generation of this step: one more than that of the last completed step.  No CTA of this step
-    // can have advanced it yet (that takes every CTA of the grid to have finished).
-    if (warp == kWarpPV && lane == 0 && p.fused_merge) {
-      atomicAdd(ws_started(p.workspace), 1);
-      misc->gen = ld_acquire(ws_generation(p.workspace)) + 1;
-    }
     ptx::bar_sync(2, kThreads);
   }
   if (tid == 0) MLA_STAMP(4, 1u, 2);
+  // Rounds: almost always exactly one; more only when a CTA's range spans more than kMaxSeg requests.
   bool first_round = true;
+  int finished = -1;
 #pragma unroll 1
   for (;;) {
     if (warp >= kWarpSoftmax0) {
       softmax_role<kSoftCap>(p, smem, tmem, tid - 32 * kWarpSoftmax0, st);
+      if (p.fused_merge && !misc->more && misc->n_slots > 0) {
+        ptx::bar_sync(5, kThreads);
+        if (misc->mode == kMergeShared) merge_weights(p, smem, tid - 32 * kWarpSoftmax0, misc->rank == 0);
+        if (tid == 128) MLA_STAMP(4, 0u, 3);
+      }
     } else if (warp == kWarpQK) {
       qk_role(p, smem, tmem, &map_q_lat, &map_q_rope, st);
     } else if (warp == kWarpPV) {
-      if (first_round && p.fused_merge) {  // (the two-kernel modes leave both to the combine kernel); the first P is far away
+      if (first_round && p.fused_merge) {  // (the two-kernel modes leave all this to the combine kernel); the first P is far away
+        // The generation of this step: one more than that of the last completed step.  No CTA of this step can have advanced it
+        // yet (that takes every CTA of the grid to have finished).
+        if (lane == 0) {
+          atomicAdd(ws_started(p.workspace), 1);
+          misc->gen = ld_acquire(ws_generation(p.workspace)) + 1;
+        }
         plan_merge(smem, 0, lane);
         zero_empty_requests(p, lane);
       }
@@ -1410,16 +1480,27 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       if (lane == 0) drain_wait(smem, kBarDrain, 0);
       __syncwarp();
       if (p.fused_merge) {
-        if (warp == kWarpPV && lane == 0 && (misc->merge[0].vtiles | misc->merge[1].vtiles)) misc->mode = merge_mode(p);
+        if (warp == kWarpPV && lane == 0) {
+          if (misc->merge[0].vtiles | misc->merge[1].vtiles) misc->mode = merge_mode(p);
+        }
         ptx::bar_sync(3, 128);
-        if (misc->n_slots > 0 && misc->mode == kMergeShared) tail_fetch(p, smem, warp, lane, true);
+        if (misc->n_slots > 0) {
+          if (misc->mode == kMergeShared) tail_fetch(p, smem, warp, lane, true);
+          __threadfence_block();
+          asm volatile("bar.arrive 5, %0;" ::"n"(kThreads) : "memory");  // every flag has been seen
+        }
         if (tid == 0) MLA_STAMP(4, 0u, 1);
+        // This CTA has no more use for the header.  (The count comes back while the merge goes on.)
+        if (warp == kWarpPV && lane == 0) finished = atomicAdd(ws_finished(p.workspace), 1);
       }
     }
     __syncthreads();  // every role is done with the staged segments
     if (!more) break;
     first_round = false;
-    if (warp == kWarpTMA) stage_segments(p, smem, lane, false);
+    if (warp == kWarpTMA) {
+      stage_segments(p, smem, lane, false, false);
+      ptx::fence_proxy_async_smem();
+    }
     __syncthreads();
   }
   if (warp == kWarpQK) {
@@ -1429,19 +1510,17 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   if (p.fused_merge) {
     if (misc->merge[0].vtiles | misc->merge[1].vtiles) {
       if (misc->mode == kMergeLast) merge_as_last(p, smem, tid);
-      else if (misc->n_slots > 0) tail_merge(p, smem, tid, 0, misc->rank == 0);
+      else if (misc->n_slots > 0) tail_merge(p, smem, tid, 0);
     }
-    // The last CTA to finish advances the generation: the next step's flags differ from all of this one's.
-    if (tid == 0) {
-      __threadfence();
-      if (atomicAdd(ws_finished(p.workspace), 1) == int(gridDim.x) - 1) {
-        *ws_finished(p.workspace) = 0;
-        *ws_started(p.workspace) = 0;
-        *ws_mode(p.workspace) = 0;
-        st_release(ws_generation(p.workspace), misc->gen);
-      }
-      MLA_STAMP(4, 1u, 3);
+    // The last CTA to have counted itself out advances the generation (the next step's flags differ from all of this one's) and
+    // resets the counters.
+    if (finished == int(gridDim.x) - 1) {
+      *ws_finished(p.workspace) = 0;
+      *ws_started(p.workspace) = 0;
+      *ws_mode(p.workspace) = 0;
+      st_release(ws_generation(p.workspace), misc->gen);
     }
+    if (tid == 0) MLA_STAMP(4, 1u, 3);
   }
 }
 
