@@ -358,34 +358,44 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
 #pragma unroll 1
     for (int t = g.tile_begin; t < g.tile_end; ++t, ++st.it) {
       const int np = min(ppt, total - t * ppt);
+      // the first four pages' ids are in hand before the waits: a slot that has come free is refilled with straight-line copies
+      int pg[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pg[i] = __shfl_sync(0xffffffffu, cur, (at + i) & 31);
+      auto for_pages = [&](auto copy) {  // copy(page, index): issued by one lane
+        if (ptx::elect_one()) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (i < np && pg[i] >= 0) copy(pg[i], i);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int i = 4; i < np; ++i) {
+          const int page = __shfl_sync(0xffffffffu, cur, at + i);
+          if (page >= 0 && ptx::elect_one()) copy(page, i);
+        }
+      };
       if (which) {  // RoPE bytes: the one buffer is free once the two RoPE MMAs of the previous tile have completed
         if (st.it >= 1) ok = wait(smem, kBarRopeEmpty, (st.it - 1) & 1);
         if (!ok) break;
         const uint32_t bar = bar_addr(smem, kBarRopeFull);
         if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * 64u);
-        uint32_t dst = smem + kOffRope;
-#pragma unroll 1
-        for (int i = 0; i < np; ++i, dst += ps * 64u) {
-          const int page = __shfl_sync(0xffffffffu, cur, at + i);
-          if (page >= 0 && ptx::elect_one()) ptx::tma_load_3d(dst, map_rope, bar, kLatent / 2, 0, page);
-        }
+        for_pages([&](int page, int i) { ptx::tma_load_3d(smem + kOffRope + uint32_t(i) * ps * 64u, map_rope, bar, kLatent / 2, 0, page); });
       }
+      const uint32_t bar = bar_addr(smem, bar_kv_full(st.slot)), dst = smem + kOffKV + st.slot * kPairBytes;
       if (st.lap >= 1) ok = wait(smem, bar_kv_empty(st.slot), (st.lap - 1) & 1);
       if (!ok) break;
       MLA_STAMP(1 + which, st.it, 0);
-      const uint32_t bar = bar_addr(smem, bar_kv_full(st.slot));
       // the transaction count of a 4-bit copy is in packed bytes: 64 per row and block
       if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * (which ? 128u : 132u));
-      uint32_t dst = smem + kOffKV + st.slot * kPairBytes;
-      uint32_t dst_sc = smem + kOffScale + (st.it & (kScaleStages - 1)) * (kTile * 4);
-#pragma unroll 1
-      for (int i = 0; i < np; ++i, dst += ps * 128u, dst_sc += ps * 4u) {
-        const int page = __shfl_sync(0xffffffffu, cur, at + i);
-        if (page >= 0 && ptx::elect_one()) {
-          ptx::tma_load_3d(dst, map_lat, bar, 256 * which, 0, page);
-          ptx::tma_load_3d(dst + kBlockBytes, map_lat, bar, 256 * which + 128, 0, page);
-          if (!which) ptx::bulk_load(dst_sc, p.kv_cache_sf + size_t(page) * ps, ps * 4u, bar);
-        }
+      const int c0 = int(256u * which);
+      for_pages([&](int page, int i) {
+        ptx::tma_load_3d(dst + uint32_t(i) * ps * 128u, map_lat, bar, c0, 0, page);
+        ptx::tma_load_3d(dst + uint32_t(i) * ps * 128u + kBlockBytes, map_lat, bar, c0 + 128, 0, page);
+      });
+      if (!which) {
+        const uint32_t dst_sc = smem + kOffScale + (st.it & (kScaleStages - 1)) * (kTile * 4);
+        for_pages([&](int page, int i) { ptx::bulk_load(dst_sc + uint32_t(i) * ps * 4u, p.kv_cache_sf + size_t(page) * ps, ps * 4u, bar); });
       }
       MLA_STAMP(1 + which, st.it, 1);
       // The rows of the tile four ahead are brought into L2: the ring holds two and a half tiles, and a pair's slot comes free
