@@ -177,7 +177,7 @@ __device__ __noinline__ bool wait_slow(uint32_t smem, int idx, uint32_t parity) 
 }
 __device__ __forceinline__ bool wait(uint32_t smem, int idx, uint32_t parity) {
   if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar_addr(smem, idx), parity))) return true;
-  return wait_slow(smem, idx, parity);
+  return __all_sync(0xffffffffu, wait_slow(smem, idx, parity));  // (already the same in all lanes; the vote says so to the compiler)
 }
 // Bounded wait that ignores the abort flag: lets in-flight asynchronous work land before exit.
 __device__ __noinline__ void drain_wait(uint32_t smem, int idx, uint32_t parity) {
@@ -342,17 +342,22 @@ __device__ __forceinline__ int page_window(const DecodeParams& p, const Segment&
   const int id = lp < min((g.seq_len - 1) / p.page_size + 1, g.tile_end * ppt) ? __ldcg(p.block_tables + size_t(g.b) * p.block_table_stride + lp) : -1;
   return int64_t(id) < p.num_pages ? id : -1;
 }
+// entry `i` of a window, in a uniform register
+__device__ __forceinline__ int uniform_page(int window, int i) { return __reduce_max_sync(0xffffffffu, int(threadIdx.x & 31) == (i & 31) ? window : -1); }
 __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, uint32_t which, const CUtensorMap* map_rope,
                                          const CUtensorMap* map_lat, RoleState& st) {
-  const int nseg = misc_of(smem)->nseg;
+  const uint32_t nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   const Segment* sg = segs_of(smem);
   const int lane = threadIdx.x & 31;
   const int ppt = kTile / p.page_size;  // pages per tile
   const uint32_t ps = uint32_t(p.page_size);
   bool ok = true;
 #pragma unroll 1
-  for (int si = 0; si < nseg && ok; ++si, ++st.seg) {
-    const Segment g = sg[si];
+  for (uint32_t si = 0; si < nseg && ok; ++si, ++st.seg) {
+    Segment g = sg[si];
+    g.tile_begin = int(ptx::uniform_u32(uint32_t(g.tile_begin)));
+    g.tile_end = int(ptx::uniform_u32(uint32_t(g.tile_end)));
+    g.seq_len = int(ptx::uniform_u32(uint32_t(g.seq_len)));
     const int total = (g.seq_len - 1) / p.page_size + 1;
     int cur = page_window(p, g, 0), nxt = page_window(p, g, 32), ahead = 64, at = 0;
 #pragma unroll 1
@@ -361,41 +366,39 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
       // the first four pages' ids are in hand before the waits: a slot that has come free is refilled with straight-line copies
       int pg[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) pg[i] = __shfl_sync(0xffffffffu, cur, (at + i) & 31);
-      auto for_pages = [&](auto copy) {  // copy(page, index): issued by one lane
-        if (ptx::elect_one()) {
+      for (int i = 0; i < 4; ++i) pg[i] = uniform_page(cur, at + i);
+      const uint32_t e = ptx::elect_one();
+      auto for_pages = [&](auto copy) {  // copy(issue, page, index)
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (i < np && pg[i] >= 0) copy(pg[i], i);
-        }
-        __syncwarp();
+        for (int i = 0; i < 4; ++i)
+          if (i < np) copy(e && pg[i] >= 0 ? 1u : 0u, pg[i], i);
 #pragma unroll 1
         for (int i = 4; i < np; ++i) {
-          const int page = __shfl_sync(0xffffffffu, cur, at + i);
-          if (page >= 0 && ptx::elect_one()) copy(page, i);
+          const int page = uniform_page(cur, at + i);
+          copy(e && page >= 0 ? 1u : 0u, page, i);
         }
       };
       if (which) {  // RoPE bytes: the one buffer is free once the two RoPE MMAs of the previous tile have completed
         if (st.it >= 1) ok = wait(smem, kBarRopeEmpty, (st.it - 1) & 1);
         if (!ok) break;
         const uint32_t bar = bar_addr(smem, kBarRopeFull);
-        if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * 64u);
-        for_pages([&](int page, int i) { ptx::tma_load_3d(smem + kOffRope + uint32_t(i) * ps * 64u, map_rope, bar, kLatent / 2, 0, page); });
+        if (e) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * 64u);
+        for_pages([&](uint32_t issue, int page, int i) { ptx::tma_load_3d_if(issue, smem + kOffRope + uint32_t(i) * ps * 64u, map_rope, bar, kLatent / 2, 0, page); });
       }
       const uint32_t bar = bar_addr(smem, bar_kv_full(st.slot)), dst = smem + kOffKV + st.slot * kPairBytes;
       if (st.lap >= 1) ok = wait(smem, bar_kv_empty(st.slot), (st.lap - 1) & 1);
       if (!ok) break;
       MLA_STAMP(1 + which, st.it, 0);
       // the transaction count of a 4-bit copy is in packed bytes: 64 per row and block
-      if (ptx::elect_one()) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * (which ? 128u : 132u));
+      if (e) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * (which ? 128u : 132u));
       const int c0 = int(256u * which);
-      for_pages([&](int page, int i) {
-        ptx::tma_load_3d(dst + uint32_t(i) * ps * 128u, map_lat, bar, c0, 0, page);
-        ptx::tma_load_3d(dst + uint32_t(i) * ps * 128u + kBlockBytes, map_lat, bar, c0 + 128, 0, page);
+      for_pages([&](uint32_t issue, int page, int i) {
+        ptx::tma_load_3d_if(issue, dst + uint32_t(i) * ps * 128u, map_lat, bar, c0, 0, page);
+        ptx::tma_load_3d_if(issue, dst + uint32_t(i) * ps * 128u + kBlockBytes, map_lat, bar, c0 + 128, 0, page);
       });
       if (!which) {
         const uint32_t dst_sc = smem + kOffScale + (st.it & (kScaleStages - 1)) * (kTile * 4);
-        for_pages([&](int page, int i) { ptx::bulk_load(dst_sc + uint32_t(i) * ps * 4u, p.kv_cache_sf + size_t(page) * ps, ps * 4u, bar); });
+        for_pages([&](uint32_t issue, int page, int i) { ptx::bulk_load_if(issue, dst_sc + uint32_t(i) * ps * 4u, p.kv_cache_sf + int64_t(page) * ps, ps * 4u, bar); });
       }
       MLA_STAMP(1 + which, st.it, 1);
       // The rows of the tile four ahead are brought into L2: the ring holds two and a half tiles, and a pair's slot comes free
@@ -432,8 +435,8 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
 }
 
 // ------------------------------------------------------------------------------------------
-// roles: MMA issue.  The whole warp runs this code with uniform control flow; only the
-// tcgen05 instructions sit under elect_one(), so their operands stay in uniform registers.
+// roles: MMA issue.  The whole warp runs this code with uniform control flow and uniform values (ptx::uniform_u32); only the
+// tcgen05 instructions are predicated on the elected lane, so their operands stay in uniform registers.
 // ------------------------------------------------------------------------------------------
 // A shared-memory descriptor as two words.  Only the 14-bit address field (bytes >> 4) in the low word
 // changes from one instruction to the next and it cannot carry out (shared memory is smaller than
@@ -452,13 +455,13 @@ __device__ __forceinline__ Desc make_desc(uint32_t addr, uint32_t lbo, uint32_t 
 // before has completed.
 __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, uint32_t tmem, const CUtensorMap* map_q_lat,
                                         const CUtensorMap* map_q_rope, RoleState& st) {
-  const int nseg = misc_of(smem)->nseg;
+  const uint32_t nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   const Segment* sg = segs_of(smem);
   const Desc rope = make_desc(smem + kOffRope, 16, 512, 4), q_rope = make_desc(smem + kOffQRope, 16, 512, 4);
   const Desc kv = make_desc(smem + kOffKV, 16, 1024, 2), q_lat = make_desc(smem + kOffQLat, 16, 1024, 2);  // K-major, 128B swizzle
   bool ok = true;
 #pragma unroll 1
-  for (int si = 0; si < nseg && ok; ++si, ++st.seg) {
+  for (uint32_t si = 0; si < nseg && ok; ++si, ++st.seg) {
     const Segment g = sg[si];
     if (st.seg >= 1 && !wait(smem, kBarQEmpty, (st.seg - 1) & 1)) break;
     int qpos, head0;
@@ -472,9 +475,10 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
         ptx::tma_load_4d(smem + kOffQLat + j * kGroupHeads * 128, map_q_lat, bar, 128 * j, head0, qpos, g.b);
     }
     __syncwarp();
+    const uint32_t n = ptx::uniform_u32(uint32_t(g.tile_end - g.tile_begin));
     ok = wait(smem, kBarQFull, st.seg & 1);
 #pragma unroll 1
-    for (int t = g.tile_begin; t < g.tile_end && ok; ++t, ++st.it) {
+    for (uint32_t t = 0; t < n && ok; ++t, ++st.it) {
       const uint32_t it = st.it, s64 = 64u * (it & 1);
       // S of this stage has been read by the softmax of tile it-2; the RoPE bytes of this tile have landed
       if (it >= 2) ok = wait(smem, bar_s_empty(it & 1), ((it >> 1) - 1) & 1);
@@ -482,11 +486,10 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
       if (!ok) break;
       MLA_STAMP(0, it, 0);
       ptx::tc_fence_after();
-      if (ptx::elect_one()) {
+      const uint32_t e = ptx::elect_one();
 #pragma unroll
-        for (uint32_t ks = 0; ks < 2; ++ks) ptx::umma_f8(tmem + kColSRope + s64, rope.at(2 * ks), q_rope.at(2 * ks), kIdescQKRope, ks);
-        ptx::umma_commit(bar_addr(smem, kBarRopeEmpty));
-      }
+      for (uint32_t ks = 0; ks < 2; ++ks) ptx::umma_f8(e, tmem + kColSRope + s64, rope.at(2 * ks), q_rope.at(2 * ks), kIdescQKRope, ks);
+      if (e) ptx::umma_commit(bar_addr(smem, kBarRopeEmpty));
       __syncwarp();
 #pragma unroll 1
       for (uint32_t pr = 0; pr < 2 && ok; ++pr) {
@@ -494,15 +497,13 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t a = st.slot * (kPairBytes >> 4), b = pr * ((2 * kGroupHeads * 128) >> 4);
-        if (ptx::elect_one()) {
 #pragma unroll
-          for (uint32_t j = 0; j < 2; ++j)
+        for (uint32_t j = 0; j < 2; ++j)
 #pragma unroll
-            for (uint32_t ks = 0; ks < 4; ++ks)
-              ptx::umma_f8(tmem + kColSLat + s64, kv.at(a + j * (kBlockBytes >> 4) + 2 * ks), q_lat.at(b + j * ((kGroupHeads * 128) >> 4) + 2 * ks),
-                           kIdescQK, (pr | j | ks) ? 1u : 0u);
-          if (pr) ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
-        }
+          for (uint32_t ks = 0; ks < 4; ++ks)
+            ptx::umma_f8(e, tmem + kColSLat + s64, kv.at(a + j * (kBlockBytes >> 4) + 2 * ks), q_lat.at(b + j * ((kGroupHeads * 128) >> 4) + 2 * ks),
+                         kIdescQK, (pr | j | ks) ? 1u : 0u);
+        if (pr && e) ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
         __syncwarp();
         st.advance(1);
       }
@@ -522,31 +523,32 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
 // role: PV issue (warp 2).  Per block of 128 dims 4 token steps x (hi, lo), which share A through the collector; the commit
 // after a pair frees its slot.
 __device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState& st) {
-  const int nseg = misc_of(smem)->nseg;
+  const uint32_t nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   const Segment* sg = segs_of(smem);
   const Desc kv = make_desc(smem + kOffKV, kBlockBytes, 1024, 2);  // V^T: MN-major, 128B swizzle; 32 tokens per step = 4 groups of 8 rows (4096 B)
   const Desc pd = make_desc(smem + kOffP, 512, 512, 4);            // P^T: MN-major (64 heads contiguous), 64B swizzle; 2048 B per step
 #pragma unroll 1
-  for (int si = 0; si < nseg; ++si, ++st.seg) {
-    const uint32_t n = uint32_t(sg[si].tile_end - sg[si].tile_begin);
+  for (uint32_t si = 0; si < nseg; ++si, ++st.seg) {
+    const uint32_t n = ptx::uniform_u32(uint32_t(sg[si].tile_end - sg[si].tile_begin));
     if (st.seg >= 1 && !wait(smem, kBarOFree, (st.seg - 1) & 1)) return;  // O^T of the previous segment has been read out
 #pragma unroll 1
     for (uint32_t t = 0; t < n; ++t, ++st.it) {
       if (!wait(smem, kBarPFull, st.it & 1)) return;
       MLA_STAMP(0, st.it, 2);
       ptx::tc_fence_after();
+      const uint32_t e = ptx::elect_one(), keep = t ? 1u : 0u;
 #pragma unroll 1
       for (uint32_t pr = 0; pr < 2; ++pr) {
         const uint32_t a = st.slot * (kPairBytes >> 4), d = tmem + kColO + 128u * pr;
-        if (ptx::elect_one()) {
 #pragma unroll
-          for (uint32_t j = 0; j < 2; ++j)
+        for (uint32_t j = 0; j < 2; ++j)
 #pragma unroll
-            for (uint32_t ks = 0; ks < 4; ++ks) {
-              const uint64_t ad = kv.at(a + j * (kBlockBytes >> 4) + 256 * ks);
-              ptx::umma_f8_a_fill(d + 64u * j, ad, pd.at(128 * ks), kIdescPV, (ks || t) ? 1u : 0u);
-              ptx::umma_f8_a_lastuse(d + 64u * j, ad, pd.at(((kTile * 64) >> 4) + 128 * ks), kIdescPV, 1u);
-            }
+          for (uint32_t ks = 0; ks < 4; ++ks) {
+            const uint64_t ad = kv.at(a + j * (kBlockBytes >> 4) + 256 * ks);
+            ptx::umma_f8_a_fill(e, d + 64u * j, ad, pd.at(128 * ks), kIdescPV, ks ? 1u : keep);
+            ptx::umma_f8_a_lastuse(e, d + 64u * j, ad, pd.at(((kTile * 64) >> 4) + 128 * ks), kIdescPV, 1u);
+          }
+        if (e) {
           ptx::umma_commit(bar_addr(smem, bar_kv_empty(st.slot)));
           if (pr) ptx::umma_commit(bar_addr(smem, kBarPvDone));
         }
@@ -1397,7 +1399,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   const uint32_t smem = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   Misc* misc = misc_of(smem);
   const int tid = threadIdx.x, lane = tid & 31;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int warp = int(ptx::uniform_u32(uint32_t(tid >> 5)));
   if (tid == 0) MLA_STAMP(4, 1u, 0);
 
   // What needs nothing an earlier kernel wrote comes first: with a programmatic dependent launch this part runs
@@ -1431,7 +1433,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem = misc->tmem_base;
+  const uint32_t tmem = ptx::uniform_u32(misc->tmem_base);
   // From here on the kernel reads what earlier kernels wrote (sequence lengths, q, the cache, the workspace).
   if (p.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
   // Let a dependent kernel start its launch and prologue early; it still waits for the end of this whole grid.

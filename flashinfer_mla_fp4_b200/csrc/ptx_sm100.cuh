@@ -59,6 +59,20 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
+// predicated instead of branched around, as the MMAs are (see umma_f8)
+__device__ __forceinline__ void tma_load_3d_if(uint32_t issue, uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "@e cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(issue)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_load_if(uint32_t issue, uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %4, 0;\n\t"
+               "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "r"(issue)
+               : "memory");
+}
 // untiled bulk copy global -> shared (both 16-byte aligned, size a multiple of 16)
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -116,36 +130,30 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---------------------------------------------------------------- UMMA
-// D[tmem] (+)= A[smem desc] * B[smem desc]; kind::f8f6f4, one CTA.  accumulate == 0 overwrites D.
-__device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
+// D[tmem] (+)= A[smem desc] * B[smem desc]; kind::f8f6f4, one CTA, issued by the lane whose `elected` is set.  accumulate == 0
+// overwrites D.  Predicated rather than branched around, so that the code stays warp-uniform: with operands that the
+// compiler knows to be uniform (uniform_u32) an MMA of 128x64x32 issues every 48 clk, the rate of its operand reads; with
+// operands moved over from vector registers inside an elected branch it was 57.
+#define MLA_UMMA_F8(NAME, USAGE)                                                                                          \
+  __device__ __forceinline__ void NAME(uint32_t elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, \
+                                       uint32_t accumulate) {                                                             \
+    asm volatile(                                                                                                         \
+        "{\n\t.reg .pred e, p;\n\t"                                                                                       \
+        "setp.ne.b32 e, %5, 0;\n\t"                                                                                      \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                                                      \
+        "@e tcgen05.mma.cta_group::1.kind::f8f6f4" USAGE " [%0], %1, %2, %3, p;\n\t}"                                    \
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)                                \
+        : "memory");                                                                                                      \
+  }
+MLA_UMMA_F8(umma_f8, "")
 // Same, keeping A in the collector buffer for the next instruction (fill) / reading it from there
 // for the last time (lastuse): two consecutive MMAs that share A fetch it from shared memory once.
-__device__ __forceinline__ void umma_f8_a_fill(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                               uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4.collector::a::fill [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_f8_a_lastuse(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                  uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4.collector::a::lastuse [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
+MLA_UMMA_F8(umma_f8_a_fill, ".collector::a::fill")
+MLA_UMMA_F8(umma_f8_a_lastuse, ".collector::a::lastuse")
+#undef MLA_UMMA_F8
+// A value that is the same in all lanes of a converged warp, through a warp reduction: the compiler may then keep it, and
+// what is computed from it, in uniform registers.
+__device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
 // mbarrier arrives once all tcgen05 operations issued so far by this thread have completed
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
