@@ -24,8 +24,10 @@
 //   * latent blocks are handled in pairs (32 KiB, five pair slots = two and a half tiles in flight): one barrier, one wait
 //     and one commit per pair;
 //   * QK^T and PV are issued by a warp each: the queue of the tensor pipe is short, so a gap in one warp's issue (a wait, the
-//     bookkeeping of a tile) is a gap of the pipe unless the other warp has something queued.  (One warp for both, in the
-//     order PV(t), QK(t+2), measured 120 us where two take XXX.)
+//     bookkeeping of a tile) is a gap of the pipe unless the other warp has something queued (one warp for both, in the order
+//     PV(t), QK(t+2), measured 106 us where two take 88).  The two take turns all the same: PV(t) follows QK(t+1), and QK(t+2)
+//     is let in when PV(t) is half issued.  That way the pipe has QK^T to work on while P(t+1), which may be stored only when
+//     PV(t) has completed, is on its way; left alone, the two streams ran side by side and then both waited (92.7 us).
 //   * two warps issue the copies of a tile (pair 0 and scales | RoPE and pair 1).  Each issues from one elected lane with
 //     page ids fetched 32 at a time.  (With per-lane copies, per-line L2 prefetches and a vote per wait, the one copy warp of
 //     an earlier version took 3500 clk per tile and bounded the whole kernel: 51.6 us for the north star, 138 us for B=2,
@@ -95,8 +97,9 @@ __device__ __forceinline__ constexpr int bar_s_full(int s) { return 2 * kRing + 
 __device__ __forceinline__ constexpr int bar_s_empty(int s) { return 2 * kRing + 2 + s; }  // ... and has been read
 constexpr int kBarRopeFull = 2 * kRing + 4, kBarRopeEmpty = 2 * kRing + 5, kBarPFull = 2 * kRing + 6, kBarPvDone = 2 * kRing + 7,
               kBarQFull = 2 * kRing + 8, kBarQEmpty = 2 * kRing + 9, kBarOFree = 2 * kRing + 10, kBarDrain = 2 * kRing + 11,
-              kBarTail = 2 * kRing + 12;
-constexpr int kNumBars = 2 * kRing + 13;
+              kBarTail = 2 * kRing + 12, kBarQkIssued = 2 * kRing + 13, kBarPvIssued = 2 * kRing + 14;
+constexpr int kNumBars = 2 * kRing + 15;
+static_assert(kNumBars <= 32, "initialised by one warp, a barrier per lane");
 constexpr uint32_t kOffTail = (kOffBars + kNumBars * 8 + 15u) & ~15u;     // merge plan: [148] slot ids
 constexpr uint32_t kOffSegs = kOffTail + kMaxCombineSlots * 4;            // Segment[kMaxSeg]
 constexpr uint32_t kOffMisc = kOffSegs + kMaxSeg * 24;
@@ -480,8 +483,11 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
 #pragma unroll 1
     for (uint32_t t = 0; t < n && ok; ++t, ++st.it) {
       const uint32_t it = st.it, s64 = 64u * (it & 1);
-      // S of this stage has been read by the softmax of tile it-2; the RoPE bytes of this tile have landed
+      // S of this stage has been read by the softmax of tile it-2; PV of tile it-2, if of this segment, is half issued; the RoPE
+      // bytes of this tile have landed.  (The two issue barriers cannot run ahead of the warp that waits for them: inside a
+      // segment PV(it-1) waits for this tile's QK^T, and QK^T of it+1 for PV(it-1).)
       if (it >= 2) ok = wait(smem, bar_s_empty(it & 1), ((it >> 1) - 1) & 1);
+      if (t >= 2) ok = ok && wait(smem, kBarPvIssued, it & 1);
       ok = ok && wait(smem, kBarRopeFull, it & 1);
       if (!ok) break;
       MLA_STAMP(0, it, 0);
@@ -503,7 +509,10 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
           for (uint32_t ks = 0; ks < 4; ++ks)
             ptx::umma_f8(e, tmem + kColSLat + s64, kv.at(a + j * (kBlockBytes >> 4) + 2 * ks), q_lat.at(b + j * ((kGroupHeads * 128) >> 4) + 2 * ks),
                          kIdescQK, (pr | j | ks) ? 1u : 0u);
-        if (pr && e) ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
+        if (pr && e) {
+          ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
+          ptx::mbar_arrive(bar_addr(smem, kBarQkIssued));
+        }
         __syncwarp();
         st.advance(1);
       }
@@ -533,6 +542,8 @@ __device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState&
     if (st.seg >= 1 && !wait(smem, kBarOFree, (st.seg - 1) & 1)) return;  // O^T of the previous segment has been read out
 #pragma unroll 1
     for (uint32_t t = 0; t < n; ++t, ++st.it) {
+      // QK^T of the segment's next tile has been issued (so it lies ahead of this PV in the queue of the tensor pipe)
+      if (t + 1 < n && !wait(smem, kBarQkIssued, (st.it + 1) & 1)) return;
       if (!wait(smem, kBarPFull, st.it & 1)) return;
       MLA_STAMP(0, st.it, 2);
       ptx::tc_fence_after();
@@ -547,6 +558,7 @@ __device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState&
             const uint64_t ad = kv.at(a + j * (kBlockBytes >> 4) + 256 * ks);
             ptx::umma_f8_a_fill(e, d + 64u * j, ad, pd.at(128 * ks), kIdescPV, ks ? 1u : keep);
             ptx::umma_f8_a_lastuse(e, d + 64u * j, ad, pd.at(((kTile * 64) >> 4) + 128 * ks), kIdescPV, 1u);
+            if (j == 0 && ks == 0 && pr && e) ptx::mbar_arrive(bar_addr(smem, kBarPvIssued));
           }
         if (e) {
           ptx::umma_commit(bar_addr(smem, bar_kv_empty(st.slot)));
