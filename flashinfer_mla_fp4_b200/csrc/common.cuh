@@ -25,7 +25,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 //     scale (the decode kernel's lanes own one dim each: with this order a warp stores 32 dims x 8 heads =
 //     512 contiguous bytes at a time; with heads innermost over all 64 it would store 16 bytes every 128).
 //   * tail of slot s (272 bytes): the base-2 LSE of the 64 heads as f32, that scale (f32), the slot's flag
-//     (int32, see below), an arrival counter (int32), 4 bytes of padding.  The tails of all slots lie side by side, so the tails of the
+//     (int32, see below), an arrival counter (int32) and the flag of the LSEs and the scale alone (int32).  The tails of all slots lie side by side, so the tails of the
 //     consecutive slots of one split request are one contiguous range (one bulk copy for a merging CTA).
 // The scale is 6 * max|token scale| * |output_scale| / 32768 rounded up to a power of two: an
 // upper bound of |O| mapped below the fp16 maximum, so the 11-bit partials can neither overflow nor
@@ -60,6 +60,7 @@ MLA_HD const float* slot_lse(const void* ws, int slot) { return reinterpret_cast
 MLA_HD float* slot_scale(void* ws, int slot) { return slot_lse(ws, slot) + kGroupHeads; }
 MLA_HD const float* slot_scale(const void* ws, int slot) { return slot_lse(ws, slot) + kGroupHeads; }
 MLA_HD int32_t* slot_flag(void* ws, int slot) { return reinterpret_cast<int32_t*>(slot_scale(ws, slot) + 1); }
+MLA_HD int32_t* slot_lse_flag(void* ws, int slot) { return slot_flag(ws, slot) + 2; }  // generation that last published the slot's LSEs and scale
 MLA_HD int32_t* slot_arrivals(void* ws, int slot) { return slot_flag(ws, slot) + 1; }  // of the request whose first writer owns the slot
 // element (dim, head) of a slot's partial O
 MLA_HD size_t slot_o_index(int dim, int head) { return (size_t(head >> 3) * kLatent + size_t(dim)) * 8 + size_t(head & 7); }

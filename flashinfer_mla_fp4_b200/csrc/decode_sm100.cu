@@ -934,7 +934,7 @@ __device__ __noinline__ void write_final_bf16(const DecodeParams& p, uint32_t sm
 
 // Normalise O^T and write it to a split-KV partial slot, as fp16 divided by the slot scale (the factors in shared memory
 // include that division).  A block of 128 dims per round, rolled.
-__device__ __noinline__ void write_partial(const DecodeParams& p, uint32_t smem, uint32_t tmem_lane, int row, int half, int tid, int slot, float slot_scale_v) {
+__device__ __noinline__ void write_partial(const DecodeParams& p, uint32_t smem, uint32_t tmem_lane, int row, int half, int slot) {
   __half* so = reinterpret_cast<__half*>(slot_o(p.workspace, slot)) + slot_o_index(row, 32 * half);
 #pragma unroll 1
   for (int jb = 0; jb < kBlocks; ++jb, so += 128 * 8) {
@@ -958,10 +958,6 @@ __device__ __noinline__ void write_partial(const DecodeParams& p, uint32_t smem,
       *reinterpret_cast<uint4*>(so + size_t(2 * hh + 1) * kLatent * 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
     }
   }
-  if (tid < kGroupHeads) {
-    slot_lse(p.workspace, slot)[tid] = lds_f32(smem + kOffLse + 4 * tid);
-    if (tid == 0) slot_scale(p.workspace, slot)[0] = slot_scale_v;
-  }
 }
 
 template <bool kSoftCap>
@@ -984,7 +980,7 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
   // this thread's P' row: two 16-byte chunks of hi and two of lo, swizzled
   const uint32_t psw = (uint32_t(row) >> 1) & 3u;
   const uint32_t p_row = smem + kOffP + uint32_t(row) * 64u;
-  int pending = 0;  // partial slots written in this call: bit 0 the even one, bit 1 the odd one
+  int pending = 0;  // partial slots written in this call: bit 0 the even one, bit 1 the odd one, bit 2 its LSEs are not out yet (the even one's)
 
 #pragma unroll 1
   for (int si = 0; si < nseg; ++si, ++st.seg) {
@@ -1084,7 +1080,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
     const float sc_warp = ptx::redux_max_f32(sc_max);
     if (lane == 0) sts_f32(smem + kOffScMax + 4 * warp, sc_warp);
     ptx::bar_sync(1, kSoftmaxThreads);
-    float slot_scale_v = 1.f;
     if (tid < kGroupHeads) {
       const float L = (lds_f32(wred + 4 * tid) + lds_f32(wred + 4 * (kGroupHeads + tid))) +
                       (lds_f32(wred + 4 * (2 * kGroupHeads + tid)) + lds_f32(wred + 4 * (3 * kGroupHeads + tid)));
@@ -1102,20 +1097,32 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
           m = mm;
         }
       }
+      float slot_scale_v = 1.f;
       if (g.slot >= 0) {  // a partial is stored divided by its slot scale
         const float4 a = lds_f32x4(smem + kOffScMax), b = lds_f32x4(smem + kOffScMax + 16);
         const float sc_all = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
         slot_scale_v = slot_scale_for(6.f * sc_all * fabsf(p.output_scale));
         fo *= __frcp_rn(slot_scale_v);  // a power of two: exact
       }
+      const float lse = __log2f(Ls) + m;
       sts_f32(smem + kOffLinv + 4 * tid, __fdividef(fo, Ls));
-      sts_f32(smem + kOffLse + 4 * tid, __log2f(Ls) + m);
+      sts_f32(smem + kOffLse + 4 * tid, lse);
+      if (g.slot >= 0) {
+        slot_lse(p.workspace, g.slot)[tid] = lse;
+        if (tid == 0) slot_scale(p.workspace, g.slot)[0] = slot_scale_v;
+        // The LSEs and the scale of a CTA's last partial go out at once: the merge weights are made from them while O is on its
+        // way.  (Not those of an earlier segment: the release would hold up the next one.)
+        if (p.fused_merge && si == nseg - 1) {
+          ptx::bar_sync(6, kGroupHeads);
+          if (tid == 0) st_release(slot_lse_flag(p.workspace, g.slot), misc->gen);
+        }
+      }
     }
     (void)wait(smem, kBarPvDone, (st.it - 1) & 1);  // the PV of the last tile
     if (tid == 0) MLA_STAMP(3, st.it - 1, 3);
     ptx::tc_fence_after();
     if (!ptx::bar_or(1, kSoftmaxThreads, misc->abort != 0)) {  // (all or none: the writers meet at barriers)
-      if (g.slot >= 0) write_partial(p, smem, tmem_lane, row, half, tid, g.slot, slot_scale_v);
+      if (g.slot >= 0) write_partial(p, smem, tmem_lane, row, half, g.slot);
       else if (p.out_dtype == MLA_FP4_OUT_BF16) write_final_bf16(p, smem, tmem_lane, quarter, half, tid, g.b, g.g);
       else if ((p.num_heads & (kGroupHeads - 1)) == 0) {  // every group is full
         if (p.out_dtype == MLA_FP4_OUT_F32) write_final<MLA_FP4_OUT_F32, true>(p, smem, tmem_lane, row, half, tid, g.b, g.g);
@@ -1128,7 +1135,7 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
     ptx::tc_fence_before();
     __syncwarp();
     if (lane == 0) ptx::mbar_arrive(bar_addr(smem, kBarOFree));
-    if (g.slot >= 0) pending |= 1 << (g.slot & 1);
+    if (g.slot >= 0) pending |= (1 << (g.slot & 1)) | (si < nseg - 1 ? 4 : 0);
     if (tid == 0) MLA_STAMP(3, st.it - 1, 4);
   }
   // Publish the partials: the tail merge of their requests' CTAs waits for these flags.  One release for all of them, after
@@ -1139,6 +1146,7 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
     ptx::bar_sync(1, kSoftmaxThreads);
     if (tid == 0) {
       const int slot = slot_of(blockIdx.x, true);
+      if (pending & 4) st_release(slot_lse_flag(p.workspace, slot), misc->gen);
       if (pending & 1) st_release(slot_flag(p.workspace, slot), misc->gen);
       if (pending & 2) st_release(slot_flag(p.workspace, slot + 1), misc->gen);
       MLA_STAMP(4, 0u, 0);
@@ -1165,7 +1173,7 @@ constexpr int kMergeShared = 1, kMergeLast = 2;
 constexpr uint32_t kTailBytes = uint32_t(kSlotTailBytes);               // a slot's tail: 64 LSEs, the slot scale, the flag, an arrival counter, padding
 constexpr uint32_t kTailStage = kOffKV;                                 // staging: [slots][this CTA's bytes of a slot], then the tails
 constexpr uint32_t kTailRed = kOffScale - kThreads * 32;                // [384][8] f32: sums of a unit that several threads share
-constexpr uint32_t kTailStageBytes = kTailRed - kTailStage;             // the KV ring, RoPE, Q and most of P
+constexpr uint32_t kTailStageBytes = kOffP - kTailStage;                // the KV ring, RoPE and Q; not P, where the last segment's output may still be in transit
 static_assert(kTailStageBytes >= 2 * (kSlotOBytes + kTailBytes), "two whole slots fit (a request cut once)");
 static_assert(kTailStageBytes >= kSlotOBytes + kSlotOBytes / 8 + kWsTailsBytes, "a request cut 148 times fits");
 
@@ -1286,13 +1294,27 @@ __device__ __forceinline__ void store_unit(const float (&acc)[8], const float4& 
 
 // The merge weights w_i = 2^(lse_i - max) * slot scale of the 64 heads, and the inverse of their sum, by the eight softmax
 // warps: four lanes per head split the slots, butterflies give all four the results.  They are computed while the shares of the
-// slots are on their way: the LSEs come straight from L2.
-__device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem, int tid, bool with_lse) {
+// slots are on their way: the LSEs come straight from L2, under flags of their own (shared form).
+__device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem, int tid, bool flags, bool with_lse) {
   Misc* misc = misc_of(smem);
   const int ns = misc->n_slots;
   const uint32_t tails = smem + kTailStage + uint32_t(ns) * (uint32_t(misc->unit1 - misc->unit0) * 16u);
   const int h = tid >> 2, j = tid & 3;
   const uint32_t col = tails + 4u * uint32_t(h);
+  if (flags) {
+    const int lane = tid & 31, gen = misc->gen;
+    const uint32_t polls = misc->polls;
+    bool all = false;
+#pragma unroll 1
+    for (uint32_t it = 0; it < polls && !all; ++it) {
+      bool up = true;
+      for (int i = lane; i < ns; i += 32) up &= ld_acquire(slot_lse_flag(p.workspace, int(lds_u32(smem + kOffTail + 4u * uint32_t(i))))) == gen;
+      all = __all_sync(0xffffffffu, up);
+      if (__any_sync(0xffffffffu, misc->abort)) break;
+    }
+    if (!all && lane == 0 && !misc->abort) flag_timeout(smem, 101, uint32_t(ns));
+    __syncwarp();
+  }
   float mx = -INFINITY;
 #pragma unroll 1
   for (int i0 = j; i0 < ns; i0 += 20) {  // five slots' loads in flight together
@@ -1365,18 +1387,25 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
     const int unit = U0 + u, hg = unit >> 9, dim = unit & 511;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (active) {
+      uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};  // pairs of heads
       uint32_t src = rows + uint32_t(s) * share + uint32_t(u) * 16u, w = tails + uint32_t(s) * kTailBytes + 32u * uint32_t(hg);
 #pragma unroll 4
       for (int i = s; i < ns; i += S) {
         const uint4 v = lds_u32x4(src);
-        const float4 w0 = lds_f32x4(w), w1 = lds_f32x4(w + 16u);
+        uint64_t wp[4];
+        lds_pairs(w, wp[0], wp[1]);
+        lds_pairs(w + 16u, wp[2], wp[3]);
         src += uint32_t(S) * share;
         w += uint32_t(S) * kTailBytes;
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
-        const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&v.z)), f3 = __half22float2(*reinterpret_cast<const __half2*>(&v.w));
-        acc[0] += w0.x * f0.x; acc[1] += w0.y * f0.y; acc[2] += w0.z * f1.x; acc[3] += w0.w * f1.y;
-        acc[4] += w1.x * f2.x; acc[5] += w1.y * f2.y; acc[6] += w1.z * f3.x; acc[7] += w1.w * f3.y;
+        const uint32_t vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&vs[e]));
+          sum[e] = fma2(wp[e], pack2(f.x, f.y), sum[e]);
+        }
       }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) unpack2(sum[e], acc[2 * e], acc[2 * e + 1]);
     }
     if (S > 1) {
       const uint32_t red = smem + kTailRed + uint32_t(tid) * 4u;  // [8][384]: conflict-free
@@ -1436,7 +1465,7 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
       }
       __syncthreads();
       if (tid < 128) tail_fetch(p, smem, tid >> 5, tid & 31, false);
-      else merge_weights(p, smem, tid - 128, r == 0);
+      else merge_weights(p, smem, tid - 128, false, r == 0);
       __syncthreads();
       tail_merge(p, smem, tid, parity);
       __syncthreads();
@@ -1519,7 +1548,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       softmax_role<kSoftCap>(p, smem, tmem, tid - 32 * kWarpSoftmax0, st);
       if (p.fused_merge && !misc->more && misc->n_slots > 0) {
         ptx::bar_sync(5, kThreads);
-        if (misc->mode == kMergeShared) merge_weights(p, smem, tid - 32 * kWarpSoftmax0, misc->rank == 0);
+        if (misc->mode == kMergeShared) merge_weights(p, smem, tid - 32 * kWarpSoftmax0, true, misc->rank == 0);
         if (tid == 128) MLA_STAMP(4, 0u, 3);
       }
     } else if (warp == kWarpQK) {
@@ -1554,9 +1583,9 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
         }
         ptx::bar_sync(3, 128);
         if (misc->n_slots > 0) {
-          if (misc->mode == kMergeShared) tail_fetch(p, smem, warp, lane, true);
           __threadfence_block();
-          asm volatile("bar.arrive 5, %0;" ::"n"(kThreads) : "memory");  // every flag has been seen
+          asm volatile("bar.arrive 5, %0;" ::"n"(kThreads) : "memory");  // the mode is known
+          if (misc->mode == kMergeShared) tail_fetch(p, smem, warp, lane, true);
         }
         if (tid == 0) MLA_STAMP(4, 0u, 1);
         // This CTA has no more use for the header.  (The count comes back while the merge goes on.)
