@@ -8,9 +8,10 @@
 // division, as the reference's fixture builder (tests/test_cute_dsl_mla_fp4.py:56-93), so the bytes
 // are identical to it; the reference leaves cache writes to the caller (README.md:81-83).
 //
-// One warp per token, 16 consecutive latent values per lane: 2 x 16-byte loads (16-bit inputs), one
-// 8-byte store of packed codes per lane (256 contiguous bytes per warp), 2 RoPE values per lane.
-// HBM-bound: 576 input elements read and 324 bytes written per token, nothing is read twice.
+// One warp per token.  A lane owns the 16-byte chunks lane, lane + 32, ... of the latent row, so every load of a warp is 512
+// contiguous bytes, and two RoPE values.  The next token's loads are issued before the current one is quantised.
+// Bound by HBM (576 input elements read and 324 bytes written per token, nothing twice) once the arithmetic is out of the way:
+// with 391 instructions per token and warp 262144 BF16 tokens took 125 us (3.1 TB/s, integer pipe 70 % busy).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -29,22 +30,38 @@ template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; 
 template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// 16 consecutive elements of a row (rows are 16-byte aligned: checked by the launcher): the raw
-// 16-byte loads of the next token are issued before the current one is converted.
+// A lane's share of a row as loaded: chunk k holds elements [kPer * (lane + 32 k), + kPer).
 template <typename T> struct Raw16 {
   static constexpr int kPer = 16 / sizeof(T);  // elements per 16-byte load
-  uint4 r[16 / kPer];
+  static constexpr int kChunks = 16 / kPer;
+  uint4 r[kChunks];
   T rope0, rope1;
   int64_t slot;
 };
-template <typename T> __device__ __forceinline__ void convert16(const Raw16<T>& raw, float (&v)[16]) {
-  constexpr int kPer = Raw16<T>::kPer;
+// Largest magnitude among a lane's 16 elements as f32 bits; NaN if there is one.
+template <typename T> __device__ __forceinline__ uint32_t amax_bits(const Raw16<T>& raw) {
+  float m = 0.f;
 #pragma unroll
-  for (int q = 0; q < 16 / kPer; ++q) {
-    const T* e = reinterpret_cast<const T*>(&raw.r[q]);
+  for (int q = 0; q < Raw16<T>::kChunks; ++q) {
+    const float* e = reinterpret_cast<const float*>(&raw.r[q]);
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) v[q * kPer + i] = to_f32<T>(e[i]);
+    for (int i = 0; i < 4; ++i) asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(fabsf(e[i])));
   }
+  return __float_as_uint(m) & 0x7fffffffu;
+}
+template <typename T2, typename T> __device__ __forceinline__ uint32_t amax_bits16(const Raw16<T>& raw) {
+  T2 m = __habs2(reinterpret_cast<const T2*>(&raw.r[0])[0]);
+#pragma unroll
+  for (int i = 1; i < 8; ++i) m = __hmax2_nan(m, __habs2(reinterpret_cast<const T2*>(&raw.r[i >> 2])[i & 3]));
+  return max(__float_as_uint(__low2float(m)) & 0x7fffffffu, __float_as_uint(__high2float(m)) & 0x7fffffffu);
+}
+template <> __device__ __forceinline__ uint32_t amax_bits<__nv_bfloat16>(const Raw16<__nv_bfloat16>& raw) { return amax_bits16<__nv_bfloat162>(raw); }
+template <> __device__ __forceinline__ uint32_t amax_bits<__half>(const Raw16<__half>& raw) { return amax_bits16<__half2>(raw); }
+constexpr uint32_t kInfBits = 0x7f800000u;
+// elements 2i and 2i + 1 of a chunk
+template <typename T> __device__ __forceinline__ float2 pair_of(const uint4& chunk, int i) {
+  const T* e = reinterpret_cast<const T*>(&chunk);
+  return make_float2(to_f32<T>(e[2 * i]), to_f32<T>(e[2 * i + 1]));
 }
 
 // E2M1 code of x / scale: magnitude = number of thresholds strictly below |n| (a tie stays on the
@@ -70,98 +87,166 @@ __device__ __forceinline__ uint32_t rope_e4m3(float x) {
   return __nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3);
 }
 
-// The same codes without the division, for all but a few values in a million.  q = x * (1/scale)
-// is within 3 units in the last place of the correctly rounded quotient n, and every rounding
-// threshold is a float whose low 21 mantissa bits are zero.  So unless bits(q) lies within 8 of a
-// multiple of 2^21, q and n fall between the same two thresholds and are not on one: round-to-
-// nearest-even and "a tie goes to the smaller magnitude" agree there, and the hardware conversion
-// cvt.rn.satfinite.e2m1x2.f32 of q gives the code (it saturates at 6 and keeps the sign of values
-// that round to magnitude zero, as the rule above does).  The fused add of +0 turns a product of
-// -0.0 into +0.0: a zero carries no sign bit.  The other values (including q = 0 from an underflow,
-// and infinity) are redone with the exact division afterwards.
-__device__ __forceinline__ bool needs_exact(float q, float x) {
-  return (((__float_as_uint(q) + 8u) & 0x1ffff0u) == 0u) && (__float_as_uint(x) << 1) != 0u;
-}
-// eight values -> eight packed codes (value 0 in the low nibble)
-__device__ __forceinline__ uint32_t e2m1x8(const float (&q)[8]) {
-  uint32_t out;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+// The same codes without the division.  x * (1/scale) is within 3 units in the last place of the correctly rounded quotient n,
+// so n lies between q_lo and q_hi, the products with 1/scale taken 2^-20 down and up.  The hardware conversion
+// cvt.rn.satfinite.e2m1x2.f32 is monotone, saturates at 6 and keeps the sign of values that round to magnitude zero, as the
+// rule above does.  (The products are fused with an addition of +0, which takes the sign off a zero.)  Where q_lo and q_hi
+// give the same code, that is the code.  Where they do not, a threshold t lies between them, and the code is that of q_hi if
+// n > t and that of q_lo if not (a tie goes to the smaller magnitude).  n > t without the division: |x| / scale must lie above
+// t by more than half of t's last place (at exactly half the quotient rounds to t, whose mantissa is even), and
+// |x| - t * scale is exact, being the small difference of a 24-bit and a 27-bit number.
+//
+// 16-bit values with scale = amax / 6 need q_lo alone, for all but one token in fifteen.  With x and amax integers of at most 11
+// bits (times powers of two) and t a multiple of 1/4, 6 x - t amax is zero or at least 2^-16 of either side, so the only
+// values with a threshold that near are x = t amax / 6 (amax / 8 is one: every other BF16 token has some).  Their quotient is
+// above t only if the rounding of amax / 6 made the scale too small by more than half of t's last place:
+// amax - 6 scale > 6 scale 2^-24 / (mantissa of t), and 1.75 is the largest mantissa.  Otherwise all of them are ties.
+//
+// What this does not cover takes the exact division for the whole token: a NaN, a scale outside [2^-100, 2^14]
+// (with which products of BF16 values could overflow or vanish), and an FP32 value below 2^-100 in magnitude, zero excepted.
+constexpr float kScaleLo = 7.8886090522101181e-31f, kScaleHi = 16384.f;
+// four values -> four packed codes (value 0 in the low nibble)
+__device__ __forceinline__ uint32_t e2m1x4(float a, float b, float c, float d) {
+  uint16_t out;
+  asm("{\n\t.reg .b8 b0, b1;\n\t"
       "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
       "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(out)
-      : "f"(q[0]), "f"(q[1]), "f"(q[2]), "f"(q[3]), "f"(q[4]), "f"(q[5]), "f"(q[6]), "f"(q[7]));
+      "mov.b16 %0, {b0, b1};\n\t}"
+      : "=h"(out)
+      : "f"(a), "f"(b), "f"(c), "f"(d));
   return out;
 }
+// a * b + 0
+__device__ __forceinline__ float2 scaled(uint64_t a, uint64_t b) {
+  float2 d;
+  asm("{\n\t.reg .b64 r;\n\tfma.rn.f32x2 r, %2, %3, %4;\n\tmov.b64 {%0, %1}, r;\n\t}" : "=f"(d.x), "=f"(d.y) : "l"(a), "l"(b), "l"(0ull));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+// What a token with a NaN gets as its largest magnitude: that of its other values.
+template <typename T> __device__ __noinline__ float amax_without_nan(const T* row, int lane) {
+  float m = 0.f;
+#pragma unroll 1
+  for (int i = lane; i < kLatent; i += 32) m = fmaxf(m, fabsf(to_f32<T>(row[i])));
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+}
+// Whether the quotient |x| / scale, rounded, is above the threshold between code magnitudes m and m + 1.
+__device__ __forceinline__ bool above(float x, float scale, uint32_t m) {
+  const uint32_t t = m < 2 ? __float_as_uint(0.25f + 0.5f * float(m)) : (m << 22) + (126u << 23) + (1u << 21);
+  const float half_ulp = __uint_as_float((t & 0x7f800000u) - (24u << 23));
+  return fmaf(-__uint_as_float(t), scale, fabsf(x)) > scale * half_ulp;
+}
+
+// Both values of a lane's RoPE pair as E4M3 bytes.
+__device__ __forceinline__ uint32_t rope_pair(float a, float b) {
+  if (fabsf(a) <= 464.f && fabsf(b) <= 464.f) return __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+  return rope_e4m3(a) | (rope_e4m3(b) << 8);
+}
+
+// CTAs per SM: what the registers of a prefetched token leave room for
+template <typename T> constexpr int kResident = sizeof(T) == 4 ? 4 : 5;
 
 template <typename T>
-__global__ void __launch_bounds__(kWriterWarps * 32)
+__global__ void __launch_bounds__(kWriterWarps * 32, kResident<T>)
 cache_write_kernel(const T* __restrict__ latent, int64_t latent_stride, const T* __restrict__ rope, int64_t rope_stride,
                    const float* __restrict__ scale_in, const int64_t* __restrict__ slot_mapping, int64_t num_tokens,
                    uint8_t* __restrict__ cache, float* __restrict__ cache_sf, int64_t num_slots) {
+  constexpr int kPer = Raw16<T>::kPer, kChunks = Raw16<T>::kChunks;
   const int lane = threadIdx.x & 31;
   const int64_t warps = int64_t(gridDim.x) * kWriterWarps;
+  // A dependent launch: its CTAs are in place when the kernel before it ends, and so are those of the kernel after it.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   auto fetch = [&](int64_t t, Raw16<T>& raw) {
-    raw.slot = slot_mapping ? __ldg(slot_mapping + t) : t;
-    const uint4* p = reinterpret_cast<const uint4*>(latent + t * latent_stride + 16 * lane);
+    raw.slot = slot_mapping ? slot_mapping[t] : t;
+    const uint4* p = reinterpret_cast<const uint4*>(latent + t * latent_stride) + lane;
 #pragma unroll
-    for (int q = 0; q < 16 / Raw16<T>::kPer; ++q) raw.r[q] = __ldg(p + q);
+    for (int q = 0; q < kChunks; ++q) raw.r[q] = p[32 * q];
     const T* rp = rope + t * rope_stride + 2 * lane;
     raw.rope0 = rp[0];
     raw.rope1 = rp[1];
   };
   int64_t t = int64_t(blockIdx.x) * kWriterWarps + (threadIdx.x >> 5);
-  Raw16<T> cur;
-  if (t < num_tokens) fetch(t, cur);
+  Raw16<T> nxt;
+  if (t < num_tokens) fetch(t, nxt);
   for (; t < num_tokens; t += warps) {
-    Raw16<T> nxt;
+    const Raw16<T> raw = nxt;
     if (t + warps < num_tokens) fetch(t + warps, nxt);  // in flight while this token is quantised
-    const Raw16<T> raw = cur;
-    cur = nxt;
     const int64_t slot = raw.slot;
     if (slot < 0 || slot >= num_slots) continue;  // padding token (negative) or out of the pool: nothing is written
-    float v[16];
-    convert16<T>(raw, v);
+    const T* src = latent + t * latent_stride;
+    const uint32_t top = __reduce_max_sync(0xffffffffu, amax_bits<T>(raw));  // non-negative floats compare as integers
     float scale;
     if (scale_in) {
       scale = scale_in[t];
     } else {
-      float amax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      scale = __fdiv_rn(amax, 6.0f);
+      scale = __fdiv_rn(top <= kInfBits ? __uint_as_float(top) : amax_without_nan<T>(src, lane), 6.0f);
       if (!(scale > 0.f)) scale = 1.0f;
     }
-    const float inv_scale = __frcp_rn(scale);
-    uint32_t w[2];
-    uint32_t redo = 0u;  // positions whose code must come from the exact division (a few per million)
+    const bool odd_token = !(scale >= kScaleLo && scale <= kScaleHi && top <= kInfBits);
+    const bool lo_alone = sizeof(T) == 2 && !scale_in && fmaf(-6.f, scale, __uint_as_float(top)) <= scale * (6.f * 0x1p-24f / 1.76f);
+    const float inv = __frcp_rn(scale), inv_lo = inv * (1.f - 0x1p-20f), inv_hi = inv * (1.f + 0x1p-20f);
+    bool odd = odd_token;
+    auto codes = [&](float f, bool look, uint32_t (&out)[2]) {  // eight codes each, in the order of the lane's elements
+      const uint64_t f2 = pack2(f, f);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float q[8];
+      for (int k = 0; k < 2; ++k) {
+        uint32_t c[2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        q[i] = fmaf(v[8 * h + i], inv_scale, 0.0f);
-        redo |= needs_exact(q[i], v[8 * h + i]) ? (1u << (8 * h + i)) : 0u;
+        for (int g = 0; g < 2; ++g) {
+          const int e = 8 * k + 4 * g;
+          const uint4& chunk = raw.r[e / kPer];
+          const float2 a = pair_of<T>(chunk, (e % kPer) / 2), b = pair_of<T>(chunk, (e % kPer) / 2 + 1);
+          const float2 qa = scaled(pack2(a.x, a.y), f2), qb = scaled(pack2(b.x, b.y), f2);
+          c[g] = e2m1x4(qa.x, qa.y, qb.x, qb.y);
+          if (sizeof(T) == 4 && look) {  // (2 * bits - 1: a zero becomes the largest word)
+            const uint32_t least = min(min(__float_as_uint(a.x) * 2u - 1u, __float_as_uint(a.y) * 2u - 1u), min(__float_as_uint(b.x) * 2u - 1u, __float_as_uint(b.y) * 2u - 1u));
+            odd |= least < 2u * __float_as_uint(kScaleLo);
+          }
+        }
+        out[k] = c[0] | (c[1] << 16);
       }
-      w[h] = e2m1x8(q);
-    }
-    while (redo) {
-      const int i = __ffs(redo) - 1;
-      redo &= redo - 1u;
-      const uint32_t code = e2m1_code(to_f32<T>(latent[t * latent_stride + 16 * lane + i]), scale);
-      const uint32_t sh = 4u * (uint32_t(i) & 7u);
-      uint32_t& word = (i >> 3) ? w[1] : w[0];
-      word = (word & ~(0xfu << sh)) | (code << sh);
+    };
+    uint32_t w[2], hi[2];
+    codes(inv_lo, true, w);
+    if (lo_alone) {
+      hi[0] = w[0];
+      hi[1] = w[1];
+    } else {
+      codes(inv_hi, false, hi);
     }
     uint8_t* row = cache + slot * kRowBytes;
-    *reinterpret_cast<uint2*>(row + 8 * lane) = make_uint2(w[0], w[1]);
-    // RoPE: two values per lane
-    const uint32_t r0 = rope_e4m3(to_f32<T>(raw.rope0)), r1 = rope_e4m3(to_f32<T>(raw.rope1));
-    *reinterpret_cast<uint16_t*>(row + kLatent / 2 + 2 * lane) = uint16_t(r0 | (r1 << 8));
+    if (odd || ((w[0] ^ hi[0]) | (w[1] ^ hi[1]))) {
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) {
+        uint32_t word = k ? w[1] : w[0];
+        const uint32_t up = k ? hi[1] : hi[0];
+        uint32_t todo = odd ? 0xffffffffu : word ^ up;
+#pragma unroll 1
+        while (todo) {
+          const int i = (__ffs(todo) - 1) >> 2;
+          const uint32_t nibble = 0xfu << (4 * i);
+          todo &= ~nibble;
+          const float x = to_f32<T>(src[kPer == 8 ? 256 * k + 8 * lane + i : 256 * k + 128 * (i >> 2) + 4 * lane + (i & 3)]);
+          if (odd) word = (word & ~nibble) | (e2m1_code(x, scale) << (4 * i));
+          else if (above(x, scale, (word >> (4 * i)) & 7u)) word = (word & ~nibble) | (up & nibble);
+        }
+        if (k) w[1] = word;
+        else w[0] = word;
+      }
+    }
+    if (kPer == 8) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) *reinterpret_cast<uint32_t*>(row + 4 * lane + 128 * q) = w[q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) *reinterpret_cast<uint16_t*>(row + 2 * lane + 64 * q) = uint16_t(w[q >> 1] >> (16 * (q & 1)));
+    }
+    *reinterpret_cast<uint16_t*>(row + kLatent / 2 + 2 * lane) = uint16_t(rope_pair(to_f32<T>(raw.rope0), to_f32<T>(raw.rope1)));
     if (lane == 0) cache_sf[slot] = scale;
   }
 }
@@ -174,13 +259,20 @@ cudaError_t launch_t(const void* latent, int64_t ls, const void* rope, int64_t r
   if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  // a whole number of waves: 8 CTAs of 8 warps per SM, fewer when the token count is small
+  // one wave of resident CTAs, fewer when the token count is small
   const int64_t want = (n + kWriterWarps - 1) / kWriterWarps;
-  const int grid = int(want < int64_t(sms) * 8 ? want : int64_t(sms) * 8);
-  cache_write_kernel<T><<<grid, kWriterWarps * 32, 0, stream>>>(
-      static_cast<const T*>(latent), ls, static_cast<const T*>(rope), rs, scale_in, slots, n,
-      static_cast<uint8_t*>(cache), sf, num_slots);
-  return cudaGetLastError();
+  const int grid = int(want < int64_t(sms) * kResident<T> ? want : int64_t(sms) * kResident<T>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kWriterWarps * 32);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, cache_write_kernel<T>, static_cast<const T*>(latent), ls, static_cast<const T*>(rope), rs, scale_in, slots, n,
+                            static_cast<uint8_t*>(cache), sf, num_slots);
 }
 
 }  // namespace

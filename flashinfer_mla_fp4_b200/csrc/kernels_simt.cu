@@ -253,6 +253,8 @@ __global__ void __launch_bounds__(256) fp32_check_kernel(DecodeParams p) {
 // the length before it reads its page id.
 __global__ void __launch_bounds__(128) step_metadata_kernel(StepMetadataParams p) {
   const int b = blockIdx.x;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (a dependent launch itself, and the writer's predecessor)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (b >= p.batch) {  // padding rows: no tokens, no cache write
     if (threadIdx.x == 0) p.dst_seq_lens[b] = 0;
     for (int j = threadIdx.x; j < p.q_len; j += blockDim.x) p.dst_slot_mapping[int64_t(b) * p.q_len + j] = -1;
@@ -307,8 +309,16 @@ cudaError_t launch_fp32_check(const DecodeParams& p, int num_ctas, cudaStream_t 
 }
 
 cudaError_t launch_step_metadata(const StepMetadataParams& p, cudaStream_t stream) {
-  step_metadata_kernel<<<unsigned(p.max_batch), 128, 0, stream>>>(p);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(p.max_batch));
+  cfg.blockDim = dim3(128);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, step_metadata_kernel, p);
 }
 
 cudaError_t launch_dequant(const void* in, void* out, int64_t n_bytes, cudaStream_t stream) {
