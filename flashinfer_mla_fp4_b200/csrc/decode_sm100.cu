@@ -83,10 +83,10 @@ constexpr uint32_t kOffQLat = kOffRope + kTile * 64;                      // [4]
 constexpr uint32_t kOffQRope = kOffQLat + kBlocks * kGroupHeads * 128;    // [64][64]      64B swizzle
 constexpr uint32_t kOffP = kOffQRope + kGroupHeads * 64;                  // [hi,lo][128][64] 64B swizzle (MN-major)
 constexpr uint32_t kOffScale = kOffP + 2 * kTile * 64;                    // [4][128] f32
-constexpr uint32_t kOffM = kOffScale + kScaleStages * kTile * 4;          // [64] f32 NEGATED reference -(M - shift)
-constexpr uint32_t kOffF = kOffM + kGroupHeads * 4;                       // [64] f32 rescale factor
-constexpr uint32_t kOffWmax = kOffF + kGroupHeads * 4;                    // [4][64] f32 per-warp column max / sum
-constexpr uint32_t kOffLinv = kOffWmax + 4 * kGroupHeads * 4;             // [64] f32 output factor; tail: 1/sum of the merge weights
+constexpr uint32_t kOffM = kOffScale + kScaleStages * kTile * 4;          // [2][64] f32 NEGATED references -(M - shift): the ones in force, and room for the next
+constexpr uint32_t kOffF = kOffM + 2 * kGroupHeads * 4;                   // [64] f32 rescale factor of a moved reference, [64] f32 by how much it moved
+constexpr uint32_t kOffNotes = kOffF + 2 * kGroupHeads * 4;               // [tile mod 3][64] s32 notes of beaten references; epilogue: [4][64] f32 row sums
+constexpr uint32_t kOffLinv = kOffNotes + 4 * kGroupHeads * 4;             // [64] f32 output factor; tail: 1/sum of the merge weights
 constexpr uint32_t kOffLse = kOffLinv + kGroupHeads * 4;                  // [64] f32
 constexpr uint32_t kOffScMax = kOffLse + kGroupHeads * 4;                 // [8] f32 per-warp largest token scale
 constexpr uint32_t kOffBars = kOffScMax + kSoftmaxWarps * 4;              // mbarriers (8 B each)
@@ -211,6 +211,7 @@ __device__ __forceinline__ void st_release(int32_t* p, int v) {
 struct RoleState {
   uint32_t it;         // tiles processed so far by this CTA (selects stages and barrier phases)
   uint32_t seg;        // segments processed so far
+  uint32_t m, mod3;    // softmax: which references are in force; it mod 3
   uint32_t slot, lap;  // pair slot of the role's next latent pair, and how many times the ring has been filled before it
   __device__ __forceinline__ void advance(uint32_t n) {
     slot += n;
@@ -340,9 +341,9 @@ __device__ __forceinline__ bool plan_still_valid(const DecodeParams& p, uint32_t
 // stage t mod 4, last read by tile t-4, is free: it needs no barrier of its own and its bytes count on the pair's barrier.
 // page id `at + lane` of a segment, -1 beyond its pages or outside the pool
 __device__ __forceinline__ int page_window(const DecodeParams& p, const Segment& g, int at) {
-  const int ppt = kTile / p.page_size;
+  const int ppt = kTile >> p.page_shift;
   const int lp = g.tile_begin * ppt + at + int(threadIdx.x & 31);
-  const int id = lp < min((g.seq_len - 1) / p.page_size + 1, g.tile_end * ppt) ? __ldcg(p.block_tables + size_t(g.b) * p.block_table_stride + lp) : -1;
+  const int id = lp < min(((g.seq_len - 1) >> p.page_shift) + 1, g.tile_end * ppt) ? __ldcg(p.block_tables + size_t(g.b) * p.block_table_stride + lp) : -1;
   return int64_t(id) < p.num_pages ? id : -1;
 }
 // entry `i` of a window, in a uniform register
@@ -352,7 +353,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
   const uint32_t nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   const Segment* sg = segs_of(smem);
   const int lane = threadIdx.x & 31;
-  const int ppt = kTile / p.page_size;  // pages per tile
+  const int ppt = kTile >> p.page_shift;  // pages per tile
   const uint32_t ps = uint32_t(p.page_size);
   bool ok = true;
 #pragma unroll 1
@@ -361,7 +362,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
     g.tile_begin = int(ptx::uniform_u32(uint32_t(g.tile_begin)));
     g.tile_end = int(ptx::uniform_u32(uint32_t(g.tile_end)));
     g.seq_len = int(ptx::uniform_u32(uint32_t(g.seq_len)));
-    const int total = (g.seq_len - 1) / p.page_size + 1;
+    const int total = ((g.seq_len - 1) >> p.page_shift) + 1;
     int cur = page_window(p, g, 0), nxt = page_window(p, g, 32), ahead = 64, at = 0;
 #pragma unroll 1
     for (int t = g.tile_begin; t < g.tile_end; ++t, ++st.it) {
@@ -682,13 +683,13 @@ __device__ __forceinline__ float tanh_approx(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-// First half of a tile's softmax, over the 32 heads this thread owns of its token: e = exp2(x*c - m) with the reference as it
-// stands; returns the largest exponent argument for the lazy-reference check.  Nothing has been summed or converted yet, so
-// a reference that turns out to be beaten costs a scaling of e, not a second pass.  The S columns of the second 16 heads are
-// on their way while the first are exponentiated.
+// First half of a tile's softmax, over the 32 heads this thread owns of its token: the exponents y = x*c - m with the reference
+// as it stands; returns the largest for the lazy-reference check.  Nothing has been exponentiated yet, so a reference that turns
+// out to be beaten, by however much, costs a subtraction.  The S columns of the second 16 heads are on their way while the
+// first are worked on.
 // kSoftCap: the raw score x = q.k passes through cap * tanh(x / cap) first (compiled only into the soft-cap kernel).
 template <bool kSoftCap>
-__device__ __forceinline__ float exp_pass(const SoftmaxTile& t, uint64_t (&e2)[kPairs]) {
+__device__ __forceinline__ float exponents(const SoftmaxTile& t, uint64_t (&y2)[kPairs]) {
   float mx = -INFINITY;
   uint32_t a[2][16], b[2][16];
   ptx::tmem_ld16(t.t_lat, a[0]);
@@ -715,88 +716,55 @@ __device__ __forceinline__ float exp_pass(const SoftmaxTile& t, uint64_t (&e2)[k
           unpack2(mul2(x2, t.rcap2), x0, x1);
           x2 = mul2(pack2(tanh_approx(x0), tanh_approx(x1)), t.cap2);
         }
-        float a0, a1;
-        unpack2(fma2(x2, t.cs2, nm[h]), a0, a1);
-        mx = max3(mx, a0, a1);
-        e2[8 * cidx + 2 * q + h] = pack2(ptx::ex2(a0), ptx::ex2(a1));
+        const uint64_t y = fma2(x2, t.cs2, nm[h]);
+        y2[8 * cidx + 2 * q + h] = y;
+        float y0, y1;
+        unpack2(y, y0, y1);
+        mx = max3(mx, y0, y1);
       }
     }
   }
   if (!t.valid) {  // token beyond seq_len: weight exactly zero, whatever its row holds (its RoPE bytes may decode to NaN)
 #pragma unroll
-    for (int q = 0; q < kPairs; ++q) e2[q] = 0ull;
+    for (int q = 0; q < kPairs; ++q) y2[q] = pack2(-INFINITY, -INFINITY);
     mx = -INFINITY;
   }
   return mx;
 }
 
-// Set the per-head reference from the scores: column max of y = x*c + log2(scale_t) over the tile's tokens,
-// m = max(m_old, colmax - shift); f = 2^(m_old - m) (0 when there was no reference yet).  Used by the first tile of a segment
-// and when a score beats the reference by so much that its exponential overflows.
-template <bool kSoftCap>
-__device__ __noinline__ void reference_from_scores(uint32_t smem, uint32_t t_lat, uint32_t t_rope, float sc, bool valid,
-                                               float cscale, float lg, bool have_m, int tid, float cap) {
-  const float rcap = kSoftCap ? 1.f / cap : 0.f;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, half = warp >> 2;  // t_lat / t_rope already point at this warp's 32 columns
-  const uint32_t wred = smem + kOffWmax;
-#pragma unroll 1
-  for (int cidx = 0; cidx < 2; ++cidx) {
-    uint32_t a[16], b[16];
-    ptx::tmem_ld16(t_lat + 16 * cidx, a);
-    ptx::tmem_ld16(t_rope + 16 * cidx, b);
-    ptx::tmem_wait_ld();
-    float mine = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float x = fmaf(__uint_as_float(a[i]), sc, __uint_as_float(b[i]));
-      if (kSoftCap) x = cap * tanh_approx(x * rcap);
-      const float y = fmaf(x, cscale, lg);
-      const float r = ptx::redux_max_f32(valid ? y : -INFINITY);
-      if ((lane & 15) == i) mine = r;
-    }
-    if (lane < 16) sts_f32(wred + 4 * (quarter * kGroupHeads + 32 * half + 16 * cidx + lane), mine);
-  }
-  ptx::bar_sync(1, kSoftmaxThreads);
-  if (tid < kGroupHeads) {
-    float mnew = fmaxf(fmaxf(lds_f32(wred + 4 * tid), lds_f32(wred + 4 * (kGroupHeads + tid))),
-                       fmaxf(lds_f32(wred + 4 * (2 * kGroupHeads + tid)), lds_f32(wred + 4 * (3 * kGroupHeads + tid)))) - kPShift;
-    const float mold = have_m ? -lds_f32(smem + kOffM + 4 * tid) : -INFINITY;
-    mnew = fmaxf(mnew, mold);
-    sts_f32(smem + kOffF + 4 * tid, have_m ? ptx::ex2(mold - mnew) : 0.f);
-    sts_f32(smem + kOffM + 4 * tid, -mnew);
-  }
-  ptx::bar_sync(1, kSoftmaxThreads);
-}
-
-// Move the references that were beaten by more than the lazy threshold, from the exponentials at hand: column max of
-// P' = e * |scale_t| over the tile's tokens; m += log2(colmax) - shift and f = its inverse for those heads, f = 1 for all others.
-__device__ __forceinline__ void refresh_beaten(uint32_t smem, const uint64_t (&e2)[kPairs], float sc_abs, int tid) {
-  const int warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, half = warp >> 2;
-  const uint32_t wred = smem + kOffWmax;
-  uint32_t mine = 0;  // lane i: head 32*half + i (non-negative floats compare as integers)
+// The references that tokens of a tile beat by more than the lazy threshold.  A warp with such a token notes the largest
+// y + log2|scale_t| of each of its heads (as integers that compare like the floats), before the vote of the softmax warps;
+// after it every warp works out the new references and factors of its 32 heads from the notes (the four warps of a half write
+// the same values): no barrier but the vote.  The first tile of a segment is the same with references of zero and every warp
+// noting.  Notes go round three places: those of tile t-1 are cleared after the vote of tile t, when nobody reads them any
+// more, and used again by tile t+2, which no warp reaches before all have voted in tile t+1.
+// (With heavy-tailed token scales a reference is beaten in every other tile, mostly by more than FP32 exponentials could hold:
+// recomputing such tiles from the scores took 1100 clk each.)
+constexpr int kNoScore = int(0x80000000u);
+__device__ __forceinline__ void note_beaten(uint32_t notes, const uint64_t (&y2)[kPairs], float lg, int lane) {
+  float mine = -INFINITY;  // lane i: head i of the warp's 32
 #pragma unroll
   for (int i = 0; i < kPairs; ++i) {
-    float e0, e1;
-    unpack2(e2[i], e0, e1);
-    const uint32_t r0 = __reduce_max_sync(0xffffffffu, __float_as_uint(e0 * sc_abs)), r1 = __reduce_max_sync(0xffffffffu, __float_as_uint(e1 * sc_abs));
-    if ((lane >> 1) == i) mine = (lane & 1) ? r1 : r0;
+    float y0, y1;
+    unpack2(y2[i], y0, y1);
+    const float r0 = ptx::redux_max_f32(y0 + lg), r1 = ptx::redux_max_f32(y1 + lg);
+    if (lane == 2 * i) mine = r0;
+    if (lane == 2 * i + 1) mine = r1;
   }
-  sts_f32(wred + 4 * (quarter * kGroupHeads + 32 * half + lane), __uint_as_float(mine));
-  ptx::bar_sync(1, kSoftmaxThreads);
-  if (tid < kGroupHeads) {
-    const float cm = fmaxf(fmaxf(lds_f32(wred + 4 * tid), lds_f32(wred + 4 * (kGroupHeads + tid))),
-                           fmaxf(lds_f32(wred + 4 * (2 * kGroupHeads + tid)), lds_f32(wred + 4 * (3 * kGroupHeads + tid))));
-    float f = 1.f;
-    if (cm > 430.f) {  // 2^(shift + threshold)
-      const float d = __log2f(cm) - kPShift;
-      f = ptx::ex2(-d);
-      sts_f32(smem + kOffM + 4 * tid, lds_f32(smem + kOffM + 4 * tid) - d);
-    }
-    sts_f32(smem + kOffF + 4 * tid, f);
-  }
-  ptx::bar_sync(1, kSoftmaxThreads);
+  const int b = __float_as_int(mine);
+  asm volatile("red.shared.max.s32 [%0], %1;" ::"r"(notes + 4 * lane), "r"(b ^ ((b >> 31) & 0x7fffffff)) : "memory");
+}
+// m += top - shift and f = 2^-(top - shift) for the heads that were beaten, f = 1 for all others.
+__device__ __forceinline__ void refresh_beaten(uint32_t smem, uint32_t notes, uint32_t cur, bool first, int half, int lane) {
+  const uint32_t at = 4u * (32u * uint32_t(half) + uint32_t(lane));
+  const int b = int(lds_u32(notes + 4 * lane));
+  const float top = __int_as_float(b ^ ((b >> 31) & 0x7fffffff));  // (a NaN where there is no note)
+  const bool beaten = first || top > kPShift + kLazyThreshold;
+  const float d = beaten ? top - kPShift : 0.f;
+  sts_f32(smem + kOffM + 256 * (cur ^ 1u) + at, lds_f32(smem + kOffM + 256 * cur + at) - d);
+  sts_f32(smem + kOffF + at, beaten ? ptx::ex2(-d) : 1.f);
+  sts_f32(smem + kOffF + 256 + at, d);
+  __syncwarp();
 }
 
 // O^T *= f per head column, in TMEM (all four 128-dim blocks of this thread's lane).  With few heads moved, as a new maximum
@@ -807,34 +775,44 @@ __device__ __noinline__ void rescale_output(uint32_t smem, uint32_t tmem_lane, u
   uint32_t moved = __ballot_sync(0xffffffffu, mine != 1.f);
   if (__popc(moved) <= 8) {
 #pragma unroll 1
-    while (moved) {
-      const uint32_t h = uint32_t(__ffs(moved)) - 1u;
+    while (moved) {  // two heads at a time (or one, twice)
+      const uint32_t h0 = uint32_t(__ffs(moved)) - 1u;
       moved &= moved - 1u;
-      const float f = __shfl_sync(0xffffffffu, mine, int(h));
-      uint32_t o[kBlocks];
+      const uint32_t h1 = moved ? uint32_t(__ffs(moved)) - 1u : h0;
+      moved &= moved - 1u;
+      const float f0 = __shfl_sync(0xffffffffu, mine, int(h0)), f1 = __shfl_sync(0xffffffffu, mine, int(h1));
+      uint32_t o[kBlocks], u[kBlocks];
 #pragma unroll
-      for (int j = 0; j < kBlocks; ++j) ptx::tmem_ld1(base + 64u * j + h, o[j]);
+      for (int j = 0; j < kBlocks; ++j) ptx::tmem_ld1(base + 64u * j + h0, o[j]);
+#pragma unroll
+      for (int j = 0; j < kBlocks; ++j) ptx::tmem_ld1(base + 64u * j + h1, u[j]);
       ptx::tmem_wait_ld();
 #pragma unroll
-      for (int j = 0; j < kBlocks; ++j) ptx::tmem_st1(base + 64u * j + h, __float_as_uint(__uint_as_float(o[j]) * f));
+      for (int j = 0; j < kBlocks; ++j) ptx::tmem_st1(base + 64u * j + h0, __float_as_uint(__uint_as_float(o[j]) * f0));
+#pragma unroll
+      for (int j = 0; j < kBlocks; ++j) ptx::tmem_st1(base + 64u * j + h1, __float_as_uint(__uint_as_float(u[j]) * f1));
     }
   } else {
 #pragma unroll 1
-    for (uint32_t jc = 0; jc < kBlocks * 2; ++jc) {
-      uint32_t o[16];
-      const uint32_t ta = base + 64u * (jc >> 1) + 16u * (jc & 1);
-      ptx::tmem_ld16(ta, o);
-      const uint32_t f = smem + kOffF + 4 * (32u * half + 16u * (jc & 1));
+    for (uint32_t jc = 0; jc < kBlocks; ++jc) {  // 16 heads of two blocks at a time
+      uint32_t o[2][16];
+      const uint32_t c = 16u * (jc & 1), ta = base + 128u * (jc >> 1) + c;
+      ptx::tmem_ld16(ta, o[0]);
+      ptx::tmem_ld16(ta + 64u, o[1]);
+      const uint32_t f = smem + kOffF + 4 * (32u * half + c);
       ptx::tmem_wait_ld();
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float4 v = lds_f32x4(f + 16 * q);
-        o[4 * q] = __float_as_uint(__uint_as_float(o[4 * q]) * v.x);
-        o[4 * q + 1] = __float_as_uint(__uint_as_float(o[4 * q + 1]) * v.y);
-        o[4 * q + 2] = __float_as_uint(__uint_as_float(o[4 * q + 2]) * v.z);
-        o[4 * q + 3] = __float_as_uint(__uint_as_float(o[4 * q + 3]) * v.w);
+        const float vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          o[0][4 * q + e] = __float_as_uint(__uint_as_float(o[0][4 * q + e]) * vs[e]);
+          o[1][4 * q + e] = __float_as_uint(__uint_as_float(o[1][4 * q + e]) * vs[e]);
+        }
       }
-      ptx::tmem_st16(ta, o);
+      ptx::tmem_st16(ta, o[0]);
+      ptx::tmem_st16(ta + 64u, o[1]);
     }
   }
   ptx::tmem_wait_st();
@@ -972,7 +950,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
   const uint32_t tmem_lane = tmem + ((uint32_t(quarter) * 32u) << 16);
   const float cscale = p.softmax_scale * kLog2e;
   SoftmaxTile t;
-  t.negm = smem + kOffM + 4 * kHalfHeads * half;
   t.cs2 = pack2(cscale, cscale);
   const float cap = kSoftCap ? p.soft_cap : 0.f;
   t.cap2 = pack2(cap, cap);
@@ -980,6 +957,8 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
   // this thread's P' row: two 16-byte chunks of hi and two of lo, swizzled
   const uint32_t psw = (uint32_t(row) >> 1) & 3u;
   const uint32_t p_row = smem + kOffP + uint32_t(row) * 64u;
+  const uint32_t notes = smem + kOffNotes + 128 * half;
+  bool noted = false;  // this warp's notes of the tile before are not cleared
   int pending = 0;  // partial slots written in this call: bit 0 the even one, bit 1 the odd one, bit 2 its LSEs are not out yet (the even one's)
 
 #pragma unroll 1
@@ -990,7 +969,7 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
     for (int h = 0; h < kPairs; ++h) l2[h] = 0ull;
     float sc_max = 0.f;  // largest |token scale| this thread has seen in the segment
 #pragma unroll 1
-    for (int tt = g.tile_begin; tt < g.tile_end; ++tt, ++st.it, st.advance(2)) {
+    for (int tt = g.tile_begin; tt < g.tile_end; ++tt, ++st.it, st.advance(2), st.mod3 = st.mod3 == 2 ? 0 : st.mod3 + 1) {
       const uint32_t it = st.it, s = it & 1;
       const bool first = tt == g.tile_begin;
       // per-token scale (it counts on the barrier of the tile's first pair)
@@ -1008,37 +987,45 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       if (tid == 0) MLA_STAMP(3, it, 0);
       ptx::tc_fence_after();
 
-      // The exponentials are taken with the reference as it stands, which holds unless some score beat it by more than the lazy
-      // threshold (P' would leave the E4M3 range; the second test catches a large score of a token with a vanishing scale).
-      // Then the references of the heads concerned are moved, and e, the sums and, below, O^T are scaled.  Latents with
-      // heavy-tailed scales do that in every other tile: recomputing the whole pass there cost 3900 clk each time.
+      // The exponents are taken with the reference as it stands, which holds unless some score beat it by more than the lazy
+      // threshold (P' would leave the E4M3 range).  Then the references of the heads concerned are moved, and the exponents, the
+      // sums and, below, O^T follow.
       uint64_t e2[kPairs];
-      bool moved = false;
-      if (first) reference_from_scores<kSoftCap>(smem, t.t_lat, t.t_rope, sc, t.valid, cscale, lg, false, tid, cap);
-#pragma unroll 1
-      for (;;) {
-        const float mx = exp_pass<kSoftCap>(t, e2);
-        if (first || moved) break;
-        if (!ptx::bar_or(1, kSoftmaxThreads, mx + lg > kPShift + kLazyThreshold || mx > 100.f)) break;
-        moved = true;
-        const bool overflow = ptx::bar_or(1, kSoftmaxThreads, mx > 100.f);
-        if (overflow) reference_from_scores<kSoftCap>(smem, t.t_lat, t.t_rope, sc, t.valid, cscale, lg, true, tid, cap);
-        else refresh_beaten(smem, e2, fabsf(sc), tid);
-#pragma unroll
-        for (int q = 0; q < kPairs / 2; ++q) {
-          uint64_t f[2];
-          lds_pairs(smem + kOffF + 4 * kHalfHeads * half + 16 * q, f[0], f[1]);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            l2[2 * q + h] = mul2(l2[2 * q + h], f[h]);
-            e2[2 * q + h] = mul2(e2[2 * q + h], f[h]);
-          }
-        }
-        if (!overflow) break;
-      }
+      t.negm = smem + kOffM + 256 * st.m + 4 * kHalfHeads * half;
+      const float mx = exponents<kSoftCap>(t, e2);
       ptx::tc_fence_before();  // orders the S reads before the arrival
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar_addr(smem, bar_s_empty(s)));
+      const bool beaten = first || mx + lg > kPShift + kLazyThreshold;
+      const bool note_now = __any_sync(0xffffffffu, beaten);
+      const uint32_t here = notes + 256 * st.mod3;
+      if (note_now) note_beaten(here, e2, lg, lane);
+      const bool moved = ptx::bar_or(1, kSoftmaxThreads, beaten);
+      if (noted) sts_f32(notes + 256 * (st.mod3 == 0 ? 2 : st.mod3 - 1) + 4 * lane, __int_as_float(kNoScore));
+      noted = note_now;
+      if (moved) {
+        refresh_beaten(smem, here, st.m, first, half, lane);
+        st.m ^= 1u;
+        const uint32_t f = smem + kOffF + 4 * kHalfHeads * half;
+        const uint64_t minus = pack2(-1.f, -1.f);
+#pragma unroll
+        for (int q = 0; q < kPairs / 2; ++q) {
+          uint64_t d[2], g2[2];
+          lds_pairs(f + 256 + 16 * q, d[0], d[1]);
+          lds_pairs(f + 16 * q, g2[0], g2[1]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            e2[2 * q + h] = fma2(d[h], minus, e2[2 * q + h]);
+            l2[2 * q + h] = mul2(l2[2 * q + h], g2[h]);
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kPairs; ++q) {
+        float y0, y1;
+        unpack2(e2[q], y0, y1);
+        e2[q] = pack2(ptx::ex2(y0), ptx::ex2(y1));
+      }
       // Second half: row sums, and P' = e * scale_t split into two E4M3 terms
       uint32_t hi[8], lo[8];
 #pragma unroll
@@ -1054,7 +1041,7 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       // The one P buffer (and, for a rescale, O^T) is free once the PV of the previous tile has completed; until then
       // this tile's P' stays in registers.
       if (it >= 1) (void)wait(smem, kBarPvDone, (it - 1) & 1);
-      if (moved) {  // O^T holds earlier tiles of the segment
+      if (moved && !first) {  // O^T holds earlier tiles of the segment
         ptx::tc_fence_after();
         rescale_output(smem, tmem_lane, uint32_t(half), lane);
       }
@@ -1075,15 +1062,22 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
 
     // ---- segment epilogue
     const float r = warp_transpose_sum32(l2, lane);  // lane L: this warp's tokens, head 32*half + L
-    const uint32_t wred = smem + kOffWmax;
+    const uint32_t wred = smem + kOffNotes;
+    ptx::bar_sync(1, kSoftmaxThreads);  // nobody reads notes any more
+    noted = false;
     sts_f32(wred + 4 * (quarter * kGroupHeads + kHalfHeads * half + lane), r);
     const float sc_warp = ptx::redux_max_f32(sc_max);
     if (lane == 0) sts_f32(smem + kOffScMax + 4 * warp, sc_warp);
     ptx::bar_sync(1, kSoftmaxThreads);
     if (tid < kGroupHeads) {
-      const float L = (lds_f32(wred + 4 * tid) + lds_f32(wred + 4 * (kGroupHeads + tid))) +
-                      (lds_f32(wred + 4 * (2 * kGroupHeads + tid)) + lds_f32(wred + 4 * (3 * kGroupHeads + tid)));
-      float m = -lds_f32(smem + kOffM + 4 * tid);
+      float L = 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        L += lds_f32(wred + 4 * (q * kGroupHeads + tid));
+        sts_f32(wred + 4 * (q * kGroupHeads + tid), __int_as_float(kNoScore));
+      }
+      float m = -lds_f32(smem + kOffM + 256 * st.m + 4 * tid);
+      sts_f32(smem + kOffM + 256 * st.m + 4 * tid, 0.f);  // for the next segment
       float Ls = L, fo = p.output_scale;
       if (p.sink && g.tile_begin == 0) {  // the sink: a virtual token with a zero value row, counted with the first tile of a request
         int qpos, head0;
@@ -1510,6 +1504,11 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     }
   } else if (warp == kWarpTMA) {
     if (p.pdl_wait) stage_segments(p, smem, lane, true, false);  // a first plan, from the lengths as they are in memory
+  } else if (warp == kWarpSoftmax0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sts_f32(smem + kOffNotes + 4 * (lane + 32 * i), __int_as_float(kNoScore));
+    sts_f32(smem + kOffM + 4 * lane, 0.f);
+    sts_f32(smem + kOffM + 4 * (lane + 32), 0.f);
   } else if (warp == kWarpTMA2 && lane == 0) {
     ptx::prefetch_tensormap(&map_q_lat);
     ptx::prefetch_tensormap(&map_q_rope);
@@ -1526,7 +1525,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (tid == 0) MLA_STAMP(4, 1u, 1);
 
-  RoleState st{0, 0, 0, 0};
+  RoleState st{};
   if (warp == kWarpTMA2) st.slot = 1;
   // The plan made before the wait stands if the lengths have not changed.  The partition is walked by the warp that issues the
   // first copies: it goes on to them without waiting for the others.
@@ -1769,6 +1768,7 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   cfg.numAttrs = p.pdl ? 1 : 0;
   DecodeParams pp = p;
   pp.pdl_wait = p.pdl;
+  pp.page_shift = __builtin_ctz(unsigned(p.page_size));
   return cudaLaunchKernelEx(&cfg, kernel, pp, map_q_lat, map_q_rope, map_rope, map_lat);
 }
 

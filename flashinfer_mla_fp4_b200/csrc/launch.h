@@ -18,6 +18,7 @@ struct DecodeParams {
   void* workspace;
   int32_t* status;
   int32_t batch, q_len, num_heads, page_size, groups;
+  int32_t page_shift;   // log2(page_size), set by the launcher
   int64_t num_pages;
   float softmax_scale, output_scale;
   int32_t out_dtype;
