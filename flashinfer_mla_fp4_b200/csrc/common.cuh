@@ -99,10 +99,10 @@ MLA_HD int capped_len(const int32_t* seq_lens, int b, int cap) {
 }
 
 // The flat space that is cut into CTA ranges counts kPhantom extra tiles in front of every non-empty
-// request: moving on to another request costs a CTA about as much as two tiles (the epilogue of the
-// old one, a fresh query, a cold pipeline), so a CTA whose range holds the start of a request gets
+// request: moving on to another request costs a CTA about as much as three tiles (the epilogue of the
+// old one, a fresh query, a first tile without a reference), so a CTA whose range holds the start of a request gets
 // that many tiles less.  A piece of a range that holds nothing but phantom tiles is no segment.
-constexpr int kPhantom = MLA_FP4_PHANTOM_TILES;  // measured: 2 and 3 are equally good, 1 and 4 worse
+constexpr int kPhantom = MLA_FP4_PHANTOM_TILES;  // measured, 1 / 2 / 3 / 4: 128 requests of 128..32768 tokens 93.8 / 89.4 / 85.8 / 85.4 us, 8x32768 34.8 / 34.8 / 34.7 / 35.3
 MLA_HD int vtiles_of(int seq_len) { return seq_len > 0 ? tiles_of(seq_len) + kPhantom : 0; }
 
 // Short requests are not split.  When no request has more than kWholeTiles tiles and there are no more (request, head
