@@ -5,6 +5,8 @@
 //   * step_metadata_kernel - a decode step's persistent metadata refreshed from the scheduler's tensors
 //   * dequant_kernel       - E2M1 -> E4M3 byte dequantisation (the routine fp32_check_kernel uses), for the
 //                            bit-exact table test; the tcgen05 kernel hands the packed codes to the MMA unchanged
+#include <climits>
+
 #include "common.cuh"
 #include "dequant.cuh"
 #include "launch.h"
@@ -249,9 +251,10 @@ __global__ void __launch_bounds__(256) fp32_check_kernel(DecodeParams p) {
 
 // One CTA per row of the persistent buffers.  The step's metadata is a few kilobytes, so the launch is all latency: the
 // torch form of it was about twenty kernels or copies and 150 us of host time.  Sources in pinned host memory are read in
-// place over PCIe; the row, the length and a given slot mapping are independent loads, and only a derived slot waits for
-// the length before it reads its page id.
+// place over PCIe, in one round trip: the row, the length and a given slot mapping are independent loads, and a derived slot is
+// written by the thread that holds its page id (read again after the length it cost a second trip, 8.1 us a launch).
 __global__ void __launch_bounds__(128) step_metadata_kernel(StepMetadataParams p) {
+  constexpr int kBatch = 4;  // page ids per thread in flight
   const int b = blockIdx.x;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (a dependent launch itself, and the writer's predecessor)
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -261,24 +264,42 @@ __global__ void __launch_bounds__(128) step_metadata_kernel(StepMetadataParams p
     return;
   }
   const int32_t* row = p.block_tables + int64_t(b) * p.block_table_stride;
-  const int64_t len = p.seq_lens_is_64 ? static_cast<const int64_t*>(p.seq_lens)[b] : int64_t(static_cast<const int32_t*>(p.seq_lens)[b]);
-  for (int j = threadIdx.x; j < p.q_len; j += blockDim.x) {
-    int64_t slot = -1;
-    if (p.slot_mapping) {
-      slot = p.slot_mapping[int64_t(b) * p.q_len + j];
-    } else {
-      const int64_t pos = len - p.q_len + j;
-      if (pos >= 0) {
-        const int64_t page = pos / p.page_size;
-        slot = int64_t(row[page < p.width ? page : p.width - 1]) * p.page_size + pos % p.page_size;
-      }
-    }
-    p.dst_slot_mapping[int64_t(b) * p.q_len + j] = slot;
-  }
-  if (threadIdx.x == 0) p.dst_seq_lens[b] = int32_t(len);
   int32_t* dst = p.dst_block_tables + int64_t(b) * p.dst_block_table_stride;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < p.width; i += blockDim.x) dst[i] = row[i];
+  int64_t* slots = p.dst_slot_mapping + int64_t(b) * p.q_len;
+  int32_t id[kBatch];
+  auto fetch = [&](int base) {
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int i = base + k * int(blockDim.x) + int(threadIdx.x);
+      id[k] = i < p.width ? row[i] : 0;
+    }
+  };
+  fetch(0);
+  const int64_t len = p.seq_lens_is_64 ? static_cast<const int64_t*>(p.seq_lens)[b] : int64_t(static_cast<const int32_t*>(p.seq_lens)[b]);
+  if (p.slot_mapping)
+    for (int j = threadIdx.x; j < p.q_len; j += blockDim.x) slots[j] = p.slot_mapping[int64_t(b) * p.q_len + j];
+  if (threadIdx.x == 0) p.dst_seq_lens[b] = int32_t(len);
+  for (int base = 0; base == 0 || base < p.width; base += kBatch * int(blockDim.x)) {
+    if (base > 0) fetch(base);
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int i = base + k * int(blockDim.x) + int(threadIdx.x);
+      if (i < p.width) dst[i] = id[k];
+    }
+    if (p.slot_mapping) continue;
+    for (int j = 0; j < p.q_len; ++j) {
+      const int64_t pos = len - p.q_len + j;
+      if (pos < 0) {
+        if (base == 0 && threadIdx.x == 0) slots[j] = -1;
+        continue;
+      }
+      const int64_t page = pos < INT_MAX ? int64_t(uint32_t(pos) / uint32_t(p.page_size)) : pos / p.page_size;
+      const int at = int(page < p.width ? page : p.width - 1) - base - int(threadIdx.x);
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (at == k * int(blockDim.x)) slots[j] = int64_t(id[k]) * p.page_size + (pos - page * p.page_size);
+    }
+  }
 }
 
 __global__ void dequant_kernel(const uint32_t* __restrict__ in, uint2* __restrict__ out, int64_t n_words) {
