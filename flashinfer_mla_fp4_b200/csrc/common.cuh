@@ -81,7 +81,8 @@ MLA_HD int out_elem_bytes(int out_dtype) { return out_dtype == MLA_FP4_OUT_F32 ?
 // A "virtual request" v = g * batch + b is request b seen by head group g (a group is 64 query
 // heads of one query position).  Request b has tiles_b = ceil(seq_len_b / 128) tiles.  All tiles
 // of all virtual requests, in v order, form a flat space of Tt = groups * sum_b tiles_b tiles.
-// CTA i of n owns the contiguous flat range [Tt*i/n, Tt*(i+1)/n).  A CTA therefore walks a list
+// CTA i of n owns the contiguous flat range [Tt*i/n, Tt*(i+1)/n); n is the grid, or, when the decode kernel merges by
+// itself, the first CTAs of the grid that it finds worth using.  A CTA therefore walks a list
 // of segments (v, tile_begin, tile_end); only its first and its last segment can cover a request
 // partially.  A partial segment writes a split-KV partial into workspace slot 2*i (first
 // segment of the CTA) or 2*i+1 (any later one); a segment that covers its request completely

@@ -1,0 +1,35 @@
+"""The number of CTAs that share a step's work: on both sides of the rule's edges, against the oracle."""
+import pytest
+import torch
+
+from oracle import mla_fp4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("lens,heads,max_ctas", [
+    ([513], 64, None),            # five tiles: the smallest request that is split, one CTA per tile
+    ([1280, 1152], 64, 5),        # 25 tiles with the phantom ones on 5 CTAs: still by the rule
+    ([1280, 1281], 64, 5),        # 27: the whole grid
+    ([3000], 64, 1),              # a grid of one
+    ([130, 0, 5000, 1, 700], 64, None),   # the walk that shares best is two tiles long; requests without work
+    ([16000], 16, None),          # many more CTAs than the rule wants
+    ([2500] * 30, 128, 7),        # rounds of many segments
+])
+def test_any_number_of_working_ctas(lens, heads, max_ctas):
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("ctas", [max(n, 1) for n in lens], heads, 64, seed=sum(lens), device=dev)
+    case.seq_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=heads, page_size=64, max_ctas=max_ctas)
+    out, lse = w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale,
+                     kv_cache_sf=case.kv_cache_sf, return_lse=True)
+    w.check_device_status()
+    ref, ref_lse = O.mla_decode(case.q, case.kv_cache, case.kv_cache_sf, case.block_tables, case.seq_lens, case.softmax_scale)
+    O.assert_parity(out, ref, "working CTAs")
+    live = torch.isfinite(ref_lse)
+    torch.testing.assert_close(lse.cpu()[live], ref_lse[live], atol=2e-3, rtol=1e-4)
