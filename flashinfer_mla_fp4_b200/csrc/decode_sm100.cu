@@ -61,6 +61,7 @@ namespace mla {
 namespace {
 
 constexpr int kWarpQK = 0, kWarpTMA = 1, kWarpPV = 2, kWarpTMA2 = 3;
+constexpr int kWarpPlan = 11;          // the softmax warp that makes the first plan while the dependency is waited for
 constexpr int kWarpSoftmax0 = 4;       // 8 warps; warp & 3 is the TMEM lane quarter the warp may access
 constexpr int kThreads = 384;          // 12 warps, three per scheduler
 constexpr int kSoftmaxWarps = 8;       // warp w works on TMEM lanes 32*(w%4).. and heads 32*(w/4)..
@@ -225,9 +226,9 @@ struct RoleState {
 // ------------------------------------------------------------------------------------------
 // Lane i looks at request base + i: a scan gives its place in the flat tile space, the overlap with the CTA's range its
 // segment, a ballot the segment's number.  The lengths are kept in shared memory (the latent ring is idle now) for the second
-// pass and for plan_still_valid; whole chunks of 32 requests outside the range are skipped with one reduction.  A sequential
+// pass and for start_work, which keeps its own reading in the other half; whole chunks of 32 requests outside the range are skipped with one reduction.  A sequential
 // walk by one thread took 2500 clk of every CTA's prologue.
-constexpr int kLensMax = int(kRing * kPairBytes / 4);
+constexpr int kLensMax = int(kRing * kPairBytes / 8);
 __device__ __forceinline__ int fresh_len(const DecodeParams& p, int i) {  // from L2: an earlier, speculative read must leave nothing in L1
   const int n = __ldcg(p.seq_lens + i);
   return n < p.seq_cap ? n : p.seq_cap;
@@ -292,7 +293,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     if (p.fused_merge) n = work_ctas(Tt, p.batch * p.groups, n);
     const flat_t cut = cta_lo(Tt, n, cta + (lane & 1));  // one division for both ends
     const flat_t lo = first_round ? __shfl_sync(0xffffffffu, cut, 0) : misc->next, hi = __shfl_sync(0xffffffffu, cut, 1);
-    int g = int(uint32_t(lo) / uint32_t(T));
+    int g = lo < T ? 0 : int(uint32_t(lo) / uint32_t(T));
 #pragma unroll 1
     for (flat_t run = flat_t(g) * T; cta < n && run < hi && !more; ++g) {
 #pragma unroll 1
@@ -342,15 +343,38 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
   __syncwarp();
 }
 
-// A plan made before the kernel ahead on the stream had ended stands if the lengths are what it was made from.
-__device__ __forceinline__ bool plan_still_valid(const DecodeParams& p, uint32_t smem, int lane) {
-  if (p.batch > kLensMax) return false;
-  const int* lens = reinterpret_cast<const int*>(smem_ptr(smem) + kOffKV);
-  bool same = true;
+// The end of the prologue: from here on the kernel reads what earlier kernels wrote (sequence lengths, q, the cache, the
+// workspace), and the plan is known.
+// The plan made before the wait stands if the lengths have not changed.  A CTA that starts late, on an SM that the kernel ahead
+// held to its end, finds nothing to wait for: there the lengths are read again while the plan is being made (1.8 us of code that
+// comes from L2 line by line).
+__device__ __forceinline__ void start_work(const DecodeParams& p, uint32_t smem, int warp, int lane) {
+  Misc* misc = misc_of(smem);
+  if (p.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
+  // Let a dependent kernel start its launch and prologue early; it still waits for the end of this whole grid.
+  if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (warp == kWarpTMA) {
+    bool stands = false;
+    if (p.pdl_wait) {
+      int* lens = reinterpret_cast<int*>(smem_ptr(smem) + kOffKV);
+      const int nb = p.batch <= kLensMax ? p.batch : 0;
 #pragma unroll 4
-  for (int i = lane; i < p.batch; i += 32) same &= fresh_len(p, i) == lens[i];
-  return __all_sync(0xffffffffu, same);
+      for (int i = lane; i < nb; i += 32) lens[kLensMax + i] = fresh_len(p, i);
+      ptx::bar_sync(8, 64);
+      bool same = true;
+#pragma unroll 1
+      for (int i = lane; i < nb; i += 32) same &= lens[kLensMax + i] == lens[i];
+      stands = __all_sync(0xffffffffu, same) && p.batch <= kLensMax && misc->Tt >= 0;
+    }
+    if (!stands) stage_segments(p, smem, lane, true, true);
+    ptx::fence_proxy_async_smem();  // the lengths give way to the first copies
+    __threadfence_block();
+    asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
+  } else {
+    ptx::bar_sync(2, kThreads);
+  }
 }
+
 // ------------------------------------------------------------------------------------------
 // role: TMA issue (warp 1: pair 0 and scales of every tile; warp 3: RoPE and pair 1)
 // ------------------------------------------------------------------------------------------
@@ -370,20 +394,31 @@ __device__ __forceinline__ int page_window(const DecodeParams& p, const Segment&
 // entry `i` of a window, in a uniform register
 __device__ __forceinline__ int uniform_page(int window, int i) { return __reduce_max_sync(0xffffffffu, int(threadIdx.x & 31) == (i & 31) ? window : -1); }
 __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, uint32_t which, const CUtensorMap* map_rope,
-                                         const CUtensorMap* map_lat, RoleState& st) {
-  const uint32_t nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
+                                         const CUtensorMap* map_lat, RoleState& st, bool starting) {
   const Segment* sg = segs_of(smem);
   const int lane = threadIdx.x & 31;
   const int ppt = kTile >> p.page_shift;  // pages per tile
   const uint32_t ps = uint32_t(p.page_size);
   bool ok = true;
+  // A kernel's instructions come from L2 line by line when it starts: the first tile's copies were in flight 1.8 us after the plan
+  // was known.  So while the plan is made, the code of a tile is gone through once with nothing to copy (`dry`: every copy
+  // predicated off, no page, no wait, no position taken).  With the plan made by another warp meanwhile: 16 requests of 200..4000
+  // tokens with 128 heads 17.0 -> 16.7 us, 61x300 11.7 -> 11.45, 8x32768 35.05 -> 34.65, 128 requests of 128..32768 88.6 -> 87.8.
+  bool dry = starting && p.pdl_wait;
+  st.slot = starting ? which : st.slot;
+  uint32_t nseg = 0;
+  if (!dry) {
+    if (starting) start_work(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+    nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
+  }
 #pragma unroll 1
-  for (uint32_t si = 0; si < nseg && ok; ++si, ++st.seg) {
-    Segment g = sg[si];
+  for (uint32_t si = 0; dry || (si < nseg && ok);) {
+    Segment g{0, 0, 0, 1, 0, -1};
+    if (!dry) g = sg[si];
     g.tile_begin = int(ptx::uniform_u32(uint32_t(g.tile_begin)));
     g.tile_end = int(ptx::uniform_u32(uint32_t(g.tile_end)));
     g.seq_len = int(ptx::uniform_u32(uint32_t(g.seq_len)));
-    const int total = ((g.seq_len - 1) >> p.page_shift) + 1;
+    const int total = dry ? ppt : ((g.seq_len - 1) >> p.page_shift) + 1;
     int cur = page_window(p, g, 0), nxt = page_window(p, g, 32), ahead = 64, at = 0;
 #pragma unroll 1
     for (int t = g.tile_begin; t < g.tile_end; ++t, ++st.it) {
@@ -392,7 +427,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
       int pg[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) pg[i] = uniform_page(cur, at + i);
-      const uint32_t e = ptx::elect_one();
+      const uint32_t e = ptx::elect_one() && !dry;
       auto for_pages = [&](auto copy) {  // copy(issue, page, index)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -445,6 +480,16 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
         nxt = page_window(p, g, ahead);
         ahead += 32;
       }
+    }
+    ++si;
+    ++st.seg;
+    if (dry) {
+      dry = false;
+      si = 0;
+      st = RoleState{};
+      st.slot = which;
+      start_work(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+      nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
     }
   }
   if (!ok && lane == 0) {  // let copies that were issued but never consumed land before exit (bounded; a refused page never does)
@@ -1521,8 +1566,14 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       misc->status = p.status;
       misc->n_slots = 0;
     }
-  } else if (warp == kWarpTMA) {
-    if (p.pdl_wait) stage_segments(p, smem, lane, true, false);  // a first plan, from the lengths as they are in memory
+  } else if (warp == kWarpPlan) {
+    asm volatile("bar.arrive 7, %0;" ::"n"(kThreads) : "memory");
+    if (p.pdl_wait) {  // a first plan, from the lengths as they are in memory; the TMA warp decides whether it stands
+      stage_segments(p, smem, lane, true, false);
+      ptx::fence_proxy_async_smem();
+      __threadfence_block();
+      asm volatile("bar.arrive 8, 64;" ::: "memory");
+    }
   } else if (warp == kWarpSoftmax0) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) sts_f32(smem + kOffNotes + 4 * (lane + 32 * i), __int_as_float(kNoScore));
@@ -1535,27 +1586,14 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     ptx::prefetch_tensormap(&map_lat);
   }
   ptx::tc_fence_before();
-  __syncthreads();
+  if (warp != kWarpPlan) ptx::bar_sync(7, kThreads);
+  RoleState st{};
+  if (warp != kWarpTMA && warp != kWarpTMA2) {  // (these two: in their role, after a first pass without effect)
+    start_work(p, smem, warp, lane);
+    if (tid == 0) MLA_STAMP(4, 1u, 1);
+  }
   ptx::tc_fence_after();
   const uint32_t tmem = ptx::uniform_u32(misc->tmem_base);
-  // From here on the kernel reads what earlier kernels wrote (sequence lengths, q, the cache, the workspace).
-  if (p.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
-  // Let a dependent kernel start its launch and prologue early; it still waits for the end of this whole grid.
-  if (p.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (tid == 0) MLA_STAMP(4, 1u, 1);
-
-  RoleState st{};
-  if (warp == kWarpTMA2) st.slot = 1;
-  // The plan made before the wait stands if the lengths have not changed.  The partition is walked by the warp that issues the
-  // first copies: it goes on to them without waiting for the others.
-  if (warp == kWarpTMA) {
-    if (!p.pdl_wait || misc->Tt < 0 || !plan_still_valid(p, smem, lane)) stage_segments(p, smem, lane, true, true);
-    ptx::fence_proxy_async_smem();  // the lengths give way to the first copies
-    __threadfence_block();
-    asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
-  } else {
-    ptx::bar_sync(2, kThreads);
-  }
   if (tid == 0) MLA_STAMP(4, 1u, 2);
   // Rounds: almost always exactly one; more only when a CTA's range spans more than kMaxSeg requests.
   bool first_round = true;
@@ -1584,7 +1622,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       }
       pv_role(smem, tmem, st);
     } else {
-      tma_role(p, smem, warp == kWarpTMA2 ? 1u : 0u, &map_rope, &map_lat, st);
+      tma_role(p, smem, warp == kWarpTMA2 ? 1u : 0u, &map_rope, &map_lat, st, first_round);
     }
     const int more = misc->more;
     if (!more && warp < kWarpSoftmax0) {
