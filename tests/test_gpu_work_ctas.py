@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
     ([3000], 64, 1),              # a grid of one
     ([130, 0, 5000, 1, 700], 64, None),   # the walk that shares best is two tiles long; requests without work
     ([16000], 16, None),          # many more CTAs than the rule wants
-    ([2500] * 30, 128, 7),        # rounds of many segments
+    ([2500] * 30, 128, 7),        # partials at both ends of most CTAs
+    ([130] * 131 + [700], 16, 2), # rounds of many segments: the partial in the first, none in the last, and the other way about
+    ([700] + [130] * 131, 16, 2),
 ])
 def test_any_number_of_working_ctas(lens, heads, max_ctas):
     if not torch.cuda.is_available():
