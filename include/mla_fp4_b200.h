@@ -101,7 +101,8 @@ typedef struct MlaFp4DecodeArgs {
   float softmax_scale, output_scale;
   int32_t out_dtype;   /* MLA_FP4_OUT_*    */
   int32_t kernel;      /* MLA_FP4_KERNEL_* */
-  int32_t num_ctas;    /* CTAs of the persistent decode grid; 0 = one per SM of the current device */
+  int32_t num_ctas;    /* CTAs of the persistent decode grid; 0 = one per SM of the current device.
+                          With few tiles the kernel lets only the first of them work */
   int32_t enable_pdl;  /* programmatic dependent launch: lets the next kernel on the stream start its
                           prologue while the decode kernel drains (0/1) */
   int32_t phase_mask;  /* two-kernel modes only: 0 = decode + combine; 1 = decode kernel only;
@@ -139,8 +140,8 @@ const char* mla_fp4_last_error(void);
 int mla_fp4_workspace_bytes(int32_t batch, int32_t q_len, int32_t num_heads, int32_t num_ctas,
                             size_t* bytes_out);
 
-/* Host copy of the work partition the decode kernel derives on the device: request b, head
-   group g and tile range of every segment of every CTA.  seq_lens is a HOST array.  Arrays
+/* Host copy of the work partition the decode kernel derives on the device, over num_ctas working
+   CTAs: request b, head group g and tile range of every segment of every CTA.  seq_lens is a HOST array.  Arrays
    hold up to max_segments entries; *num_segments receives the count (the required count when
    it exceeds max_segments).  Stands in for the reference's split heuristic + static tile
    scheduler (flashinfer cute_dsl/attention/scheduler/mla_persistent.py:137-282).  Host only. */
