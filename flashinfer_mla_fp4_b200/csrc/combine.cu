@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kCombThreads) combine_kernel(CombineParams p) 
   // all LSEs of the request in one round of independent loads
   for (int idx = tid; idx < ns * kGroupHeads; idx += kCombThreads) {
     const int i = idx >> 6, h = idx & 63;
-    lse_s[i][h] = slot_word_value(slot_words(ws, slot_list[i])[h]);
+    lse_s[i][h] = slot_lse(ws, slot_list[i])[h];
   }
   __syncthreads();
   if (tid < kGroupHeads) {
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kCombThreads) combine_kernel(CombineParams p) 
     const float inv = dsum > 0.f ? 1.f / dsum : 0.f;
     for (int i = 0; i < ns; ++i) {  // the LSEs become the weights (times the slot's fp16 scale)
       const float l = lse_s[i][tid];
-      lse_s[i][tid] = (l == -INFINITY) ? 0.f : exp2f(l - m) * inv * slot_word_value(slot_words(ws, slot_list[i])[kGroupHeads]);
+      lse_s[i][tid] = (l == -INFINITY) ? 0.f : exp2f(l - m) * inv * slot_scale(ws, slot_list[i])[0];
     }
     if (dchunk == 0 && p.lse && tid < heads_here) p.lse[row0 + tid] = (dsum > 0.f) ? (log2f(dsum) + m) : -INFINITY;
   }

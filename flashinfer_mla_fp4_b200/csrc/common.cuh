@@ -24,15 +24,14 @@ constexpr float kLog2e = 1.4426950408889634f;
 //   * partial O of slot s: normalised O as fp16 [8 head groups][512 dims][8 heads] divided by a per-slot
 //     scale (the decode kernel's lanes own one dim each: with this order a warp stores 32 dims x 8 heads =
 //     512 contiguous bytes at a time; with heads innermost over all 64 it would store 16 bytes every 128).
-//   * tail of slot s (528 bytes): 64 words of 8 bytes, a head's base-2 LSE (f32) and a tag, the same with that scale, the
-//     slot's flag (int32, see below) and an arrival counter (int32).  A tag is the generation of the step that wrote the word
-//     (0 in the two-kernel mode): whoever reads a word knows whether it is this step's, and no release, flag and second
-//     trip to L2 stand between the LSEs and the merge weights.
+//   * tail of slot s (272 bytes): the base-2 LSE of the 64 heads as f32, that scale (f32), the slot's flag
+//     (int32, see below), an arrival counter (int32) and the flag of the LSEs and the scale alone (int32).  The tails of all slots lie side by side, so the tails of the
+//     consecutive slots of one split request are one contiguous range (one bulk copy for a merging CTA).
 // The scale is 6 * max|token scale| * |output_scale| / 32768 rounded up to a power of two: an
 // upper bound of |O| mapped below the fp16 maximum, so the 11-bit partials can neither overflow nor
 // lose the small values (fp16 spans 29 binades below that bound).  Half the bytes of f32 partials.
 constexpr size_t kSlotOBytes = size_t(kLatent) * kGroupHeads * 2;
-constexpr size_t kSlotTailBytes = (kGroupHeads + 2) * 8;
+constexpr size_t kSlotTailBytes = kGroupHeads * sizeof(float) + 16;
 constexpr size_t kSlotBytes = kSlotOBytes + kSlotTailBytes;  // per slot, tail and partial O together
 constexpr float kSlotHalfRange = 32768.f;
 // A request can be split over at most this many CTAs (= the largest decode grid accepted).
@@ -56,10 +55,12 @@ MLA_HD int32_t* ws_started(void* ws) { return static_cast<int32_t*>(ws) + 2; }
 MLA_HD int32_t* ws_mode(void* ws) { return static_cast<int32_t*>(ws) + 3; }
 MLA_HD uint16_t* slot_o(void* ws, int slot) { return reinterpret_cast<uint16_t*>(static_cast<char*>(ws) + kWsFixedBytes + size_t(slot) * kSlotOBytes); }
 MLA_HD const uint16_t* slot_o(const void* ws, int slot) { return reinterpret_cast<const uint16_t*>(static_cast<const char*>(ws) + kWsFixedBytes + size_t(slot) * kSlotOBytes); }
-// words of a slot's tail: 64 LSEs, the slot scale
-MLA_HD uint64_t* slot_words(void* ws, int slot) { return reinterpret_cast<uint64_t*>(static_cast<char*>(ws) + kWsHeaderBytes + size_t(slot) * kSlotTailBytes); }
-MLA_HD const uint64_t* slot_words(const void* ws, int slot) { return reinterpret_cast<const uint64_t*>(static_cast<const char*>(ws) + kWsHeaderBytes + size_t(slot) * kSlotTailBytes); }
-MLA_HD int32_t* slot_flag(void* ws, int slot) { return reinterpret_cast<int32_t*>(slot_words(ws, slot) + kGroupHeads + 1); }
+MLA_HD float* slot_lse(void* ws, int slot) { return reinterpret_cast<float*>(static_cast<char*>(ws) + kWsHeaderBytes + size_t(slot) * kSlotTailBytes); }
+MLA_HD const float* slot_lse(const void* ws, int slot) { return reinterpret_cast<const float*>(static_cast<const char*>(ws) + kWsHeaderBytes + size_t(slot) * kSlotTailBytes); }
+MLA_HD float* slot_scale(void* ws, int slot) { return slot_lse(ws, slot) + kGroupHeads; }
+MLA_HD const float* slot_scale(const void* ws, int slot) { return slot_lse(ws, slot) + kGroupHeads; }
+MLA_HD int32_t* slot_flag(void* ws, int slot) { return reinterpret_cast<int32_t*>(slot_scale(ws, slot) + 1); }
+MLA_HD int32_t* slot_lse_flag(void* ws, int slot) { return slot_flag(ws, slot) + 2; }  // generation that last published the slot's LSEs and scale
 MLA_HD int32_t* slot_arrivals(void* ws, int slot) { return slot_flag(ws, slot) + 1; }  // of the request whose first writer owns the slot
 // element (dim, head) of a slot's partial O
 MLA_HD size_t slot_o_index(int dim, int head) { return (size_t(head >> 3) * kLatent + size_t(dim)) * 8 + size_t(head & 7); }
@@ -67,8 +68,6 @@ MLA_HD size_t slot_o_index(int dim, int head) { return (size_t(head >> 3) * kLat
 __host__ __device__ constexpr size_t workspace_bytes_for(int num_ctas) { return kWsFixedBytes + size_t(2) * size_t(num_ctas) * kSlotOBytes; }
 // power-of-two scale that maps `bound` (an upper bound of |O|) to at most kSlotHalfRange
 #ifdef __CUDACC__
-__device__ __forceinline__ uint64_t slot_word(float value, int tag) { return (uint64_t(uint32_t(tag)) << 32) | __float_as_uint(value); }
-__device__ __forceinline__ float slot_word_value(uint64_t w) { return __uint_as_float(uint32_t(w)); }
 __device__ __forceinline__ float slot_scale_for(float bound) {  // (round up to the next power of two: carry the mantissa into the exponent)
   return __uint_as_float((__float_as_uint(fmaxf(bound, 1e-30f) / kSlotHalfRange) + 0x7fffffu) & 0x7f800000u);
 }

@@ -89,8 +89,8 @@ constexpr uint32_t kOffM = kOffScale + kScaleStages * kTile * 4;          // [2]
 constexpr uint32_t kOffF = kOffM + 2 * kGroupHeads * 4;                   // [64] f32 rescale factor of a moved reference, [64] f32 by how much it moved
 constexpr uint32_t kOffNotes = kOffF + 2 * kGroupHeads * 4;               // [tile mod 3][64] s32 notes of beaten references; epilogue: [4][64] f32 row sums
 constexpr uint32_t kOffLinv = kOffNotes + 4 * kGroupHeads * 4;             // [64] f32 output factor; tail: 1/sum of the merge weights
-constexpr uint32_t kOffLse = kOffLinv + kGroupHeads * 4;                  // [64] f32, and the slot scale of a partial
-constexpr uint32_t kOffScMax = kOffLse + kGroupHeads * 4 + 16;            // [8] f32 per-warp largest token scale
+constexpr uint32_t kOffLse = kOffLinv + kGroupHeads * 4;                  // [64] f32
+constexpr uint32_t kOffScMax = kOffLse + kGroupHeads * 4;                 // [8] f32 per-warp largest token scale
 constexpr uint32_t kOffBars = kOffScMax + kSoftmaxWarps * 4;              // mbarriers (8 B each)
 // barrier indices
 __device__ __forceinline__ constexpr int bar_kv_full(int slot) { return slot; }            // a pair (and, pair 0, the tile's scales) has landed
@@ -199,12 +199,6 @@ __device__ __noinline__ void drain_wait(uint32_t smem, int idx, uint32_t parity)
 __device__ __forceinline__ int ld_acquire(const int32_t* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed(uint64_t* p, uint64_t v) { asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory"); }
-__device__ __forceinline__ uint64_t ld_relaxed(const uint64_t* p) {
-  uint64_t v;
-  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ int ld_relaxed(const int32_t* p) {
@@ -992,18 +986,7 @@ __device__ __noinline__ void write_final_bf16(const DecodeParams& p, uint32_t sm
 
 // Normalise O^T and write it to a split-KV partial slot, as fp16 divided by the slot scale (the factors in shared memory
 // include that division).  A block of 128 dims per round, rolled.
-// The LSEs and the scale of a partial, tagged, before O: the merge weights are made from them while O is on its way.  (Whoever
-// gets here has waited for a PV, so misc->gen is there.)
-__device__ __forceinline__ void write_words(const DecodeParams& p, uint32_t smem, int tid, int slot) {
-  if (tid >= kGroupHeads) return;
-  const int tag = p.fused_merge ? misc_of(smem)->gen : 0;
-  uint64_t* at = slot_words(p.workspace, slot) + tid;
-  st_relaxed(at, slot_word(lds_f32(smem + kOffLse + 4 * tid), tag));
-  if (tid == 0) st_relaxed(at + kGroupHeads, slot_word(lds_f32(smem + kOffLse + 4 * kGroupHeads), tag));  // the scale
-}
-__device__ __noinline__ void write_partial(const DecodeParams& p, uint32_t smem, uint32_t tmem_lane, int row, int half, int slot, bool all) {
-  write_words(p, smem, 128 * half + row, slot);
-  if (!all) return;
+__device__ __noinline__ void write_partial(const DecodeParams& p, uint32_t smem, uint32_t tmem_lane, int row, int half, int slot) {
   __half* so = reinterpret_cast<__half*>(slot_o(p.workspace, slot)) + slot_o_index(row, 32 * half);
 #pragma unroll 1
   for (int jb = 0; jb < kBlocks; ++jb, so += 128 * 8) {
@@ -1188,17 +1171,23 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
         const float sc_all = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(a.z, a.w)), fmaxf(fmaxf(b.x, b.y), fmaxf(b.z, b.w)));
         slot_scale_v = slot_scale_for(6.f * sc_all * fabsf(p.output_scale));
         fo *= __frcp_rn(slot_scale_v);  // a power of two: exact
-        if (tid == 0) sts_f32(smem + kOffLse + 4 * kGroupHeads, slot_scale_v);
       }
       const float lse = __log2f(Ls) + m;
       sts_f32(smem + kOffLinv + 4 * tid, __fdividef(fo, Ls));
       sts_f32(smem + kOffLse + 4 * tid, lse);
+      if (g.slot >= 0) {
+        slot_lse(p.workspace, g.slot)[tid] = lse;
+        if (tid == 0) slot_scale(p.workspace, g.slot)[0] = slot_scale_v;
+        // The LSEs and the scale of a CTA's last partial go out at once (publish): the merge weights are made from them while O is
+        // on its way.
+        if (p.fused_merge && si == nseg - 1 && !misc->more) asm volatile("bar.arrive 6, %0;" ::"n"(kGroupHeads + 32) : "memory");
+      }
     }
     (void)wait(smem, kBarPvDone, (st.it - 1) & 1);  // the PV of the last tile
     if (tid == 0) MLA_STAMP(3, st.it - 1, 3);
     ptx::tc_fence_after();
     if (!ptx::bar_or(1, kSoftmaxThreads, misc->abort != 0)) {  // (all or none: the writers meet at barriers)
-      if (g.slot >= 0) write_partial(p, smem, tmem_lane, row, half, g.slot, true);
+      if (g.slot >= 0) write_partial(p, smem, tmem_lane, row, half, g.slot);
       else if (p.out_dtype == MLA_FP4_OUT_BF16) {
         if (p.num_heads <= 32) write_final_bf16<1>(p, smem, tmem_lane, quarter, half, tid, g.b, g.g);
         else write_final_bf16<0>(p, smem, tmem_lane, quarter, half, tid, g.b, g.g);
@@ -1210,8 +1199,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
         if (p.out_dtype == MLA_FP4_OUT_F32) write_final<MLA_FP4_OUT_F32, false>(p, smem, tmem_lane, row, half, tid, g.b, g.g);
         else write_final<MLA_FP4_OUT_E4M3, false>(p, smem, tmem_lane, row, half, tid, g.b, g.g);
       }
-    } else if (g.slot >= 0) {  // (nobody is to wait for its words)
-      write_partial(p, smem, tmem_lane, row, half, g.slot, false);
     }
     ptx::tc_fence_before();
     __syncwarp();
@@ -1221,10 +1208,14 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
   }
   if (pending && p.fused_merge) {
     if (!misc->more) {  // (publish)
-      asm volatile("bar.arrive 6, %0;" ::"n"(kSoftmaxThreads + 32) : "memory");
+      asm volatile("bar.arrive 9, %0;" ::"n"(kSoftmaxThreads + 32) : "memory");
     } else {  // a round of whole segments but for the first: others follow
       ptx::bar_sync(1, kSoftmaxThreads);
-      if (tid == 0) st_release(slot_flag(p.workspace, slot_of(blockIdx.x, true)), misc->gen);
+      if (tid == 0) {
+        const int slot = slot_of(blockIdx.x, true);
+        st_release(slot_lse_flag(p.workspace, slot), misc->gen);
+        st_release(slot_flag(p.workspace, slot), misc->gen);
+      }
     }
   }
 }
@@ -1232,21 +1223,30 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
 // Publishing the partials, by the QK warp in the last round: the merging CTAs wait for these flags.  A release takes a microsecond,
 // until every store before it is in L2, and the softmax warps have the merge weights to make meanwhile.  One release for O of
 // both partials, after the last segment: nobody can use a partial before this CTA, itself a writer of the later request, is
-// done anyway.  The barrier orders the writers' stores before lane 0's release, and a release is cumulative.
-// With the softmax warps no longer waiting for it: 4x4096 tokens (64 heads) 14.0 -> 13.25 us, 8x32768 34.8 -> 33.85, 128 requests of
+// done anyway.  The barriers order the writers' stores before lane 0's release, and a release is cumulative.
+// With the softmax warps no longer waiting for either: 4x4096 tokens (64 heads) 14.0 -> 13.25 us, 8x32768 34.8 -> 33.85, 128 requests of
 // 128..32768 88.2 -> 87.2, 32 requests with 128 heads 40.9 -> 39.9.
+// (On the way, the commit for kBarDrain: nobody can have advanced the generation before this CTA counts itself out, which it does
+// after the drain.)
 __device__ __noinline__ void publish(const DecodeParams& p, uint32_t smem, int lane) {
-  Misc* misc = misc_of(smem);
-  const int nseg = misc->nseg;
-  if (nseg == 0) return;
+  const int nseg = misc_of(smem)->nseg;
   const Segment* sg = segs_of(smem);  // (only a round's first and last segment can be partial)
-  const int even = slot_of(blockIdx.x, true);
-  const bool head = sg[0].slot == even, tail = sg[nseg - 1].slot == even + 1;
+  const int even = slot_of(blockIdx.x, true), first = nseg > 0 ? sg[0].slot : -1, last = nseg > 0 ? sg[nseg - 1].slot : -1;
+  const bool head = first == even, tail = last == even + 1;
+  const int gen = head || tail ? ld_acquire(ws_generation(p.workspace)) + 1 : 0;
+  if (ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
+  __syncwarp();
   if (!head && !tail) return;
-  ptx::bar_sync(6, kSoftmaxThreads + 32);
+  if (last >= 0) {
+    ptx::bar_sync(6, kGroupHeads + 32);
+    if (lane == 0) st_release(slot_lse_flag(p.workspace, last), gen);
+    __syncwarp();
+  }
+  ptx::bar_sync(9, kSoftmaxThreads + 32);
   if (lane == 0) {
-    if (head) st_release(slot_flag(p.workspace, even), misc->gen);
-    if (tail) st_release(slot_flag(p.workspace, even + 1), misc->gen);
+    if (head && last != even) st_release(slot_lse_flag(p.workspace, even), gen);
+    if (head) st_release(slot_flag(p.workspace, even), gen);
+    if (tail) st_release(slot_flag(p.workspace, even + 1), gen);
     MLA_STAMP(4, 0u, 0);
   }
   __syncwarp();
@@ -1268,12 +1268,12 @@ __device__ __noinline__ void publish(const DecodeParams& p, uint32_t smem, int l
 // case whenever the grid has the GPU to itself for a moment.  A cooperative launch gave the same guarantee and cost 3.3 us
 // per step launched outside a graph (it does not overlap the kernel before it): 22.7 -> 19.4 us for 4 x 4096 tokens.
 constexpr int kMergeShared = 1, kMergeLast = 2;
-constexpr uint32_t kTailBytes = kGroupHeads * 4 + 16;                   // a slot's tail as staged: 64 LSEs, the slot scale, padding
+constexpr uint32_t kTailBytes = uint32_t(kSlotTailBytes);               // a slot's tail: 64 LSEs, the slot scale, the flag, an arrival counter, padding
 constexpr uint32_t kTailStage = kOffKV;                                 // staging: [slots][this CTA's bytes of a slot], then the tails
 constexpr uint32_t kTailRed = kOffScale - kThreads * 32;                // [384][8] f32: sums of a unit that several threads share
 constexpr uint32_t kTailStageBytes = kOffP - kTailStage;                // the KV ring, RoPE and Q; not P, where the last segment's output may still be in transit
 static_assert(kTailStageBytes >= 2 * (kSlotOBytes + kTailBytes), "two whole slots fit (a request cut once)");
-static_assert(kTailStageBytes >= kSlotOBytes + kSlotOBytes / 8 + kMaxSlots * kTailBytes, "a request cut 148 times fits");
+static_assert(kTailStageBytes >= kSlotOBytes + kSlotOBytes / 8 + kWsTailsBytes, "a request cut 148 times fits");
 
 // Requests without tokens: zero rows and LSE -inf (the sink's logit when there is a sink).
 __device__ __noinline__ void zero_empty_requests(const DecodeParams& p, int lane) {
@@ -1390,49 +1390,48 @@ __device__ __forceinline__ void store_unit(const float (&acc)[8], const float4& 
 
 // The merge weights w_i = 2^(lse_i - max) * slot scale of the 64 heads, and the inverse of their sum, by the eight softmax
 // warps: four lanes per head split the slots, butterflies give all four the results.  They are computed while the shares of the
-// slots are on their way: the tagged LSEs and scales are polled in L2 until they are this step's (in the last-writer form
-// they are).  Under a release and a flag of their own they cost a microsecond and a trip to L2 more: 1x16000 tokens 16.3 -> 15.5 us,
-// 7 ragged requests of up to 3000 tokens 13.2 -> 12.7, 4x4096 13.25 -> 13.1.  Four slots' loads in flight: with five the main loop spilled.
-__device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem, int tid, bool with_lse) {
+// slots are on their way: the LSEs come straight from L2, under flags of their own (shared form).
+__device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem, int tid, bool flags, bool with_lse) {
   Misc* misc = misc_of(smem);
   const int ns = misc->n_slots;
   const uint32_t tails = smem + kTailStage + uint32_t(ns) * (uint32_t(misc->unit1 - misc->unit0) * 16u);
   const int h = tid >> 2, j = tid & 3;
   const uint32_t col = tails + 4u * uint32_t(h);
-  const uint32_t gen = uint32_t(misc->gen), polls = misc->polls;
-  float mx = -INFINITY;
+  if (flags) {
+    const int lane = tid & 31, gen = misc->gen;
+    const uint32_t polls = misc->polls;
+    bool all = false;
 #pragma unroll 1
-  for (int i0 = j; i0 - j < ns; i0 += 16) {  // four slots' loads in flight together
-    const uint64_t* tail[4];
-    uint64_t l[4], sc[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) tail[k] = slot_words(p.workspace, int(lds_u32(smem + kOffTail + 4u * uint32_t(min(i0 + 4 * k, ns - 1)))));
-    bool up = false;
-#pragma unroll 1
-    for (uint32_t it = 0; it < polls && !up; ++it) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        l[k] = ld_relaxed(tail[k] + h);
-        sc[k] = ld_relaxed(tail[k] + kGroupHeads);  // the slot scale
-      }
-      up = true;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) up &= uint32_t(l[k] >> 32) == gen && uint32_t(sc[k] >> 32) == gen;
-      up = __all_sync(0xffffffffu, up);
+    for (uint32_t it = 0; it < polls && !all; ++it) {
+      bool up = true;
+      for (int i = lane; i < ns; i += 32) up &= ld_acquire(slot_lse_flag(p.workspace, int(lds_u32(smem + kOffTail + 4u * uint32_t(i))))) == gen;
+      all = __all_sync(0xffffffffu, up);
       if (__any_sync(0xffffffffu, misc->abort)) break;
     }
-    if (!up && (tid & 31) == 0 && !misc->abort) flag_timeout(smem, 101, uint32_t(ns));
+    if (!all && lane == 0 && !misc->abort) flag_timeout(smem, 101, uint32_t(ns));
+    __syncwarp();
+  }
+  float mx = -INFINITY;
+#pragma unroll 1
+  for (int i0 = j; i0 < ns; i0 += 20) {  // five slots' loads in flight together
+    const float* tail[5];
+    float l[5], sc[5];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 0; k < 5; ++k) tail[k] = slot_lse(p.workspace, int(lds_u32(smem + kOffTail + 4u * uint32_t(min(i0 + 4 * k, ns - 1)))));
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      l[k] = __ldcg(tail[k] + h);
+      sc[k] = __ldcg(tail[k] + kGroupHeads);  // the slot scale
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
       const int i = i0 + 4 * k;
-      const float v = slot_word_value(l[k]);
-      mx = fmaxf(mx, v);  // (a repeated last slot changes nothing)
+      mx = fmaxf(mx, l[k]);  // (a repeated last slot changes nothing)
       if (i < ns) {
-        sts_f32(col + uint32_t(i) * kTailBytes, v);
-        if (h == 0) sts_f32(tails + uint32_t(i) * kTailBytes + 4u * kGroupHeads, slot_word_value(sc[k]));
+        sts_f32(col + uint32_t(i) * kTailBytes, l[k]);
+        if (h == 0) sts_f32(tails + uint32_t(i) * kTailBytes + 4u * kGroupHeads, sc[k]);
       }
     }
-    if (!up) break;
   }
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
@@ -1562,7 +1561,7 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
       }
       __syncthreads();
       if (tid < 32 * kFetchWarps) tail_fetch(p, smem, tid >> 5, tid & 31, false);
-      else if (tid >= 128) merge_weights(p, smem, tid - 128, r == 0);
+      else if (tid >= 128) merge_weights(p, smem, tid - 128, false, r == 0);
       __syncthreads();
       tail_merge(p, smem, tid, parity);
       __syncthreads();
@@ -1643,7 +1642,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       softmax_role<kSoftCap>(p, smem, tmem, tid - 32 * kWarpSoftmax0, st);
       if (p.fused_merge && !misc->more && misc->n_slots > 0) {
         ptx::bar_sync(5, kThreads - 32);
-        if (misc->mode == kMergeShared) merge_weights(p, smem, tid - 32 * kWarpSoftmax0, misc->rank == 0);
+        if (misc->mode == kMergeShared) merge_weights(p, smem, tid - 32 * kWarpSoftmax0, true, misc->rank == 0);
         if (tid == 128) MLA_STAMP(4, 0u, 3);
       }
     } else if (warp == kWarpQK) {
@@ -1651,7 +1650,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     } else if (warp == kWarpPV) {
       if (first_round && p.fused_merge) {  // (the two-kernel modes leave all this to the combine kernel); the first P is far away
         // The generation of this step: one more than that of the last completed step.  No CTA of this step can have advanced it
-        // yet (that takes every CTA of the grid to have finished).  Whoever uses it has waited for a PV of this warp.
+        // yet (that takes every CTA of the grid to have finished).
         if (lane == 0) {
           atomicAdd(ws_started(p.workspace), 1);
           misc->gen = ld_acquire(ws_generation(p.workspace)) + 1;
@@ -1669,7 +1668,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       // a commit covers the MMAs of the thread that executes it), then these warps, idle from here on, publish this CTA's
       // partials and fetch those of the request it merges while the softmax warps finish with its own.
       const bool publishes = warp == kWarpQK && p.fused_merge;
-      if ((warp == kWarpQK || warp == kWarpPV) && ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
+      if (((warp == kWarpQK && !publishes) || warp == kWarpPV) && ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
       __syncwarp();
       if (publishes) {
         publish(p, smem, lane);

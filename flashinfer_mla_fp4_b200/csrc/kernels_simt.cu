@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(256) fp32_check_kernel(DecodeParams p) {
         so[slot_o_index(tid, h)] = __float2half_rn(o0[h] * inv);
         so[slot_o_index(tid + 256, h)] = __float2half_rn(o1[h] * inv);
       }
-      if (tid == 0) slot_words(p.workspace, s.slot)[kGroupHeads] = slot_word(sscale, 0);
-      if (tid < kGroupHeads) slot_words(p.workspace, s.slot)[tid] = slot_word(log2f(l_s[tid]) + m_s[tid], 0);
+      if (tid == 0) slot_scale(p.workspace, s.slot)[0] = sscale;
+      if (tid < kGroupHeads) slot_lse(p.workspace, s.slot)[tid] = log2f(l_s[tid]) + m_s[tid];
     }
   }
 }

@@ -50,7 +50,7 @@ extern "C" {
 
 /* The workspace starts with a header of this many bytes (the generation of the last decode step
    that completed on it and a count of the CTAs that have finished the running one), followed by
-   296 slot tails of 528 bytes (64 tagged LSEs, the slot scale, and a flag: the generation that last
+   296 slot tails of 272 bytes (64 LSEs, the slot scale, and a flag: the generation that last
    published the slot) and then the partial slots of 65536 bytes.  Header and tails must be zero
    before the first decode step on that workspace (mla_fp4_workspace_init); completed steps keep
    them consistent by themselves.  After a step that reported MLA_FP4_ERR_DEVICE_TIMEOUT call
@@ -254,7 +254,7 @@ int mla_fp4_step_metadata(const int32_t* block_tables, int64_t block_table_strid
 /* Largest decode grid the allocation-free variant below accepts, and the bytes of device memory
    its built-in scratch occupies on every GPU that loads the library (until the process exits). */
 #define MLA_FP4_STATIC_MAX_CTAS 148
-#define MLA_FP4_STATIC_SCRATCH_BYTES (MLA_FP4_WORKSPACE_HEADER_BYTES + 2 * MLA_FP4_STATIC_MAX_CTAS * 66064)
+#define MLA_FP4_STATIC_SCRATCH_BYTES (MLA_FP4_WORKSPACE_HEADER_BYTES + 2 * MLA_FP4_STATIC_MAX_CTAS * 65808)
 
 /* No counterpart in the reference.  Same decode step as mla_fp4_decode, for callers that may not
    allocate device memory and have no workspace buffer to lend: plugins running inside an engine
