@@ -235,17 +235,18 @@ __device__ __forceinline__ int fresh_len(const DecodeParams& p, int i) {  // fro
   return n < p.seq_cap ? n : p.seq_cap;
 }
 // How many CTAs share the work when the decode kernel merges by itself.  A CTA more shortens everybody's walk, but every partial of a
-// request is one more for all its writers to weigh and sum: with Tt tiles over n CTAs, 1.25 us * Tt / n + 0.07 us * n / pairs,
-// which is least at n = 4.2 sqrt(Tt * pairs).  Then the longest walk k is kept and n lowered as far as k allows: CTAs
+// request is one more for all its writers to weigh and sum: with Tt tiles over n CTAs, 1.25 us * Tt / n + 0.05 us * n / pairs,
+// which is least at n = 5 sqrt(Tt * pairs).  Then the longest walk k is kept and n lowered as far as k allows: CTAs
 // that cannot shorten the longest walk only add partials, and a CTA without work does not hold the step up when it starts late.
-// On 148 SMs, 64 heads, before -> after: 1x16000 tokens 21.3 -> 17.5 us, 1x32768 22.9 -> 19.5, 4x4096 15.1 -> 14.1, 2x1024 14.0 -> 12.0;
-// beyond five tiles a CTA the whole grid works (8x32768, 128 requests).  Approximate arithmetic will do: every CTA takes the same
-// steps, and any 1 <= n <= Tt is right.
+// On 148 SMs, 64 heads, the whole grid -> as many as this: 1x16000 tokens 21.3 -> 17.5 us, 1x32768 22.9 -> 19.5, 4x4096 15.1 -> 14.1,
+// 2x1024 14.0 -> 12.0; beyond five tiles a CTA the whole grid works (8x32768, 128 requests).  4 / 5 / 6 sqrt(Tt * pairs), with today's
+// merge: 1x32768 18.45 / 17.2 / 18.2, 1x8192 14.15 / 13.3 / 13.3, 2x32768 19.6 / 18.6 / 18.6, 4x4096 13.2 / 13.2 / 13.55, 2x16000 17.5 /
+// 17.4 / 15.8.  Approximate arithmetic will do: every CTA takes the same steps, and any 1 <= n <= Tt is right.
 __device__ __forceinline__ int work_ctas(flat_t Tt, int pairs, int n) {
   if (Tt > 5 * n && pairs > 1) return n;  // the whole grid, and next to nothing to gain from the rounding
   const float tiles = float(Tt);
   float best, r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(best) : "f"(16.f * tiles * float(pairs)));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(best) : "f"(25.f * tiles * float(pairs)));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fminf(float(n), best)));
   const float k = float(__float2int_ru(tiles * r - 1e-3f));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(k));
