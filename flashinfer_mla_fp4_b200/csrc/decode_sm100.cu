@@ -822,7 +822,8 @@ __device__ __forceinline__ void note_beaten(uint32_t notes, const uint64_t (&y2)
   const int b = __float_as_int(mine);
   asm volatile("red.shared.max.s32 [%0], %1;" ::"r"(notes + 4 * lane), "r"(b ^ ((b >> 31) & 0x7fffffff)) : "memory");
 }
-// m += top - shift and f = 2^-(top - shift) for the heads that were beaten, f = 1 for all others.
+// m += top - shift and f = 2^-(top - shift) for the heads that were beaten, f = 1 for all others.  In the first tile of a segment
+// there are no sums yet, and f is 0: a first top far below zero would make it infinite, and infinity times the empty sums a NaN.
 __device__ __forceinline__ void refresh_beaten(uint32_t smem, uint32_t notes, uint32_t cur, bool first, int half, int lane) {
   const uint32_t at = 4u * (32u * uint32_t(half) + uint32_t(lane));
   const int b = int(lds_u32(notes + 4 * lane));
@@ -830,7 +831,7 @@ __device__ __forceinline__ void refresh_beaten(uint32_t smem, uint32_t notes, ui
   const bool beaten = first || top > kPShift + kLazyThreshold;
   const float d = beaten ? top - kPShift : 0.f;
   sts_f32(smem + kOffM + 256 * (cur ^ 1u) + at, lds_f32(smem + kOffM + 256 * cur + at) - d);
-  sts_f32(smem + kOffF + at, beaten ? ptx::ex2(-d) : 1.f);
+  sts_f32(smem + kOffF + at, first ? 0.f : (beaten ? ptx::ex2(-d) : 1.f));
   sts_f32(smem + kOffF + 256 + at, d);
   __syncwarp();
 }
