@@ -74,9 +74,8 @@ constexpr int kPairBytes = 2 * kBlockBytes;
 constexpr int kScaleStages = 4;            // per-token scales; a stage is free when the pair slots of its tile come round (see tma_role)
 constexpr int kMaxSeg = 16;                // segments staged per round
 constexpr float kPShift = 4.0f;            // P' = 2^(y - M + 4): keeps the E4M3 lo term out of the subnormals
-constexpr float kLazyThreshold = 4.75f;    // the reference is refreshed only when beaten by 2^4.75: P' <= 2^8.75 = 430.5, just inside
-                                           // E4M3 (448).  A refresh costs a CTA a tile and a half, and the CTAs that had one set the
-                                           // kernel's end; at 2^4 the north-star data had eight of them, at 2^4.75 none.
+constexpr float kLazyThreshold = 4.75f;    // the references move only when one is beaten by 2^4.75: P' <= 2^8.75 = 430.5, just inside E4M3 (448)
+constexpr float kNoteMargin = 2.0f;        // a warp whose best token beats its reference by 2^2 has its say in how they move (note_tops)
 
 // shared memory map (bytes from a 1024-aligned base)
 constexpr uint32_t kOffKV = 0;                                            // [5][2][16384]
@@ -800,16 +799,22 @@ __device__ __forceinline__ float exponents(const SoftmaxTile& t, uint64_t (&y2)[
   return mx;
 }
 
-// The references that tokens of a tile beat by more than the lazy threshold.  A warp with such a token notes the largest
-// y + log2|scale_t| of each of its heads (as integers that compare like the floats), before the vote of the softmax warps;
-// after it every warp works out the new references and factors of its 32 heads from the notes (the four warps of a half write
-// the same values): no barrier but the vote.  The first tile of a segment is the same with references of zero and every warp
-// noting.  Notes go round three places: those of tile t-1 are cleared after the vote of tile t, when nobody reads them any
-// more, and used again by tile t+2, which no warp reaches before all have voted in tile t+1.
+// How the references move.  A head's best token should have a P' of exactly 2^kPShift, which has no rounding error: that counts
+// where few tokens carry the weight.  So when a token beats a reference by more than the lazy threshold, not its head alone is
+// moved, but every head to the top of the tokens that the warps have noted: each warp with a token that beats some reference by
+// 2^kNoteMargin, or by the threshold, notes the largest y + log2|scale_t| of each of its heads (as integers that compare like the
+// floats) before the vote of the softmax warps.  After it every warp works out the new references and factors of its 32 heads from the
+// notes (the four warps of a half write the same values): no barrier but the vote.  The first tile of a segment is the same with
+// references of zero and every warp noting.  Notes go round three places: those of tile t-1 are cleared after the vote of tile t,
+// when nobody reads them any more, and used again by tile t+2, which no warp reaches before all have voted in tile t+1.
+// Error against 64 bits (FP32 output) and time with the beaten heads alone moved -> this: 2x256 tokens, 16 heads, logits eight times as
+// large 2.97e-4 -> 1.81e-4, 8.43 -> 8.46 us; 128 requests of 128..32768 tokens with outliers 2.14e-4 -> 1.92e-4, 93.9 -> 95.2 us.  All heads
+// by the tokens of all warps that are above a reference: as exact, with those notes before the vote (a margin of 0) 95.9 us
+// and 2x131072 tokens, 128 heads, q_len 2 89.8 -> 93 us; behind the vote and another barrier 104.4 us.
 // (With heavy-tailed token scales a reference is beaten in every other tile, mostly by more than FP32 exponentials could hold:
 // recomputing such tiles from the scores took 1100 clk each.)
 constexpr int kNoScore = int(0x80000000u);
-__device__ __forceinline__ void note_beaten(uint32_t notes, const uint64_t (&y2)[kPairs], float lg, int lane) {
+__device__ __forceinline__ void note_tops(uint32_t notes, const uint64_t (&y2)[kPairs], float lg, int lane) {
   float mine = -INFINITY;  // lane i: head i of the warp's 32
 #pragma unroll
   for (int i = 0; i < kPairs; ++i) {
@@ -822,16 +827,16 @@ __device__ __forceinline__ void note_beaten(uint32_t notes, const uint64_t (&y2)
   const int b = __float_as_int(mine);
   asm volatile("red.shared.max.s32 [%0], %1;" ::"r"(notes + 4 * lane), "r"(b ^ ((b >> 31) & 0x7fffffff)) : "memory");
 }
-// m += top - shift and f = 2^-(top - shift) for the heads that were beaten, f = 1 for all others.  In the first tile of a segment
-// there are no sums yet, and f is 0: a first top far below zero would make it infinite, and infinity times the empty sums a NaN.
-__device__ __forceinline__ void refresh_beaten(uint32_t smem, uint32_t notes, uint32_t cur, bool first, int half, int lane) {
+// m += d and f = 2^-d with d = top - shift, where that is positive; d = 0 and f = 1 for all other heads.  In the first tile of a
+// segment d = top - shift whatever its sign, and f is 0: there are no sums yet, and a first top far below zero would make f
+// infinite and the empty sums NaN.
+__device__ __forceinline__ void refresh_references(uint32_t smem, uint32_t notes, uint32_t cur, bool first, int half, int lane) {
   const uint32_t at = 4u * (32u * uint32_t(half) + uint32_t(lane));
   const int b = int(lds_u32(notes + 4 * lane));
-  const float top = __int_as_float(b ^ ((b >> 31) & 0x7fffffff));  // (a NaN where there is no note)
-  const bool beaten = first || top > kPShift + kLazyThreshold;
-  const float d = beaten ? top - kPShift : 0.f;
+  const float above = __int_as_float(b ^ ((b >> 31) & 0x7fffffff)) - kPShift;
+  const float d = first ? above : fmaxf(above, 0.f);
   sts_f32(smem + kOffM + 256 * (cur ^ 1u) + at, lds_f32(smem + kOffM + 256 * cur + at) - d);
-  sts_f32(smem + kOffF + at, first ? 0.f : (beaten ? ptx::ex2(-d) : 1.f));
+  sts_f32(smem + kOffF + at, first ? 0.f : ptx::ex2(-d));
   sts_f32(smem + kOffF + 256 + at, d);
   __syncwarp();
 }
@@ -1064,8 +1069,8 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       ptx::tc_fence_after();
 
       // The exponents are taken with the reference as it stands, which holds unless some score beat it by more than the lazy
-      // threshold (P' would leave the E4M3 range).  Then the references of the heads concerned are moved, and the exponents, the
-      // sums and, below, O^T follow.
+      // threshold (P' would leave the E4M3 range).  Then the references are moved, and the exponents, the sums and, below, O^T
+      // follow.
       uint64_t e2[kPairs];
       t.negm = smem + kOffM + 256 * st.m + 4 * kHalfHeads * half;
       const float mx = exponents<kSoftCap>(t, e2);
@@ -1073,14 +1078,14 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar_addr(smem, bar_s_empty(s)));
       const bool beaten = first || mx + lg > kPShift + kLazyThreshold;
-      const bool note_now = __any_sync(0xffffffffu, beaten);
+      const bool note = __any_sync(0xffffffffu, first || mx + lg > kPShift + kNoteMargin);
       const uint32_t here = notes + 256 * st.mod3;
-      if (note_now) note_beaten(here, e2, lg, lane);
+      if (note) note_tops(here, e2, lg, lane);
       const bool moved = ptx::bar_or(1, kSoftmaxThreads, beaten);
       if (noted) sts_f32(notes + 256 * (st.mod3 == 0 ? 2 : st.mod3 - 1) + 4 * lane, __int_as_float(kNoScore));
-      noted = note_now;
+      noted = note;
       if (moved) {
-        refresh_beaten(smem, here, st.m, first, half, lane);
+        refresh_references(smem, here, st.m, first, half, lane);
         st.m ^= 1u;
         const uint32_t f = smem + kOffF + 4 * kHalfHeads * half;
         const uint64_t minus = pack2(-1.f, -1.f);
