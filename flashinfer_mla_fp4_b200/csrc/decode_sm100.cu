@@ -1460,8 +1460,9 @@ __device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem,
   }
 }
 
-// out = sum_i w_i * O_i / sum, over the staged shares, in slot order whatever the order of arrival (bit-reproducible).  All
-// threads of the CTA; the weights are there.
+// out = sum_i w_i * O_i / sum, over the staged shares, in an order that depends on the number of slots and units alone and not on
+// the order of arrival: both forms cut the units into the same shares, so they agree to the bit.  All threads of the CTA; the
+// weights are there.
 __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, int tid, uint32_t parity) {
   Misc* misc = misc_of(smem);
   const int ns = misc->n_slots;
@@ -1546,7 +1547,7 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
     if (__syncthreads_or(misc->abort)) return;
     if (tid < 32) plan_merge(smem, which, tid);
     __syncthreads();
-    const int ns = misc->n_slots, part = max(ns - 1, 1);
+    const int ns = misc->n_slots, part = misc->n_part;  // (the shares of the shared form, so that both sum in the same order)
     if (tid == 0) {
       int32_t* arrivals = slot_arrivals(p.workspace, int(lds_u32(smem + kOffTail)));
       __threadfence();  // this CTA's partial (published after a barrier of its writers) before the count

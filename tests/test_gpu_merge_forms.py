@@ -39,3 +39,29 @@ def test_both_merge_forms(lens, heads, page_size, max_ctas):
         torch.testing.assert_close(lse.cpu()[live], ref_lse[live], atol=2e-3, rtol=1e-4)
     for i, j in ((0, 3), (1, 2)):
         assert torch.equal(got[i][0], got[j][0]) and torch.equal(got[i][1], got[j][1])
+
+
+@pytest.mark.parametrize("lens,heads", [
+    ([16384], 64),       # 43 partials: several threads per unit, a different number of them in shares of 42 and of 43
+    ([4500], 64),        # 22 or so
+    ([115000], 40),      # every CTA
+    ([2500, 6000, 900], 64),
+])
+def test_both_merge_forms_agree_to_the_bit(lens, heads):
+    """Which form runs depends on what else holds the GPU at that moment: the result must not."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("forms", lens, heads, 64, seed=lens[0], device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=heads, page_size=64, out_dtype=torch.float32)
+    got = []
+    for mask in (0, 4):
+        w._phase_mask = mask
+        got.append(w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale,
+                         kv_cache_sf=case.kv_cache_sf, return_lse=True))
+        torch.cuda.synchronize()
+        w.check_device_status()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
