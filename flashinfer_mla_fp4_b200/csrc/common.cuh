@@ -45,7 +45,8 @@ constexpr int kMaxSlots = 2 * kMaxCombineSlots;
 // generation g = header[0] + 1.  A writer stamps the flag of a slot with g once the slot's bytes are
 // visible; a merger waits until the flags of a request's slots equal g.  Flags of earlier steps never
 // match, so nothing has to be reset between steps, and a step that gave up on a wait leaves the workspace
-// consistent (its last CTA still advances the generation).  Each flag has a cache line of its own.
+// consistent: its CTAs publish and count themselves in and out all the same, and the last one advances the generation.
+// Each flag has a cache line of its own.
 constexpr size_t kWsHeaderBytes = MLA_FP4_WORKSPACE_HEADER_BYTES;
 constexpr size_t kWsTailsBytes = size_t(kMaxSlots) * kSlotTailBytes;
 constexpr size_t kWsFixedBytes = kWsHeaderBytes + kWsTailsBytes;  // what mla_fp4_workspace_init zeroes

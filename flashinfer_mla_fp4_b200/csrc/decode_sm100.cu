@@ -1538,13 +1538,13 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
 }
 
 // The last-writer form: for each request this CTA wrote a partial of, count it in; the last to arrive merges it, share by share.
+// A CTA that has given up counts itself in all the same: the counters are back to zero after every step, whatever became of it.
 __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem, int tid) {
   Misc* misc = misc_of(smem);
   uint32_t parity = 0;
 #pragma unroll 1
   for (int which = 0; which < 2; ++which) {
     if (misc->merge[which].vtiles == 0) continue;
-    if (__syncthreads_or(misc->abort)) return;
     if (tid < 32) plan_merge(smem, which, tid);
     __syncthreads();
     const int ns = misc->n_slots, part = misc->n_part;  // (the shares of the shared form, so that both sum in the same order)
@@ -1559,6 +1559,7 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
     if (!misc->last) continue;
 #pragma unroll 1
     for (int r = 0; r < part; ++r, parity ^= 1u) {
+      if (__syncthreads_or(misc->abort)) break;
       if (tid == 0) {
         misc->unit0 = (4096 * r) / part;
         misc->unit1 = (4096 * (r + 1)) / part;

@@ -50,11 +50,11 @@ extern "C" {
 
 /* The workspace starts with a header of this many bytes (the generation of the last decode step
    that completed on it and a count of the CTAs that have finished the running one), followed by
-   296 slot tails of 272 bytes (64 LSEs, the slot scale, and a flag: the generation that last
-   published the slot) and then the partial slots of 65536 bytes.  Header and tails must be zero
-   before the first decode step on that workspace (mla_fp4_workspace_init); completed steps keep
-   them consistent by themselves.  After a step that reported MLA_FP4_ERR_DEVICE_TIMEOUT call
-   mla_fp4_workspace_init again. */
+   296 slot tails of 272 bytes (64 LSEs, the slot scale, the generation that last published the
+   slot, an arrival counter, the generation that last published the LSEs and the scale) and then
+   the partial slots of 65536 bytes.  Header and tails must be zero before the first decode step on
+   that workspace (mla_fp4_workspace_init); every step whose kernel returns leaves them consistent,
+   one that reported MLA_FP4_ERR_DEVICE_TIMEOUT included. */
 #define MLA_FP4_WORKSPACE_HEADER_BYTES 2048
 
 /* input element types of mla_fp4_cache_write */

@@ -65,3 +65,41 @@ def test_both_merge_forms_agree_to_the_bit(lens, heads):
         torch.cuda.synchronize()
         w.check_device_status()
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+def test_a_step_that_gave_up_leaves_the_last_writer_form_consistent():
+    """One block-table entry of a split request names a page outside the pool (the copy is never issued and a bounded wait runs out).
+    The CTA that gives up counts itself into its requests all the same, so every arrival counter is back to zero: the next step on
+    the same workspace, which nothing has initialised since, must not merge before the last partial is there."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, _cabi, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("gave up", [3000, 5000], 64, 64, seed=21, device=dev)
+    ws = torch.empty(32 << 20, dtype=torch.int8, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(ws)
+    w.plan(num_heads=64, page_size=64)
+    w._phase_mask = 4
+    head = _cabi.WORKSPACE_HEADER_BYTES
+    tails = ws[head: head + 296 * 272].view(torch.int32).reshape(296, 68)  # 64 LSEs, scale, flag, arrival counter, flag of the LSEs
+
+    def step(q, tables):
+        out = w.run(q, case.kv_cache, tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
+        torch.cuda.synchronize()
+        return out
+
+    other = case.q.flip(2).contiguous()  # (the slots hold the partials of the step before: the queries have to differ)
+    good = [step(q, case.block_tables) for q in (case.q, other)]
+    w.check_device_status()
+    bad = case.block_tables.clone()
+    bad[1, 40] = case.kv_cache.shape[0] + 5
+    w._wait_polls = 2000
+    step(case.q, bad)
+    assert w.device_status()[0] == _cabi.ERR_DEVICE_TIMEOUT
+    assert int(tails[:, 66].abs().max()) == 0
+    w._wait_polls = 0
+    w._status.zero_()
+    for q, want in ((case.q, good[0]), (other, good[1]), (case.q, good[0])):
+        assert torch.equal(step(q, case.block_tables), want)
+    assert w.device_status()[0] == 0
