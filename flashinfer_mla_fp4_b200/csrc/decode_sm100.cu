@@ -553,7 +553,7 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
       const uint32_t it = st.it, s64 = 64u * (it & 1);
       // S of this stage has been read by the softmax of tile it-2; PV of tile it-2, if of this segment, is half issued; the RoPE
       // bytes of this tile have landed.  (The two issue barriers cannot run ahead of the warp that waits for them: inside a
-      // segment PV(it-1) waits for this tile's QK^T, and QK^T of it+1 for PV(it-1).)
+      // segment PV(it-1) waits for this tile's QK^T, and QK^T of it+1 for PV(it-1).  tests/test_issue_order.py tries every interleaving.)
       if (it >= 2) ok = wait(smem, bar_s_empty(it & 1), ((it >> 1) - 1) & 1);
       if (t >= 2) ok = ok && wait(smem, kBarPvIssued, it & 1);
       ok = ok && wait(smem, kBarRopeFull, it & 1);
@@ -578,8 +578,8 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
             ptx::umma_f8(e, tmem + kColSLat + s64, kv.at(a + j * (kBlockBytes >> 4) + 2 * ks), q_lat.at(b + j * ((kGroupHeads * 128) >> 4) + 2 * ks),
                          kIdescQK, (pr | j | ks) ? 1u : 0u);
         if (pr && e) {
+          ptx::mbar_arrive(bar_addr(smem, kBarQkIssued));  // (first: who has seen what follows from S finds it done)
           ptx::umma_commit(bar_addr(smem, bar_s_full(it & 1)));
-          ptx::mbar_arrive(bar_addr(smem, kBarQkIssued));
         }
         __syncwarp();
         st.advance(1);
@@ -610,9 +610,11 @@ __device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState&
     if (st.seg >= 1 && !wait(smem, kBarOFree, (st.seg - 1) & 1)) return;  // O^T of the previous segment has been read out
 #pragma unroll 1
     for (uint32_t t = 0; t < n; ++t, ++st.it) {
-      // QK^T of the segment's next tile has been issued (so it lies ahead of this PV in the queue of the tensor pipe)
-      if (t + 1 < n && !wait(smem, kBarQkIssued, (st.it + 1) & 1)) return;
+      // P of this tile, and QK^T of the segment's next tile has been issued (so it lies ahead of this PV in the queue of the tensor
+      // pipe).  In this order: P says that QK^T of this tile was reported as issued, so the phase before the one waited for is over and
+      // its parity cannot be taken for an older phase's.  (The other way round, tile 0 found the barrier untouched and did not wait.)
       if (!wait(smem, kBarPFull, st.it & 1)) return;
+      if (t + 1 < n && !wait(smem, kBarQkIssued, (st.it + 1) & 1)) return;
       MLA_STAMP(0, st.it, 2);
       ptx::tc_fence_after();
       const uint32_t e = ptx::elect_one(), keep = t ? 1u : 0u;
