@@ -1370,10 +1370,11 @@ __device__ __noinline__ void tail_fetch(const DecodeParams& p, uint32_t smem, in
     bool done = i >= ns;
 #pragma unroll 1
     for (uint32_t it = 0; it < polls; ++it) {
-      // acquire: the slot's bytes, written before the flag, are read after it.  The copies read them from L2, where the
-      // writer's release put them: no proxy fence is needed for that (a full one here cost microseconds).
+      // acquire: the slot's bytes, written before the flag, are read after it; they were written by ordinary stores and the copy
+      // belongs to the async proxy, hence the fence (of global memory alone: 0.05 us; a full one cost microseconds here).
       if (!done && (!flags || ld_acquire(slot_flag(ws, slot)) == gen)) {
         done = true;
+        ptx::fence_proxy_async_global();
         ptx::mbar_expect_tx(bar, share);
         ptx::bulk_load(rows + uint32_t(i) * share, reinterpret_cast<const char*>(slot_o(ws, slot)) + size_t(U0) * 16, share, bar);
       }
@@ -1571,6 +1572,7 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
       else if (tid >= 128) merge_weights(p, smem, tid - 128, false, r == 0);
       __syncthreads();
       tail_merge(p, smem, tid, parity);
+      ptx::fence_proxy_async_smem();  // the weights written here and the shares read give way to the copies of the next share
       __syncthreads();
     }
   }

@@ -113,3 +113,12 @@ def test_no_wait_passes_for_another_phase(segments):
 def test_the_model_finds_the_waits_that_run_ahead(waits, arrivals):
     faults = explore((5,), waits, arrivals)
     assert "qk_issued phase 1 passed with 0 complete" in faults and "deadlock" in faults
+
+
+def test_proxy_fences_of_the_merge():
+    """What no run can be relied on to show: bulk copies of bytes that ordinary stores wrote, or over them, come behind a proxy fence."""
+    text = SOURCE.read_text()
+    fetch = re.search(r"void tail_fetch\(.*?\n}\n", text, re.S).group(0)
+    assert fetch.index("ld_acquire(slot_flag") < fetch.index("fence_proxy_async_global()") < fetch.index("ptx::bulk_load(")
+    last = re.search(r"void merge_as_last\(.*?\n}\n", text, re.S).group(0)  # one share after the other through the same buffer
+    assert re.search(r"tail_merge\(p, smem, tid, parity\);\s*ptx::fence_proxy_async_smem\(\);[^\n]*\s*__syncthreads\(\);", last)
