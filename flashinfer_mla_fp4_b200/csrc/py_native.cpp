@@ -7,6 +7,9 @@
 // not of the common form: another layout or dtype, a host tensor, an argument that is wrong.  The Python caller then
 // goes through its own checks, which also word the error messages, and through ctypes.
 //
+// The GIL is let go around allocations and launches: a launch blocks while the stream's queue is full, and what is queued may wait
+// for another Python thread (a host callback, say).
+//
 // The kernels stay behind the C ABI: bind() receives the addresses of its functions from the loaded library, so this
 // module works with whichever build of the library was loaded and links against none.
 #define PY_SSIZE_T_CLEAN
@@ -34,6 +37,15 @@ struct Abi {
   decltype(&mla_fp4_step_metadata) step_metadata = nullptr;
   decltype(&mla_fp4_last_error) last_error = nullptr;
 } abi;
+
+// Without the GIL for as long as it lives.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  NoGil() = default;
+  NoGil(const NoGil&) = delete;
+  NoGil& operator=(const NoGil&) = delete;
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
 
 // The exception that the Python binding raises for a status (_cabi.check).
 PyObject* raise_status(int rc) {
@@ -140,8 +152,6 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (pdl < 0) return nullptr;
 
   c10::cuda::CUDAGuard guard(dev);
-  if (!given) out = at::empty(at::IntArrayRef(shape, 4), at::TensorOptions().dtype(out_type).device(dev));
-  if (want_lse && !lse_given) lse = at::empty(at::IntArrayRef(shape, 3), at::TensorOptions().dtype(at::kFloat).device(dev));
   MlaFp4DecodeArgs d = {};
   d.q = q->data_ptr();
   d.q_stride_batch = q->stride(0); d.q_stride_qpos = q->stride(1); d.q_stride_head = q->stride(2);
@@ -150,8 +160,6 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   d.block_tables = static_cast<const int32_t*>(bt->data_ptr());
   d.block_table_stride = bt->stride(0);
   d.seq_lens = static_cast<const int32_t*>(sl->data_ptr());
-  d.out = out.data_ptr();
-  d.lse = want_lse ? static_cast<float*>(lse.data_ptr()) : nullptr;
   d.workspace = ws->data_ptr();
   d.workspace_bytes = size_t(ws->numel());
   d.status = static_cast<int32_t*>(status->data_ptr());
@@ -165,7 +173,15 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   d.wait_polls = int32_t(polls);
   d.logits_soft_cap = float(cap);
   d.sink = sink ? static_cast<const float*>(sink->data_ptr()) : nullptr;
-  const int rc = abi.decode(&d);
+  int rc;
+  {
+    NoGil released;
+    if (!given) out = at::empty(at::IntArrayRef(shape, 4), at::TensorOptions().dtype(out_type).device(dev));
+    if (want_lse && !lse_given) lse = at::empty(at::IntArrayRef(shape, 3), at::TensorOptions().dtype(at::kFloat).device(dev));
+    d.out = out.data_ptr();
+    d.lse = want_lse ? static_cast<float*>(lse.data_ptr()) : nullptr;
+    rc = abi.decode(&d);
+  }
   if (rc != MLA_FP4_OK) return raise_status(rc);
   PyObject* po = given ? Py_NewRef(a[19]) : THPVariable_Wrap(std::move(out));
   if (!po || !want_lse) return po;
@@ -206,10 +222,18 @@ PyObject* write_tokens(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (slots && (slots->scalar_type() != at::kLong || slots->numel() != tokens || !slots->is_contiguous())) Py_RETURN_FALSE;
   if (ts && (ts->scalar_type() != at::kFloat || ts->numel() != tokens || !ts->is_contiguous())) Py_RETURN_FALSE;
   c10::cuda::CUDAGuard guard(dev);
-  const int rc = abi.cache_write(lat->data_ptr(), lat->stride(0), rope->data_ptr(), rope->stride(0), in_type,
-                                 ts ? static_cast<const float*>(ts->data_ptr()) : nullptr,
-                                 slots ? static_cast<const int64_t*>(slots->data_ptr()) : nullptr, tokens, kv->data_ptr(),
-                                 static_cast<float*>(sf->data_ptr()), num_slots, c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+  const void *lat_p = lat->data_ptr(), *rope_p = rope->data_ptr();
+  const int64_t lat_stride = lat->stride(0), rope_stride = rope->stride(0);
+  const float* ts_p = ts ? static_cast<const float*>(ts->data_ptr()) : nullptr;
+  const int64_t* slots_p = slots ? static_cast<const int64_t*>(slots->data_ptr()) : nullptr;
+  void* kv_p = kv->data_ptr();
+  float* sf_p = static_cast<float*>(sf->data_ptr());
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  int rc;
+  {
+    NoGil released;
+    rc = abi.cache_write(lat_p, lat_stride, rope_p, rope_stride, in_type, ts_p, slots_p, tokens, kv_p, sf_p, num_slots, stream);
+  }
   if (rc != MLA_FP4_OK) return raise_status(rc);
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
@@ -247,15 +271,24 @@ PyObject* step_metadata(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const void *pbt = readable(*bt, dev), *psl = readable(*sl, dev), *psm = sm ? readable(*sm, dev) : nullptr;
   if (!pbt || !psl || (sm && !psm)) Py_RETURN_FALSE;
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  const int rc = abi.step_metadata(
-      static_cast<const int32_t*>(pbt), bt->stride(0), int32_t(bt->size(1)), psl, sl->scalar_type() == at::kLong ? 1 : 0,
-      static_cast<const int64_t*>(psm), int32_t(bt->size(0)), int32_t(page), int32_t(q_len), static_cast<int32_t*>(dbt->data_ptr()),
-      dbt->stride(0), static_cast<int32_t*>(dsl->data_ptr()), static_cast<int64_t*>(dsm->data_ptr()), int32_t(dsl->size(0)),
-      stream.stream());
+  const int64_t bt_stride = bt->stride(0), dbt_stride = dbt->stride(0);
+  const int32_t width = int32_t(bt->size(1)), batch = int32_t(bt->size(0)), max_batch = int32_t(dsl->size(0)), wide = sl->scalar_type() == at::kLong ? 1 : 0;
+  int32_t *dbt_p = static_cast<int32_t*>(dbt->data_ptr()), *dsl_p = static_cast<int32_t*>(dsl->data_ptr());
+  int64_t* dsm_p = static_cast<int64_t*>(dsm->data_ptr());
+  at::Tensor pinned[3];  // kept while they are handed to the allocator
+  int n_pinned = 0;
+  for (const at::Tensor* t : {bt, sl, sm})
+    if (t && !t->is_cuda()) pinned[n_pinned++] = *t;
+  int rc;
+  {
+    NoGil released;
+    rc = abi.step_metadata(static_cast<const int32_t*>(pbt), bt_stride, width, psl, wide, static_cast<const int64_t*>(psm), batch, int32_t(page),
+                           int32_t(q_len), dbt_p, dbt_stride, dsl_p, dsm_p, max_batch, stream.stream());
+    if (rc == MLA_FP4_OK)
+      for (int i = 0; i < n_pinned; ++i)  // pinned memory that the caller lets go now is not handed out again before the kernel has read it
+        at::getHostAllocator(at::kCUDA)->record_event(pinned[i].data_ptr(), pinned[i].storage().data_ptr().get_context(), stream);
+  }
   if (rc != MLA_FP4_OK) return raise_status(rc);
-  for (const at::Tensor* t : {bt, sl, sm})  // pinned memory that the caller lets go now is not handed out again before the kernel has read it
-    if (t && !t->is_cuda())
-      at::getHostAllocator(at::kCUDA)->record_event(t->data_ptr(), t->storage().data_ptr().get_context(), stream);
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }

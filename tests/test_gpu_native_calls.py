@@ -1,0 +1,65 @@
+"""The native call path of the Python entry points: what it owes to other Python threads and to its callers."""
+import ctypes
+import subprocess
+import threading
+import time
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev():
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    return torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("call", ["decode", "write_tokens", "step_metadata"])
+def test_other_python_threads_run_during_a_launch(call, tmp_path):
+    """A launch that blocks (a full queue; here a stand-in of the library's function that sleeps) must not hold the interpreter."""
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, FP4MLADecodeBackend, FP4MLAPagedCache, _cabi, synth
+    from flashinfer_mla_fp4_b200.kvcache import write_tokens
+
+    dev = _dev()
+    (tmp_path / "slow.c").write_text("#include <unistd.h>\nint slow(void) { usleep(300000); return 0; }\n")
+    subprocess.run(["cc", "-shared", "-fPIC", str(tmp_path / "slow.c"), "-o", str(tmp_path / "slow.so")], check=True)
+    slow = ctypes.cast(ctypes.CDLL(str(tmp_path / "slow.so")).slow, ctypes.c_void_p).value
+    names = ("mla_fp4_decode", "mla_fp4_workspace_bytes", "mla_fp4_cache_write", "mla_fp4_step_metadata", "mla_fp4_last_error")
+    real = [ctypes.cast(getattr(_cabi.lib, n), ctypes.c_void_p).value for n in names]
+
+    case = synth.build_case("gil", [100], 16, 64, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=16, page_size=64)
+    cache = FP4MLAPagedCache(2, 64, dev)
+    backend = FP4MLADecodeBackend(16, 64, 2, 128, 0.1, dev)
+    lat, rope = torch.zeros(3, 512, dtype=torch.bfloat16, device=dev), torch.zeros(3, 64, dtype=torch.bfloat16, device=dev)
+    calls = {
+        "decode": lambda: w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale,
+                                kv_cache_sf=case.kv_cache_sf),
+        "write_tokens": lambda: write_tokens(lat, rope, torch.arange(3, device=dev), cache.kv_cache, cache.kv_cache_sf),
+        "step_metadata": lambda: backend.prepare(torch.zeros(1, 1, dtype=torch.int32).pin_memory(), torch.ones(1, dtype=torch.int32).pin_memory()),
+    }
+    calls[call]()
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.monotonic())
+            time.sleep(0.001)
+
+    t = threading.Thread(target=tick)
+    _cabi.native.bind(slow, real[1], slow, slow, real[4])
+    try:
+        t.start()
+        begin = time.monotonic()
+        calls[call]()
+        end = time.monotonic()
+    finally:
+        stop.set()
+        t.join()
+        _cabi.native.bind(*real)
+    assert end - begin > 0.25  # the stand-in was called
+    assert sum(begin + 0.02 < x < end - 0.02 for x in ticks) > 20
