@@ -252,6 +252,14 @@ const void* readable(const at::Tensor& t, const at::Device& dev) {
   return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
+// Whether the memory that `rows` [n, width] (or [n]) at p spans meets that of a contiguous tensor.
+bool meets(const void* p, const at::Tensor& rows, const at::Tensor& buffer) {
+  int64_t elements = 1;
+  for (int64_t d = 0; d < rows.dim(); ++d) elements += (rows.size(d) - 1) * rows.stride(d);
+  const auto a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(buffer.data_ptr());
+  return a < b + size_t(buffer.numel()) * buffer.element_size() && b < a + size_t(elements) * rows.element_size();
+}
+
 // step_metadata(block_tables, seq_lens, slot_mapping, dst_block_tables, dst_seq_lens, dst_slot_mapping, page_size, q_len)
 // -> whether it was launched; the caller has checked the shapes against its buffers
 PyObject* step_metadata(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -270,6 +278,10 @@ PyObject* step_metadata(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c10::cuda::CUDAGuard guard(dev);
   const void *pbt = readable(*bt, dev), *psl = readable(*sl, dev), *psm = sm ? readable(*sm, dev) : nullptr;
   if (!pbt || !psl || (sm && !psm)) Py_RETURN_FALSE;
+  // Sources inside the buffers (a backend's own rows, moved up, say) are the general path's: one kernel would read what it writes.
+  if (sl->numel() == 0 || (sm && sm->numel() == 0)) Py_RETURN_FALSE;
+  for (const at::Tensor* dst : {dbt, dsl, dsm})
+    if (meets(pbt, *bt, *dst) || meets(psl, *sl, *dst) || (sm && meets(psm, *sm, *dst))) Py_RETURN_FALSE;
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(dev.index());
   const int64_t bt_stride = bt->stride(0), dbt_stride = dbt->stride(0);
   const int32_t width = int32_t(bt->size(1)), batch = int32_t(bt->size(0)), max_batch = int32_t(dsl->size(0)), wide = sl->scalar_type() == at::kLong ? 1 : 0;

@@ -63,3 +63,21 @@ def test_other_python_threads_run_during_a_launch(call, tmp_path):
         _cabi.native.bind(*real)
     assert end - begin > 0.25  # the stand-in was called
     assert sum(begin + 0.02 < x < end - 0.02 for x in ticks) > 20
+
+
+def test_prepare_from_the_backends_own_buffers():
+    """Rows of the persistent buffers as sources: refused where they lie across their places (a copy would), kept where they are the same."""
+    from flashinfer_mla_fp4_b200 import FP4MLADecodeBackend
+
+    dev = _dev()
+    backend = FP4MLADecodeBackend(16, 16, 5, 1024, 0.1, dev)
+    tables = torch.arange(4 * backend.max_pages, dtype=torch.int32, device=dev).reshape(4, -1)
+    lens = torch.tensor([700, 1, 90, 1024], dtype=torch.int32, device=dev)
+    backend.prepare(tables, lens)
+    slots = backend.slot_mapping.clone()
+    for bt, sl in ((backend.block_tables[1:4], lens[1:]), (tables[1:], backend.seq_lens[1:4])):
+        with pytest.raises(RuntimeError, match="clone"):
+            backend.prepare(bt, sl)
+    backend.prepare(tables, lens)
+    backend.prepare(backend.block_tables[:4], backend.seq_lens[:4])
+    assert torch.equal(backend.block_tables[:4], tables) and torch.equal(backend.seq_lens[:4], lens) and torch.equal(backend.slot_mapping, slots)
