@@ -94,7 +94,7 @@ class FP4MLADecodeBackend:
         self.seq_lens = torch.zeros(max_batch, dtype=torch.int32, device=self.device)
         self.slot_mapping = torch.full((max_batch * q_len,), -1, dtype=torch.int64, device=self.device)
         self._step_metadata = _cabi.native.step_metadata
-        self._views = (0, None, None, None)  # (batch, block_tables, seq_lens, slot_mapping) of the last forward()
+        self._views = (0, None, None, None, None, None, None)  # of the last forward(): batch, rows of the three buffers, the buffers
 
     # ------------------------------------------------------------------ metadata
     def clear(self) -> None:
@@ -158,9 +158,10 @@ class FP4MLADecodeBackend:
             raise ValueError(f"latent must be [{n}, {LATENT_DIM}] and rope [{n}, {ROPE_DIM}]")
         if cache.page_size != self.page_size:
             raise ValueError(f"cache page size {cache.page_size} does not match the backend's {self.page_size}")
-        views = self._views  # one attribute read: a batch and the views of the same batch, whatever another thread does
-        if views[0] != batch or views[1] is None:
-            views = self._views = (batch, self.block_tables[:batch], self.seq_lens[:batch], self.slot_mapping[:n])
+        bt, sl, sm = self.block_tables, self.seq_lens, self.slot_mapping
+        views = self._views  # one attribute read: a batch and the rows of the same batch, whatever another thread does
+        if views[0] != batch or views[4] is not bt or views[5] is not sl or views[6] is not sm:
+            views = self._views = (batch, bt[:batch], sl[:batch], sm[:n], bt, sl, sm)
         write_tokens(latent, rope, views[3], cache.kv_cache, cache.kv_cache_sf)
         return self._runner.run(q, cache.kv_cache, views[1], views[2], self.max_seq_len, self.softmax_scale,
                                 output_scale=self.output_scale, out=out, kv_cache_sf=cache.kv_cache_sf)

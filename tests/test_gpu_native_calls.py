@@ -81,3 +81,28 @@ def test_prepare_from_the_backends_own_buffers():
     backend.prepare(tables, lens)
     backend.prepare(backend.block_tables[:4], backend.seq_lens[:4])
     assert torch.equal(backend.block_tables[:4], tables) and torch.equal(backend.seq_lens[:4], lens) and torch.equal(backend.slot_mapping, slots)
+
+
+def test_forward_reads_the_buffers_that_the_backend_has():
+    """The rows kept from one forward() to the next belong to the buffers they were cut from: replaced buffers count at once."""
+    from flashinfer_mla_fp4_b200 import FP4MLADecodeBackend, FP4MLAPagedCache, synth
+
+    dev = _dev()
+    case = synth.build_case("buffers", [300, 70], 16, 64, device=dev)
+    lat, rope = torch.randn(2, 512, dtype=torch.bfloat16, device=dev), torch.randn(2, 64, dtype=torch.bfloat16, device=dev)
+
+    def outputs(lens, replace):
+        cache = FP4MLAPagedCache(case.kv_cache.shape[0], 64, dev)
+        cache.kv_cache.copy_(case.kv_cache)
+        cache.kv_cache_sf.copy_(case.kv_cache_sf)
+        backend = FP4MLADecodeBackend(16, 64, 2, 320, case.softmax_scale, dev)
+        backend.prepare(case.block_tables, case.seq_lens)
+        backend.forward(case.q, lat, rope, cache)
+        if replace:
+            backend.block_tables, backend.seq_lens, backend.slot_mapping = (t.clone() for t in (backend.block_tables, backend.seq_lens, backend.slot_mapping))
+        backend.prepare(case.block_tables, lens)
+        return backend.forward(case.q, lat + 1, rope, cache), cache.kv_cache, cache.kv_cache_sf
+
+    lens = torch.tensor([200, 64], dtype=torch.int32, device=dev)
+    for a, b in zip(outputs(lens, False), outputs(lens, True)):
+        assert torch.equal(a, b)
