@@ -252,16 +252,19 @@ const void* readable(const at::Tensor& t, const at::Device& dev) {
   return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
-// Whether the memory that `rows` [n, width] (or [n]) at p spans meets that of a contiguous tensor.
-bool meets(const void* p, const at::Tensor& rows, const at::Tensor& buffer) {
+// Whether the memory that a tensor at p spans meets that of another (neither is empty).
+size_t span(const at::Tensor& t) {
   int64_t elements = 1;
-  for (int64_t d = 0; d < rows.dim(); ++d) elements += (rows.size(d) - 1) * rows.stride(d);
+  for (int64_t d = 0; d < t.dim(); ++d) elements += (t.size(d) - 1) * t.stride(d);
+  return size_t(elements) * t.element_size();
+}
+bool meets(const void* p, const at::Tensor& t, const at::Tensor& buffer) {
   const auto a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(buffer.data_ptr());
-  return a < b + size_t(buffer.numel()) * buffer.element_size() && b < a + size_t(elements) * rows.element_size();
+  return a < b + span(buffer) && b < a + span(t);
 }
 
 // step_metadata(block_tables, seq_lens, slot_mapping, dst_block_tables, dst_seq_lens, dst_slot_mapping, page_size, q_len)
-// -> whether it was launched; the caller has checked the shapes against its buffers
+// -> whether it was launched
 PyObject* step_metadata(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 8) return PyErr_Format(PyExc_TypeError, "step_metadata takes 8 arguments");
@@ -275,6 +278,12 @@ PyObject* step_metadata(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (sm && (sm->scalar_type() != at::kLong || !sm->is_contiguous())) Py_RETURN_FALSE;
   if (!dsl->is_cuda()) Py_RETURN_FALSE;
   const at::Device dev = dsl->device();
+  // The buffers are public attributes of the backend: what is not of the form it made them in is the general path's.
+  if (!on(*dbt, dev) || dbt->dim() != 2 || dbt->scalar_type() != at::kInt || dbt->stride(1) != 1 || dbt->size(0) < bt->size(0) ||
+      dbt->size(1) < bt->size(1) || (dbt->size(0) > 1 && dbt->stride(0) < dbt->size(1)) || dsl->dim() != 1 || dsl->scalar_type() != at::kInt ||
+      !dsl->is_contiguous() || dsl->size(0) < sl->size(0) || bt->size(0) != sl->size(0) || !on(*dsm, dev) || dsm->scalar_type() != at::kLong ||
+      !dsm->is_contiguous() || q_len <= 0 || dsm->numel() != dsl->size(0) * q_len || (sm && sm->numel() != bt->size(0) * q_len))
+    Py_RETURN_FALSE;
   c10::cuda::CUDAGuard guard(dev);
   const void *pbt = readable(*bt, dev), *psl = readable(*sl, dev), *psm = sm ? readable(*sm, dev) : nullptr;
   if (!pbt || !psl || (sm && !psm)) Py_RETURN_FALSE;

@@ -106,3 +106,24 @@ def test_forward_reads_the_buffers_that_the_backend_has():
     lens = torch.tensor([200, 64], dtype=torch.int32, device=dev)
     for a, b in zip(outputs(lens, False), outputs(lens, True)):
         assert torch.equal(a, b)
+
+
+def test_prepare_into_buffers_of_another_form():
+    """Replaced buffers that the one-kernel form was not made for: wider types and rows with a pitch are filled, too narrow ones refused."""
+    from flashinfer_mla_fp4_b200 import FP4MLADecodeBackend
+
+    dev = _dev()
+    tables = torch.arange(12, dtype=torch.int32, device=dev).reshape(3, 4)
+    lens = torch.tensor([60, 1, 33], dtype=torch.int32, device=dev)
+    backend = FP4MLADecodeBackend(16, 16, 4, 64, 0.1, dev)
+    backend.prepare(tables, lens)
+    slots = backend.slot_mapping.clone()
+    backend.seq_lens = torch.full((4,), -7, dtype=torch.int64, device=dev)
+    backend.block_tables = torch.zeros(4, 9, dtype=torch.int32, device=dev)[:, :4]
+    backend.prepare(tables, lens)
+    assert backend.seq_lens.tolist() == [60, 1, 33, 0]
+    assert torch.equal(backend.block_tables[:3], tables) and torch.equal(backend.slot_mapping, slots)
+    backend.seq_lens = backend.seq_lens.int()
+    backend.block_tables = torch.zeros(4, 3, dtype=torch.int32, device=dev)
+    with pytest.raises(RuntimeError):
+        backend.prepare(tables, lens)
