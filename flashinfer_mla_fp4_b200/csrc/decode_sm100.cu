@@ -238,9 +238,11 @@ __device__ __forceinline__ int fresh_len(const DecodeParams& p, int i) {  // fro
 // which is least at n = 5 sqrt(Tt * pairs).  Then the longest walk k is kept and n lowered as far as k allows: CTAs
 // that cannot shorten the longest walk only add partials, and a CTA without work does not hold the step up when it starts late.
 // On 148 SMs, 64 heads, the whole grid -> as many as this: 1x16000 tokens 21.3 -> 17.5 us, 1x32768 22.9 -> 19.5, 4x4096 15.1 -> 14.1,
-// 2x1024 14.0 -> 12.0; beyond five tiles a CTA the whole grid works (8x32768, 128 requests).  4 / 5 / 6 sqrt(Tt * pairs), with today's
+// 2x1024 14.0 -> 12.0; with several requests or head groups the whole grid works beyond five tiles a CTA (8x32768, 128 requests).  4 / 5 / 6 sqrt(Tt * pairs), with today's
 // merge: 1x32768 18.45 / 17.2 / 18.2, 1x8192 14.15 / 13.3 / 13.3, 2x32768 19.6 / 18.6 / 18.6, 4x4096 13.2 / 13.2 / 13.55, 2x16000 17.5 /
-// 17.4 / 15.8.  Approximate arithmetic will do: every CTA takes the same steps, and any 1 <= n <= Tt is right.
+// 17.4 / 15.8.  Approximate arithmetic will do: every CTA takes the same steps, and any 1 <= n <= Tt is right.  (The host's form of this
+// rule, mla_fp4_work_ctas, is exact; the two agree while no walk is longer than a thousand tiles: where the root decides, Tt * pairs is
+// below n^2 / 25, so that its argument keeps clear of the squares by more than the 1e-3 allows for.)
 __device__ __forceinline__ int work_ctas(flat_t Tt, int pairs, int n) {
   if (Tt > 5 * n && pairs > 1) return n;  // the whole grid, and next to nothing to gain from the rounding
   const float tiles = float(Tt);

@@ -2,7 +2,9 @@
 
 The decode kernel derives its partition on the device from ``seq_lens``; this
 module asks the library for the same partition computed on the host, for
-inspection, tests and capacity planning.  It replaces the reference's
+inspection, tests and capacity planning: ``plan_partition`` over the CTAs that
+``work_ctas`` counts for the default kernel, which leaves part of the grid idle
+when there are few tiles, or over the whole grid for the two-kernel mode.  It replaces the reference's
 ``mla_get_split_kv_simplified`` + static tile scheduler (flashinfer
 ``cute_dsl/attention/scheduler/mla_persistent.py:137-282``), which split every
 request the same number of times whatever its length.
@@ -34,8 +36,16 @@ def tiles_of(seq_len: int) -> int:
     return (seq_len + _cabi.TILE_TOKENS - 1) // _cabi.TILE_TOKENS if seq_len > 0 else 0
 
 
+def work_ctas(seq_lens: Sequence[int], q_len: int, num_heads: int, num_ctas: int) -> int:
+    """How many CTAs of a grid of ``num_ctas`` the default kernel (which merges by itself) shares the tiles among."""
+    arr = (C.c_int32 * max(len(seq_lens), 1))(*[int(x) for x in seq_lens])
+    out = C.c_int32(0)
+    _cabi.check(_cabi.lib.mla_fp4_work_ctas(arr, len(seq_lens), q_len, num_heads, num_ctas, C.byref(out)))
+    return out.value
+
+
 def plan_partition(seq_lens: Sequence[int], q_len: int, num_heads: int, num_ctas: int) -> List[Segment]:
-    """All segments of all CTAs, in CTA order."""
+    """All segments of ``num_ctas`` working CTAs, in CTA order."""
     n = len(seq_lens)
     arr = (C.c_int32 * max(n, 1))(*[int(x) for x in seq_lens])
     count = C.c_int32(0)

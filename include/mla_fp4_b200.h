@@ -151,8 +151,16 @@ int mla_fp4_plan_partition(const int32_t* seq_lens_host, int32_t batch, int32_t 
                            int32_t* seg_tile_begin, int32_t* seg_tile_end, int32_t* seg_slot,
                            int32_t* num_segments);
 
-/* Zero the header of a workspace (an asynchronous memset on `stream`).  Call once after
-   allocating the workspace, and again after a step that reported MLA_FP4_ERR_DEVICE_TIMEOUT.
+/* How many CTAs of a grid of num_ctas share a step's tiles when the decode kernel merges by itself
+   (MLA_FP4_KERNEL_TCGEN05): with few tiles, fewer than the grid, since each CTA more is a partial
+   more to merge.  mla_fp4_plan_partition over this many CTAs is that kernel's partition; the
+   other kernels use the whole grid.  (Beyond a thousand tiles a CTA, some 19 M tokens in one
+   request, the kernel's number may be one off.) */
+int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len, int32_t num_heads,
+                      int32_t num_ctas, int32_t* work_ctas);
+
+/* Zero the header and the slot tails of a workspace (an asynchronous memset on `stream`).  Call
+   once after allocating the workspace.
    The reference's workspace needs no preparation (wrappers/batch_mla_fp4.py:413-420). */
 int mla_fp4_workspace_init(void* workspace, size_t workspace_bytes, void* stream);
 

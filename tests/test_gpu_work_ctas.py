@@ -35,3 +35,28 @@ def test_any_number_of_working_ctas(lens, heads, max_ctas):
     O.assert_parity(out, ref, "working CTAs")
     live = torch.isfinite(ref_lse)
     torch.testing.assert_close(lse.cpu()[live], ref_lse[live], atol=2e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("lens,heads,q_len,max_ctas", [
+    ([513], 64, 1, None), ([16000], 64, 1, None), ([16000] + [0] * 32, 64, 1, None), ([4096] * 4, 64, 1, None), ([3000, 1500], 128, 2, None),
+    ([130, 0, 5000, 1, 700], 40, 1, 31), ([2500] * 30, 128, 1, 7), ([512] * 6, 64, 1, None), ([60000], 8, 1, 100), ([9000, 100], 16, 3, 148),
+    ([1280, 1152], 64, 1, 5), ([1280, 1281], 64, 1, 5),
+])
+def test_the_planner_describes_the_kernels_partition(lens, heads, q_len, max_ctas):
+    """The partial slots that a step publishes are those of the host's partition over the host's number of working CTAs."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, _cabi, planner, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("slots", [max(n, 1) for n in lens], heads, 64, q_len=q_len, seed=1, device=dev)
+    case.seq_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
+    ws = torch.empty(32 << 20, dtype=torch.int8, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(ws)
+    w.plan(num_heads=heads, page_size=64, max_ctas=max_ctas)  # (zeroes the slots' flags)
+    w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
+    w.check_device_status()
+    head = _cabi.WORKSPACE_HEADER_BYTES
+    published = ws[head: head + 296 * 272].view(torch.int32).reshape(296, 68)[:, 65].nonzero().flatten().tolist()
+    n = planner.work_ctas(lens, q_len, heads, w._num_ctas)
+    assert published == sorted(s.slot for s in planner.plan_partition(lens, q_len, heads, n) if s.slot >= 0)

@@ -254,3 +254,27 @@ def test_partition_beyond_32_bits_is_refused():
     with pytest.raises(ValueError, match="32 bits"):
         planner.plan_partition([2**31 - 1] * 64, 1, 64, 148)
     assert planner.plan_partition([2**20] * 64, 1, 64, 148)  # 64 M tokens: fits
+
+
+@pytest.mark.parametrize("seq_lens,heads,ctas,expect", [
+    ([], 64, 148, 148),
+    ([0, 0], 64, 148, 148),
+    ([512] * 3, 64, 148, 148),          # short requests stay whole: no rule
+    ([513], 64, 148, 8),                # 8 tiles with the phantom ones: below 5 sqrt(8), so one a CTA
+    ([16000], 64, 148, 43),             # 128 tiles, 5 sqrt(128) = 56.6: walks of three
+    ([4096] * 4, 64, 148, 70),          # 140 tiles, 5 sqrt(140 * 4) > 70: walks of one would need 140 CTAs of 118, so two
+    ([32768] * 8, 64, 148, 148),        # beyond five tiles a CTA, several requests: the whole grid
+    ([2500], 64, 3, 3),
+])
+def test_number_of_working_ctas(seq_lens, heads, ctas, expect):
+    """The default kernel's own CTA count: n = 5 sqrt(tiles * pairs) at most, then the fewest CTAs with the same longest walk."""
+    from flashinfer_mla_fp4_b200 import planner
+
+    assert planner.work_ctas(seq_lens, 1, heads, ctas) == expect
+
+
+def test_working_ctas_of_a_tile_space_beyond_32_bits_are_refused():
+    from flashinfer_mla_fp4_b200 import planner
+
+    with pytest.raises(ValueError, match="32 bits"):
+        planner.work_ctas([2**31 - 1] * 64, 1, 64, 148)
