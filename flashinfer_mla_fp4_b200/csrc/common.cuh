@@ -25,8 +25,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 //     scale (the decode kernel's lanes own one dim each: with this order a warp stores 32 dims x 8 heads =
 //     512 contiguous bytes at a time; with heads innermost over all 64 it would store 16 bytes every 128).
 //   * tail of slot s (272 bytes): the base-2 LSE of the 64 heads as f32, that scale (f32), the slot's flag
-//     (int32, see below), an arrival counter (int32) and the flag of the LSEs and the scale alone (int32).  The tails of all slots lie side by side, so the tails of the
-//     consecutive slots of one split request are one contiguous range (one bulk copy for a merging CTA).
+//     (int32, see below), an arrival counter (int32) and the flag of the LSEs and the scale alone (int32).
 // The scale is 6 * max|token scale| * |output_scale| / 32768 rounded up to a power of two: an
 // upper bound of |O| mapped below the fp16 maximum, so the 11-bit partials can neither overflow nor
 // lose the small values (fp16 spans 29 binades below that bound).  Half the bytes of f32 partials.

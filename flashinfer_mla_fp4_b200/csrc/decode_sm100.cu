@@ -18,9 +18,10 @@
 // RoPE bytes, per-token scales and Q arrive by TMA as well.
 //
 // What bounds it (measured with one MMA form at a time, operands in shared memory): at N = 64 an MMA reads A (4 KiB) and
-// B (2 KiB) at the 128 B/clk of shared memory, 48 clk, and a PV pair that shares A through the collector takes 79: 18 x 48
-// + 16 x 79 = 2130 clk of tensor pipe per tile, beside 72 KiB of TMA writes (560 clk of the same port).  Everything else
-// is arranged to stay under that:
+// B (2 KiB) at the 128 B/clk of shared memory, 48 clk, and a PV pair that shares A through the collector takes 78: the 18 + 32
+// MMAs of a tile measured alone take 863 + 1248 = 2111 clk of tensor pipe, beside 72 KiB of TMA writes (560 clk of the same port).  A
+// tile takes 2500 in the steady state: the pipe also waits for P', whose one buffer is free when the last PV has completed.
+// Everything else is arranged to stay under that:
 //   * latent blocks are handled in pairs (32 KiB, five pair slots = two and a half tiles in flight): one barrier, one wait
 //     and one commit per pair;
 //   * QK^T and PV are issued by a warp each: the queue of the tensor pipe is short, so a gap in one warp's issue (a wait, the
@@ -150,9 +151,6 @@ __device__ __forceinline__ uint8_t* smem_ptr(uint32_t smem) { return static_cast
 __device__ __forceinline__ Misc* misc_of(uint32_t smem) { return reinterpret_cast<Misc*>(smem_ptr(smem) + kOffMisc); }
 __device__ __forceinline__ const Segment* segs_of(uint32_t smem) { return reinterpret_cast<const Segment*>(smem_ptr(smem) + kOffSegs); }
 __device__ __forceinline__ uint32_t bar_addr(uint32_t smem, int idx) { return smem + kOffBars + 8u * idx; }
-#ifndef MLA_STAMP
-#define MLA_STAMP(role, tile, ev)
-#endif
 
 // A bounded wait expired: flag the CTA (every role then stops issuing and drains) and leave a record.
 __device__ __noinline__ void flag_timeout(uint32_t smem, int idx, uint32_t parity) {
@@ -451,7 +449,6 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
       const uint32_t bar = bar_addr(smem, bar_kv_full(st.slot)), dst = smem + kOffKV + st.slot * kPairBytes;
       if (st.lap >= 1) ok = wait(smem, bar_kv_empty(st.slot), (st.lap - 1) & 1);
       if (!ok) break;
-      MLA_STAMP(1 + which, st.it, 0);
       // the transaction count of a 4-bit copy is in packed bytes: 64 per row and block
       if (e) ptx::mbar_arrive_expect_tx(bar, uint32_t(np) * ps * (which ? 128u : 132u));
       const int c0 = int(256u * which);
@@ -463,8 +460,8 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
         const uint32_t dst_sc = smem + kOffScale + (st.it & (kScaleStages - 1)) * (kTile * 4);
         for_pages([&](uint32_t issue, int page, int i) { ptx::bulk_load_if(issue, dst_sc + uint32_t(i) * ps * 4u, p.kv_cache_sf + int64_t(page) * ps, ps * 4u, bar); });
       }
-      MLA_STAMP(1 + which, st.it, 1);
-      // The rows of the tile four ahead are brought into L2: the ring holds two and a half tiles, and a pair's slot comes free
+      // The rows of the tile four ahead are brought into L2 (page ids in hand reach 32 to 64 pages: with pages of 8 tokens, sixteen to a
+      // tile, that is not four tiles, and nothing is prefetched): the ring holds two and a half tiles, and a pair's slot comes free
       // two tiles before the pair is needed, so a load that comes from DRAM (2000 clk instead of 900) shows in every tile:
       // 2x131072 tokens, H=128, q_len=2: 97.5 -> 92.6 us; 8x32768: 37.6 -> 36.8.
       if (which) {
@@ -560,7 +557,6 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
       if (t >= 2) ok = ok && wait(smem, kBarPvIssued, it & 1);
       ok = ok && wait(smem, kBarRopeFull, it & 1);
       if (!ok) break;
-      MLA_STAMP(0, it, 0);
       ptx::tc_fence_after();
       const uint32_t e = ptx::elect_one();
 #pragma unroll
@@ -586,7 +582,6 @@ __device__ __forceinline__ void qk_role(const DecodeParams& p, uint32_t smem, ui
         __syncwarp();
         st.advance(1);
       }
-      MLA_STAMP(0, it, 1);
     }
     // every QK^T of this segment has been issued: Q may be overwritten once they complete
     if (ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarQEmpty));
@@ -617,7 +612,6 @@ __device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState&
       // its parity cannot be taken for an older phase's.  (The other way round, tile 0 found the barrier untouched and did not wait.)
       if (!wait(smem, kBarPFull, st.it & 1)) return;
       if (t + 1 < n && !wait(smem, kBarQkIssued, (st.it + 1) & 1)) return;
-      MLA_STAMP(0, st.it, 2);
       ptx::tc_fence_after();
       const uint32_t e = ptx::elect_one(), keep = t ? 1u : 0u;
 #pragma unroll 1
@@ -639,7 +633,6 @@ __device__ __forceinline__ void pv_role(uint32_t smem, uint32_t tmem, RoleState&
         __syncwarp();
         st.advance(1);
       }
-      MLA_STAMP(0, st.it, 3);
     }
   }
 }
@@ -1069,7 +1062,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       t.t_rope = tmem_lane + kColSRope + 64u * s + uint32_t(kHalfHeads * half);
 
       (void)wait(smem, bar_s_full(s), (it >> 1) & 1);
-      if (tid == 0) MLA_STAMP(3, it, 0);
       ptx::tc_fence_after();
 
       // The exponents are taken with the reference as it stands, which holds unless some score beat it by more than the lazy
@@ -1122,7 +1114,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
         l2[2 * q] = add2(l2[2 * q], e2[2 * q]);
         l2[2 * q + 1] = add2(l2[2 * q + 1], e2[2 * q + 1]);
       }
-      if (tid == 0) MLA_STAMP(3, it, 1);
       // The one P buffer (and, for a rescale, O^T) is free once the PV of the previous tile has completed; until then
       // this tile's P' stays in registers.
       if (it >= 1) (void)wait(smem, kBarPvDone, (it - 1) & 1);
@@ -1142,7 +1133,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       ptx::tc_fence_before();  // orders the O^T writes of a rescale before the arrival
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(bar_addr(smem, kBarPFull));
-      if (tid == 0) MLA_STAMP(3, it, 2);
     }
 
     // ---- segment epilogue
@@ -1195,7 +1185,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
       }
     }
     (void)wait(smem, kBarPvDone, (st.it - 1) & 1);  // the PV of the last tile
-    if (tid == 0) MLA_STAMP(3, st.it - 1, 3);
     ptx::tc_fence_after();
     if (!ptx::bar_or(1, kSoftmaxThreads, misc->abort != 0)) {  // (all or none: the writers meet at barriers)
       if (g.slot >= 0) write_partial(p, smem, tmem_lane, row, half, g.slot);
@@ -1215,7 +1204,6 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
     __syncwarp();
     if (lane == 0) ptx::mbar_arrive(bar_addr(smem, kBarOFree));
     pending |= g.slot >= 0;
-    if (tid == 0) MLA_STAMP(3, st.it - 1, 4);
   }
   if (pending && p.fused_merge) {
     if (!misc->more) {  // (publish)
@@ -1258,7 +1246,6 @@ __device__ __noinline__ void publish(const DecodeParams& p, uint32_t smem, int l
     if (head && last != even) st_release(slot_lse_flag(p.workspace, even), gen);
     if (head) st_release(slot_flag(p.workspace, even), gen);
     if (tail) st_release(slot_flag(p.workspace, even + 1), gen);
-    MLA_STAMP(4, 0u, 0);
   }
   __syncwarp();
 }
@@ -1279,7 +1266,7 @@ __device__ __noinline__ void publish(const DecodeParams& p, uint32_t smem, int l
 // case whenever the grid has the GPU to itself for a moment.  A cooperative launch gave the same guarantee and cost 3.3 us
 // per step launched outside a graph (it does not overlap the kernel before it): 22.7 -> 19.4 us for 4 x 4096 tokens.
 constexpr int kMergeShared = 1, kMergeLast = 2;
-constexpr uint32_t kTailBytes = uint32_t(kSlotTailBytes);               // a slot's tail: 64 LSEs, the slot scale, the flag, an arrival counter, padding
+constexpr uint32_t kTailBytes = uint32_t(kSlotTailBytes);               // a slot's tail: 64 LSEs, the slot scale, the flag, an arrival counter, the flag of the LSEs
 constexpr uint32_t kTailStage = kOffKV;                                 // staging: [slots][this CTA's bytes of a slot], then the tails
 constexpr uint32_t kTailRed = kOffScale - kThreads * 32;                // [384][8] f32: sums of a unit that several threads share
 constexpr uint32_t kTailStageBytes = kOffP - kTailStage;                // the KV ring, RoPE and Q; not P, where the last segment's output may still be in transit
@@ -1480,7 +1467,6 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
   const uint32_t share = uint32_t(nu) * 16u, rows = smem + kTailStage, tails = rows + uint32_t(ns) * share;
   const bool landed = wait(smem, kBarTail, parity);
   if (!landed && (tid & 31) == 0) drain_wait(smem, kBarTail, parity);  // giving up: copies in flight land first
-  if (tid == 0) MLA_STAMP(4, 0u, 2);
   if (__syncthreads_or(!landed || misc->abort)) return;  // (uniform: there is a barrier below)
   // A thread per unit, or, when there are fewer units than threads, S threads per unit, each with every S-th slot.
   const int S = min(max(kThreads / nu, 1), ns);
@@ -1539,7 +1525,6 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
       store_unit(acc, i0, i1, heads, [&](int e, float v) { d[e * kLatent] = __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3); });
     }
   }
-  if (tid == 0) MLA_STAMP(4, 0u, 4);
 }
 
 // The last-writer form: for each request this CTA wrote a partial of, count it in; the last to arrive merges it, share by share.
@@ -1593,7 +1578,6 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   Misc* misc = misc_of(smem);
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = int(ptx::uniform_u32(uint32_t(tid >> 5)));
-  if (tid == 0) MLA_STAMP(4, 1u, 0);
 
   // What needs nothing an earlier kernel wrote comes first: with a programmatic dependent launch this part runs
   // while the kernel before this one on the stream is still draining.
@@ -1639,11 +1623,9 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   RoleState st{};
   if (warp != kWarpTMA && warp != kWarpTMA2) {  // (these two: in their role, after a first pass without effect)
     start_work(p, smem, warp, lane);
-    if (tid == 0) MLA_STAMP(4, 1u, 1);
   }
   ptx::tc_fence_after();
   const uint32_t tmem = ptx::uniform_u32(misc->tmem_base);
-  if (tid == 0) MLA_STAMP(4, 1u, 2);
   // Rounds: almost always exactly one; more only when a CTA's range spans more than kMaxSeg requests.
   bool first_round = true;
   int finished = -1;
@@ -1654,7 +1636,6 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       if (p.fused_merge && !misc->more && misc->n_slots > 0) {
         ptx::bar_sync(5, kThreads - 32);
         if (misc->mode == kMergeShared) merge_weights(p, smem, tid - 32 * kWarpSoftmax0, true, misc->rank == 0);
-        if (tid == 128) MLA_STAMP(4, 0u, 3);
       }
     } else if (warp == kWarpQK) {
       qk_role(p, smem, tmem, &map_q_lat, &map_q_rope, st);
@@ -1697,7 +1678,6 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
           asm volatile("bar.arrive 5, %0;" ::"n"(kThreads - 32) : "memory");  // the mode is known
           if (misc->mode == kMergeShared) tail_fetch(p, smem, warp - kWarpTMA, lane, true);
         }
-        if (warp == kWarpPV) MLA_STAMP(4, 0u, 1);
         // This CTA has no more use for the header.  (The count comes back while the merge goes on.)
         if (warp == kWarpPV && lane == 0) finished = atomicAdd(ws_finished(p.workspace), 1);
       }
@@ -1728,7 +1708,6 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       *ws_mode(p.workspace) = 0;
       st_release(ws_generation(p.workspace), misc->gen);
     }
-    if (tid == 0) MLA_STAMP(4, 1u, 3);
   }
 }
 
