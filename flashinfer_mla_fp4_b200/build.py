@@ -14,7 +14,7 @@ LIB_PATH = Path(os.environ.get("MLA_FP4_B200_LIB") or (PKG_DIR / "libmla_fp4_b20
 SOURCES = ["abi.cu", "kernels_simt.cu", "combine.cu", "cache_write.cu", "cp_exchange.cu", "decode_sm100.cu"]
 NATIVE_PATH = PKG_DIR / "_native.so"
 NATIVE_SOURCE = CSRC / "py_native.cpp"
-HEADERS = ["common.cuh", "dequant.cuh", "launch.h", "ptx_sm100.cuh", "../../include/mla_fp4_b200.h"]
+HEADERS = ["common.cuh", "decode_pair.cuh", "dequant.cuh", "launch.h", "ptx_sm100.cuh", "../../include/mla_fp4_b200.h"]
 
 
 def _nvcc() -> str:

@@ -118,7 +118,9 @@ int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len
   if (!work_ctas || (batch > 0 && !seq_lens_host)) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
   if (batch < 0 || q_len <= 0 || num_heads <= 0 || num_ctas <= 0)
     return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/num_ctas out of range");
-  const int64_t groups = mla::num_groups(q_len, num_heads), pairs = groups * batch, n = num_ctas;
+  const int64_t groups = mla::num_groups(q_len, num_heads), pairs = groups * batch;
+  const int pair_grid = mla::pair_ctas(int(groups), num_ctas);
+  const int64_t n = pair_grid ? pair_grid : num_ctas;
   int64_t T = 0;
   int max_tiles = 0;
   for (int b = 0; b < batch; ++b) {
@@ -126,12 +128,13 @@ int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len
     max_tiles = std::max(max_tiles, mla::tiles_of(seq_lens_host[b]));
   }
   if (!mla::partition_fits(T, num_ctas)) return fail(MLA_FP4_ERR_UNSUPPORTED, "the work partition is computed in 32 bits: too many tiles x CTAs");
-  *work_ctas = num_ctas;
-  if (T == 0 || mla::whole_requests(max_tiles, pairs, num_ctas) || (T > 5 * n && pairs > 1)) return MLA_FP4_OK;
+  *work_ctas = int32_t(n);
+  if (T == 0 || mla::whole_requests(max_tiles, pairs, int(n)) || (T > 5 * n && pairs > 1)) return MLA_FP4_OK;
   // the longest walk: k >= T / n and k >= T / (5 sqrt(T * pairs)); then the fewest CTAs whose walks are no longer
   int64_t k = (T + n - 1) / n;
   while (25 * pairs * k * k < T) ++k;
   *work_ctas = int32_t(std::min(n, (T + k - 1) / k));
+  if (pair_grid) *work_ctas = int32_t((*work_ctas + groups - 1) / groups * groups);  // (every group is shared by as many)
   return MLA_FP4_OK;
 }
 

@@ -23,7 +23,8 @@ constexpr float kLog2e = 1.4426950408889634f;
 // Split-KV partials in the workspace.  Layout:  header | tails [296] | partial O [slots]
 //   * partial O of slot s: normalised O as fp16 [8 head groups][512 dims][8 heads] divided by a per-slot
 //     scale (the decode kernel's lanes own one dim each: with this order a warp stores 32 dims x 8 heads =
-//     512 contiguous bytes at a time; with heads innermost over all 64 it would store 16 bytes every 128).
+//     512 contiguous bytes at a time; with heads innermost over all 64 it would store 16 bytes every 128).  In a step
+//     of the pair kernel, whose lanes own a head each: fp16 [64 heads][512 dims].
 //   * tail of slot s (272 bytes): the base-2 LSE of the 64 heads as f32, that scale (f32), the slot's flag
 //     (int32, see below), an arrival counter (int32) and the flag of the LSEs and the scale alone (int32).
 // The scale is 6 * max|token scale| * |output_scale| / 32768 rounded up to a power of two: an
@@ -115,6 +116,14 @@ MLA_HD bool whole_requests(int max_real_tiles, int64_t pairs, int n) { return ma
 
 MLA_HD int num_groups(int q_len, int num_heads) {
   return q_len * ((num_heads + kGroupHeads - 1) / kGroupHeads);
+}
+
+// The grid where the decode kernel for pairs of head groups (decode_pair.cuh) can be used, or 0: an even number of groups, and as many CTAs
+// as the groups can share evenly, unless that leaves too many of `num_ctas` idle (more than that kernel gains).
+MLA_HD int pair_ctas(int groups, int num_ctas) {
+  if (groups & 1) return 0;
+  const int n = num_ctas / groups * groups;
+  return 8 * n >= 7 * num_ctas ? n : 0;
 }
 
 // Positions in the flat tile space are 32-bit: a 64-bit division is a subroutine of a hundred instructions and these

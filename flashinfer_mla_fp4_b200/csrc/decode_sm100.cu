@@ -47,6 +47,7 @@
 // Every wait is bounded: when a wait expires the CTA records MLA_FP4_ERR_DEVICE_TIMEOUT in the
 // status words, stops issuing work, drains and exits normally.
 #include <atomic>
+#include <climits>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -99,8 +100,9 @@ __device__ __forceinline__ constexpr int bar_s_full(int s) { return 2 * kRing + 
 __device__ __forceinline__ constexpr int bar_s_empty(int s) { return 2 * kRing + 2 + s; }  // ... and has been read
 constexpr int kBarRopeFull = 2 * kRing + 4, kBarRopeEmpty = 2 * kRing + 5, kBarPFull = 2 * kRing + 6, kBarPvDone = 2 * kRing + 7,
               kBarQFull = 2 * kRing + 8, kBarQEmpty = 2 * kRing + 9, kBarOFree = 2 * kRing + 10, kBarDrain = 2 * kRing + 11,
-              kBarTail = 2 * kRing + 12, kBarQkIssued = 2 * kRing + 13, kBarPvIssued = 2 * kRing + 14;
-constexpr int kNumBars = 2 * kRing + 15;
+              kBarTail = 2 * kRing + 12, kBarQkIssued = 2 * kRing + 13, kBarPvIssued = 2 * kRing + 14,
+              kBarScale = 2 * kRing + 15;  // pair kernel: scales of a tile, four stages
+constexpr int kNumBars = 2 * kRing + 15 + kScaleStages;
 static_assert(kNumBars <= 32, "initialised by one warp, a barrier per lane");
 constexpr uint32_t kOffTail = (kOffBars + kNumBars * 8 + 15u) & ~15u;     // merge plan: [148] slot ids
 constexpr uint32_t kOffSegs = kOffTail + kMaxCombineSlots * 4;            // Segment[kMaxSeg]
@@ -144,6 +146,7 @@ struct Misc {
   int mode;           // how the split requests of this step are merged: kMergeShared or kMergeLast
   int32_t gen;        // generation of this decode step, fetched once per CTA
   int last;           // kMergeLast: this CTA is the last writer of the request
+  int cta;            // pair kernel: this CTA's place in the partition (cta_in_partition)
 };
 static_assert(sizeof(Misc) <= 256, "misc area");
 
@@ -251,11 +254,24 @@ __device__ __forceinline__ int work_ctas(flat_t Tt, int pairs, int n) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(k));
   return min(n, max(1, __float2int_ru(tiles * r - 1e-3f)));
 }
+// This CTA's place in the partition.  In the pair kernel the two CTAs of a cluster walk the same tiles for two neighbouring head groups.
+// There the working CTAs are a multiple of the groups, so that every group is shared by as many, `per`, in ranges of its own tiles that are
+// the same for all groups: cluster w takes range w mod per of the groups 2 (w / per) and 2 (w / per) + 1.  (Short requests: `per` is the
+// batch.)  The partition is thus the one of the other kernel, on other CTAs.
+template <bool kPair>
+__device__ __forceinline__ int cta_in_partition(int per, int groups) {
+  if (!kPair) return blockIdx.x;
+  const int w = int(blockIdx.x >> 1), gp = int(uint32_t(w) / uint32_t(per));
+  return 2 * gp < groups ? (2 * gp + int(blockIdx.x & 1)) * per + (w - gp * per) : per * groups;  // (beyond the last: no work)
+}
+template <bool kPair>
+__device__ __forceinline__ int cta_of(const Misc* misc) { return kPair ? misc->cta : int(blockIdx.x); }
+template <bool kPair>
 __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem, int lane, bool first_round, bool report) {
   Misc* misc = misc_of(smem);
   Segment* out = reinterpret_cast<Segment*>(smem_ptr(smem) + kOffSegs);
   int* lens = reinterpret_cast<int*>(smem_ptr(smem) + kOffKV);
-  const int cta = blockIdx.x;
+  int cta = blockIdx.x;
   int n = gridDim.x;
   auto len_of = [&](int i) { return i < kLensMax ? lens[i] : fresh_len(p, i); };
   unsigned long long acc = 0;
@@ -280,6 +296,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     if (lane == 0 && p.status && report) atomicCAS(p.status, 0, MLA_FP4_ERR_UNSUPPORTED);
   } else if (whole_requests(mx > 0 ? int(mx) - kPhantom : 0, int64_t(p.batch) * p.groups, n)) {  // CTA v: pair v, whole
     Tt = flat_t(T64) * p.groups;
+    cta = cta_in_partition<kPair>(p.batch, p.groups);
     if (cta < p.batch * p.groups) {
       const int g = cta / p.batch, b = cta - g * p.batch;
       const int len = len_of(b);
@@ -292,6 +309,8 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     const flat_t T = flat_t(T64);
     Tt = T * p.groups;
     if (p.fused_merge) n = work_ctas(Tt, p.batch * p.groups, n);
+    if (p.share > 1) n = (n + p.share - 1) / p.share * p.share;  // (the grid is a multiple, and so is Tt)
+    cta = cta_in_partition<kPair>(kPair ? n / p.groups : 1, p.groups);
     const flat_t cut = cta_lo(Tt, n, cta + (lane & 1));  // one division for both ends
     const flat_t lo = first_round ? __shfl_sync(0xffffffffu, cut, 0) : misc->next, hi = __shfl_sync(0xffffffffu, cut, 1);
     int g = lo < T ? 0 : int(uint32_t(lo) / uint32_t(T));
@@ -340,6 +359,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     misc->next = next;
     misc->Tt = Tt;
     misc->n = n;
+    if (kPair) misc->cta = cta;
   }
   __syncwarp();
 }
@@ -349,6 +369,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
 // The plan made before the wait stands if the lengths have not changed.  A CTA that starts late, on an SM that the kernel ahead
 // held to its end, finds nothing to wait for: there the lengths are read again while the plan is being made (1.8 us of code that
 // comes from L2 line by line).
+template <bool kPair>
 __device__ __forceinline__ void start_work(const DecodeParams& p, uint32_t smem, int warp, int lane) {
   Misc* misc = misc_of(smem);
   if (p.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -367,7 +388,7 @@ __device__ __forceinline__ void start_work(const DecodeParams& p, uint32_t smem,
       for (int i = lane; i < nb; i += 32) same &= lens[kLensMax + i] == lens[i];
       stands = __all_sync(0xffffffffu, same) && p.batch <= kLensMax && misc->Tt >= 0;
     }
-    if (!stands) stage_segments(p, smem, lane, true, true);
+    if (!stands) stage_segments<kPair>(p, smem, lane, true, true);
     ptx::fence_proxy_async_smem();  // the lengths give way to the first copies
     __threadfence_block();
     asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
@@ -409,7 +430,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
   st.slot = starting ? which : st.slot;
   uint32_t nseg = 0;
   if (!dry) {
-    if (starting) start_work(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+    if (starting) start_work<false>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
     nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   }
 #pragma unroll 1
@@ -488,7 +509,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
       si = 0;
       st = RoleState{};
       st.slot = which;
-      start_work(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+      start_work<false>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
       nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
     }
   }
@@ -1227,13 +1248,18 @@ __device__ __forceinline__ void softmax_role(const DecodeParams& p, uint32_t sme
 // 128..32768 88.2 -> 87.2, 32 requests with 128 heads 40.9 -> 39.9.
 // (On the way, the commit for kBarDrain: nobody can have advanced the generation before this CTA counts itself out, which it does
 // after the drain.)
+template <bool kPair>
 __device__ __noinline__ void publish(const DecodeParams& p, uint32_t smem, int lane) {
   const int nseg = misc_of(smem)->nseg;
   const Segment* sg = segs_of(smem);  // (only a round's first and last segment can be partial)
-  const int even = slot_of(blockIdx.x, true), first = nseg > 0 ? sg[0].slot : -1, last = nseg > 0 ? sg[nseg - 1].slot : -1;
+  const int even = slot_of(cta_of<kPair>(misc_of(smem)), true), first = nseg > 0 ? sg[0].slot : -1, last = nseg > 0 ? sg[nseg - 1].slot : -1;
   const bool head = first == even, tail = last == even + 1;
   const int gen = head || tail ? ld_acquire(ws_generation(p.workspace)) + 1 : 0;
-  if (ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
+  if (!kPair) {
+    if (ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
+  } else if (!(blockIdx.x & 1)) {
+    if (ptx::elect_one()) ptx::umma_commit_pair(bar_addr(smem, kBarDrain));
+  }
   __syncwarp();
   if (!head && !tail) return;
   if (last >= 0) {
@@ -1298,6 +1324,7 @@ __device__ __noinline__ void zero_empty_requests(const DecodeParams& p, int lane
 // the shared form (those whose partial was their first segment: every CTA then takes part in at most one merge) and this
 // CTA's place among them.  The writers are the CTAs whose range holds a real tile; they are consecutive, as no CTA that shares
 // the work is without a tile.
+template <bool kPair>
 __device__ __noinline__ void plan_merge(uint32_t smem, int which, int lane) {
   Misc* misc = misc_of(smem);
   const MergeReq m = misc->merge[which];
@@ -1305,7 +1332,7 @@ __device__ __noinline__ void plan_merge(uint32_t smem, int which, int lane) {
     if (lane == 0) misc->n_slots = 0;
     return;
   }
-  const int n = misc->n, cta = blockIdx.x;
+  const int n = misc->n, cta = cta_of<kPair>(misc);
   const flat_t Tt = misc->Tt;
   const flat_t f0 = m.start + kPhantom;
   const int ends = cta_of_tile(Tt, n, (lane & 1) ? m.start + m.vtiles - 1 : f0);
@@ -1387,6 +1414,28 @@ __device__ __forceinline__ void store_unit(const float (&acc)[8], const float4& 
     if (e < heads) store(e, acc[e] * inv[e]);
 }
 
+// eight dims of one head
+__device__ __forceinline__ void store_dims(const DecodeParams& p, const float (&acc)[8], float inv, size_t at) {
+  if (p.out_dtype == MLA_FP4_OUT_F32) {
+    float4* d = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at);
+    d[0] = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+    d[1] = make_float4(acc[4] * inv, acc[5] * inv, acc[6] * inv, acc[7] * inv);
+  } else {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (p.out_dtype == MLA_FP4_OUT_BF16) {
+        const __nv_bfloat162 t = __floats2bfloat162_rn(acc[2 * i] * inv, acc[2 * i + 1] * inv);
+        w[i] = *reinterpret_cast<const uint32_t*>(&t);
+      } else {
+        w[i] = __nv_cvt_float2_to_fp8x2(make_float2(acc[2 * i] * inv, acc[2 * i + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+      }
+    }
+    if (p.out_dtype == MLA_FP4_OUT_BF16) *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out) + at) = make_uint4(w[0], w[1], w[2], w[3]);
+    else *reinterpret_cast<uint2*>(static_cast<uint8_t*>(p.out) + at) = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+  }
+}
+
 // The merge weights w_i = 2^(lse_i - max) * slot scale of the 64 heads, and the inverse of their sum, by the eight softmax
 // warps: four lanes per head split the slots, butterflies give all four the results.  They are computed while the shares of the
 // slots are on their way: the LSEs come straight from L2, under flags of their own (shared form).
@@ -1455,7 +1504,8 @@ __device__ __noinline__ void merge_weights(const DecodeParams& p, uint32_t smem,
 // out = sum_i w_i * O_i / sum, over the staged shares, in an order that depends on the number of slots and units alone and not on
 // the order of arrival: both forms cut the units into the same shares, so they agree to the bit.  All threads of the CTA; the
 // weights are there.
-__device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, int tid, uint32_t parity) {
+template <bool kPair>
+__device__ __noinline__ void tail_merge_of(const DecodeParams& p, uint32_t smem, int tid, uint32_t parity) {
   Misc* misc = misc_of(smem);
   const int ns = misc->n_slots;
   const MergeReq m = misc->m;
@@ -1475,17 +1525,23 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
   for (int u0 = 0; u0 < nu; u0 += kThreads) {  // (one pass when S > 1)
     const int u = u0 + tid - s * nu;
     bool active = s < S && u < nu;
-    const int unit = U0 + u, hg = unit >> 9, dim = unit & 511;
+    // (a unit is eight heads of a dim, or, in the pair kernel, eight dims of a head)
+    const int unit = U0 + u, hg = unit >> 9, dim = unit & 511, head = unit >> 6;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (active) {
       uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};  // pairs of heads
-      uint32_t src = rows + uint32_t(s) * share + uint32_t(u) * 16u, w = tails + uint32_t(s) * kTailBytes + 32u * uint32_t(hg);
+      uint32_t src = rows + uint32_t(s) * share + uint32_t(u) * 16u, w = tails + uint32_t(s) * kTailBytes + (kPair ? 4u * uint32_t(head) : 32u * uint32_t(hg));
 #pragma unroll 4
       for (int i = s; i < ns; i += S) {
         const uint4 v = lds_u32x4(src);
         uint64_t wp[4];
-        lds_pairs(w, wp[0], wp[1]);
-        lds_pairs(w + 16u, wp[2], wp[3]);
+        if (kPair) {
+          const float wh = lds_f32(w);
+          wp[0] = wp[1] = wp[2] = wp[3] = pack2(wh, wh);
+        } else {
+          lds_pairs(w, wp[0], wp[1]);
+          lds_pairs(w + 16u, wp[2], wp[3]);
+        }
         src += uint32_t(S) * share;
         w += uint32_t(S) * kTailBytes;
         const uint32_t vs[4] = {v.x, v.y, v.z, v.w};
@@ -1511,6 +1567,10 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
           for (int e = 0; e < 8; ++e) acc[e] += lds_f32(red + uint32_t(e) * (kThreads * 4) + uint32_t(k * nu) * 4u);
     }
     if (!active) continue;
+    if (kPair) {
+      if (head < heads_here) store_dims(p, acc, lds_f32(smem + kOffLinv + 4u * uint32_t(head)), (row0 + head) * kLatent + 8 * (unit & 63));
+      continue;
+    }
     const float4 i0 = lds_f32x4(smem + kOffLinv + 32u * uint32_t(hg)), i1 = lds_f32x4(smem + kOffLinv + 32u * uint32_t(hg) + 16u);
     const size_t idx = (row0 + 8 * hg) * kLatent + dim;
     const int heads = heads_here - 8 * hg;
@@ -1529,13 +1589,15 @@ __device__ __noinline__ void tail_merge(const DecodeParams& p, uint32_t smem, in
 
 // The last-writer form: for each request this CTA wrote a partial of, count it in; the last to arrive merges it, share by share.
 // A CTA that has given up counts itself in all the same: the counters are back to zero after every step, whatever became of it.
+template <bool kPair>
 __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem, int tid) {
+  constexpr auto& tail_merge = tail_merge_of<kPair>;
   Misc* misc = misc_of(smem);
   uint32_t parity = 0;
 #pragma unroll 1
   for (int which = 0; which < 2; ++which) {
     if (misc->merge[which].vtiles == 0) continue;
-    if (tid < 32) plan_merge(smem, which, tid);
+    if (tid < 32) plan_merge<kPair>(smem, which, tid);
     __syncthreads();
     const int ns = misc->n_slots, part = misc->n_part;  // (the shares of the shared form, so that both sum in the same order)
     if (tid == 0) {
@@ -1602,7 +1664,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   } else if (warp == kWarpPlan) {
     asm volatile("bar.arrive 7, %0;" ::"n"(kThreads) : "memory");
     if (p.pdl_wait) {  // a first plan, from the lengths as they are in memory; the TMA warp decides whether it stands
-      stage_segments(p, smem, lane, true, false);
+      stage_segments<false>(p, smem, lane, true, false);
       ptx::fence_proxy_async_smem();
       __threadfence_block();
       asm volatile("bar.arrive 8, 64;" ::: "memory");
@@ -1622,7 +1684,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   if (warp != kWarpPlan) ptx::bar_sync(7, kThreads);
   RoleState st{};
   if (warp != kWarpTMA && warp != kWarpTMA2) {  // (these two: in their role, after a first pass without effect)
-    start_work(p, smem, warp, lane);
+    start_work<false>(p, smem, warp, lane);
   }
   ptx::tc_fence_after();
   const uint32_t tmem = ptx::uniform_u32(misc->tmem_base);
@@ -1647,7 +1709,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
           atomicAdd(ws_started(p.workspace), 1);
           misc->gen = ld_acquire(ws_generation(p.workspace)) + 1;
         }
-        plan_merge(smem, 0, lane);
+        plan_merge<false>(smem, 0, lane);
         zero_empty_requests(p, lane);
       }
       pv_role(smem, tmem, st);
@@ -1663,7 +1725,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       if (((warp == kWarpQK && !publishes) || warp == kWarpPV) && ptx::elect_one()) ptx::umma_commit(bar_addr(smem, kBarDrain));
       __syncwarp();
       if (publishes) {
-        publish(p, smem, lane);
+        publish<false>(p, smem, lane);
       } else {
         if (lane == 0) drain_wait(smem, kBarDrain, 0);
         __syncwarp();
@@ -1686,7 +1748,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     if (!more) break;
     first_round = false;
     if (warp == kWarpTMA) {
-      stage_segments(p, smem, lane, false, false);
+      stage_segments<false>(p, smem, lane, false, false);
       ptx::fence_proxy_async_smem();
     }
     __syncthreads();
@@ -1697,8 +1759,8 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   }
   if (p.fused_merge) {
     if (misc->merge[0].vtiles | misc->merge[1].vtiles) {
-      if (misc->mode == kMergeLast) merge_as_last(p, smem, tid);
-      else if (misc->n_slots > 0) tail_merge(p, smem, tid, 0);
+      if (misc->mode == kMergeLast) merge_as_last<false>(p, smem, tid);
+      else if (misc->n_slots > 0) tail_merge_of<false>(p, smem, tid, 0);
     }
     // The last CTA to have counted itself out advances the generation (the next step's flags differ from all of this one's) and
     // resets the counters.
@@ -1710,6 +1772,8 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     }
   }
 }
+
+#include "decode_pair.cuh"  // (in this namespace: it is the other half of this file)
 
 // ------------------------------------------------------------------------------------------ host
 
@@ -1758,8 +1822,8 @@ struct QKey {
 struct KvKey {
   const void* kv;
   int64_t num_pages;
-  int32_t page_size, dev;
-  bool operator==(const KvKey& o) const { return kv == o.kv && num_pages == o.num_pages && page_size == o.page_size && dev == o.dev; }
+  int32_t page_size, rows, dev;  // rows: of a box
+  bool operator==(const KvKey& o) const { return kv == o.kv && num_pages == o.num_pages && page_size == o.page_size && rows == o.rows && dev == o.dev; }
 };
 template <typename Key>
 struct MapPair {
@@ -1784,20 +1848,32 @@ bool encode_q_maps(const DecodeParams& p, CUtensorMap* lat, CUtensorMap* rope) {
          encode_map(rope, p.q, 4, dims, strides, box_rope, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 // the RoPE bytes of a page, and the cache as 4-bit elements: 640 per row (the 512 latent codes, then the RoPE bytes seen as
-// nibbles and never fetched through this map), page_size rows per page; a box is one 128-dim block of one page
-bool encode_kv_maps(const DecodeParams& p, CUtensorMap* lat, CUtensorMap* rope) {
+// nibbles and never fetched through this map), page_size rows per page; a box is one 128-dim block of `rows` rows of a page
+bool encode_kv_maps(const DecodeParams& p, uint32_t rows, CUtensorMap* lat, CUtensorMap* rope) {
   const uint64_t dims[3] = {uint64_t(kRowBytes), uint64_t(p.page_size), uint64_t(p.num_pages)};
   const uint64_t strides[2] = {uint64_t(kRowBytes), uint64_t(kRowBytes) * uint64_t(p.page_size)};
-  const uint32_t box[3] = {64, uint32_t(p.page_size), 1};
+  const uint32_t box[3] = {64, rows, 1};
   if (!encode_map(rope, p.kv_cache, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B)) return false;
   EncodeTiledFn fn = get_encode_fn();
   cuuint64_t gd[3] = {cuuint64_t(2 * kRowBytes), cuuint64_t(p.page_size), cuuint64_t(p.num_pages)};
   cuuint64_t gs[2] = {cuuint64_t(kRowBytes), cuuint64_t(kRowBytes) * cuuint64_t(p.page_size)};
-  cuuint32_t bx[3] = {128, cuuint32_t(p.page_size), 1};
+  cuuint32_t bx[3] = {128, cuuint32_t(rows), 1};
   cuuint32_t es[3] = {1, 1, 1};
   return fn(lat, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, const_cast<void*>(p.kv_cache), gd, gs, bx, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Where the pair kernel is used, as far as the caller's longest length (the width of its block tables) tells.  From twenty tiles a CTA on, where
+// the main loop counts: single -> pair 2x131072 tokens, 128 heads, q_len 2 105.7 -> 96.8 us, 32x(1024..16384), 128 heads 49.7 -> 47.6, 3x30000,
+// 128 heads, q_len 3 52.4 -> 47.5.  And for requests too short to be split, whose rows leave faster: 32x(100..500), 128 heads 13.0 -> 11.4, 1x200
+// 9.7 -> 8.7, 37x(64..512) 13.7 -> 12.6; not with pages of 8 tokens, sixteen copies one after the other for 64 tokens of K (6x110 10.4 -> 10.5).
+// Between the two a pair, whose CTAs wait for each other at every change of request and whose first tiles take longer (four warps a tile), is
+// faster or slower by as much: 1x16000, 128 heads 18.2 -> 16.9, 8x2000 16.8 -> 16.2, 16x(200..4000) 16.6 -> 16.7, 60x(100..2000) 24.4 -> 25.2,
+// 1x4096, 64 heads, q_len 2 13.2 -> 13.5, 2x(924..17749), 64 heads, q_len 2 13.3 -> 13.9.
+bool pair_pays(const DecodeParams& p, int grid) {
+  const int64_t pairs = int64_t(p.batch) * p.groups, tiles = (int64_t(p.seq_cap) + kTile - 1) / kTile;  // at most, of a request
+  return whole_requests(int(tiles < INT_MAX ? tiles : INT_MAX), pairs, grid) ? p.page_size >= 16 : pairs * tiles >= 20 * int64_t(grid);
 }
 
 }  // namespace
@@ -1812,7 +1888,12 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   MapPair<QKey>& qm = q_maps[map_slot(p.q)];
   MapPair<KvKey>& km = kv_maps[map_slot(p.kv_cache)];
   const QKey qkey{p.q, p.q_stride_batch, p.q_stride_qpos, p.q_stride_head, p.batch, p.q_len, p.num_heads, dev};
-  const KvKey kvkey{p.kv_cache, p.num_pages, p.page_size, dev};
+  // Which kernel: see pair_pays.  (Where the pair kernel could be used, the grid and the partition are such as it needs, whichever runs.)
+  const int even_grid = p.fused_merge ? pair_ctas(p.groups, num_ctas) : 0;
+  const int grid = even_grid ? even_grid : num_ctas;
+  const bool pair = even_grid && pair_pays(p, grid);
+  const uint32_t rows = pair && p.page_size > 64 ? 64u : uint32_t(p.page_size);
+  const KvKey kvkey{p.kv_cache, p.num_pages, p.page_size, int32_t(rows), dev};
   if (!(qm.valid && qm.key == qkey)) {
     qm.valid = false;
     if (!encode_q_maps(p, &qm.a, &qm.b)) {
@@ -1824,7 +1905,7 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   }
   if (!(km.valid && km.key == kvkey)) {
     km.valid = false;
-    if (!encode_kv_maps(p, &km.a, &km.b)) {
+    if (!encode_kv_maps(p, rows, &km.a, &km.b)) {
       *err = "cuTensorMapEncodeTiled failed for kv_cache (it must be 32-byte aligned)";
       return cudaErrorInvalidValue;
     }
@@ -1839,13 +1920,18 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
       if (e != cudaSuccess) return e;
       e = cudaFuncSetAttribute(mla_fp4_decode_sm100_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
       if (e != cudaSuccess) return e;
+      e = cudaFuncSetAttribute(mla_fp4_decode_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
+      if (e != cudaSuccess) return e;
+      e = cudaFuncSetAttribute(mla_fp4_decode_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
+      if (e != cudaSuccess) return e;
       if (dev >= 0 && dev < 64) attr_done[dev].store(true, std::memory_order_release);
     }
   }
   // the attention variant with a score transform is a kernel of its own: the standard one carries none of its instructions
-  auto* kernel = p.soft_cap > 0.f ? mla_fp4_decode_sm100_kernel<true> : mla_fp4_decode_sm100_kernel<false>;
+  auto* kernel = pair ? (p.soft_cap > 0.f ? mla_fp4_decode_pair_kernel<true> : mla_fp4_decode_pair_kernel<false>)
+                           : (p.soft_cap > 0.f ? mla_fp4_decode_sm100_kernel<true> : mla_fp4_decode_sm100_kernel<false>);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(num_ctas);
+  cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemAlloc;
   cfg.stream = stream;
@@ -1858,6 +1944,7 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   cfg.numAttrs = p.pdl ? 1 : 0;
   DecodeParams pp = p;
   pp.pdl_wait = p.pdl;
+  pp.share = even_grid ? p.groups : 1;
   pp.page_shift = __builtin_ctz(unsigned(p.page_size));
   return cudaLaunchKernelEx(&cfg, kernel, pp, map_q_lat, map_q_rope, map_rope, map_lat);
 }

@@ -153,7 +153,7 @@ int mla_fp4_plan_partition(const int32_t* seq_lens_host, int32_t batch, int32_t 
 
 /* How many CTAs of a grid of num_ctas share a step's tiles when the decode kernel merges by itself
    (MLA_FP4_KERNEL_TCGEN05): with few tiles, fewer than the grid, since each CTA more is a partial
-   more to merge.  mla_fp4_plan_partition over this many CTAs is that kernel's partition; the
+   more to merge (with an even number of head groups, a multiple of the groups).  mla_fp4_plan_partition over this many CTAs is that kernel's partition; the
    other kernels use the whole grid.  (Beyond a thousand tiles a CTA, some 19 M tokens in one
    request, the kernel's number may be one off.) */
 int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len, int32_t num_heads,

@@ -1,0 +1,100 @@
+"""The decode kernel for an even number of head groups (two CTAs, two groups of the same tiles) where it can go wrong: edges of tiles,
+half tiles and pages, many requests in one pair's walk, heads that fill no group, every output type and variant, both merge
+forms, references that move, a wait that runs out.  Against the oracle, and against the other kernel (the two-kernel mode uses it).  The grids are
+so small that there are twenty tiles or more to a CTA, or the requests so
+short that they are not split: there this kernel is used."""
+import pytest
+import torch
+
+from oracle import mla_fp4_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(lens, heads, page, q_len, max_ctas=None, out_dtype=None, variant=None, sharp=1.0, latent="normal", forms=(0, 4), **ref_kw):
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, _cabi, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("pair", [max(n, 1) for n in lens], heads, page, q_len=q_len, seed=sum(lens) + heads, device=dev, latent_dist=latent)
+    case.seq_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=heads, page_size=page, max_ctas=max_ctas, out_dtype=out_dtype, variant=variant)
+    scale, got = case.softmax_scale * sharp, []
+    for kernel, mask in [(_cabi.KERNEL_TCGEN05, f) for f in forms] + [(_cabi.KERNEL_TCGEN05_2PASS, 0)]:
+        w._kernel, w._phase_mask = kernel, mask
+        got.append(w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, scale, kv_cache_sf=case.kv_cache_sf, return_lse=True))
+        torch.cuda.synchronize()
+        w.check_device_status()
+    ref, ref_lse = O.mla_decode(case.q, case.kv_cache, case.kv_cache_sf, case.block_tables, case.seq_lens, scale, **ref_kw)
+    return got, ref, ref_lse
+
+
+@pytest.mark.parametrize("lens,heads,page,q_len,max_ctas", [
+    ([1, 63, 64, 65, 127, 128, 129, 0, 512], 128, 64, 1, 2),   # half tiles with and without tokens
+    ([1, 63, 64, 65, 127, 128, 129, 1025], 65, 128, 1, 2),            # one pair walks them all; pages copied by halves; one head in a group
+    ([57, 120, 513, 1025], 100, 8, 2, 4),
+    ([130] * 37 + [900], 128, 16, 1, 2),                          # more requests than a round holds
+    ([640, 2304, 5000], 40, 32, 2, 8),                            # partials at both ends of a walk
+    ([30000, 500, 9000], 128, 64, 3, None),                             # six groups: 144 of the 148 CTAs
+    ([50000], 128, 64, 1, 36),
+    ([300, 400, 500, 512, 100, 200, 300, 64, 65], 128, 64, 1, 36), # short requests, whole
+])
+@pytest.mark.parametrize("latent,sharp", [("normal", 1.0), ("student_t3", 8.0)])
+def test_pairs_of_groups(lens, heads, page, q_len, max_ctas, latent, sharp):
+    got, ref, ref_lse = _run(lens, heads, page, q_len, max_ctas, torch.float32, sharp=sharp, latent=latent)
+    live = torch.isfinite(ref_lse)
+    for out, lse in got:
+        O.assert_parity(out, ref, "pairs")
+        torch.testing.assert_close(lse.cpu()[live], ref_lse[live], atol=2e-3, rtol=1e-4)
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])  # both merge forms
+    # P' has about eight bits on either side: the parity bar against the oracle, twice
+    diff = (got[0][0] - got[2][0]).float().cpu()
+    assert float(diff.abs().max()) <= 2 * O.MAXABS_OVER_RMS_BAR * float(ref.float().pow(2).mean(-1).sqrt().max())
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32, torch.float8_e4m3fn])
+@pytest.mark.parametrize("lens,max_ctas", [([90, 300], None), ([5000, 700], 16)])
+def test_pairs_output_types_and_variants(out_dtype, lens, max_ctas):
+    from flashinfer_mla_fp4_b200 import SoftCappingAttention
+
+    sink = torch.linspace(-3.0, 3.0, 96)
+    got, ref, ref_lse = _run(lens, 96, 64, 2, max_ctas, out_dtype, SoftCappingAttention(25.0, sink.cuda()), forms=(0,), sink=sink, logits_soft_cap=25.0)
+    if out_dtype == torch.float8_e4m3fn:  # half a unit in the last place of E4M3 (2^-4 of the value, 2^-10 below its normal range) beside P'
+        err = (got[0][0].float().cpu() - ref.float()).abs()
+        assert bool((err <= ref.float().abs() * 0.0625 + 2.0 ** -10 + 2e-2 * ref.float().pow(2).mean(-1, keepdim=True).sqrt()).all())
+    else:
+        O.assert_parity(got[0][0], ref, "pairs, variants")
+    torch.testing.assert_close(got[0][1].cpu(), ref_lse, atol=2e-3, rtol=1e-4)
+
+
+def test_a_pair_that_gave_up_leaves_the_workspace_consistent():
+    """A page id outside the pool: the copy is never issued (for CTA 0's or CTA 1's half of a tile), CTA 0's bounded wait runs out and takes
+    the partner along; the next step on the same workspace is right."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, _cabi, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("gave up", [3000, 5000], 128, 64, seed=21, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=128, page_size=64, max_ctas=8)
+
+    def step(tables):
+        out = w.run(case.q, case.kv_cache, tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
+        torch.cuda.synchronize()
+        return out
+
+    good = step(case.block_tables)
+    w.check_device_status()
+    for page in (40, 41):
+        bad = case.block_tables.clone()
+        bad[1, page] = case.kv_cache.shape[0] + 5
+        w._wait_polls = 2000
+        step(bad)
+        assert w.device_status()[0] == _cabi.ERR_DEVICE_TIMEOUT
+        w._wait_polls = 0
+        w._status.zero_()
+        assert torch.equal(step(case.block_tables), good)
+        assert w.device_status()[0] == 0
