@@ -102,7 +102,7 @@ constexpr int kBarRopeFull = 2 * kRing + 4, kBarRopeEmpty = 2 * kRing + 5, kBarP
               kBarQFull = 2 * kRing + 8, kBarQEmpty = 2 * kRing + 9, kBarOFree = 2 * kRing + 10, kBarDrain = 2 * kRing + 11,
               kBarTail = 2 * kRing + 12, kBarQkIssued = 2 * kRing + 13, kBarPvIssued = 2 * kRing + 14,
               kBarScale = 2 * kRing + 15;  // pair kernel: scales of a tile, four stages
-constexpr int kNumBars = 2 * kRing + 15 + kScaleStages;
+constexpr int kNumBars = kBarScale + kScaleStages;
 static_assert(kNumBars <= 32, "initialised by one warp, a barrier per lane");
 constexpr uint32_t kOffTail = (kOffBars + kNumBars * 8 + 15u) & ~15u;     // merge plan: [148] slot ids
 constexpr uint32_t kOffSegs = kOffTail + kMaxCombineSlots * 4;            // Segment[kMaxSeg]
@@ -244,7 +244,8 @@ __device__ __forceinline__ int fresh_len(const DecodeParams& p, int i) {  // fro
 // 17.4 / 15.8.  Approximate arithmetic will do: every CTA takes the same steps, and any 1 <= n <= Tt is right.  (The host's form of this
 // rule, mla_fp4_work_ctas, is exact; the two agree while no walk is longer than a thousand tiles: where the root decides, Tt * pairs is
 // below n^2 / 25, so that its argument keeps clear of the squares by more than the 1e-3 allows for.)
-__device__ __forceinline__ int work_ctas(flat_t Tt, int pairs, int n) {
+// With an even number of groups the number is a multiple of them (share): that many times what one group's tiles, T, need for the same walk.
+__device__ __forceinline__ int work_ctas(flat_t Tt, flat_t T, int share, int pairs, int n) {
   if (Tt > 5 * n && pairs > 1) return n;  // the whole grid, and next to nothing to gain from the rounding
   const float tiles = float(Tt);
   float best, r;
@@ -252,15 +253,13 @@ __device__ __forceinline__ int work_ctas(flat_t Tt, int pairs, int n) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fminf(float(n), best)));
   const float k = float(__float2int_ru(tiles * r - 1e-3f));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(k));
-  return min(n, max(1, __float2int_ru(tiles * r - 1e-3f)));
+  return min(n, share * max(1, __float2int_ru(float(share > 1 ? T : Tt) * r - 1e-3f)));
 }
 // This CTA's place in the partition.  In the pair kernel the two CTAs of a cluster walk the same tiles for two neighbouring head groups.
 // There the working CTAs are a multiple of the groups, so that every group is shared by as many, `per`, in ranges of its own tiles that are
 // the same for all groups: cluster w takes range w mod per of the groups 2 (w / per) and 2 (w / per) + 1.  (Short requests: `per` is the
 // batch.)  The partition is thus the one of the other kernel, on other CTAs.
-template <bool kPair>
 __device__ __forceinline__ int cta_in_partition(int per, int groups) {
-  if (!kPair) return blockIdx.x;
   const int w = int(blockIdx.x >> 1), gp = int(uint32_t(w) / uint32_t(per));
   return 2 * gp < groups ? (2 * gp + int(blockIdx.x & 1)) * per + (w - gp * per) : per * groups;  // (beyond the last: no work)
 }
@@ -296,7 +295,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     if (lane == 0 && p.status && report) atomicCAS(p.status, 0, MLA_FP4_ERR_UNSUPPORTED);
   } else if (whole_requests(mx > 0 ? int(mx) - kPhantom : 0, int64_t(p.batch) * p.groups, n)) {  // CTA v: pair v, whole
     Tt = flat_t(T64) * p.groups;
-    cta = cta_in_partition<kPair>(p.batch, p.groups);
+    if (kPair) cta = cta_in_partition(p.batch, p.groups);
     if (cta < p.batch * p.groups) {
       const int g = cta / p.batch, b = cta - g * p.batch;
       const int len = len_of(b);
@@ -308,9 +307,8 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
   } else if (T64 > 0) {
     const flat_t T = flat_t(T64);
     Tt = T * p.groups;
-    if (p.fused_merge) n = work_ctas(Tt, p.batch * p.groups, n);
-    if (p.share > 1) n = (n + p.share - 1) / p.share * p.share;  // (the grid is a multiple, and so is Tt)
-    cta = cta_in_partition<kPair>(kPair ? n / p.groups : 1, p.groups);
+    if (p.fused_merge) n = work_ctas(Tt, T, p.share, p.batch * p.groups, n);
+    if (kPair) cta = cta_in_partition(n / p.groups, p.groups);
     const flat_t cut = cta_lo(Tt, n, cta + (lane & 1));  // one division for both ends
     const flat_t lo = first_round ? __shfl_sync(0xffffffffu, cut, 0) : misc->next, hi = __shfl_sync(0xffffffffu, cut, 1);
     int g = lo < T ? 0 : int(uint32_t(lo) / uint32_t(T));
