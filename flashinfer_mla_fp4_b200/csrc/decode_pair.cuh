@@ -20,7 +20,10 @@
 // four threads share a head.
 //
 // CTA 0 of the cluster issues all MMAs.  What it waits for it is told by both CTAs at its own barriers (remote arrivals, copies that
-// report to it); what both wait for arrives as a commit with multicast.  The roles and the merge are those of the other kernel; the two issue
+// report to it); what both wait for arrives as a commit with multicast.  An arrival at the other CTA that stands for work done (S read, P' stored, O
+// rescaled or read out) releases at cluster scope, behind its proxy and tcgen05 fences, and every wait acquires at that scope.  The release is a
+// fence of shared memory alone: 2x131072 tokens, 128 heads, q_len 2 95.9 us without it, 95.8 with it, 1x200 8.68 and 8.72; as
+// mbarrier.arrive.release.cluster, which waits for stores to global memory too, 142, and passed on by the idle issue warps of CTA 1 102.6.  The roles and the merge are those of the other kernel; the two issue
 // warps take no turns (with QK^T held to two tiles ahead of PV a tile took 2670 to 2800 clk, without 1840).
 
 // shared memory map of the big part; from kOffP on as in the other kernel
@@ -48,13 +51,13 @@ constexpr uint32_t kPairIdescQK = ptx::idesc_e4m3(128, 128, false, false) | kFmt
 constexpr uint32_t kPairIdescPV = ptx::idesc_e4m3(128, 256, false, true) | kFmtE2M1B;
 
 __device__ __forceinline__ uint32_t leader_bar(uint32_t smem, int idx) { return ptx::mapa(bar_addr(smem, idx), 0); }
-// Bounded wait as in the other kernel; a CTA that gives up takes its partner along.
+// Bounded wait as in the other kernel, acquiring at cluster scope; a CTA that gives up takes its partner along.
 __device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t parity) {
   Misc* m = misc_of(smem);
   const uint32_t bar = bar_addr(smem, idx), polls = m->polls;
 #pragma unroll 1
   for (uint32_t i = 0; i < polls; ++i) {
-    if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar, parity))) return true;
+    if (__all_sync(0xffffffffu, ptx::mbar_try_wait_cluster(bar, parity))) return true;
     if (__any_sync(0xffffffffu, m->abort)) return false;
     if (i > 4096) __nanosleep(128);
   }
@@ -66,7 +69,7 @@ __device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t par
   return false;
 }
 __device__ __forceinline__ bool pair_wait(uint32_t smem, int idx, uint32_t parity) {
-  if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar_addr(smem, idx), parity))) return true;
+  if (__all_sync(0xffffffffu, ptx::mbar_try_wait_cluster(bar_addr(smem, idx), parity))) return true;
   return __all_sync(0xffffffffu, pair_wait_slow(smem, idx, parity));
 }
 
@@ -126,14 +129,14 @@ __device__ __forceinline__ void pair_tma_role(const DecodeParams& p, uint32_t sm
         }
       };
       if (which && st.it == 0) scales();
-      if (st.it >= 2) ok = wait(smem, which ? pbar_pv_empty(s) : pbar_qk_empty(s), ((st.it >> 1) - 1) & 1);
+      if (st.it >= 2) ok = pair_wait(smem, which ? pbar_pv_empty(s) : pbar_qk_empty(s), ((st.it >> 1) - 1) & 1);
       if (!ok) break;
       const int full = which ? pbar_pv_full(s) : pbar_qk_full(s);
       // the bytes of both CTAs (a 4-bit copy counts its packed bytes: 64 per row and block)
       if (e && rank == 0) ptx::mbar_arrive_expect_tx(bar_addr(smem, full), uint32_t(subs) * sub * (which ? 256u : 320u));
       const uint32_t bar = leader_bar(smem, full);
       // (CTA 1 may have nothing to copy for QK^T, in a tile of at most 64 tokens; CTA 0 must not run ahead of this warp's waits then)
-      if (e && rank && !which) ptx::mbar_arrive_cluster(bar);
+      if (e && rank && !which) ptx::mbar_arrive_relaxed_cluster(bar);
       const uint32_t dst = smem + (which ? kPairOffPv + s * kPairPvBytes : kPairOffQk + s * kPairQkBytes);
       auto copy = [&](uint32_t issue, int page, int i) {
         const uint32_t rows = uint32_t(i) * sub;                                          // in the destination
@@ -406,7 +409,7 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
     for (int tt = g.tile_begin + ((int(it0) ^ grp) & 1); tt < g.tile_end; tt += 2) {
       const uint32_t it = it0 + uint32_t(tt - g.tile_begin), half_it = it >> 1;
       const bool first = tt == g.tile_begin;
-      (void)wait(smem, kBarScale + int(it & (kScaleStages - 1)), (it / kScaleStages) & 1);
+      (void)pair_wait(smem, kBarScale + int(it & (kScaleStages - 1)), (it / kScaleStages) & 1);
       const int live = g.seq_len - (tt * kTile + 64 * upper);  // tokens of this warp's 64 that exist (any number)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -417,7 +420,7 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
         sts_f32(tok + 256 + 128 * i + 4 * lane, __log2f(fmaxf(fabsf(sc), 8.67361738e-19f)));  // floor 2^-60
       }
       __syncwarp();
-      (void)wait(smem, bar_s_full(grp), half_it & 1);
+      (void)pair_wait(smem, bar_s_full(grp), half_it & 1);
       ptx::tc_fence_after();
       // The scores, and the largest x c + log2|scale|.
       uint64_t x2[2 * kPairs];
@@ -458,7 +461,7 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
       }
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(bar_s);
+      if (lane == 0) ptx::mbar_arrive_release_cluster(bar_s);
       if (live < 64) {  // tokens beyond seq_len have no say
         mx = -INFINITY;
 #pragma unroll
@@ -522,9 +525,9 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
         t2[1] = add2(t2[1], x2[2 * q + 1]);
       }
       l2 = add2(l2, add2(t2[0], t2[1]));
-      if (it >= 2) (void)wait(smem, pbar_pv_empty(uint32_t(grp)), (half_it - 1) & 1);  // this group's P buffer is free
+      if (it >= 2) (void)pair_wait(smem, pbar_pv_empty(uint32_t(grp)), (half_it - 1) & 1);  // this group's P buffer is free
       if (moved && !first && __any_sync(0xffffffffu, f != 1.f)) {  // O holds earlier tiles of the segment, all of them now
-        (void)wait(smem, pbar_pv_empty(uint32_t(grp ^ 1)), ((it - 1) >> 1) & 1);
+        (void)pair_wait(smem, pbar_pv_empty(uint32_t(grp ^ 1)), ((it - 1) >> 1) & 1);
         ptx::tc_fence_after();
         pair_rescale(tmem_lane, f);
       }
@@ -537,7 +540,7 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
       ptx::fence_proxy_async_smem();
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(bar_p);
+      if (lane == 0) ptx::mbar_arrive_release_cluster(bar_p);
     }
     st.it = it0 + uint32_t(g.tile_end - g.tile_begin);
     r += uint32_t(g.tile_end - g.tile_begin);
@@ -586,7 +589,7 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
         if (si == nseg - 1 && !misc->more) asm volatile("bar.arrive 6, %0;" ::"n"(kGroupHeads + 32) : "memory");
       }
     }
-    (void)wait(smem, pbar_pv_empty((st.it - 1) & 1), ((st.it - 1) >> 1) & 1);  // the PV of the last tile
+    (void)pair_wait(smem, pbar_pv_empty((st.it - 1) & 1), ((st.it - 1) >> 1) & 1);  // the PV of the last tile
     ptx::tc_fence_after();
     if (!ptx::bar_or(1, kSoftmaxThreads, misc->abort != 0)) {
       if (g.slot >= 0) {
@@ -605,7 +608,7 @@ __device__ __forceinline__ void pair_softmax_role(const DecodeParams& p, uint32_
     }
     ptx::tc_fence_before();
     __syncwarp();
-    if (lane == 0) ptx::mbar_arrive_cluster(bar_o);
+    if (lane == 0) ptx::mbar_arrive_release_cluster(bar_o);
     if (si + 1 < nseg) ptx::bar_sync(1, kSoftmaxThreads);  // the rows of all warps have left the P buffer
     pending |= g.slot >= 0;
   }
@@ -710,7 +713,7 @@ mla_fp4_decode_pair_kernel(const __grid_constant__ DecodeParams p, const __grid_
       if (warp == kWarpQK) {
         publish<true>(p, smem, lane);
       } else {
-        if (lane == 0) drain_wait(smem, kBarDrain, 0);
+        if (lane == 0) drain_wait<true>(smem, kBarDrain, 0);
         __syncwarp();
         if (warp == kWarpPV && lane == 0) {
           if (misc->merge[0].vtiles | misc->merge[1].vtiles) misc->mode = merge_mode(p);

@@ -186,12 +186,13 @@ __device__ __forceinline__ bool wait(uint32_t smem, int idx, uint32_t parity) {
   return __all_sync(0xffffffffu, wait_slow(smem, idx, parity));  // (already the same in all lanes; the vote says so to the compiler)
 }
 // Bounded wait that ignores the abort flag: lets in-flight asynchronous work land before exit.
+template <bool kCluster = false>
 __device__ __noinline__ void drain_wait(uint32_t smem, int idx, uint32_t parity) {
   const uint32_t bar = bar_addr(smem, idx), polls = misc_of(smem)->polls;
   const uint32_t limit = polls < (1u << 20) ? polls : (1u << 20);
 #pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
-    if (ptx::mbar_try_wait(bar, parity)) return;
+    if (kCluster ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity)) return;
     __nanosleep(64);
   }
 }

@@ -11,7 +11,13 @@ SOURCE = Path(__file__).resolve().parent.parent / "flashinfer_mla_fp4_b200" / "c
 COUNTS = {"qk_full": 2, "pv_full": 2, "q_full": 2, "s_empty": 2, "p_full": 2, "o_free": 4, "epilogue": 2}  # (a group of softmax warps counts once)
 
 
-def programs(segments, both_copy=True):
+def both_cta_report_k():
+    """Whether the K copy warp of CTA 1 arrives at CTA 0's barrier for every tile, as the source has it."""
+    role = re.search(r"void pair_tma_role\(.*?\n}\n", SOURCE.read_text(), re.S).group(0)
+    return bool(re.search(r"if \([^)]*rank && !which\) ptx::mbar_arrive", role))
+
+
+def programs(segments, both_copy):
     """Roles: QK^T, PV, Q loads of CTA 1, two softmax groups, a K copy warp (with the scales) and a V copy warp in each CTA."""
     qk, pv, q1, load_v, load_k = [], [], [], [[], []], [[], []]
     soft = [[[], []], [[], []]]  # [CTA][parity of the tile]
@@ -97,10 +103,24 @@ def explore(roles):
 
 @pytest.mark.parametrize("segments", [(1, 1, 1), (5,), (2, 1), (1, 2), (3, 1)])
 def test_no_wait_passes_for_another_phase(segments):
-    assert explore(programs(segments)) == set()
+    assert explore(programs(segments, both_cta_report_k())) == set()
 
 
 def test_the_model_finds_a_copy_warp_left_behind():
     """Without an arrival of CTA 1 for tiles of which it copies nothing, CTA 0 runs ahead of that warp's waits."""
     assert "deadlock" in explore(programs((3,), both_copy=False))
-    assert "if (e && rank && !which) ptx::mbar_arrive_cluster(bar);" in SOURCE.read_text()
+
+
+def test_what_passes_between_the_ctas_is_ordered_between_them():
+    """What no run can be relied on to show: an arrival at the other CTA's barrier that stands for work done releases at cluster scope, and
+    every wait acquires at that scope (without a scope both would hold within a CTA alone)."""
+    ptx = (SOURCE.parent / "ptx_sm100.cuh").read_text()
+    for op in re.findall(r"mbarrier\.arrive\S*shared::cluster\S*", ptx):
+        assert op.startswith(("mbarrier.arrive.release.cluster.", "mbarrier.arrive.relaxed.cluster.")), op
+    release = re.search(r"void mbar_arrive_release_cluster\(.*?\n}", ptx, re.S).group(0)
+    assert release.index("fence.release.sync_restrict::shared::cta.cluster;") < release.index("mbarrier.arrive.relaxed.cluster")
+    assert ".acquire.cluster." in re.search(r"bool mbar_try_wait_cluster\(.*?\n}", ptx, re.S).group(0)
+    text = SOURCE.read_text()
+    assert "mbar_try_wait(" not in text and not re.search(r"[^_]wait\(smem", text)
+    relaxed = re.findall(r".*mbar_arrive_relaxed_cluster.*", text)
+    assert len(relaxed) == 1 and "!which" in relaxed[0]  # (a count alone: the copies report for themselves)
