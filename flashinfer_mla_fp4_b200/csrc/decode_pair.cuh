@@ -51,7 +51,10 @@ constexpr uint32_t kPairIdescQK = ptx::idesc_e4m3(128, 128, false, false) | kFmt
 constexpr uint32_t kPairIdescPV = ptx::idesc_e4m3(128, 256, false, true) | kFmtE2M1B;
 
 __device__ __forceinline__ uint32_t leader_bar(uint32_t smem, int idx) { return ptx::mapa(bar_addr(smem, idx), 0); }
-// Bounded wait as in the other kernel, acquiring at cluster scope; a CTA that gives up takes its partner along.
+// Bounded wait as in the other kernel, acquiring at cluster scope.  A CTA that gives up takes its partner along, whichever role's wait it was, and
+// the partner is flagged first: once a CTA is, its softmax warps run through the rest of their tiles and still report them, two of which CTA 0
+// could take for one of both CTAs'; but whatever CTA 0 does after such a report, it does as a flagged CTA, which writes no rows.  (Softmax warps that
+// report nothing after a failed wait instead: 1x200 8.69 -> 8.84 us, by the flag, -> 8.92, by the waits' results.)
 __device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t parity) {
   Misc* m = misc_of(smem);
   const uint32_t bar = bar_addr(smem, idx), polls = m->polls;
@@ -62,8 +65,9 @@ __device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t par
     if (i > 4096) __nanosleep(128);
   }
   if ((threadIdx.x & 31) == 0) {
-    flag_timeout(smem, idx, parity);
     ptx::st_cluster_u32(ptx::mapa(smem + kOffMisc + uint32_t(offsetof(Misc, abort)), ptx::cluster_ctarank() ^ 1u), 1u);
+    ptx::fence_cluster();
+    flag_timeout(smem, idx, parity);
   }
   __syncwarp();
   return false;

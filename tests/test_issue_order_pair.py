@@ -35,6 +35,7 @@ def programs(segments, both_copy):
                 qk.append(("wait", f"s_empty{s}", half - 1))
             qk += [("wait", f"qk_full{s}", half), ("mma", tuple(f"{b}{s}.{c}" for b in ("s_full", "qk_empty") for c in (0, 1)))]
             pv += [("wait", f"pv_full{s}", half), ("wait", f"p_full{s}", half)]
+            pv += [("seen", "tiles_of.0", it + 1), ("seen", "tiles_of.1", it + 1)]  # (P' of this tile, of both CTAs)
             pv += [("mma", (f"pv_empty{s}.0", f"pv_empty{s}.1"))]
             for c in (0, 1):
                 load_k[c] += [("wait", f"qk_empty{s}.{c}", half - 1)] if it >= 2 else []
@@ -46,7 +47,7 @@ def programs(segments, both_copy):
                 ops += ([("wait", f"ref{1 - s}.{c}", (it - 1) >> 1)] if it else []) + ([("arrive", f"ref{s}.{c}")] if it + 1 < total else [])
                 ops += [("wait", f"pv_empty{s}.{c}", half - 1)] if it >= 2 else []
                 ops += [("wait", f"pv_empty{1 - s}.{c}", (it - 1) >> 1)] if t else []  # (where O is rescaled)
-                ops.append(("arrive", f"p_full{s}"))
+                ops += [("arrive", f"p_full{s}"), ("arrive", f"tiles_of.{c}")]
             it += 1
         qk.append(("mma", ("q_empty.0", "q_empty.1")))
         for c in (0, 1):
@@ -83,7 +84,10 @@ def explore(roles):
             if pcs[r] == len(ops):
                 continue
             op, q = ops[pcs[r]], pipe
-            if op[0] == "wait":
+            if op[0] == "seen":
+                if done[at[op[1]]] < op[2] and not ("flag.0" in at and done[at["flag.0"]]):  # (a flagged CTA writes nothing)
+                    faults.add(f"{op[1]}: {done[at[op[1]]]} of {op[2]}")
+            elif op[0] == "wait":
                 phases = done[at[op[1]]] // count[at[op[1]]]
                 if (phases & 1) == (op[2] & 1):  # the phase of this parity is the running one
                     continue
@@ -109,6 +113,23 @@ def test_no_wait_passes_for_another_phase(segments):
 def test_the_model_finds_a_copy_warp_left_behind():
     """Without an arrival of CTA 1 for tiles of which it copies nothing, CTA 0 runs ahead of that warp's waits."""
     assert "deadlock" in explore(programs((3,), both_copy=False))
+
+
+@pytest.mark.parametrize("partner_first", [None, False])
+def test_a_cta_that_gave_up_takes_its_partner_along(partner_first):
+    """Softmax warps of CTA 1 whose waits fail go through the rest of their tiles at once and report them: CTA 0 may take two tiles of theirs
+    for one of both CTAs', but only if it has been flagged by then."""
+    slow = re.search(r"bool pair_wait_slow\(.*?\n}\n", SOURCE.read_text(), re.S).group(0)
+    order = [slow.find(t) for t in ("ptx::st_cluster_u32(", "ptx::fence_cluster()", "flag_timeout(")]
+    if partner_first is None:  # as the source has it
+        partner_first = -1 < order[0] < order[1] < order[2]
+        assert partner_first
+    roles = programs((4,), True)
+    for ops in roles[-2:]:  # CTA 1's softmax groups
+        ops[:] = [("wait", "flag.1", 0)] + [op for op in ops if op[0] == "arrive"]
+    flags = [("arrive", "flag.0"), ("seen", "flag.0", 0), ("arrive", "flag.1")]  # (a point at which others may run)
+    roles.append(flags if partner_first else flags[::-1])
+    assert any(f.startswith("tiles_of.0") for f in explore(roles)) != partner_first
 
 
 def test_what_passes_between_the_ctas_is_ordered_between_them():
