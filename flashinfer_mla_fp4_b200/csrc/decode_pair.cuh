@@ -55,11 +55,12 @@ __device__ __forceinline__ uint32_t leader_bar(uint32_t smem, int idx) { return 
 // the partner is flagged first: once a CTA is, its softmax warps run through the rest of their tiles and still report them, two of which CTA 0
 // could take for one of both CTAs'; but whatever CTA 0 does after such a report, it does as a flagged CTA, which writes no rows.  (Softmax warps that
 // report nothing after a failed wait instead: 1x200 8.69 -> 8.84 us, by the flag, -> 8.92, by the waits' results.)
-__device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t parity) {
+__device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t parity, uint32_t tiles) {
   Misc* m = misc_of(smem);
-  const uint32_t bar = bar_addr(smem, idx), polls = m->polls;
+  const uint32_t bar = bar_addr(smem, idx);
+  const uint64_t polls = uint64_t(m->polls) * tiles;
 #pragma unroll 1
-  for (uint32_t i = 0; i < polls; ++i) {
+  for (uint64_t i = 0; i < polls; ++i) {
     if (__all_sync(0xffffffffu, ptx::mbar_try_wait_cluster(bar, parity))) return true;
     if (__any_sync(0xffffffffu, m->abort)) return false;
     if (i > 4096) __nanosleep(128);
@@ -72,9 +73,10 @@ __device__ __noinline__ bool pair_wait_slow(uint32_t smem, int idx, uint32_t par
   __syncwarp();
   return false;
 }
-__device__ __forceinline__ bool pair_wait(uint32_t smem, int idx, uint32_t parity) {
+// tiles: how many tiles the wait may span (the budget of polls is that of one)
+__device__ __forceinline__ bool pair_wait(uint32_t smem, int idx, uint32_t parity, uint32_t tiles = 1) {
   if (__all_sync(0xffffffffu, ptx::mbar_try_wait_cluster(bar_addr(smem, idx), parity))) return true;
-  return __all_sync(0xffffffffu, pair_wait_slow(smem, idx, parity));
+  return __all_sync(0xffffffffu, pair_wait_slow(smem, idx, parity, tiles));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -212,10 +214,11 @@ __device__ __forceinline__ void pair_qk_role(const DecodeParams& p, uint32_t sme
   const Desc q_rope = make_desc(smem + kOffQRope, 16, 512, 4), q_lat = make_desc(smem + kOffQLat, 16, 1024, 2);
   const Desc k_lat = make_desc(smem + kPairOffQk, 16, 1024, 2), k_rope = make_desc(smem + kPairOffQk + kBlocks * 8192, 16, 512, 4);
   bool ok = true;
+  uint32_t spans = 1;  // CTA 1 has no QK^T to issue: its wait for the end of a segment's spans all of its tiles
 #pragma unroll 1
   for (uint32_t si = 0; si < nseg && ok; ++si, ++st.seg) {
     const Segment g = sg[si];
-    if (st.seg >= 1 && !pair_wait(smem, kBarQEmpty, (st.seg - 1) & 1)) break;
+    if (st.seg >= 1 && !pair_wait(smem, kBarQEmpty, (st.seg - 1) & 1, spans)) break;
     int qpos, head0;
     group_coords(g.g, p.num_heads, qpos, head0);
     if (ptx::elect_one()) {
@@ -227,8 +230,11 @@ __device__ __forceinline__ void pair_qk_role(const DecodeParams& p, uint32_t sme
         ptx::tma_load_4d_pair(smem + kOffQLat + j * kGroupHeads * 128, map_q_lat, bar, 128 * j, head0, qpos, g.b);
     }
     __syncwarp();
-    if (rank) continue;
     const uint32_t n = ptx::uniform_u32(uint32_t(g.tile_end - g.tile_begin));
+    if (rank) {
+      spans = n + 1;
+      continue;
+    }
     ok = pair_wait(smem, kBarQFull, st.seg & 1);
 #pragma unroll 1
     for (uint32_t t = 0; t < n && ok; ++t, ++st.it) {

@@ -113,8 +113,8 @@ typedef struct MlaFp4DecodeArgs {
      beyond it: a seq_lens entry larger than max_pages_per_request * page_size is treated as
      that many tokens.  0 = not given (rows are trusted to cover seq_lens). */
   int32_t max_pages_per_request;
-  /* Poll budget of every bounded device-side wait (0 = the default, 2^22).  When a wait runs
-     out the kernel records MLA_FP4_ERR_DEVICE_TIMEOUT in the status words and returns. */
+  /* Poll budget of every bounded device-side wait (0 = the default, 2^22); a wait that spans several
+     tiles of other warps' work has it once per tile.  When a wait runs out the kernel records MLA_FP4_ERR_DEVICE_TIMEOUT in the status words and returns. */
   int32_t wait_polls;
   /* Attention variants, compiled into the kernels (the reference passes an AttentionVariant object whose hooks are
      traced into its kernel, wrappers/batch_mla_fp4.py:237-253; the two hooks in use there are restated as data):

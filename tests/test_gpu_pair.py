@@ -98,3 +98,28 @@ def test_a_pair_that_gave_up_leaves_the_workspace_consistent():
         w._status.zero_()
         assert torch.equal(step(case.block_tables), good)
         assert w.device_status()[0] == 0
+
+
+def test_a_small_poll_budget_is_a_budget_of_tiles():
+    """CTA 1's QK^T warp has nothing to issue and waits for a whole segment at a time: a long correct step runs to its end with a budget
+    that covers a tile."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("polls", [200000, 200], 128, 64, seed=3, device=dev)  # one pair of CTAs: 1563 tiles, then two
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=128, page_size=64, max_ctas=2)
+
+    def step():
+        out = w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
+        torch.cuda.synchronize()
+        return out
+
+    expect = step()
+    w.check_device_status()
+    w._wait_polls = 32
+    got, status = step(), w.device_status()
+    assert status[0] == 0, status
+    assert torch.equal(got, expect)
