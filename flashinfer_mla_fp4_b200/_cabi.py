@@ -71,6 +71,7 @@ EXPORTS = (
     "mla_fp4_workspace_init",
     "mla_fp4_plan_partition",
     "mla_fp4_work_ctas",
+    "mla_fp4_decode_plan",
     "mla_fp4_decode",
     "mla_fp4_merge_partials",
     "mla_fp4_dequant_e2m1_to_e4m3",
@@ -109,6 +110,8 @@ def _load() -> C.CDLL:
     lib.mla_fp4_plan_partition.restype = C.c_int
     lib.mla_fp4_work_ctas.argtypes = [i32p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, i32p]
     lib.mla_fp4_work_ctas.restype = C.c_int
+    lib.mla_fp4_decode_plan.argtypes = [C.c_int32] * 6 + [i32p] * 4
+    lib.mla_fp4_decode_plan.restype = C.c_int
     lib.mla_fp4_decode.argtypes = [C.POINTER(DecodeArgs)]
     lib.mla_fp4_decode.restype = C.c_int
     lib.mla_fp4_decode_static.argtypes = [C.POINTER(DecodeArgs)]

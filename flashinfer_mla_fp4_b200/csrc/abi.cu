@@ -31,6 +31,32 @@ int sm_count(int* out) {
 
 bool page_size_ok(int ps) { return ps >= 8 && ps <= 128 && (128 % ps) == 0; }
 
+// The most tokens that a block-table row of this many pages can hold (0: not given).
+int seq_cap_of(int max_pages, int page_size) {
+  const int64_t cap = int64_t(max_pages) * page_size;
+  return cap > 0 && cap < INT_MAX ? int(cap) : INT_MAX;
+}
+
+// How many CTAs of a grid of n share a step's tiles (decode_sm100.cu: work_ctas, in exact arithmetic): a multiple of `share`, the groups or 1.
+int count_work_ctas(const int32_t* seq_lens, int cap, int batch, int groups, int n, int share, int32_t* out) {
+  const int64_t pairs = int64_t(groups) * batch;
+  int64_t T = 0;
+  int max_tiles = 0;
+  for (int b = 0; b < batch; ++b) {
+    const int len = std::min(seq_lens[b], cap);
+    T += int64_t(groups) * mla::vtiles_of(len);
+    max_tiles = std::max(max_tiles, mla::tiles_of(len));
+  }
+  if (!mla::partition_fits(T, n)) return fail(MLA_FP4_ERR_UNSUPPORTED, "the work partition is computed in 32 bits: too many tiles x CTAs");
+  *out = n;
+  if (T == 0 || mla::whole_requests(max_tiles, pairs, n) || (T > 5 * int64_t(n) && pairs > 1)) return MLA_FP4_OK;
+  // the longest walk: k >= T / n and k >= T / (5 sqrt(T * pairs)); then the fewest CTAs whose walks are no longer
+  int64_t k = (T + n - 1) / n;
+  while (25 * pairs * k * k < T) ++k;
+  *out = int32_t(std::min<int64_t>(n, (T / share + k - 1) / k * share));
+  return MLA_FP4_OK;
+}
+
 // Zero the header (generation, finished count) and the tails of all slots (their flags): one asynchronous memset.
 int clear_workspace(void* ws, size_t bytes, cudaStream_t stream) {
   if (bytes < mla::kWsFixedBytes) return fail(MLA_FP4_ERR_WORKSPACE_TOO_SMALL, "workspace is smaller than its header and slot tails");
@@ -118,24 +144,21 @@ int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len
   if (!work_ctas || (batch > 0 && !seq_lens_host)) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
   if (batch < 0 || q_len <= 0 || num_heads <= 0 || num_ctas <= 0)
     return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/num_ctas out of range");
-  const int64_t groups = mla::num_groups(q_len, num_heads), pairs = groups * batch;
-  const int pair_grid = mla::pair_ctas(int(groups), num_ctas);
-  const int64_t n = pair_grid ? pair_grid : num_ctas;
-  int64_t T = 0;
-  int max_tiles = 0;
-  for (int b = 0; b < batch; ++b) {
-    T += groups * mla::vtiles_of(seq_lens_host[b]);
-    max_tiles = std::max(max_tiles, mla::tiles_of(seq_lens_host[b]));
-  }
-  if (!mla::partition_fits(T, num_ctas)) return fail(MLA_FP4_ERR_UNSUPPORTED, "the work partition is computed in 32 bits: too many tiles x CTAs");
-  *work_ctas = int32_t(n);
-  if (T == 0 || mla::whole_requests(max_tiles, pairs, int(n)) || (T > 5 * n && pairs > 1)) return MLA_FP4_OK;
-  // the longest walk: k >= T / n and k >= T / (5 sqrt(T * pairs)); then the fewest CTAs whose walks are no longer
-  int64_t k = (T + n - 1) / n;
-  while (25 * pairs * k * k < T) ++k;
-  *work_ctas = int32_t(std::min(n, (T + k - 1) / k));
-  if (pair_grid) *work_ctas = int32_t((*work_ctas + groups - 1) / groups * groups);  // (every group is shared by as many)
-  return MLA_FP4_OK;
+  const int groups = mla::num_groups(q_len, num_heads), grid = mla::shared_grid(groups, num_ctas, false);
+  return count_work_ctas(seq_lens_host, INT_MAX, batch, groups, grid ? grid : num_ctas, grid ? groups : 1, work_ctas);
+}
+
+int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size, int32_t max_pages_per_request, int32_t num_ctas,
+                        const int32_t* seq_lens_host, int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas) {
+  if (!groups_per_cluster || !grid || (work_ctas && batch > 0 && !seq_lens_host)) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
+  if (batch < 0 || q_len <= 0 || num_heads <= 0 || num_ctas <= 0 || max_pages_per_request < 0)
+    return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/num_ctas/max_pages_per_request out of range");
+  if (!page_size_ok(page_size)) return fail(MLA_FP4_ERR_UNSUPPORTED, "page_size must be one of 8, 16, 32, 64, 128");
+  const int groups = mla::num_groups(q_len, num_heads), cap = seq_cap_of(max_pages_per_request, page_size);
+  const mla::DecodeForm f = mla::decode_form(batch, groups, page_size, cap, num_ctas);
+  *groups_per_cluster = f.pair ? 2 : 1;
+  *grid = f.grid;
+  return work_ctas ? count_work_ctas(seq_lens_host, cap, batch, groups, f.grid, f.share, work_ctas) : MLA_FP4_OK;
 }
 
 int mla_fp4_workspace_init(void* workspace, size_t workspace_bytes, void* stream) {
@@ -186,11 +209,7 @@ int mla_fp4_decode(const MlaFp4DecodeArgs* a) {
   p.softmax_scale = a->softmax_scale; p.output_scale = a->output_scale;
   p.out_dtype = a->out_dtype; p.pdl = a->enable_pdl ? 1 : 0;
   if (a->max_pages_per_request < 0 || a->wait_polls < 0) return fail(MLA_FP4_ERR_BAD_ARG, "max_pages_per_request/wait_polls must not be negative");
-  p.seq_cap = INT_MAX;
-  if (a->max_pages_per_request > 0) {
-    const int64_t cap = int64_t(a->max_pages_per_request) * a->page_size;
-    p.seq_cap = cap < INT_MAX ? int32_t(cap) : INT_MAX;
-  }
+  p.seq_cap = seq_cap_of(a->max_pages_per_request, a->page_size);
   p.wait_polls = a->wait_polls > 0 ? uint32_t(a->wait_polls) : (1u << 22);
   if (!(a->logits_soft_cap >= 0.f)) return fail(MLA_FP4_ERR_BAD_ARG, "logits_soft_cap must be >= 0 (0 = off)");
   p.soft_cap = a->logits_soft_cap;

@@ -118,12 +118,41 @@ MLA_HD int num_groups(int q_len, int num_heads) {
   return q_len * ((num_heads + kGroupHeads - 1) / kGroupHeads);
 }
 
-// The grid where the decode kernel for pairs of head groups (decode_pair.cuh) can be used, or 0: an even number of groups, and as many CTAs
-// as the groups can share evenly, unless that leaves too many of `num_ctas` idle (more than that kernel gains).
-MLA_HD int pair_ctas(int groups, int num_ctas) {
-  if (groups & 1) return 0;
+// An even number of groups: as many CTAs as the groups can share evenly, so that every group is cut into the same ranges, or 0 where that would
+// leave too many of `num_ctas` idle.  The kernel for pairs of head groups (decode_pair.cuh) needs such a grid and makes up for some idle CTAs:
+// 16x(1000..8000) tokens, ten groups on 140 of 148 CTAs 55.1 -> 52.0 us.  The other kernel gains a few partials, and nothing with two groups, whose
+// walks are the same either way; it is given such a grid where next to no CTA idles, from 31/32 of them on: four groups 2x7104 18.65 -> 17.5 us, six
+// (144 CTAs) 2x4736 18.95 -> 18.0, 30x(315..880) 27.85 -> 27.3.  With more CTAs idle it gains or loses: ten groups 2x2841 18.5 -> 17.2 but
+// 30x(378..1060) 38.4 -> 39.5, 22 (132) 8x(645..1800) 33.85 -> 35.8, 26 (130) 8x(546..1530) 35.6 -> 37.5.
+MLA_HD int shared_grid(int groups, int num_ctas, bool pair) {
+  if ((groups & 1) || (groups < 4 && !pair)) return 0;  // (two groups on an even grid: the same walks either way)
   const int n = num_ctas / groups * groups;
-  return 8 * n >= 7 * num_ctas ? n : 0;
+  return (pair ? 8 * n >= 7 * num_ctas : 32 * n >= 31 * num_ctas) ? n : 0;
+}
+
+// Where the pair kernel is used, as far as the caller's longest length (the width of its block tables) tells.  From twenty tiles a CTA on, where
+// the main loop counts: single -> pair 2x131072 tokens, 128 heads, q_len 2 105.7 -> 96.8 us, 32x(1024..16384), 128 heads 49.7 -> 47.6, 3x30000,
+// 128 heads, q_len 3 52.4 -> 47.5.  And for requests too short to be split, whose rows leave faster: 32x(100..500), 128 heads 13.0 -> 11.4, 1x200
+// 9.7 -> 8.7, 37x(64..512) 13.7 -> 12.6; not with pages of 8 tokens, sixteen copies one after the other for 64 tokens of K (6x110 10.4 -> 10.5).
+// Between the two a pair, whose CTAs wait for each other at every change of request and whose first tiles take longer (four warps a tile), is
+// faster or slower by as much: 1x16000, 128 heads 18.2 -> 16.9, 8x2000 16.8 -> 16.2, 16x(200..4000) 16.6 -> 16.7, 60x(100..2000) 24.4 -> 25.2,
+// 1x4096, 64 heads, q_len 2 13.2 -> 13.5, 2x(924..17749), 64 heads, q_len 2 13.3 -> 13.9.
+inline bool pair_pays(int batch, int groups, int page_size, int seq_cap, int grid) {
+  const int64_t pairs = int64_t(batch) * groups, tiles = (int64_t(seq_cap) + kTile - 1) / kTile;  // at most, of a request
+  return whole_requests(int(tiles), pairs, grid) ? page_size >= 16 : pairs * tiles >= 20 * int64_t(grid);
+}
+
+// Which decode kernel a step runs when it merges by itself, and on which grid.
+struct DecodeForm {
+  bool pair;  // the kernel for pairs of head groups
+  int grid;
+  int share;  // the number of working CTAs is a multiple of this: the groups where they share the grid evenly, or 1
+};
+inline DecodeForm decode_form(int batch, int groups, int page_size, int seq_cap, int num_ctas) {
+  const int pair_grid = shared_grid(groups, num_ctas, true);
+  const bool pair = pair_grid && pair_pays(batch, groups, page_size, seq_cap, pair_grid);
+  const int grid = pair ? pair_grid : shared_grid(groups, num_ctas, false);
+  return grid ? DecodeForm{pair, grid, groups} : DecodeForm{false, num_ctas, 1};
 }
 
 // Positions in the flat tile space are 32-bit: a 64-bit division is a subroutine of a hundred instructions and these

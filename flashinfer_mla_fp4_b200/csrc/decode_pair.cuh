@@ -99,7 +99,7 @@ __device__ __forceinline__ void pair_tma_role(const DecodeParams& p, uint32_t sm
   bool dry = starting && p.pdl_wait;  // (as in the other kernel)
   uint32_t nseg = 0;
   if (!dry) {
-    if (starting) start_work<true>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+    if (starting) start_work<kFormPair>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
     nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   }
 #pragma unroll 1
@@ -187,7 +187,7 @@ __device__ __forceinline__ void pair_tma_role(const DecodeParams& p, uint32_t sm
       dry = false;
       si = 0;
       st = RoleState{};
-      start_work<true>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+      start_work<kFormPair>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
       nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
     }
   }
@@ -680,14 +680,14 @@ mla_fp4_decode_pair_kernel(const __grid_constant__ DecodeParams p, const __grid_
   ptx::tc_fence_before();
   ptx::cluster_arrive();  // (from here on the partner may arrive at this CTA's barriers)
   if (warp == kWarpPlan && p.pdl_wait) {
-    stage_segments<true>(p, smem, lane, true, false);
+    stage_segments<kFormPair>(p, smem, lane, true, false);
     ptx::fence_proxy_async_smem();
     __threadfence_block();
     asm volatile("bar.arrive 8, 64;" ::: "memory");
   }
   ptx::cluster_wait();
   RoleState st{};
-  if (warp != kWarpTMA && warp != kWarpTMA2) start_work<true>(p, smem, warp, lane);
+  if (warp != kWarpTMA && warp != kWarpTMA2) start_work<kFormPair>(p, smem, warp, lane);
   ptx::tc_fence_after();
   const uint32_t tmem = ptx::uniform_u32(misc->tmem_base);
   bool first_round = true;
@@ -741,7 +741,7 @@ mla_fp4_decode_pair_kernel(const __grid_constant__ DecodeParams p, const __grid_
     if (!more) break;
     first_round = false;
     if (warp == kWarpTMA) {
-      stage_segments<true>(p, smem, lane, false, false);
+      stage_segments<kFormPair>(p, smem, lane, false, false);
       ptx::fence_proxy_async_smem();
     }
     __syncthreads();

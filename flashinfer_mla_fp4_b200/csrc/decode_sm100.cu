@@ -47,7 +47,6 @@
 // Every wait is bounded: when a wait expires the CTA records MLA_FP4_ERR_DEVICE_TIMEOUT in the
 // status words, stops issuing work, drains and exits normally.
 #include <atomic>
-#include <climits>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -211,6 +210,10 @@ __device__ __forceinline__ void st_release(int32_t* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// The kernel's forms: one head group per CTA, over any CTAs or over as many for each group (shared_grid); two groups on a pair of CTAs.  The
+// first carries none of the second's arithmetic, which stands in the prologue of every CTA (4x4096 tokens, 64 heads 13.45 -> 13.50 us).
+enum Form { kFormAlone, kFormShared, kFormPair };
+
 // running position of a role across rounds
 struct RoleState {
   uint32_t it;         // tiles processed so far by this CTA (selects stages and barrier phases)
@@ -245,8 +248,9 @@ __device__ __forceinline__ int fresh_len(const DecodeParams& p, int i) {  // fro
 // 17.4 / 15.8.  Approximate arithmetic will do: every CTA takes the same steps, and any 1 <= n <= Tt is right.  (The host's form of this
 // rule, mla_fp4_work_ctas, is exact; the two agree while no walk is longer than a thousand tiles: where the root decides, Tt * pairs is
 // below n^2 / 25, so that its argument keeps clear of the squares by more than the 1e-3 allows for.)
-// With an even number of groups the number is a multiple of them (share): that many times what one group's tiles, T, need for the same walk.
-__device__ __forceinline__ int work_ctas(flat_t Tt, flat_t T, int share, int pairs, int n) {
+// Where the groups share the CTAs evenly (shared_grid) the number is a multiple of them: that many times what one group's tiles, T, need for the same walk.
+template <Form F>
+__device__ __forceinline__ int work_ctas(flat_t Tt, flat_t T, int groups, int pairs, int n) {
   if (Tt > 5 * n && pairs > 1) return n;  // the whole grid, and next to nothing to gain from the rounding
   const float tiles = float(Tt);
   float best, r;
@@ -254,7 +258,8 @@ __device__ __forceinline__ int work_ctas(flat_t Tt, flat_t T, int share, int pai
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fminf(float(n), best)));
   const float k = float(__float2int_ru(tiles * r - 1e-3f));
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(k));
-  return min(n, share * max(1, __float2int_ru(float(share > 1 ? T : Tt) * r - 1e-3f)));
+  if (F != kFormAlone) return min(n, groups * max(1, __float2int_ru(float(T) * r - 1e-3f)));
+  return min(n, max(1, __float2int_ru(tiles * r - 1e-3f)));
 }
 // This CTA's place in the partition.  In the pair kernel the two CTAs of a cluster walk the same tiles for two neighbouring head groups.
 // There the working CTAs are a multiple of the groups, so that every group is shared by as many, `per`, in ranges of its own tiles that are
@@ -266,7 +271,7 @@ __device__ __forceinline__ int cta_in_partition(int per, int groups) {
 }
 template <bool kPair>
 __device__ __forceinline__ int cta_of(const Misc* misc) { return kPair ? misc->cta : int(blockIdx.x); }
-template <bool kPair>
+template <Form F>
 __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem, int lane, bool first_round, bool report) {
   Misc* misc = misc_of(smem);
   Segment* out = reinterpret_cast<Segment*>(smem_ptr(smem) + kOffSegs);
@@ -296,7 +301,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     if (lane == 0 && p.status && report) atomicCAS(p.status, 0, MLA_FP4_ERR_UNSUPPORTED);
   } else if (whole_requests(mx > 0 ? int(mx) - kPhantom : 0, int64_t(p.batch) * p.groups, n)) {  // CTA v: pair v, whole
     Tt = flat_t(T64) * p.groups;
-    if (kPair) cta = cta_in_partition(p.batch, p.groups);
+    if (F == kFormPair) cta = cta_in_partition(p.batch, p.groups);
     if (cta < p.batch * p.groups) {
       const int g = cta / p.batch, b = cta - g * p.batch;
       const int len = len_of(b);
@@ -308,8 +313,8 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
   } else if (T64 > 0) {
     const flat_t T = flat_t(T64);
     Tt = T * p.groups;
-    if (p.fused_merge) n = work_ctas(Tt, T, p.share, p.batch * p.groups, n);
-    if (kPair) cta = cta_in_partition(n / p.groups, p.groups);
+    if (p.fused_merge) n = work_ctas<F>(Tt, T, p.groups, p.batch * p.groups, n);
+    if (F == kFormPair) cta = cta_in_partition(n / p.groups, p.groups);
     const flat_t cut = cta_lo(Tt, n, cta + (lane & 1));  // one division for both ends
     const flat_t lo = first_round ? __shfl_sync(0xffffffffu, cut, 0) : misc->next, hi = __shfl_sync(0xffffffffu, cut, 1);
     int g = lo < T ? 0 : int(uint32_t(lo) / uint32_t(T));
@@ -358,7 +363,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
     misc->next = next;
     misc->Tt = Tt;
     misc->n = n;
-    if (kPair) misc->cta = cta;
+    if (F == kFormPair) misc->cta = cta;
   }
   __syncwarp();
 }
@@ -368,7 +373,7 @@ __device__ __noinline__ void stage_segments(const DecodeParams& p, uint32_t smem
 // The plan made before the wait stands if the lengths have not changed.  A CTA that starts late, on an SM that the kernel ahead
 // held to its end, finds nothing to wait for: there the lengths are read again while the plan is being made (1.8 us of code that
 // comes from L2 line by line).
-template <bool kPair>
+template <Form F>
 __device__ __forceinline__ void start_work(const DecodeParams& p, uint32_t smem, int warp, int lane) {
   Misc* misc = misc_of(smem);
   if (p.pdl_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -387,7 +392,7 @@ __device__ __forceinline__ void start_work(const DecodeParams& p, uint32_t smem,
       for (int i = lane; i < nb; i += 32) same &= lens[kLensMax + i] == lens[i];
       stands = __all_sync(0xffffffffu, same) && p.batch <= kLensMax && misc->Tt >= 0;
     }
-    if (!stands) stage_segments<kPair>(p, smem, lane, true, true);
+    if (!stands) stage_segments<F>(p, smem, lane, true, true);
     ptx::fence_proxy_async_smem();  // the lengths give way to the first copies
     __threadfence_block();
     asm volatile("bar.arrive 2, %0;" ::"n"(kThreads) : "memory");
@@ -414,6 +419,7 @@ __device__ __forceinline__ int page_window(const DecodeParams& p, const Segment&
 }
 // entry `i` of a window, in a uniform register
 __device__ __forceinline__ int uniform_page(int window, int i) { return __reduce_max_sync(0xffffffffu, int(threadIdx.x & 31) == (i & 31) ? window : -1); }
+template <Form F>
 __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, uint32_t which, const CUtensorMap* map_rope,
                                          const CUtensorMap* map_lat, RoleState& st, bool starting) {
   const Segment* sg = segs_of(smem);
@@ -429,7 +435,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
   st.slot = starting ? which : st.slot;
   uint32_t nseg = 0;
   if (!dry) {
-    if (starting) start_work<false>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+    if (starting) start_work<F>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
     nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
   }
 #pragma unroll 1
@@ -508,7 +514,7 @@ __device__ __forceinline__ void tma_role(const DecodeParams& p, uint32_t smem, u
       si = 0;
       st = RoleState{};
       st.slot = which;
-      start_work<false>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
+      start_work<F>(p, smem, which ? kWarpTMA2 : kWarpTMA, lane);
       nseg = ptx::uniform_u32(uint32_t(misc_of(smem)->nseg));
     }
   }
@@ -1629,7 +1635,7 @@ __device__ __noinline__ void merge_as_last(const DecodeParams& p, uint32_t smem,
 // ------------------------------------------------------------------------------------------
 // kernel
 // ------------------------------------------------------------------------------------------
-template <bool kSoftCap>
+template <bool kSoftCap, Form F>
 __global__ void __launch_bounds__(kThreads, 1)
 mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__ CUtensorMap map_q_lat,
                             const __grid_constant__ CUtensorMap map_q_rope, const __grid_constant__ CUtensorMap map_rope,
@@ -1663,7 +1669,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   } else if (warp == kWarpPlan) {
     asm volatile("bar.arrive 7, %0;" ::"n"(kThreads) : "memory");
     if (p.pdl_wait) {  // a first plan, from the lengths as they are in memory; the TMA warp decides whether it stands
-      stage_segments<false>(p, smem, lane, true, false);
+      stage_segments<F>(p, smem, lane, true, false);
       ptx::fence_proxy_async_smem();
       __threadfence_block();
       asm volatile("bar.arrive 8, 64;" ::: "memory");
@@ -1683,7 +1689,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
   if (warp != kWarpPlan) ptx::bar_sync(7, kThreads);
   RoleState st{};
   if (warp != kWarpTMA && warp != kWarpTMA2) {  // (these two: in their role, after a first pass without effect)
-    start_work<false>(p, smem, warp, lane);
+    start_work<F>(p, smem, warp, lane);
   }
   ptx::tc_fence_after();
   const uint32_t tmem = ptx::uniform_u32(misc->tmem_base);
@@ -1713,7 +1719,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
       }
       pv_role(smem, tmem, st);
     } else {
-      tma_role(p, smem, warp == kWarpTMA2 ? 1u : 0u, &map_rope, &map_lat, st, first_round);
+      tma_role<F>(p, smem, warp == kWarpTMA2 ? 1u : 0u, &map_rope, &map_lat, st, first_round);
     }
     const int more = misc->more;
     if (!more && warp < kWarpSoftmax0) {
@@ -1747,7 +1753,7 @@ mla_fp4_decode_sm100_kernel(const __grid_constant__ DecodeParams p, const __grid
     if (!more) break;
     first_round = false;
     if (warp == kWarpTMA) {
-      stage_segments<false>(p, smem, lane, false, false);
+      stage_segments<F>(p, smem, lane, false, false);
       ptx::fence_proxy_async_smem();
     }
     __syncthreads();
@@ -1863,18 +1869,6 @@ bool encode_kv_maps(const DecodeParams& p, uint32_t rows, CUtensorMap* lat, CUte
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Where the pair kernel is used, as far as the caller's longest length (the width of its block tables) tells.  From twenty tiles a CTA on, where
-// the main loop counts: single -> pair 2x131072 tokens, 128 heads, q_len 2 105.7 -> 96.8 us, 32x(1024..16384), 128 heads 49.7 -> 47.6, 3x30000,
-// 128 heads, q_len 3 52.4 -> 47.5.  And for requests too short to be split, whose rows leave faster: 32x(100..500), 128 heads 13.0 -> 11.4, 1x200
-// 9.7 -> 8.7, 37x(64..512) 13.7 -> 12.6; not with pages of 8 tokens, sixteen copies one after the other for 64 tokens of K (6x110 10.4 -> 10.5).
-// Between the two a pair, whose CTAs wait for each other at every change of request and whose first tiles take longer (four warps a tile), is
-// faster or slower by as much: 1x16000, 128 heads 18.2 -> 16.9, 8x2000 16.8 -> 16.2, 16x(200..4000) 16.6 -> 16.7, 60x(100..2000) 24.4 -> 25.2,
-// 1x4096, 64 heads, q_len 2 13.2 -> 13.5, 2x(924..17749), 64 heads, q_len 2 13.3 -> 13.9.
-bool pair_pays(const DecodeParams& p, int grid) {
-  const int64_t pairs = int64_t(p.batch) * p.groups, tiles = (int64_t(p.seq_cap) + kTile - 1) / kTile;  // at most, of a request
-  return whole_requests(int(tiles < INT_MAX ? tiles : INT_MAX), pairs, grid) ? p.page_size >= 16 : pairs * tiles >= 20 * int64_t(grid);
-}
-
 }  // namespace
 
 cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_t stream, const char** err) {
@@ -1887,10 +1881,8 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   MapPair<QKey>& qm = q_maps[map_slot(p.q)];
   MapPair<KvKey>& km = kv_maps[map_slot(p.kv_cache)];
   const QKey qkey{p.q, p.q_stride_batch, p.q_stride_qpos, p.q_stride_head, p.batch, p.q_len, p.num_heads, dev};
-  // Which kernel: see pair_pays.  (Where the pair kernel could be used, the grid and the partition are such as it needs, whichever runs.)
-  const int even_grid = p.fused_merge ? pair_ctas(p.groups, num_ctas) : 0;
-  const int grid = even_grid ? even_grid : num_ctas;
-  const bool pair = even_grid && pair_pays(p, grid);
+  const DecodeForm form = p.fused_merge ? decode_form(p.batch, p.groups, p.page_size, p.seq_cap, num_ctas) : DecodeForm{false, num_ctas, 1};
+  const bool pair = form.pair;
   const uint32_t rows = pair && p.page_size > 64 ? 64u : uint32_t(p.page_size);
   const KvKey kvkey{p.kv_cache, p.num_pages, p.page_size, int32_t(rows), dev};
   if (!(qm.valid && qm.key == qkey)) {
@@ -1912,25 +1904,28 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
     km.valid = true;
   }
   const CUtensorMap &map_q_lat = qm.a, &map_q_rope = qm.b, &map_rope = km.b, &map_lat = km.a;
+  // the attention variant with a score transform is a kernel of its own, as is each form: none carries another's instructions
+  using Kernel = void (*)(DecodeParams, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap);
+  static constexpr Kernel kernels[3][2] = {
+      {mla_fp4_decode_sm100_kernel<false, kFormAlone>, mla_fp4_decode_sm100_kernel<true, kFormAlone>},
+      {mla_fp4_decode_sm100_kernel<false, kFormShared>, mla_fp4_decode_sm100_kernel<true, kFormShared>},
+      {mla_fp4_decode_pair_kernel<false>, mla_fp4_decode_pair_kernel<true>}};
   {
+    // (all of them with the first step: a later one may be under capture, where no kernel should be loaded)
     static std::atomic<bool> attr_done[64];  // zero-initialised; setting the attribute twice is harmless
     if (dev < 0 || dev >= 64 || !attr_done[dev].load(std::memory_order_acquire)) {
-      e = cudaFuncSetAttribute(mla_fp4_decode_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
-      if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(mla_fp4_decode_sm100_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
-      if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(mla_fp4_decode_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
-      if (e != cudaSuccess) return e;
-      e = cudaFuncSetAttribute(mla_fp4_decode_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
-      if (e != cudaSuccess) return e;
+      for (const Kernel(&forms)[2] : kernels) {
+        for (const Kernel k : forms) {
+          e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemAlloc));
+          if (e != cudaSuccess) return e;
+        }
+      }
       if (dev >= 0 && dev < 64) attr_done[dev].store(true, std::memory_order_release);
     }
   }
-  // the attention variant with a score transform is a kernel of its own: the standard one carries none of its instructions
-  auto* kernel = pair ? (p.soft_cap > 0.f ? mla_fp4_decode_pair_kernel<true> : mla_fp4_decode_pair_kernel<false>)
-                           : (p.soft_cap > 0.f ? mla_fp4_decode_sm100_kernel<true> : mla_fp4_decode_sm100_kernel<false>);
+  const Kernel kernel = kernels[pair ? kFormPair : (form.share > 1 ? kFormShared : kFormAlone)][p.soft_cap > 0.f];
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = dim3(form.grid);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemAlloc;
   cfg.stream = stream;
@@ -1943,7 +1938,6 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   cfg.numAttrs = p.pdl ? 1 : 0;
   DecodeParams pp = p;
   pp.pdl_wait = p.pdl;
-  pp.share = even_grid ? p.groups : 1;
   pp.page_shift = __builtin_ctz(unsigned(p.page_size));
   return cudaLaunchKernelEx(&cfg, kernel, pp, map_q_lat, map_q_rope, map_rope, map_lat);
 }

@@ -19,7 +19,6 @@ struct DecodeParams {
   int32_t* status;
   int32_t batch, q_len, num_heads, page_size, groups;
   int32_t page_shift;   // log2(page_size), set by the launcher
-  int32_t share;        // set by the launcher: the number of working CTAs is a multiple of this
   int64_t num_pages;
   float softmax_scale, output_scale;
   int32_t out_dtype;

@@ -152,12 +152,21 @@ int mla_fp4_plan_partition(const int32_t* seq_lens_host, int32_t batch, int32_t 
                            int32_t* num_segments);
 
 /* How many CTAs of a grid of num_ctas share a step's tiles when the decode kernel merges by itself
-   (MLA_FP4_KERNEL_TCGEN05): with few tiles, fewer than the grid, since each CTA more is a partial
-   more to merge (with an even number of head groups, a multiple of the groups).  mla_fp4_plan_partition over this many CTAs is that kernel's partition; the
-   other kernels use the whole grid.  (Beyond a thousand tiles a CTA, some 19 M tokens in one
-   request, the kernel's number may be one off.) */
+   (MLA_FP4_KERNEL_TCGEN05, one head group per CTA): with few tiles, fewer than the grid, since each CTA more
+   is a partial more to merge; with an even number of head groups that nearly fills the grid, a multiple of
+   the groups.  mla_fp4_plan_partition over this many CTAs is that kernel's partition; the other kernels use
+   the whole grid.  (Beyond a thousand tiles a CTA, some 19 M tokens in one request, the kernel may count one
+   tile more or less to the longest walk, and its number differ accordingly.) */
 int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len, int32_t num_heads,
                       int32_t num_ctas, int32_t* work_ctas);
+
+/* What a call of mla_fp4_decode with MLA_FP4_KERNEL_TCGEN05 and these arguments launches: *groups_per_cluster is 1
+   (a CTA decodes one group of 64 heads) or 2 (a pair of CTAs decodes two groups of the same tiles), *grid the CTAs
+   launched and *work_ctas (may be NULL, seq_lens_host then too) how many of them share the tiles: the partition is
+   mla_fp4_plan_partition over that many.  num_ctas as resolved (not 0).  Host only. */
+int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size,
+                        int32_t max_pages_per_request, int32_t num_ctas, const int32_t* seq_lens_host,
+                        int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas);
 
 /* Zero the header and the slot tails of a workspace (an asynchronous memset on `stream`).  Call
    once after allocating the workspace.

@@ -60,3 +60,32 @@ def test_the_planner_describes_the_kernels_partition(lens, heads, q_len, max_cta
     published = ws[head: head + 296 * 272].view(torch.int32).reshape(296, 68)[:, 65].nonzero().flatten().tolist()
     n = planner.work_ctas(lens, q_len, heads, w._num_ctas)
     assert published == sorted(s.slot for s in planner.plan_partition(lens, q_len, heads, n) if s.slot >= 0)
+
+
+@pytest.mark.parametrize("lens,heads,q_len,max_ctas,pair,grid", [
+    ([2000] * 4, 128, 5, None, 1, 148),      # ten groups do not fill 148 CTAs evenly: the kernel with a group per CTA has them all
+    ([1500, 700], 128, 3, None, 1, 144),     # six nearly do
+    ([3000, 1500], 128, 2, None, 1, 148),
+    ([9000] * 20, 128, 5, None, 2, 140),     # a pair of groups per cluster, on as many CTAs as ten groups share evenly
+    ([30000, 500, 9000], 128, 3, None, 2, 144),
+    ([5000, 700, 0, 1], 40, 2, 12, 2, 12),
+])
+def test_the_decode_plan_describes_the_step(lens, heads, q_len, max_ctas, pair, grid):
+    """Which kernel, which grid, and the partial slots that the step publishes."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, _cabi, planner, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("plan", [max(n, 1) for n in lens], heads, 64, q_len=q_len, seed=2, device=dev)
+    case.seq_lens = torch.tensor(lens, dtype=torch.int32, device=dev)
+    ws = torch.empty(32 << 20, dtype=torch.int8, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(ws)
+    w.plan(num_heads=heads, page_size=64, max_ctas=max_ctas)
+    plan = planner.decode_plan(lens, q_len, heads, 64, case.block_tables.shape[1], w._num_ctas)
+    assert (plan.groups_per_cluster, plan.grid) == (pair, grid)
+    w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
+    w.check_device_status()
+    head = _cabi.WORKSPACE_HEADER_BYTES
+    published = ws[head: head + 296 * 272].view(torch.int32).reshape(296, 68)[:, 65].nonzero().flatten().tolist()
+    assert published == sorted(s.slot for s in planner.plan_partition(lens, q_len, heads, plan.work_ctas) if s.slot >= 0)

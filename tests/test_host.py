@@ -278,3 +278,20 @@ def test_working_ctas_of_a_tile_space_beyond_32_bits_are_refused():
 
     with pytest.raises(ValueError, match="32 bits"):
         planner.work_ctas([2**31 - 1] * 64, 1, 64, 148)
+
+
+@pytest.mark.parametrize("seq_lens,heads,q_len,ctas,expect", [
+    ([3000] * 8, 64, 1, 148, (1, 148, 108)),    # 216 tiles with the phantom ones: no walk is shorter than two
+    ([3000] * 8, 128, 3, 148, (1, 144, 144)),   # six groups: 144 CTAs, as many each
+    ([3000] * 8, 128, 5, 148, (1, 148, 148)),   # ten groups would leave eight CTAs idle, which the kernel with a group per CTA does not make up for
+    ([700] * 8, 128, 13, 148, (1, 148, 148)),
+    ([9000] * 20, 128, 5, 148, (2, 140, 140)),  # the kernel for pairs of groups does
+    ([2500] * 30, 128, 1, 7, (1, 7, 7)),        # six of seven would do for neither
+])
+def test_decode_plan(seq_lens, heads, q_len, ctas, expect):
+    from flashinfer_mla_fp4_b200 import planner
+
+    p = planner.decode_plan(seq_lens, q_len, heads, 64, -(-max(seq_lens) // 64), ctas)
+    assert (p.groups_per_cluster, p.grid, p.work_ctas) == expect
+    if p.groups_per_cluster == 1:
+        assert p.work_ctas == planner.work_ctas(seq_lens, q_len, heads, ctas)
