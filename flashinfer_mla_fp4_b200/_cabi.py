@@ -60,7 +60,7 @@ class DecodeArgs(C.Structure):
         ("stream", C.c_void_p),
         ("max_pages_per_request", C.c_int32),
         ("wait_polls", C.c_int32),
-        ("logits_soft_cap", C.c_float), ("sink", C.c_void_p),
+        ("logits_soft_cap", C.c_float), ("max_seq_len", C.c_int32), ("sink", C.c_void_p),
     ]
 
 
@@ -110,7 +110,7 @@ def _load() -> C.CDLL:
     lib.mla_fp4_plan_partition.restype = C.c_int
     lib.mla_fp4_work_ctas.argtypes = [i32p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, i32p]
     lib.mla_fp4_work_ctas.restype = C.c_int
-    lib.mla_fp4_decode_plan.argtypes = [C.c_int32] * 6 + [i32p] * 4
+    lib.mla_fp4_decode_plan.argtypes = [C.c_int32] * 7 + [i32p] * 4
     lib.mla_fp4_decode_plan.restype = C.c_int
     lib.mla_fp4_decode.argtypes = [C.POINTER(DecodeArgs)]
     lib.mla_fp4_decode.restype = C.c_int

@@ -93,6 +93,10 @@ class FP4MLADecodeBackend:
         self.block_tables = torch.zeros(max_batch, self.max_pages, dtype=torch.int32, device=self.device)
         self.seq_lens = torch.zeros(max_batch, dtype=torch.int32, device=self.device)
         self.slot_mapping = torch.full((max_batch * q_len,), -1, dtype=torch.int64, device=self.device)
+        # The longest request that a step's kernel is chosen for, where there are two (a hint; run()'s max_seq_len): what the tables last given to prepare() can hold,
+        # in a graph what capture() was told, else the capacity.
+        self._longest = self._longest_captured = max_seq_len
+        self._two_kernels = q_len * -(-num_heads // _cabi.GROUP_HEADS) % 2 == 0
         self._step_metadata = _cabi.native.step_metadata
         self._views = (0, None, None, None, None, None, None)  # of the last forward(): batch, rows of the three buffers, the buffers
 
@@ -101,6 +105,7 @@ class FP4MLADecodeBackend:
         """Make every row padding (what the buffers hold before the first ``prepare``)."""
         self.seq_lens.zero_()
         self.slot_mapping.fill_(-1)
+        self._longest = self.max_seq_len
 
     @api_logged
     def prepare(self, block_tables: torch.Tensor, seq_lens: torch.Tensor, slot_mapping: Optional[torch.Tensor] = None) -> int:
@@ -119,6 +124,8 @@ class FP4MLADecodeBackend:
             raise ValueError(f"block_tables must be [batch, <= {self.max_pages}], got {tuple(block_tables.shape)}")
         if slot_mapping is not None and slot_mapping.numel() != batch * self.q_len:
             raise ValueError(f"slot_mapping must hold batch * q_len = {batch * self.q_len} slots")
+        if self._two_kernels:
+            self._longest = min(self.max_seq_len, block_tables.shape[1] * self.page_size) or self.max_seq_len
         # Device or pinned host tensors of the usual types: one kernel writes all three buffers.
         if self._step_metadata(block_tables, seq_lens, slot_mapping, self.block_tables, self.seq_lens, self.slot_mapping,
                                self.page_size, self.q_len):
@@ -163,17 +170,27 @@ class FP4MLADecodeBackend:
         if views[0] != batch or views[4] is not bt or views[5] is not sl or views[6] is not sm:
             views = self._views = (batch, bt[:batch], sl[:batch], sm[:n], bt, sl, sm)
         write_tokens(latent, rope, views[3], cache.kv_cache, cache.kv_cache_sf)
-        return self._runner.run(q, cache.kv_cache, views[1], views[2], self.max_seq_len, self.softmax_scale,
+        longest = self._longest
+        if longest != self.max_seq_len and torch.cuda.is_current_stream_capturing():  # (the graph is for other steps than this one)
+            longest = self._longest_captured
+        return self._runner.run(q, cache.kv_cache, views[1], views[2], longest, self.softmax_scale,
                                 output_scale=self.output_scale, out=out, kv_cache_sf=cache.kv_cache_sf)
 
     def capture(self, cache: FP4MLAPagedCache, batch: Optional[int] = None, in_dtype: torch.dtype = torch.bfloat16,
-                warmup: int = 2) -> "CapturedDecodeStep":
+                warmup: int = 2, expected_seq_len: Optional[int] = None) -> "CapturedDecodeStep":
         """Record ``forward`` for ``batch`` (default ``max_batch``) requests in a CUDA graph.
 
         The warm-up runs and the capture see padding metadata only, so they touch neither the cache nor
         any request; afterwards fill ``step.q / step.latent / step.rope``, call ``prepare()`` and
         ``step.replay()`` each step and read ``step.out``.
+
+        The graph serves requests of any length up to ``max_seq_len``.  ``expected_seq_len`` (default ``max_seq_len``) is the length
+        that the longest requests usually have: with an even number of 64-head groups the graph holds the kernel that is faster for
+        a batch of that length (``wrapper.run``; the other one is up to a tenth slower, and differs in the last bits).  Give it where
+        ``max_seq_len`` is a model's limit and requests are mostly far shorter.
         """
+        if expected_seq_len is not None and not 1 <= expected_seq_len <= self.max_seq_len:
+            raise ValueError(f"expected_seq_len must be in [1, {self.max_seq_len}], got {expected_seq_len}")
         batch = self.max_batch if batch is None else batch
         n = batch * self.q_len
         step = CapturedDecodeStep()
@@ -182,15 +199,20 @@ class FP4MLADecodeBackend:
         step.rope = torch.zeros(n, ROPE_DIM, dtype=in_dtype, device=self.device)
         step.out = torch.empty(batch, self.q_len, self.num_heads, LATENT_DIM, dtype=self.wrapper._o_dtype, device=self.device)
         self.clear()
-        side = torch.cuda.Stream(device=self.device)
-        side.wait_stream(torch.cuda.current_stream(self.device))
-        with torch.cuda.stream(side):
-            for _ in range(warmup):
+        if expected_seq_len is not None:
+            self._longest = self._longest_captured = int(expected_seq_len)
+        try:
+            side = torch.cuda.Stream(device=self.device)
+            side.wait_stream(torch.cuda.current_stream(self.device))
+            with torch.cuda.stream(side):
+                for _ in range(warmup):
+                    self.forward(step.q, step.latent, step.rope, cache, out=step.out)
+            torch.cuda.current_stream(self.device).wait_stream(side)
+            step.graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(step.graph):
                 self.forward(step.q, step.latent, step.rope, cache, out=step.out)
-        torch.cuda.current_stream(self.device).wait_stream(side)
-        step.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(step.graph):
-            self.forward(step.q, step.latent, step.rope, cache, out=step.out)
+        finally:
+            self._longest = self._longest_captured = self.max_seq_len
         return step
 
 

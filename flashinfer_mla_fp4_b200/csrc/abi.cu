@@ -37,6 +37,12 @@ int seq_cap_of(int max_pages, int page_size) {
   return cap > 0 && cap < INT_MAX ? int(cap) : INT_MAX;
 }
 
+// The longest request as far as the caller tells: what it states, and what its block tables can hold; 0: neither is known.
+int longest_of(int max_seq_len, int cap) {
+  if (max_seq_len <= 0) return cap < INT_MAX ? cap : 0;
+  return std::min(max_seq_len, cap);
+}
+
 // How many CTAs of a grid of n share a step's tiles (decode_sm100.cu: work_ctas, in exact arithmetic): a multiple of `share`, the groups or 1.
 int count_work_ctas(const int32_t* seq_lens, int cap, int batch, int groups, int n, int share, int32_t* out) {
   const int64_t pairs = int64_t(groups) * batch;
@@ -148,14 +154,14 @@ int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len
   return count_work_ctas(seq_lens_host, INT_MAX, batch, groups, grid ? grid : num_ctas, grid ? groups : 1, work_ctas);
 }
 
-int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size, int32_t max_pages_per_request, int32_t num_ctas,
-                        const int32_t* seq_lens_host, int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas) {
+int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size, int32_t max_pages_per_request, int32_t max_seq_len,
+                        int32_t num_ctas, const int32_t* seq_lens_host, int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas) {
   if (!groups_per_cluster || !grid || (work_ctas && batch > 0 && !seq_lens_host)) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
   if (batch < 0 || q_len <= 0 || num_heads <= 0 || num_ctas <= 0 || max_pages_per_request < 0)
     return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/num_ctas/max_pages_per_request out of range");
   if (!page_size_ok(page_size)) return fail(MLA_FP4_ERR_UNSUPPORTED, "page_size must be one of 8, 16, 32, 64, 128");
   const int groups = mla::num_groups(q_len, num_heads), cap = seq_cap_of(max_pages_per_request, page_size);
-  const mla::DecodeForm f = mla::decode_form(batch, groups, page_size, cap, num_ctas);
+  const mla::DecodeForm f = mla::decode_form(batch, groups, page_size, longest_of(max_seq_len, cap), num_ctas);
   *groups_per_cluster = f.pair ? 2 : 1;
   *grid = f.grid;
   return work_ctas ? count_work_ctas(seq_lens_host, cap, batch, groups, f.grid, f.share, work_ctas) : MLA_FP4_OK;
@@ -210,6 +216,7 @@ int mla_fp4_decode(const MlaFp4DecodeArgs* a) {
   p.out_dtype = a->out_dtype; p.pdl = a->enable_pdl ? 1 : 0;
   if (a->max_pages_per_request < 0 || a->wait_polls < 0) return fail(MLA_FP4_ERR_BAD_ARG, "max_pages_per_request/wait_polls must not be negative");
   p.seq_cap = seq_cap_of(a->max_pages_per_request, a->page_size);
+  p.longest = longest_of(a->max_seq_len, p.seq_cap);
   p.wait_polls = a->wait_polls > 0 ? uint32_t(a->wait_polls) : (1u << 22);
   if (!(a->logits_soft_cap >= 0.f)) return fail(MLA_FP4_ERR_BAD_ARG, "logits_soft_cap must be >= 0 (0 = off)");
   p.soft_cap = a->logits_soft_cap;

@@ -130,16 +130,21 @@ MLA_HD int shared_grid(int groups, int num_ctas, bool pair) {
   return (pair ? 8 * n >= 7 * num_ctas : 32 * n >= 31 * num_ctas) ? n : 0;
 }
 
-// Where the pair kernel is used, as far as the caller's longest length (the width of its block tables) tells.  From twenty tiles a CTA on, where
-// the main loop counts: single -> pair 2x131072 tokens, 128 heads, q_len 2 105.7 -> 96.8 us, 32x(1024..16384), 128 heads 49.7 -> 47.6, 3x30000,
-// 128 heads, q_len 3 52.4 -> 47.5.  And for requests too short to be split, whose rows leave faster: 32x(100..500), 128 heads 13.0 -> 11.4, 1x200
-// 9.7 -> 8.7, 37x(64..512) 13.7 -> 12.6; not with pages of 8 tokens, sixteen copies one after the other for 64 tokens of K (6x110 10.4 -> 10.5).
-// Between the two a pair, whose CTAs wait for each other at every change of request and whose first tiles take longer (four warps a tile), is
-// faster or slower by as much: 1x16000, 128 heads 18.2 -> 16.9, 8x2000 16.8 -> 16.2, 16x(200..4000) 16.6 -> 16.7, 60x(100..2000) 24.4 -> 25.2,
-// 1x4096, 64 heads, q_len 2 13.2 -> 13.5, 2x(924..17749), 64 heads, q_len 2 13.3 -> 13.9.
-inline bool pair_pays(int batch, int groups, int page_size, int seq_cap, int grid) {
-  const int64_t pairs = int64_t(batch) * groups, tiles = (int64_t(seq_cap) + kTile - 1) / kTile;  // at most, of a request
-  return whole_requests(int(tiles), pairs, grid) ? page_size >= 16 : pairs * tiles >= 20 * int64_t(grid);
+// Where the pair kernel is used, by the longest request: the lengths themselves are on the device, so what the caller says of it (the least of the
+// max_seq_len it states and what its block tables can hold; 0: neither is known).  Single -> pair, 128 heads, BF16 output unless said:
+//  * requests too short to be split, whose rows leave faster: 32x(100..500) 13.0 -> 11.5 us, 1x200 9.85 -> 8.75, 8x512 12.65 -> 11.25, with pages of 16
+//    13.7 -> 12.7, of 8 17.85 -> 16.1; 6x110 with pages of 8 and FP32 output 10.65 -> 10.7.
+//  * from twenty tiles a CTA on, where the main loop counts, with pages of 64 and 128 tokens: 16x16000 51.95 -> 48.85, 24x8000 42.8 -> 42.0, 64x3000 47.55 ->
+//    45.2, 32x(1024..16384) 43.1 -> 39.85, 3x30000, q_len 3 52.4 -> 47.9; 2x131072, q_len 2 105.5 -> 97.  With smaller pages the copies of K, every byte of
+//    which is fetched by both CTAs of a pair as K of one and V of both, take longer: 16x16000 with pages of 32 52.55 -> 52.85, of 16 60.35 -> 62.6, of 8 89.0 -> 89.7.
+//  * not between the two: a pair's CTAs wait for each other at every change of request, and its first tiles take longer (four warps a tile).
+//    4x4000 14.4 -> 15.65, 2x8000 14.8 -> 16.05, 60x(100..2000) 24.45 -> 25.4, 8x8000 23.4 -> 23.7, 2x(20000..60000), 64 heads, q_len 2 22.6 -> 23.9; the same at about
+//    thirteen tiles a CTA (2x64000 33.2 -> 32.6, 32x4000 35.05 -> 34.7).  Lengths far below the longest come out there too:
+//    24x(100..16384) 27.7 -> 28.7, but 64x(200..4000) 31.8 -> 31.8, 64x(500..8000) 44.5 -> 42.4.
+inline bool pair_pays(int batch, int groups, int page_size, int longest, int grid) {
+  const int64_t pairs = int64_t(batch) * groups, tiles = (int64_t(longest) + kTile - 1) / kTile;
+  if (longest <= 0) return false;
+  return whole_requests(int(tiles), pairs, grid) || (page_size >= 64 && pairs * tiles >= 20 * int64_t(grid));
 }
 
 // Which decode kernel a step runs when it merges by itself, and on which grid.
@@ -148,9 +153,9 @@ struct DecodeForm {
   int grid;
   int share;  // the number of working CTAs is a multiple of this: the groups where they share the grid evenly, or 1
 };
-inline DecodeForm decode_form(int batch, int groups, int page_size, int seq_cap, int num_ctas) {
+inline DecodeForm decode_form(int batch, int groups, int page_size, int longest, int num_ctas) {
   const int pair_grid = shared_grid(groups, num_ctas, true);
-  const bool pair = pair_grid && pair_pays(batch, groups, page_size, seq_cap, pair_grid);
+  const bool pair = pair_grid && pair_pays(batch, groups, page_size, longest, pair_grid);
   const int grid = pair ? pair_grid : shared_grid(groups, num_ctas, false);
   return grid ? DecodeForm{pair, grid, groups} : DecodeForm{false, num_ctas, 1};
 }

@@ -170,6 +170,7 @@ PyObject* decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   d.enable_pdl = pdl; d.phase_mask = int32_t(phase);
   d.stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   d.max_pages_per_request = int32_t(bt->size(1));
+  d.max_seq_len = int32_t(max_len < INT32_MAX ? max_len : INT32_MAX);
   d.wait_polls = int32_t(polls);
   d.logits_soft_cap = float(cap);
   d.sink = sink ? static_cast<const float*>(sink->data_ptr()) : nullptr;

@@ -51,11 +51,13 @@ class DecodePlan:
     work_ctas: int
 
 
-def decode_plan(seq_lens: Sequence[int], q_len: int, num_heads: int, page_size: int, max_pages: int, num_ctas: int) -> DecodePlan:
-    """Which decode kernel a call with block tables of ``max_pages`` pages runs, its grid and how many of its CTAs share the tiles."""
+def decode_plan(seq_lens: Sequence[int], q_len: int, num_heads: int, page_size: int, max_pages: int, num_ctas: int,
+                max_seq_len: int = 0) -> DecodePlan:
+    """Which decode kernel a call with block tables of ``max_pages`` pages (0: not given) and this ``max_seq_len`` (0: not given) runs, its
+    grid and how many of its CTAs share the tiles."""
     arr = (C.c_int32 * max(len(seq_lens), 1))(*[int(x) for x in seq_lens])
     out = [C.c_int32(0) for _ in range(3)]
-    _cabi.check(_cabi.lib.mla_fp4_decode_plan(len(seq_lens), q_len, num_heads, page_size, max_pages, num_ctas, arr, *map(C.byref, out)))
+    _cabi.check(_cabi.lib.mla_fp4_decode_plan(len(seq_lens), q_len, num_heads, page_size, max_pages, max_seq_len, num_ctas, arr, *map(C.byref, out)))
     return DecodePlan(*(x.value for x in out))
 
 

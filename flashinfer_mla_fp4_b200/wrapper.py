@@ -162,6 +162,10 @@ class BatchMLADecodeCuteDSLFP4Wrapper:
     ) -> Union[torch.Tensor, Tuple[torch.Tensor, torch.Tensor]]:
         """One decode step on torch's current stream; asynchronous, CUDA-graph capturable.
 
+        ``max_seq_len`` bounds nothing on the device (the block tables do).  With an even number of 64-head groups (65 to 128 heads, or an
+        even ``q_len``) it decides which of two kernels runs: state the longest length of the step where it is known.  The two differ in
+        the last bits of their results.
+
         ``lse_out`` (f32, contiguous [batch, q_len, num_heads], on q's device) receives the base-2 LSE in
         place when ``return_lse`` is set, instead of a freshly allocated tensor."""
         if not self._planned:
@@ -263,6 +267,7 @@ class BatchMLADecodeCuteDSLFP4Wrapper:
         a.enable_pdl = 1 if self._enable_pdl else 0
         a.phase_mask = self._phase_mask
         a.max_pages_per_request = block_tables.shape[1]
+        a.max_seq_len = min(int(max_seq_len), 2**31 - 1)
         a.logits_soft_cap = self._soft_cap
         a.sink = self._sink.data_ptr() if self._sink is not None else None
         a.wait_polls = self._wait_polls

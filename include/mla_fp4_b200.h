@@ -124,6 +124,10 @@ typedef struct MlaFp4DecodeArgs {
        compared with the scaled scores) and a zero value row: it only adds exp(sink[h]) to the softmax denominator
        (the update_statistics hook of the sink variant, applied with the first tile of a request). */
   float logits_soft_cap;
+  /* The longest entry of seq_lens, as far as the caller knows (the max_seq_len of run()); 0 or less = not given.  A
+     hint: with max_pages_per_request it decides which of two kernels runs with an even number of head groups (they differ in
+     speed and in the last bits of the results).  It bounds nothing.  (The place was padding before.) */
+  int32_t max_seq_len;
   const float* sink;
 } MlaFp4DecodeArgs;
 
@@ -163,9 +167,10 @@ int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len
 /* What a call of mla_fp4_decode with MLA_FP4_KERNEL_TCGEN05 and these arguments launches: *groups_per_cluster is 1
    (a CTA decodes one group of 64 heads) or 2 (a pair of CTAs decodes two groups of the same tiles), *grid the CTAs
    launched and *work_ctas (may be NULL, seq_lens_host then too) how many of them share the tiles: the partition is
-   mla_fp4_plan_partition over that many.  num_ctas as resolved (not 0).  Host only. */
+   mla_fp4_plan_partition over that many.  max_pages_per_request and max_seq_len as in MlaFp4DecodeArgs, num_ctas as
+   resolved (not 0).  Host only. */
 int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size,
-                        int32_t max_pages_per_request, int32_t num_ctas, const int32_t* seq_lens_host,
+                        int32_t max_pages_per_request, int32_t max_seq_len, int32_t num_ctas, const int32_t* seq_lens_host,
                         int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas);
 
 /* Zero the header and the slot tails of a workspace (an asynchronous memset on `stream`).  Call

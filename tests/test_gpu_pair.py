@@ -123,3 +123,49 @@ def test_a_small_poll_budget_is_a_budget_of_tiles():
     got, status = step(), w.device_status()
     assert status[0] == 0, status
     assert torch.equal(got, expect)
+
+
+def test_a_backend_chooses_by_the_lengths_it_is_told():
+    """A backend sized for a model's limit: the kernel of a step is chosen by the tables that prepare() was given, that of a graph by the
+    length that capture() was told."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    from flashinfer_mla_fp4_b200 import FP4MLADecodeBackend, FP4MLAPagedCache, planner, synth
+
+    dev, lens, limit = torch.device("cuda:0"), [4000, 200, 1500, 2000], 131072
+    case = synth.build_case("backend", lens, 128, 64, seed=8, device=dev)
+    backend = FP4MLADecodeBackend(128, 64, len(lens), limit, case.softmax_scale, dev)
+    cache = FP4MLAPagedCache(case.kv_cache.shape[0], 64, dev)
+    cache.kv_cache.copy_(case.kv_cache)
+    cache.kv_cache_sf.copy_(case.kv_cache_sf)
+    told, run = [], backend.wrapper.run
+    backend.wrapper.run = lambda *a, **k: told.append(a[4]) or run(*a, **k)
+    lat, rope = torch.randn(4, 512, device=dev), torch.randn(4, 64, device=dev)
+
+    def eager():
+        backend.prepare(case.block_tables, case.seq_lens)
+        return backend.forward(case.q, lat, rope, cache).clone()
+
+    def replayed(step):
+        backend.prepare(case.block_tables, case.seq_lens)
+        step.q.copy_(case.q), step.latent.copy_(lat), step.rope.copy_(rope)
+        return step.replay().clone()
+
+    width = case.block_tables.shape[1] * 64
+    first = eager()
+    assert told == [width] and planner.decode_plan(lens, 1, 128, 64, limit // 64, 148, width).groups_per_cluster == 1
+    short = backend.capture(cache, in_dtype=torch.float32, expected_seq_len=4000)
+    assert set(told[1:]) == {4000}
+    del told[:]
+    full = backend.capture(cache, in_dtype=torch.float32)
+    assert set(told) == {limit} and planner.decode_plan(lens, 1, 128, 64, limit // 64, 148, limit).groups_per_cluster == 2
+    assert torch.equal(replayed(short), first) and torch.equal(eager(), first)
+    O.assert_parity(replayed(full), first.float().cpu(), "the other kernel")
+    del told[:]
+    graph = torch.cuda.CUDAGraph()  # a caller's own capture: for any later step, not for the one prepared last
+    with torch.cuda.graph(graph):
+        backend.forward(case.q, lat, rope, cache)
+    assert told == [limit]
+    with pytest.raises(ValueError, match="expected_seq_len"):
+        backend.capture(cache, expected_seq_len=limit + 1)
+    backend.wrapper.check_device_status()

@@ -295,3 +295,27 @@ def test_decode_plan(seq_lens, heads, q_len, ctas, expect):
     assert (p.groups_per_cluster, p.grid, p.work_ctas) == expect
     if p.groups_per_cluster == 1:
         assert p.work_ctas == planner.work_ctas(seq_lens, q_len, heads, ctas)
+
+
+@pytest.mark.parametrize("batch,q_len,page,max_pages,max_seq_len,pair", [
+    (16, 1, 64, 2048, 131072, True),
+    (16, 1, 64, 2048, 4000, False),   # wide tables, requests stated as short: what is stated counts
+    (16, 1, 64, 63, 131072, False),   # ... and so does what the tables can hold
+    (16, 1, 64, 0, 0, False),         # nothing is known
+    (16, 1, 64, 0, 16384, True),
+    (16, 1, 64, 256, 0, True),
+    (16, 1, 64, 2048, 500, True),     # too short to be split
+    (80, 1, 64, 2048, 500, False),    # more pairs than CTAs: split, few tiles
+    (16, 1, 32, 2048, 131072, False),  # pages below 64 tokens: only where nothing is split
+    (16, 1, 8, 2048, 512, True),
+    (16, 1, 8, 64, 0, True),
+    (16, 1, 8, 2048, 513, False),
+    (15, 1, 64, 100, 0, False),       # below twenty tiles a CTA
+    (30, 1, 64, 100, 0, True),
+    (15, 1, 64, 100, -7, False),      # a hint that is none
+])
+def test_choice_of_the_decode_kernel(batch, q_len, page, max_pages, max_seq_len, pair):
+    from flashinfer_mla_fp4_b200 import planner
+
+    p = planner.decode_plan([100] * batch, q_len, 128, page, max_pages, 148, max_seq_len)
+    assert (p.groups_per_cluster == 2) == pair
