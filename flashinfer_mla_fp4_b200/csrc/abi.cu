@@ -161,7 +161,7 @@ int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t
     return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/num_ctas/max_pages_per_request out of range");
   if (!page_size_ok(page_size)) return fail(MLA_FP4_ERR_UNSUPPORTED, "page_size must be one of 8, 16, 32, 64, 128");
   const int groups = mla::num_groups(q_len, num_heads), cap = seq_cap_of(max_pages_per_request, page_size);
-  const mla::DecodeForm f = mla::decode_form(batch, groups, page_size, longest_of(max_seq_len, cap), num_ctas);
+  const mla::DecodeForm f = mla::decode_form(batch, groups, page_size, longest_of(max_seq_len, cap), 0, num_ctas);
   *groups_per_cluster = f.pair ? 2 : 1;
   *grid = f.grid;
   return work_ctas ? count_work_ctas(seq_lens_host, cap, batch, groups, f.grid, f.share, work_ctas) : MLA_FP4_OK;
@@ -226,6 +226,7 @@ int mla_fp4_decode(const MlaFp4DecodeArgs* a) {
   cudaError_t e = cudaSuccess;
   const bool fused = a->kernel == MLA_FP4_KERNEL_TCGEN05;
   p.fused_merge = fused ? 1 : 0;
+  p.phase_mask = a->phase_mask;
   p.merge_last = fused && (a->phase_mask & 4) ? 1 : 0;
   const bool do_decode = fused || a->phase_mask == 0 || (a->phase_mask & 1);
   const bool do_combine = !fused && (a->phase_mask == 0 || (a->phase_mask & 2));

@@ -153,9 +153,11 @@ struct DecodeForm {
   int grid;
   int share;  // the number of working CTAs is a multiple of this: the groups where they share the grid evenly, or 1
 };
-inline DecodeForm decode_form(int batch, int groups, int page_size, int longest, int num_ctas) {
+// phase_mask (MlaFp4DecodeArgs): 8 = pairs wherever they can be used, 16 = never.
+inline DecodeForm decode_form(int batch, int groups, int page_size, int longest, int phase_mask, int num_ctas) {
   const int pair_grid = shared_grid(groups, num_ctas, true);
-  const bool pair = pair_grid && pair_pays(batch, groups, page_size, longest, pair_grid);
+  const bool pays = phase_mask & 8 ? true : (phase_mask & 16 ? false : pair_pays(batch, groups, page_size, longest, pair_grid));
+  const bool pair = pair_grid && pays;
   const int grid = pair ? pair_grid : shared_grid(groups, num_ctas, false);
   return grid ? DecodeForm{pair, grid, groups} : DecodeForm{false, num_ctas, 1};
 }

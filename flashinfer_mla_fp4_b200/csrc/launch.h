@@ -27,6 +27,7 @@ struct DecodeParams {
   int32_t fused_merge;  // the decode kernel merges the split-KV partials itself
   int32_t merge_last;   // ... always by the last writer of a request (tests; otherwise only when the grid is not resident at once)
   int32_t longest;      // the longest request as far as the caller tells (decode_form), 0 when it does not
+  int32_t phase_mask;   // as in MlaFp4DecodeArgs
   int32_t seq_cap;      // most tokens a request may have: block-table width * page_size (INT_MAX when not given)
   uint32_t wait_polls;  // poll budget of every bounded wait
   float soft_cap;       // > 0: raw scores pass through cap * tanh(s / cap)

@@ -107,7 +107,8 @@ typedef struct MlaFp4DecodeArgs {
                           prologue while the decode kernel drains (0/1) */
   int32_t phase_mask;  /* two-kernel modes only: 0 = decode + combine; 1 = decode kernel only;
                           2 = combine kernel only (profiling).  MLA_FP4_KERNEL_TCGEN05: 4 = merge split
-                          requests by their last writer even when the whole grid is resident (tests) */
+                          requests by their last writer even when the whole grid is resident, 8 = two head groups
+                          on a pair of CTAs wherever an even number of groups allows it, 16 = nowhere (tests) */
   void* stream;        /* cudaStream_t */
   /* Width of a block-table row in pages (block_tables.shape[1]).  The kernels never read a row
      beyond it: a seq_lens entry larger than max_pages_per_request * page_size is treated as

@@ -1,14 +1,20 @@
 """The decode kernel for an even number of head groups (two CTAs, two groups of the same tiles) where it can go wrong: edges of tiles,
 half tiles and pages, many requests in one pair's walk, heads that fill no group, every output type and variant, both merge
-forms, references that move, a wait that runs out.  Against the oracle, and against the other kernel (the two-kernel mode uses it).  The grids are
-so small that there are twenty tiles or more to a CTA, or the requests so
-short that they are not split: there this kernel is used."""
+forms, references that move, a wait that runs out, steps under capture and on two streams.  Against the oracle, and against the other
+kernel (the two-kernel mode uses it).  The calls ask for this kernel (phase mask 8), whatever the rule between the two says of them."""
 import pytest
 import torch
 
 from oracle import mla_fp4_oracle as O
 
 pytestmark = pytest.mark.gpu
+PAIRS = 8
+
+
+def takes_pairs(w, q_len):
+    """Whether a call of this wrapper can take the kernel under test: an even number of groups, and a grid that they nearly fill evenly."""
+    groups = q_len * -(-w._num_heads // 64)
+    assert groups % 2 == 0 and 8 * (w._num_ctas // groups * groups) >= 7 * w._num_ctas
 
 
 def _run(lens, heads, page, q_len, max_ctas=None, out_dtype=None, variant=None, sharp=1.0, latent="normal", forms=(0, 4), **ref_kw):
@@ -22,7 +28,8 @@ def _run(lens, heads, page, q_len, max_ctas=None, out_dtype=None, variant=None, 
     w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
     w.plan(num_heads=heads, page_size=page, max_ctas=max_ctas, out_dtype=out_dtype, variant=variant)
     scale, got = case.softmax_scale * sharp, []
-    for kernel, mask in [(_cabi.KERNEL_TCGEN05, f) for f in forms] + [(_cabi.KERNEL_TCGEN05_2PASS, 0)]:
+    takes_pairs(w, q_len)
+    for kernel, mask in [(_cabi.KERNEL_TCGEN05, PAIRS | f) for f in forms] + [(_cabi.KERNEL_TCGEN05_2PASS, 0)]:
         w._kernel, w._phase_mask = kernel, mask
         got.append(w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, scale, kv_cache_sf=case.kv_cache_sf, return_lse=True))
         torch.cuda.synchronize()
@@ -80,6 +87,7 @@ def test_a_pair_that_gave_up_leaves_the_workspace_consistent():
     case = synth.build_case("gave up", [3000, 5000], 128, 64, seed=21, device=dev)
     w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
     w.plan(num_heads=128, page_size=64, max_ctas=8)
+    w._phase_mask = PAIRS
 
     def step(tables):
         out = w.run(case.q, case.kv_cache, tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
@@ -111,6 +119,7 @@ def test_a_small_poll_budget_is_a_budget_of_tiles():
     case = synth.build_case("polls", [200000, 200], 128, 64, seed=3, device=dev)  # one pair of CTAs: 1563 tiles, then two
     w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
     w.plan(num_heads=128, page_size=64, max_ctas=2)
+    w._phase_mask = PAIRS
 
     def step():
         out = w.run(case.q, case.kv_cache, case.block_tables, case.seq_lens, case.max_seq_len, case.softmax_scale, kv_cache_sf=case.kv_cache_sf)
@@ -123,6 +132,72 @@ def test_a_small_poll_budget_is_a_budget_of_tiles():
     got, status = step(), w.device_status()
     assert status[0] == 0, status
     assert torch.equal(got, expect)
+
+
+def _pair_case(lens, heads, q_len, max_ctas, seed):
+    from flashinfer_mla_fp4_b200 import BatchMLADecodeCuteDSLFP4Wrapper, synth
+
+    dev = torch.device("cuda:0")
+    case = synth.build_case("pair", lens, heads, 64, q_len=q_len, seed=seed, device=dev)
+    w = BatchMLADecodeCuteDSLFP4Wrapper(torch.empty(32 << 20, dtype=torch.int8, device=dev))
+    w.plan(num_heads=heads, page_size=64, max_ctas=max_ctas)
+    takes_pairs(w, q_len)
+    w._phase_mask = PAIRS
+    return w, lambda seq_lens, out=None: w.run(case.q, case.kv_cache, case.block_tables, seq_lens, case.max_seq_len, case.softmax_scale, out=out,
+                                               kv_cache_sf=case.kv_cache_sf), case
+
+
+@pytest.mark.parametrize("batch", [1, 32, 33, 130])  # lanes of one warp, one more, several rounds of segments
+def test_pairs_and_lengths_changed_by_the_kernel_ahead(batch):
+    """Each CTA of a pair makes its own plan, before the kernel ahead has ended: both must see the lengths that it leaves."""
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    w, run, case = _pair_case([700] * batch, 128, 1, None, batch)
+    lens = [torch.full((batch,), v, dtype=torch.int32, device="cuda:0") for v in (700, 65)]
+    lens[1][-1] = 640  # (only the last one differs from the third step's)
+    lens.append(lens[1].clone())
+    lens[2][-1] = 1
+    want = []
+    for x in lens:
+        want.append(run(x))
+        torch.cuda.synchronize()
+    now = lens[0].clone()
+    for k in (0, 1, 2, 1, 0):  # steps back to back
+        now.copy_(lens[k])
+        run(lens[2])
+        assert torch.equal(run(now), want[k])
+    w.check_device_status()
+
+
+def test_pairs_in_a_graph_and_on_two_streams():
+    if not torch.cuda.is_available():
+        pytest.fail("a CUDA device is required for -m gpu tests")
+    both = [_pair_case([9000, 700, 3000], 128, 2, None, 4), _pair_case([300] * 40, 100, 1, None, 5)]
+    want, graphs, streams = [], [], [torch.cuda.Stream() for _ in both]
+    for w, run, case in both:
+        shorter = case.seq_lens - 200
+        want.append((run(case.seq_lens), run(shorter), shorter))
+        now, out = case.seq_lens.clone(), torch.empty_like(want[-1][0])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run(now, out)
+        graphs.append((graph, now, out))
+    torch.cuda.synchronize()
+    for lens in (0, 1, 0):  # one graph, other lengths
+        for (graph, now, out), (a, b, shorter), (w, run, case) in zip(graphs, want, both):
+            now.copy_(shorter if lens else case.seq_lens)
+            graph.replay()
+            assert torch.equal(out, b if lens else a)
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(20):  # steps of two workspaces side by side
+        for i, (w, run, case) in enumerate(both):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(run(case.seq_lens))
+    torch.cuda.synchronize()
+    for i, (w, run, case) in enumerate(both):
+        w.check_device_status()
+        assert all(torch.equal(x, want[i][0]) for x in got[i])
 
 
 def test_a_backend_chooses_by_the_lengths_it_is_told():
