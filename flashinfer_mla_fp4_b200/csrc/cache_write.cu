@@ -279,27 +279,33 @@ template <typename T2, typename T> __device__ __forceinline__ uint32_t amax_bits
 template <typename T> struct PairOf;
 template <> struct PairOf<__half> { using type = __half2; };
 template <> struct PairOf<__nv_bfloat16> { using type = __nv_bfloat162; };
-// (as amax_without_nan, each lane of the token's group on its own)
-template <typename T> __device__ __noinline__ float amax_without_nan_alone(const T* row) {
-  float m = 0.f;
-#pragma unroll 1
-  for (int i = 0; i < kLatent; ++i) m = fmaxf(m, fabsf(to_f32<T>(row[i])));
-  return m;
-}
-// The codes of a chunk that the fast form leaves open: all of them by division (`exact`), or those in which q_lo and q_hi (word
-// and up) differ.  e: the chunk's first element.
-template <typename T> __device__ __noinline__ uint32_t settle(const T* e, float scale, uint32_t word, uint32_t up, bool exact) {
-  uint32_t todo = exact ? 0xffffffffu : word ^ up;
+// The codes of a chunk in which q_lo and q_hi (word and up) differ.  e: the chunk's first element.
+template <typename T> __device__ __noinline__ uint32_t settle(const T* e, float scale, uint32_t word, uint32_t up) {
+  uint32_t todo = word ^ up;
 #pragma unroll 1
   while (todo) {
     const int i = (__ffs(todo) - 1) >> 2;
     const uint32_t nibble = 0xfu << (4 * i);
     todo &= ~nibble;
-    const float x = to_f32<T>(e[i]);
-    if (exact) word = (word & ~nibble) | (e2m1_code(x, scale) << (4 * i));
-    else if (above(x, scale, (word >> (4 * i)) & 7u)) word = (word & ~nibble) | (up & nibble);
+    if (above(to_f32<T>(e[i]), scale, (word >> (4 * i)) & 7u)) word = (word & ~nibble) | (up & nibble);
   }
   return word;
+}
+// A token that takes the exact division for all its codes, by the whole warp: 16 of them a lane, as in cache_write_kernel.
+template <typename T> __device__ __noinline__ void write_exactly(const T* src, float scale, uint8_t* row, int lane) {
+#pragma unroll 1
+  for (int q = 0; q < 2; ++q) {
+    const T* e = src + 256 * q + 8 * lane;
+    uint32_t word = 0;
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i) word |= e2m1_code(to_f32<T>(e[i]), scale) << (4 * i);
+    *reinterpret_cast<uint32_t*>(row + 4 * lane + 128 * q) = word;
+  }
+}
+
+// another lane's pointer
+template <typename P> __device__ __forceinline__ P* of_lane(P* p, int lane) {
+  return reinterpret_cast<P*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), lane));
 }
 
 template <typename T>
@@ -307,14 +313,14 @@ __global__ void __launch_bounds__(kManyWarps * 32, kManyResident)
 cache_write_many_kernel(const T* __restrict__ latent, int64_t latent_stride, const T* __restrict__ rope, int64_t rope_stride,
                         const float* __restrict__ scale_in, const int64_t* __restrict__ slot_mapping, int64_t num_tokens,
                         uint8_t* __restrict__ cache, float* __restrict__ cache_sf, int64_t num_slots, bool rope_16) {
-  const int lane = threadIdx.x & (kManyLanes - 1);
+  const int lane = threadIdx.x & (kManyLanes - 1), group = (threadIdx.x & 31) / kManyLanes;
   constexpr int kPerCta = kManyWarps * 32 / kManyLanes;
   const int64_t step = int64_t(gridDim.x) * kPerCta;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // (a warp's groups stay together: those past the end go over the last token again and write nothing)
   int64_t t = int64_t(blockIdx.x) * kPerCta + threadIdx.x / kManyLanes;
-  int64_t t0 = t - (threadIdx.x & 31) / kManyLanes;
+  int64_t t0 = t - group;
 #pragma unroll 1
   for (; t0 < num_tokens; t += step, t0 += step) {
     const int64_t at = t < num_tokens ? t : num_tokens - 1;
@@ -335,11 +341,20 @@ cache_write_many_kernel(const T* __restrict__ latent, int64_t latent_stride, con
     uint32_t top = amax_bits_many<typename PairOf<T>::type, T>(raw);    // non-negative floats compare as integers
 #pragma unroll
     for (int o = kManyLanes / 2; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (!__any_sync(0xffffffffu, live)) continue;
     float scale;
     if (scale_in) {
       scale = scale_in[at];
     } else {
-      scale = __fdiv_rn(top <= kInfBits ? __uint_as_float(top) : amax_without_nan_alone<T>(latent + at * latent_stride), 6.0f);
+      float amax = __uint_as_float(top);
+#pragma unroll 1
+      for (uint32_t nans = __ballot_sync(0xffffffffu, top > kInfBits && live); nans;) {  // one token after the other, by the whole warp
+        const int g = (__ffs(nans) - 1) / kManyLanes;
+        nans &= ~(((1u << kManyLanes) - 1u) << (kManyLanes * g));
+        const float m = amax_without_nan<T>(of_lane(src, kManyLanes * g), threadIdx.x & 31);
+        if (g == group) amax = m;
+      }
+      scale = __fdiv_rn(amax, 6.0f);
       if (!(scale > 0.f)) scale = 1.0f;
     }
     const bool odd = !(scale >= kScaleLo && scale <= kScaleHi && top <= kInfBits);
@@ -362,8 +377,8 @@ cache_write_many_kernel(const T* __restrict__ latent, int64_t latent_stride, con
       };
       uint32_t w = codes(lo2), up = w;
       if (both && !lo_alone) up = codes(hi2);
-      if (odd || w != up) w = settle<T>(src + 8 * kManyLanes * q, scale, w, up, odd);
-      if (live) *reinterpret_cast<uint32_t*>(row + 4 * (lane + kManyLanes * q)) = w;
+      if (w != up && !odd) w = settle<T>(src + 8 * kManyLanes * q, scale, w, up);
+      if (live && !odd) *reinterpret_cast<uint32_t*>(row + 4 * (lane + kManyLanes * q)) = w;
     }
     uint32_t r8[2];
 #pragma unroll
@@ -375,11 +390,18 @@ cache_write_many_kernel(const T* __restrict__ latent, int64_t latent_stride, con
       *reinterpret_cast<uint2*>(row + kLatent / 2 + kManyRope * lane) = make_uint2(r8[0], r8[1]);
       if (lane == 0) cache_sf[slot] = scale;
     }
+#pragma unroll 1
+    for (uint32_t rest = __ballot_sync(0xffffffffu, odd && live); rest;) {
+      const int from = __ffs(rest) - 1;  // (lane 0 of a token's group)
+      rest &= ~(((1u << kManyLanes) - 1u) << from);
+      write_exactly<T>(of_lane(src, from), __shfl_sync(0xffffffffu, scale, from), of_lane(row, from), threadIdx.x & 31);
+    }
   }
 }
 
 // From how many tokens of a 16-bit type on four go to a warp: one a warp -> four, inputs that are not in L2: 8191 tokens 5.17 -> 5.04 us,
-// 16384 7.94 -> 8.58, 30000 10.82 -> 10.04, 60000 19.2 -> 16.2, 262144 75.3 -> 59.3; 61 tokens 1.68 -> 2.33.
+// 16384 7.94 -> 8.58, 24576 9.6 -> 9.2 (FP16 9.0 -> 8.2), 30000 11.2 -> 10.3, 60000 19.2 -> 16.2, 262144 75.3 -> 59.3; 61 tokens 1.68 -> 2.33.
+// Strided rows 24576 9.95 -> 9.65; nine of ten tokens padding 6.9 -> 7.5, 200000 39.1 -> 37.1; all of them 6.05 -> 5.55; a NaN in every token 46.0 -> 44.9.
 constexpr int64_t kManyTokens = 24576;
 template <typename T>
 cudaError_t launch_t(const void* latent, int64_t ls, const void* rope, int64_t rs, const float* scale_in,

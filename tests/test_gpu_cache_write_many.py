@@ -9,7 +9,7 @@ MANY = 24576  # from here on in one call: the form under test
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("extra", [0, 1, 6])
-@pytest.mark.parametrize("form", ["plain", "strided", "given"])
+@pytest.mark.parametrize("form", ["plain", "strided", "given", "nans", "padding"])
 def test_many_tokens_as_in_pieces(dtype, extra, form):
     if not torch.cuda.is_available():
         pytest.fail("a CUDA device is required for -m gpu tests")
@@ -27,6 +27,9 @@ def test_many_tokens_as_in_pieces(dtype, extra, form):
     latent[::7] *= 2.0 ** -10
     latent[11], latent[n - 1, 3] = 0.0, -0.0
     latent[17, 100], latent[18, 0], latent[23] = float("nan"), float("inf"), 1e-30  # (the last is zero in FP16)
+    if form == "nans":  # one to four tokens of a warp; runs of them
+        latent[rnd(n) > 0.5, 7] = float("nan")
+        latent[1000:1064, 500] = float("nan")
     rope = rnd(n, 64) * 200
     stride = 520 if form == "strided" else 512
     lat = torch.empty(n, stride, dtype=dtype, device=dev)[:, :512].copy_(latent)
@@ -37,6 +40,8 @@ def test_many_tokens_as_in_pieces(dtype, extra, form):
     pages = n // page + 40
     slots = torch.randperm(pages * page, generator=g, device=dev)[:n]
     slots[5], slots[n - 2], slots[300] = -1, pages * page, -7  # padding and out of the pool: nothing is written
+    if form == "padding":  # whole warps and parts of them
+        slots[rnd(n) > 0], slots[2000:3001] = -1, -1
 
     def written(step):
         cache = torch.full((pages, page, 320), 0xAB, dtype=torch.uint8, device=dev)
