@@ -76,6 +76,7 @@ EXPORTS = (
     "mla_fp4_merge_partials",
     "mla_fp4_dequant_e2m1_to_e4m3",
     "mla_fp4_cache_write",
+    "mla_fp4_cache_write_plan",
     "mla_fp4_decode_static",
     "mla_fp4_static_reset",
     "mla_fp4_cp_exchange_bytes",
@@ -139,6 +140,8 @@ def _load() -> C.CDLL:
     lib.mla_fp4_cache_write.argtypes = [C.c_void_p, C.c_int64, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p,
                                         C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
     lib.mla_fp4_cache_write.restype = C.c_int
+    lib.mla_fp4_cache_write_plan.argtypes = [C.c_int32, C.c_int64, C.c_int32, i32p]
+    lib.mla_fp4_cache_write_plan.restype = C.c_int
     lib.mla_fp4_step_metadata.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_int32,
                                           C.c_int32, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]
     lib.mla_fp4_step_metadata.restype = C.c_int

@@ -416,6 +416,14 @@ int mla_fp4_cp_exchange_merge(void* const* blocks, int32_t world, int32_t rank, 
   return MLA_FP4_OK;
 }
 
+int mla_fp4_cache_write_plan(int32_t in_dtype, int64_t num_tokens, int32_t scales_given, int32_t* tokens_per_warp) {
+  if (!tokens_per_warp || num_tokens < 0) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer or num_tokens out of range");
+  if (in_dtype != MLA_FP4_IN_BF16 && in_dtype != MLA_FP4_IN_F16 && in_dtype != MLA_FP4_IN_F32)
+    return fail(MLA_FP4_ERR_UNSUPPORTED, "in_dtype must be MLA_FP4_IN_BF16, MLA_FP4_IN_F16 or MLA_FP4_IN_F32");
+  *tokens_per_warp = mla::cache_write_tokens_per_warp(in_dtype != MLA_FP4_IN_F32, num_tokens, scales_given != 0);
+  return MLA_FP4_OK;
+}
+
 int mla_fp4_cache_write(const void* latent, int64_t latent_stride, const void* rope, int64_t rope_stride,
                         int32_t in_dtype, const float* token_scale, const int64_t* slot_mapping,
                         int64_t num_tokens, void* kv_cache, float* kv_cache_sf, int64_t num_slots, void* stream) {

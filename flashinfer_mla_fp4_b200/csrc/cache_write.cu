@@ -401,8 +401,15 @@ cache_write_many_kernel(const T* __restrict__ latent, int64_t latent_stride, con
 
 // From how many tokens of a 16-bit type on four go to a warp: one a warp -> four, inputs that are not in L2: 8191 tokens 5.17 -> 5.04 us,
 // 16384 7.94 -> 8.58, 24576 9.6 -> 9.2 (FP16 9.0 -> 8.2), 30000 11.2 -> 10.3, 60000 19.2 -> 16.2, 262144 75.3 -> 59.3; 61 tokens 1.68 -> 2.33.
+// With the scales given every token is converted twice (see lo_alone), which weighs more where a lane has four times the work: 24576 10.6 ->
+// 12.3, 40000 15.3 -> 16.4, 57344 20.2 -> 20.35 (FP16 18.35 -> 18.55), 200000 62.8 -> 55.2 (57.0 -> 51.1).
 // Strided rows 24576 9.95 -> 9.65; nine of ten tokens padding 6.9 -> 7.5, 200000 39.1 -> 37.1; all of them 6.05 -> 5.55; a NaN in every token 46.0 -> 44.9.
-constexpr int64_t kManyTokens = 24576;
+constexpr int64_t kManyTokens = 24576, kManyTokensScaled = 65536;
+}  // namespace
+int cache_write_tokens_per_warp(bool half, int64_t n, bool scales_given) {
+  return half && n >= (scales_given ? kManyTokensScaled : kManyTokens) ? 4 : 1;
+}
+namespace {
 template <typename T>
 cudaError_t launch_t(const void* latent, int64_t ls, const void* rope, int64_t rs, const float* scale_in,
                      const int64_t* slots, int64_t n, void* cache, float* sf, int64_t num_slots, cudaStream_t stream) {
@@ -419,7 +426,7 @@ cudaError_t launch_t(const void* latent, int64_t ls, const void* rope, int64_t r
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if constexpr (sizeof(T) == 2) {
-    if (n >= kManyTokens) {
+    if (cache_write_tokens_per_warp(true, n, scale_in != nullptr) > 1) {
       constexpr int64_t per = kManyWarps * 32 / kManyLanes;
       const int64_t want = (n + per - 1) / per;
       cfg.gridDim = dim3(unsigned(want < 0x7fffffff ? want : 0x7fffffff));

@@ -82,6 +82,7 @@ cudaError_t launch_fp32_check(const DecodeParams& p, int num_ctas, cudaStream_t 
 cudaError_t launch_cache_write(const void* latent, int64_t latent_stride, const void* rope, int64_t rope_stride, int in_dtype,
                                const float* scale_in, const int64_t* slot_mapping, int64_t num_tokens, void* cache,
                                float* cache_sf, int64_t num_slots, cudaStream_t stream);
+int cache_write_tokens_per_warp(bool half, int64_t n, bool scales_given);  // which of the writer's two forms launch_cache_write takes
 struct StepMetadataParams {
   const int32_t* block_tables;
   int64_t block_table_stride;

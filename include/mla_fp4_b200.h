@@ -261,6 +261,10 @@ int mla_fp4_cache_write(const void* latent, int64_t latent_stride, const void* r
                         int64_t num_tokens, void* kv_cache, float* kv_cache_sf, int64_t num_slots,
                         void* stream);
 
+/* Which of its two forms mla_fp4_cache_write takes: *tokens_per_warp is 1 or, for many tokens of a 16-bit type, 4.
+   The bytes they write are the same.  Host only. */
+int mla_fp4_cache_write_plan(int32_t in_dtype, int64_t num_tokens, int32_t scales_given, int32_t* tokens_per_warp);
+
 /* Refresh the persistent metadata of a decode step (what a captured step reads) from a scheduler's tensors, in one
    launch: block_tables int32 [batch][width] with row stride block_table_stride -> dst_block_tables (row stride
    dst_block_table_stride, columns beyond width untouched); seq_lens [batch] (int32, or int64 when seq_lens_is_64) ->

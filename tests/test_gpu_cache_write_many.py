@@ -4,7 +4,17 @@ import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
-MANY = 24576  # from here on in one call: the form under test
+MANY = {False: 24576, True: 65536}  # from here on in one call: the form under test (scales given or not)
+
+
+def tokens_per_warp(dtype, n, given):
+    import ctypes as C
+
+    from flashinfer_mla_fp4_b200 import _cabi
+
+    out = C.c_int32(0)
+    _cabi.check(_cabi.lib.mla_fp4_cache_write_plan({torch.bfloat16: _cabi.IN_BF16, torch.float16: _cabi.IN_F16}[dtype], n, int(given), C.byref(out)))
+    return out.value
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -15,7 +25,8 @@ def test_many_tokens_as_in_pieces(dtype, extra, form):
         pytest.fail("a CUDA device is required for -m gpu tests")
     from flashinfer_mla_fp4_b200.kvcache import write_tokens
 
-    dev, n, page = torch.device("cuda:0"), MANY + extra, 16
+    dev, n, page = torch.device("cuda:0"), MANY[form == "given"] + extra, 16
+    assert [tokens_per_warp(dtype, k, form == "given") for k in (n, MANY[form == "given"] - 1, 5000)] == [4, 1, 1]
     g = torch.Generator(device=dev).manual_seed(extra + 5)
 
     def rnd(*shape):

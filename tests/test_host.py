@@ -319,3 +319,18 @@ def test_choice_of_the_decode_kernel(batch, q_len, page, max_pages, max_seq_len,
 
     p = planner.decode_plan([100] * batch, q_len, 128, page, max_pages, 148, max_seq_len)
     assert (p.groups_per_cluster == 2) == pair
+
+
+@pytest.mark.parametrize("dtype,tokens,given,expect", [
+    ("IN_BF16", 24575, 0, 1), ("IN_BF16", 24576, 0, 4), ("IN_F16", 24576, 0, 4), ("IN_F32", 262144, 0, 1),
+    ("IN_BF16", 30000, 1, 1), ("IN_F16", 65535, 1, 1), ("IN_F16", 65536, 1, 4), ("IN_BF16", 0, 0, 1),
+])
+def test_form_of_the_cache_writer(dtype, tokens, given, expect):
+    """With the scales given, which makes a token dearer, four tokens a warp pay later."""
+    import ctypes as C
+
+    from flashinfer_mla_fp4_b200 import _cabi
+
+    out = C.c_int32(0)
+    _cabi.check(_cabi.lib.mla_fp4_cache_write_plan(getattr(_cabi, dtype), tokens, given, C.byref(out)))
+    assert out.value == expect
