@@ -258,11 +258,11 @@ cache_write_kernel(const T* __restrict__ latent, int64_t latent_stride, const T*
 // reciprocal, the tests: a third of the 241 instructions a token cost a warp) is shared by four tokens, and a warp has 4.5 KiB of loads
 // in flight before it waits, so that the next token's need not be kept in registers beside this one's.  CTAs of two warps and
 // no loop over the tokens (but for the largest grids): the hardware fills the place of a CTA as soon as it is done.
-// 262144 BF16 tokens 75.3 -> 59.3 us, 6.56 TB/s, the rate of a plain copy (with a loop: 24 warps a SM 63.2; the next tokens in registers 74.9;
+// 262144 BF16 tokens 75.3 -> 58.7 us, 6.63 TB/s, the rate of a plain copy (with a loop: 24 warps a SM 63.2; the next tokens in registers 74.9;
 // staged with cp.async 64.8).  Fewer tokens take longer this way, a lane having four times the work one after the other:
 // see launch_t.  FP32 rows gain nothing: a warp per token runs at 6.58 TB/s.
 constexpr int kManyWarps = 2;
-constexpr int kManyResident = 14;  // CTAs per SM: 72 registers a thread hold a token's share without spills
+constexpr int kManyResident = 14;  // CTAs per SM, which leave 72 registers a thread: they hold a token's share without spills (BF16 70, FP16 66)
 constexpr int kManyLanes = 8, kManyChunks = kLatent / (8 * kManyLanes), kManyRope = kRope / kManyLanes;
 template <typename T> struct ManyShare {
   static_assert(sizeof(T) == 2, "a 16-byte chunk is eight elements");
@@ -400,7 +400,7 @@ cache_write_many_kernel(const T* __restrict__ latent, int64_t latent_stride, con
 }
 
 // From how many tokens of a 16-bit type on four go to a warp: one a warp -> four, inputs that are not in L2: 8191 tokens 5.17 -> 5.04 us,
-// 16384 7.94 -> 8.58, 24576 9.6 -> 9.2 (FP16 9.0 -> 8.2), 30000 11.2 -> 10.3, 60000 19.2 -> 16.2, 262144 75.3 -> 59.3; 61 tokens 1.68 -> 2.33.
+// 16384 7.94 -> 8.58, 24576 9.6 -> 9.2 (FP16 9.0 -> 8.2), 30000 11.2 -> 10.3, 60000 19.2 -> 16.2, 262144 75.3 -> 58.7; 61 tokens 1.68 -> 2.33.
 // With the scales given every token is converted twice (see lo_alone), which weighs more where a lane has four times the work: 24576 10.6 ->
 // 12.3, 40000 15.3 -> 16.4, 57344 20.2 -> 20.35 (FP16 18.35 -> 18.55), 200000 62.8 -> 55.2 (57.0 -> 51.1).
 // Strided rows 24576 9.95 -> 9.65; nine of ten tokens padding 6.9 -> 7.5, 200000 39.1 -> 37.1; all of them 6.05 -> 5.55; a NaN in every token 46.0 -> 44.9.

@@ -12,8 +12,8 @@
 // so every latent byte is read twice from L2, once by the CTA that has its token and once by the one that has its dim, as often
 // as by two CTAs with a group each, and the operand reads from shared memory, which bound the other kernel (decode_sm100.cu), are a third
 // less: 4 KiB an MMA of QK^T and 5 of PV (P' read once for both halves of the dims) for as many products as take 6 and 8 there.
-// Measured back to back, a tile's MMAs take 576 + 1040 = 1617 clk (the rate of the tensor cores; 2111 there).  2x131072 tokens, 128 heads,
-// q_len 2: 105.7 -> 96.8 us (1000 W cap).
+// Measured back to back, a tile's MMAs take 576 + 1040 = 1616 clk (the rate of the tensor cores; 2111 there); in the kernel a tile takes 1780 (2300
+// there).  2x131072 tokens, 128 heads, q_len 2: 105.4 -> 96.5 us, at 1.38 GHz under the 1000 W cap.
 //
 // An accumulator of 64 rows per CTA lies in all 128 TMEM lanes: lanes 0-63 hold the heads for the first half of the columns, lanes
 // 64-127 the same heads for the second.  A softmax thread has one head and 64 tokens of every second tile: its reference and its sum are scalars, and
@@ -24,7 +24,7 @@
 // rescaled or read out) releases at cluster scope, behind its proxy and tcgen05 fences, and every wait acquires at that scope.  The release is a
 // fence of shared memory alone: 2x131072 tokens, 128 heads, q_len 2 95.9 us without it, 95.8 with it, 1x200 8.68 and 8.72; as
 // mbarrier.arrive.release.cluster, which waits for stores to global memory too, 142, and passed on by the idle issue warps of CTA 1 102.6.  The roles and the merge are those of the other kernel; the two issue
-// warps take no turns (with QK^T held to two tiles ahead of PV a tile took 2670 to 2800 clk, without 1840).
+// warps take no turns (with QK^T held to two tiles ahead of PV a tile took 2670 to 2800 clk).
 
 // shared memory map of the big part; from kOffP on as in the other kernel
 constexpr uint32_t kPairQkBytes = kBlocks * 64 * 128 + 64 * 64;  // 36 KiB: 64 tokens, four blocks [64][128 B] and RoPE [64][64 B]
@@ -305,7 +305,7 @@ __device__ __forceinline__ void pair_pv_role(uint32_t smem, uint32_t tmem, RoleS
 // ------------------------------------------------------------------------------------------
 // Two groups of four warps, one for the even tiles and one for the odd: a tile's chain of waits (S, the vote, P's buffer, fences) is
 // longer than a tile of the tensor pipe, and with all warps on the same tile nothing else runs meanwhile (2400 clk a tile, now
-// 1840).  What passes from tile to tile is the heads' references alone: the scores are made without them, and a group takes
+// 1780).  What passes from tile to tile is the heads' references alone: the scores are made without them, and a group takes
 // them over when the other one has moved them (or not), by a named barrier each way.  A group's row sums are relative to the
 // reference that it last saw.
 // Rows of the accumulators, scaled, to memory: head h of the CTA at dst + h * 512 elements.  A warp's 32 lanes are 32 heads, so a direct

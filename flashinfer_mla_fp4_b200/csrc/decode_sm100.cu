@@ -20,7 +20,7 @@
 // What bounds it (measured with one MMA form at a time, operands in shared memory): at N = 64 an MMA reads A (4 KiB) and
 // B (2 KiB) at the 128 B/clk of shared memory, 48 clk, and a PV pair that shares A through the collector takes 78: the 18 + 32
 // MMAs of a tile measured alone take 863 + 1248 = 2111 clk of tensor pipe, beside 72 KiB of TMA writes (560 clk of the same port).  A
-// tile takes 2500 in the steady state: the pipe also waits for P', whose one buffer is free when the last PV has completed.
+// tile takes 2300 (8x32768 tokens, from a CTA's fifth tile to its last): the pipe also waits for P', whose one buffer is free when the last PV has completed.
 // Everything else is arranged to stay under that:
 //   * latent blocks are handled in pairs (32 KiB, five pair slots = two and a half tiles in flight): one barrier, one wait
 //     and one commit per pair;
