@@ -184,11 +184,12 @@ __device__ __forceinline__ bool wait(uint32_t smem, int idx, uint32_t parity) {
   if (__all_sync(0xffffffffu, ptx::mbar_try_wait(bar_addr(smem, idx), parity))) return true;
   return __all_sync(0xffffffffu, wait_slow(smem, idx, parity));  // (already the same in all lanes; the vote says so to the compiler)
 }
-// Bounded wait that ignores the abort flag: lets in-flight asynchronous work land before exit.
+// Bounded wait that ignores the abort flag: lets in-flight asynchronous work land before exit.  Its bound has a floor (some milliseconds): however
+// small a budget the caller gave the other waits, a copy must not land in the shared memory of a CTA that has left.
 template <bool kCluster = false>
 __device__ __noinline__ void drain_wait(uint32_t smem, int idx, uint32_t parity) {
   const uint32_t bar = bar_addr(smem, idx), polls = misc_of(smem)->polls;
-  const uint32_t limit = polls < (1u << 20) ? polls : (1u << 20);
+  const uint32_t limit = min(max(polls, 1u << 10), 1u << 20);
 #pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
     if (kCluster ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity)) return;

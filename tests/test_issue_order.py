@@ -122,3 +122,9 @@ def test_proxy_fences_of_the_merge():
     assert fetch.index("ld_acquire(slot_flag") < fetch.index("fence_proxy_async_global()") < fetch.index("ptx::bulk_load(")
     last = re.search(r"void merge_as_last\(.*?\n}\n", text, re.S).group(0)  # one share after the other through the same buffer
     assert re.search(r"tail_merge\(p, smem, tid, parity\);\s*ptx::fence_proxy_async_smem\(\);[^\n]*\s*__syncthreads\(\);", last)
+
+
+def test_a_small_poll_budget_does_not_shorten_the_drain():
+    """A CTA that gave up stays until its copies have landed, whatever the budget of the waits that ran out."""
+    drain = re.search(r"void drain_wait\(.*?\n}\n", SOURCE.read_text(), re.S).group(0)
+    assert re.search(r"limit = min\(max\(polls, 1u << 10\), 1u << 20\);", drain) and "i < limit" in drain
