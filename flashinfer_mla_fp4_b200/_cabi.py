@@ -111,7 +111,7 @@ def _load() -> C.CDLL:
     lib.mla_fp4_plan_partition.restype = C.c_int
     lib.mla_fp4_work_ctas.argtypes = [i32p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, i32p]
     lib.mla_fp4_work_ctas.restype = C.c_int
-    lib.mla_fp4_decode_plan.argtypes = [C.c_int32] * 7 + [i32p] * 4
+    lib.mla_fp4_decode_plan.argtypes = [C.POINTER(DecodeArgs)] + [i32p] * 4
     lib.mla_fp4_decode_plan.restype = C.c_int
     lib.mla_fp4_decode.argtypes = [C.POINTER(DecodeArgs)]
     lib.mla_fp4_decode.restype = C.c_int

@@ -154,17 +154,23 @@ int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len
   return count_work_ctas(seq_lens_host, INT_MAX, batch, groups, grid ? grid : num_ctas, grid ? groups : 1, work_ctas);
 }
 
-int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size, int32_t max_pages_per_request, int32_t max_seq_len,
-                        int32_t num_ctas, const int32_t* seq_lens_host, int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas) {
-  if (!groups_per_cluster || !grid || (work_ctas && batch > 0 && !seq_lens_host)) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
-  if (batch < 0 || q_len <= 0 || num_heads <= 0 || num_ctas <= 0 || max_pages_per_request < 0)
-    return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/num_ctas/max_pages_per_request out of range");
-  if (!page_size_ok(page_size)) return fail(MLA_FP4_ERR_UNSUPPORTED, "page_size must be one of 8, 16, 32, 64, 128");
-  const int groups = mla::num_groups(q_len, num_heads), cap = seq_cap_of(max_pages_per_request, page_size);
-  const mla::DecodeForm f = mla::decode_form(batch, groups, page_size, longest_of(max_seq_len, cap), 0, num_ctas);
+int mla_fp4_decode_plan(const MlaFp4DecodeArgs* a, const int32_t* seq_lens_host, int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas) {
+  if (!a || !groups_per_cluster || !grid || (work_ctas && a->batch > 0 && !seq_lens_host)) return fail(MLA_FP4_ERR_BAD_ARG, "null pointer");
+  if (a->batch < 0 || a->q_len <= 0 || a->num_heads <= 0 || a->max_pages_per_request < 0)
+    return fail(MLA_FP4_ERR_BAD_ARG, "batch/q_len/num_heads/max_pages_per_request out of range");
+  if (!page_size_ok(a->page_size)) return fail(MLA_FP4_ERR_UNSUPPORTED, "page_size must be one of 8, 16, 32, 64, 128");
+  if (a->kernel != MLA_FP4_KERNEL_TCGEN05) return fail(MLA_FP4_ERR_UNSUPPORTED, "the plan is that of MLA_FP4_KERNEL_TCGEN05");
+  int num_ctas = a->num_ctas;
+  if (num_ctas <= 0) {
+    int rc = sm_count(&num_ctas);
+    if (rc) return rc;
+  }
+  const int groups = mla::num_groups(a->q_len, a->num_heads), cap = seq_cap_of(a->max_pages_per_request, a->page_size);
+  const mla::DecodeForm f = mla::decode_form({a->batch, groups, a->num_heads, a->page_size, longest_of(a->max_seq_len, cap), num_ctas, a->out_dtype,
+                                              a->logits_soft_cap > 0.f, a->phase_mask});
   *groups_per_cluster = f.pair ? 2 : 1;
   *grid = f.grid;
-  return work_ctas ? count_work_ctas(seq_lens_host, cap, batch, groups, f.grid, f.share, work_ctas) : MLA_FP4_OK;
+  return work_ctas ? count_work_ctas(seq_lens_host, cap, a->batch, groups, f.grid, f.share, work_ctas) : MLA_FP4_OK;
 }
 
 int mla_fp4_workspace_init(void* workspace, size_t workspace_bytes, void* stream) {

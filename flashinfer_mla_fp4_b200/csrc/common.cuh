@@ -132,8 +132,13 @@ MLA_HD int shared_grid(int groups, int num_ctas, bool pair) {
 
 // Where the pair kernel is used, by the longest request: the lengths themselves are on the device, so what the caller says of it (the least of the
 // max_seq_len it states and what its block tables can hold; 0: neither is known).  Single -> pair, 128 heads, BF16 output unless said:
-//  * requests too short to be split, whose rows leave faster: 32x(100..500) 13.0 -> 11.5 us, 1x200 9.85 -> 8.75, 8x512 12.65 -> 11.25, with pages of 16
-//    13.7 -> 12.7, of 8 17.85 -> 16.1; 6x110 with pages of 8 and FP32 output 10.65 -> 10.7.
+//  * requests too short to be split (whole_requests), by what their rows cost either kernel (1400 calls with both, ratios of the times; where pairs are taken
+//    0.90 in the mean, above 1.03 in one of 200):
+//      - FP32 rows of full groups never (one tile 1.11, more 1.01); groups that are not full, whose 8- and 32-bit rows the other kernel stores value by
+//        value, always with E4M3 (0.81; two tiles 0.79) and, from two tiles on, with FP32 (0.91);
+//      - from two tiles on with all else (BF16 0.93, E4M3 0.90; 20x512 13.05 -> 12.0 us, 1x200 9.85 -> 8.8), unless the pairs nearly fill the grid (1.03);
+//      - one tile, half of which is nothing to CTA 1, only with few of them: 8- and 32-bit rows up to a seventh of the grid (0.95; 1.02 beyond), FP32
+//        rows of at most 32 heads as above (0.93), full groups of BF16 rows up to a sixteenth (0.97; 1.02 beyond, with a soft cap 1.03).
 //  * from twenty tiles a CTA on, where the main loop counts, with pages of 64 and 128 tokens: 16x16000 51.95 -> 48.85, 24x8000 42.8 -> 42.0, 64x3000 47.55 ->
 //    45.2, 32x(1024..16384) 43.1 -> 39.85, 3x30000, q_len 3 52.4 -> 47.9; 2x131072, q_len 2 105.5 -> 97.  With smaller pages the copies of K, every byte of
 //    which is fetched by both CTAs of a pair as K of one and V of both, take longer: 16x16000 with pages of 32 52.55 -> 52.85, of 16 60.35 -> 62.6, of 8 89.0 -> 89.7.
@@ -141,10 +146,23 @@ MLA_HD int shared_grid(int groups, int num_ctas, bool pair) {
 //    4x4000 14.4 -> 15.65, 2x8000 14.8 -> 16.05, 60x(100..2000) 24.45 -> 25.4, 8x8000 23.4 -> 23.7, 2x(20000..60000), 64 heads, q_len 2 22.6 -> 23.9; the same at about
 //    thirteen tiles a CTA (2x64000 33.2 -> 32.6, 32x4000 35.05 -> 34.7).  Lengths far below the longest come out there too:
 //    24x(100..16384) 27.7 -> 28.7, but 64x(200..4000) 31.8 -> 31.8, 64x(500..8000) 44.5 -> 42.4.
-inline bool pair_pays(int batch, int groups, int page_size, int longest, int grid) {
-  const int64_t pairs = int64_t(batch) * groups, tiles = (int64_t(longest) + kTile - 1) / kTile;
-  if (longest <= 0) return false;
-  return whole_requests(int(tiles), pairs, grid) || (page_size >= 64 && pairs * tiles >= 20 * int64_t(grid));
+struct DecodeCall {
+  int batch, groups, heads, page_size, longest, num_ctas, out_dtype;
+  bool soft_cap;
+  int phase_mask;  // as in MlaFp4DecodeArgs: 8 = pairs wherever they can be used, 16 = never
+};
+inline bool pair_pays_short(const DecodeCall& c, bool one_tile, int64_t pairs, int grid) {
+  const bool full = c.heads % kGroupHeads == 0, f32 = c.out_dtype == MLA_FP4_OUT_F32, e4m3 = c.out_dtype == MLA_FP4_OUT_E4M3;
+  if (f32 && full) return false;
+  if (!full && (e4m3 || (f32 && !one_tile))) return true;
+  if (!one_tile || (f32 && c.heads <= kGroupHeads / 2)) return 4 * pairs <= 3 * int64_t(grid);
+  return f32 || e4m3 ? 7 * pairs <= grid : full && !c.soft_cap && 16 * pairs <= grid;
+}
+inline bool pair_pays(const DecodeCall& c, int grid) {
+  const int64_t pairs = int64_t(c.batch) * c.groups, tiles = (int64_t(c.longest) + kTile - 1) / kTile;
+  if (c.longest <= 0) return false;
+  if (whole_requests(int(tiles), pairs, grid)) return pair_pays_short(c, tiles == 1, pairs, grid);
+  return c.page_size >= 64 && pairs * tiles >= 20 * int64_t(grid);
 }
 
 // Which decode kernel a step runs when it merges by itself, and on which grid.
@@ -153,13 +171,11 @@ struct DecodeForm {
   int grid;
   int share;  // the number of working CTAs is a multiple of this: the groups where they share the grid evenly, or 1
 };
-// phase_mask (MlaFp4DecodeArgs): 8 = pairs wherever they can be used, 16 = never.
-inline DecodeForm decode_form(int batch, int groups, int page_size, int longest, int phase_mask, int num_ctas) {
-  const int pair_grid = shared_grid(groups, num_ctas, true);
-  const bool pays = phase_mask & 8 ? true : (phase_mask & 16 ? false : pair_pays(batch, groups, page_size, longest, pair_grid));
-  const bool pair = pair_grid && pays;
-  const int grid = pair ? pair_grid : shared_grid(groups, num_ctas, false);
-  return grid ? DecodeForm{pair, grid, groups} : DecodeForm{false, num_ctas, 1};
+inline DecodeForm decode_form(const DecodeCall& c) {
+  const int pair_grid = shared_grid(c.groups, c.num_ctas, true);
+  const bool pair = pair_grid && !(c.phase_mask & 16) && ((c.phase_mask & 8) || pair_pays(c, pair_grid));
+  const int grid = pair ? pair_grid : shared_grid(c.groups, c.num_ctas, false);
+  return grid ? DecodeForm{pair, grid, c.groups} : DecodeForm{false, c.num_ctas, 1};
 }
 
 // Positions in the flat tile space are 32-bit: a 64-bit division is a subroutine of a hundred instructions and these

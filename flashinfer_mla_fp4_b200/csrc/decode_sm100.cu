@@ -1882,7 +1882,8 @@ cudaError_t launch_decode_sm100(const DecodeParams& p, int num_ctas, cudaStream_
   MapPair<QKey>& qm = q_maps[map_slot(p.q)];
   MapPair<KvKey>& km = kv_maps[map_slot(p.kv_cache)];
   const QKey qkey{p.q, p.q_stride_batch, p.q_stride_qpos, p.q_stride_head, p.batch, p.q_len, p.num_heads, dev};
-  const DecodeForm form = p.fused_merge ? decode_form(p.batch, p.groups, p.page_size, p.longest, p.phase_mask, num_ctas) : DecodeForm{false, num_ctas, 1};
+  const DecodeForm form = p.fused_merge ? decode_form({p.batch, p.groups, p.num_heads, p.page_size, p.longest, num_ctas, p.out_dtype, p.soft_cap > 0.f, p.phase_mask})
+                                        : DecodeForm{false, num_ctas, 1};
   const bool pair = form.pair;
   const uint32_t rows = pair && p.page_size > 64 ? 64u : uint32_t(p.page_size);
   const KvKey kvkey{p.kv_cache, p.num_pages, p.page_size, int32_t(rows), dev};

@@ -52,12 +52,14 @@ class DecodePlan:
 
 
 def decode_plan(seq_lens: Sequence[int], q_len: int, num_heads: int, page_size: int, max_pages: int, num_ctas: int,
-                max_seq_len: int = 0) -> DecodePlan:
+                max_seq_len: int = 0, out_dtype: int = _cabi.OUT_BF16, soft_cap: float = 0.0) -> DecodePlan:
     """Which decode kernel a call with block tables of ``max_pages`` pages (0: not given) and this ``max_seq_len`` (0: not given) runs, its
     grid and how many of its CTAs share the tiles."""
+    a = _cabi.DecodeArgs(batch=len(seq_lens), q_len=q_len, num_heads=num_heads, page_size=page_size, num_ctas=num_ctas, out_dtype=out_dtype,
+                         max_pages_per_request=max_pages, max_seq_len=max_seq_len, logits_soft_cap=soft_cap)
     arr = (C.c_int32 * max(len(seq_lens), 1))(*[int(x) for x in seq_lens])
     out = [C.c_int32(0) for _ in range(3)]
-    _cabi.check(_cabi.lib.mla_fp4_decode_plan(len(seq_lens), q_len, num_heads, page_size, max_pages, max_seq_len, num_ctas, arr, *map(C.byref, out)))
+    _cabi.check(_cabi.lib.mla_fp4_decode_plan(C.byref(a), arr, *map(C.byref, out)))
     return DecodePlan(*(x.value for x in out))
 
 

@@ -165,14 +165,12 @@ int mla_fp4_plan_partition(const int32_t* seq_lens_host, int32_t batch, int32_t 
 int mla_fp4_work_ctas(const int32_t* seq_lens_host, int32_t batch, int32_t q_len, int32_t num_heads,
                       int32_t num_ctas, int32_t* work_ctas);
 
-/* What a call of mla_fp4_decode with MLA_FP4_KERNEL_TCGEN05 and these arguments launches: *groups_per_cluster is 1
-   (a CTA decodes one group of 64 heads) or 2 (a pair of CTAs decodes two groups of the same tiles), *grid the CTAs
-   launched and *work_ctas (may be NULL, seq_lens_host then too) how many of them share the tiles: the partition is
-   mla_fp4_plan_partition over that many.  max_pages_per_request and max_seq_len as in MlaFp4DecodeArgs, num_ctas as
-   resolved (not 0).  Host only. */
-int mla_fp4_decode_plan(int32_t batch, int32_t q_len, int32_t num_heads, int32_t page_size,
-                        int32_t max_pages_per_request, int32_t max_seq_len, int32_t num_ctas, const int32_t* seq_lens_host,
-                        int32_t* groups_per_cluster, int32_t* grid, int32_t* work_ctas);
+/* What mla_fp4_decode(args) with MLA_FP4_KERNEL_TCGEN05 launches: *groups_per_cluster is 1 (a CTA decodes one group of
+   64 heads) or 2 (a pair of CTAs decodes two groups of the same tiles), *grid the CTAs launched and *work_ctas (may be
+   NULL, seq_lens_host then too) how many of them share the tiles: the partition is mla_fp4_plan_partition over that many.
+   The pointers of args are not looked at; num_ctas 0 asks the current device, otherwise host only. */
+int mla_fp4_decode_plan(const MlaFp4DecodeArgs* args, const int32_t* seq_lens_host, int32_t* groups_per_cluster,
+                        int32_t* grid, int32_t* work_ctas);
 
 /* Zero the header and the slot tails of a workspace (an asynchronous memset on `stream`).  Call
    once after allocating the workspace.

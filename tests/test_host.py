@@ -306,9 +306,15 @@ def test_decode_plan(seq_lens, heads, q_len, ctas, expect):
     (16, 1, 64, 256, 0, True),
     (16, 1, 64, 2048, 500, True),     # too short to be split
     (80, 1, 64, 2048, 500, False),    # more pairs than CTAs: split, few tiles
+    (70, 1, 64, 2048, 500, False),    # they nearly fill the grid
+    (55, 1, 64, 2048, 500, True),
+    (16, 1, 64, 2048, 128, False),    # of one tile
+    (4, 1, 64, 2048, 128, True),      # ... few of them
+    (16, 1, 64, 2048, 129, True),
     (16, 1, 32, 2048, 131072, False),  # pages below 64 tokens: only where nothing is split
     (16, 1, 8, 2048, 512, True),
     (16, 1, 8, 64, 0, True),
+    (16, 1, 8, 16, 0, False),
     (16, 1, 8, 2048, 513, False),
     (15, 1, 64, 100, 0, False),       # below twenty tiles a CTA
     (30, 1, 64, 100, 0, True),
@@ -334,3 +340,24 @@ def test_form_of_the_cache_writer(dtype, tokens, given, expect):
     out = C.c_int32(0)
     _cabi.check(_cabi.lib.mla_fp4_cache_write_plan(getattr(_cabi, dtype), tokens, given, C.byref(out)))
     assert out.value == expect
+
+
+@pytest.mark.parametrize("batch,heads,longest,out,cap,pair", [
+    (16, 128, 300, "OUT_E4M3", 0.0, True), (16, 128, 300, "OUT_F32", 0.0, False), (16, 128, 300, "OUT_BF16", 30.0, True),
+    (16, 128, 100, "OUT_E4M3", 0.0, False), (10, 128, 100, "OUT_E4M3", 0.0, True), (4, 128, 100, "OUT_BF16", 30.0, False),
+    (70, 100, 100, "OUT_E4M3", 30.0, True), (70, 100, 300, "OUT_F32", 0.0, True), (70, 100, 300, "OUT_BF16", 0.0, False),
+    (16, 100, 100, "OUT_F32", 0.0, False), (10, 100, 100, "OUT_F32", 0.0, True), (4, 100, 100, "OUT_BF16", 0.0, False),
+    (16, 128, 131072, "OUT_F32", 30.0, True),  # (long requests: none of that counts)
+])
+def test_choice_of_the_decode_kernel_by_output_and_variant(batch, heads, longest, out, cap, pair):
+    from flashinfer_mla_fp4_b200 import _cabi, planner
+
+    p = planner.decode_plan([100] * batch, 1, heads, 64, 0, 148, longest, getattr(_cabi, out), cap)
+    assert (p.groups_per_cluster == 2) == pair
+
+
+def test_choice_of_the_decode_kernel_with_few_heads():
+    from flashinfer_mla_fp4_b200 import _cabi, planner
+
+    for batch, heads, pair in ((40, 32, True), (60, 32, False), (40, 40, False)):  # one tile, FP32 rows
+        assert (planner.decode_plan([100] * batch, 2, heads, 64, 0, 148, 100, _cabi.OUT_F32).groups_per_cluster == 2) == pair
